@@ -237,6 +237,38 @@ def _zeros(*shape):
     return torch.zeros(shape, device="cuda", dtype=torch.float64)
 
 
+def _operator_calls(s):
+    """One CalculateTendency and UpdateGRK of SELF_CompressibleIdealGas2D by the drop-in entry points: (call, arguments)
+    with the pointers that a Fortran program keeps in its c_ptr variables."""
+    L, w = s["geo"].interp, S.lib()
+    N, n, geo, mesh = L.N, s["n"], s["geo"], s["mesh"]
+
+    def p(t):
+        return S._lib.pp(t.data_ptr())
+
+    bM, dgM, qw = p(L.device("bMatrix")), p(L.device("dgMatrix")), p(L.device("qWeights"))
+    nh, ns, si, rank = p(geo.nHat), p(geo.nScale), p(mesh.sideInfo_d), p(s["rank"])
+    a = {k: p(v) for k, v in s.items() if isinstance(v, torch.Tensor)}
+    calls = [(w.CalculateDiagnostics_CompressibleIdealGas2D_gpu_wrapper, (a["q"], a["diag"], GAMMA, 1.0, N, 4, 4, n)),
+             (w.ConservativeToPrimitive_CompressibleIdealGas2D_gpu_wrapper, (a["q"], a["prim"], GAMMA, N, 4, n))]
+    for f, b, x in (("q", "qb", "qx"), ("prim", "pb", "px"), ("diag", "db", "dx")):
+        calls += [(w.ScalarBoundaryInterp_2D_gpu_wrapper, (bM, a[f], a[b], N, 4, n)),
+                  (w.SideExchange_MappedScalar2D_gpu_wrapper, (a[x], a[b], si, rank, 0, 0, N, 4, n))]
+    calls += [
+        (w.SetBoundaryCondition_CompressibleIdealGas2D_gpu_wrapper,
+         (a["qb"], a["qx"], a["qp"], a["pb"], a["px"], a["pp"], a["db"], a["dx"], a["dp"], nh, si, N, 4, 4, n)),
+        (w.Source_CompressibleIdealGas2D_gpu_wrapper, (a["src"], a["q"], a["env"], N, 4, n)),
+        (w.NaiveLLF_CompressibleIdealGas2D_gpu_wrapper,
+         (a["fb"], a["qb"], a["qx"], a["pb"], a["px"], a["db"], a["dx"], nh, ns, N, 4, 4, n)),
+        (w.Flux_CompressibleIdealGas2D_gpu_wrapper, (a["flux"], a["q"], a["prim"], N, 4, n)),
+        (w.ContravariantProjection_MappedVector2D_gpu_wrapper, (a["flux"], p(geo.dsdx), N, 4, n)),
+        (w.VectorDGDivergence_2D_gpu_wrapper, (dgM, bM, qw, a["flux"], a["fb"], a["div"], N, 4, n)),
+        (w.JacobianWeight_MappedScalar2D_gpu_wrapper, (a["div"], p(geo.J), N, 4, n)),
+        (w.CalculateDSDt_Model2D_gpu_wrapper, (a["div"], a["src"], a["dSdt"], N, 4, n)),
+        (w.UpdateGRK_Model2D_gpu_wrapper, (a["G"], a["q"], a["dSdt"], RK_A[0], RK_G[0], s["dt"], 4, N, 4, n))]
+    return calls
+
+
 def prepare(case, seed):
     kind = case["kind"]
     st = {"case": case}
@@ -264,6 +296,7 @@ def prepare(case, seed):
         st["flux"] = _zeros(n, 4, P, P, 2)
         for k in ("qb", "qx", "qp", "pb", "px", "pp", "db", "dx", "dp", "fb"):
             st[k] = _zeros(n, 4, 4, P)
+        st["calls"] = _operator_calls(st)
     elif kind == "fields":
         N, nVar = case["N"], case["nVar"]
         c = dict(case, walls=False, perturb=0.02)
@@ -290,34 +323,8 @@ def prepare(case, seed):
 
 # ------------------------------------------------------------------- one pass
 def _operators(s):
-    """One CalculateTendency and UpdateGRK of SELF_CompressibleIdealGas2D by the drop-in entry points."""
-    L, w = s["geo"].interp, S.lib()
-    N, n, geo, mesh = L.N, s["n"], s["geo"], s["mesh"]
-
-    def p(t):
-        return S._lib.pp(t.data_ptr())
-
-    bM, dgM, qw = p(L.device("bMatrix")), p(L.device("dgMatrix")), p(L.device("qWeights"))
-    nh, ns, si, rank = p(geo.nHat), p(geo.nScale), p(mesh.sideInfo_d), p(s["rank"])
-    s["q"].copy_(s["q0"])
-    q, prim, diag, flux = p(s["q"]), p(s["prim"]), p(s["diag"]), p(s["flux"])
-    w.CalculateDiagnostics_CompressibleIdealGas2D_gpu_wrapper(q, diag, GAMMA, 1.0, N, 4, 4, n)
-    w.ConservativeToPrimitive_CompressibleIdealGas2D_gpu_wrapper(q, prim, GAMMA, N, 4, n)
-    for f, b, x in (("q", "qb", "qx"), ("prim", "pb", "px"), ("diag", "db", "dx")):
-        w.ScalarBoundaryInterp_2D_gpu_wrapper(bM, p(s[f]), p(s[b]), N, 4, n)
-        w.SideExchange_MappedScalar2D_gpu_wrapper(p(s[x]), p(s[b]), si, rank, 0, 0, N, 4, n)
-    w.SetBoundaryCondition_CompressibleIdealGas2D_gpu_wrapper(
-        p(s["qb"]), p(s["qx"]), p(s["qp"]), p(s["pb"]), p(s["px"]), p(s["pp"]), p(s["db"]), p(s["dx"]), p(s["dp"]),
-        nh, si, N, 4, 4, n)
-    w.Source_CompressibleIdealGas2D_gpu_wrapper(p(s["src"]), q, p(s["env"]), N, 4, n)
-    w.NaiveLLF_CompressibleIdealGas2D_gpu_wrapper(p(s["fb"]), p(s["qb"]), p(s["qx"]), p(s["pb"]), p(s["px"]),
-                                                  p(s["db"]), p(s["dx"]), nh, ns, N, 4, 4, n)
-    w.Flux_CompressibleIdealGas2D_gpu_wrapper(flux, q, prim, N, 4, n)
-    w.ContravariantProjection_MappedVector2D_gpu_wrapper(flux, p(geo.dsdx), N, 4, n)
-    w.VectorDGDivergence_2D_gpu_wrapper(dgM, bM, qw, flux, p(s["fb"]), p(s["div"]), N, 4, n)
-    w.JacobianWeight_MappedScalar2D_gpu_wrapper(p(s["div"]), p(geo.J), N, 4, n)
-    w.CalculateDSDt_Model2D_gpu_wrapper(p(s["div"]), p(s["src"]), p(s["dSdt"]), N, 4, n)
-    w.UpdateGRK_Model2D_gpu_wrapper(p(s["G"]), q, p(s["dSdt"]), RK_A[0], RK_G[0], s["dt"], 4, N, 4, n)
+    for call, args in s["calls"]:
+        call(*args)
     return {"dSdt": s["dSdt"], "q": s["q"]}
 
 
@@ -366,6 +373,7 @@ def run(st):
             torch.cuda.current_stream().wait_stream(h["stream"])
         return {"N%d" % N: h["model"].solution for N, h in st["ens"].handles.items()}
     if kind == "operators":
+        st["q"].copy_(st["q0"])
         return _operators(st)
     return _fields(st) if kind == "fields" else _learn(st)
 
