@@ -67,7 +67,8 @@ __global__ void k_pack_geometry(const double* __restrict__ dsdx, const double* _
       const int s = (b - gr.oJ) / 8;
       v = kind == GEO_REF ? J[PP * e + s] : 1.0 / J[PP * e + s];
     } else {
-      out[k] = (uint32_t)sideInfo[20 * e + (b - gr.oSi) / 4];
+      const int s = (b - gr.oSi) / 4;
+      out[k] = s < 20 ? (uint32_t)sideInfo[20 * e + s] : 0u;  // the record's padding
       continue;
     }
     const unsigned long long u = (unsigned long long)__double_as_longlong(v);

@@ -24,7 +24,7 @@
 // Two kernels implement this: k_fused_stage (below; one CTA of P*P-thread
 // element groups, plain loads; any degree) and k_fused_stage_tma
 // (fused_stage_tma.cuh; persistent, bulk-async copies into a shared-memory
-// ring; even P).  Both share the model policies and the trace-cache layout.
+// ring).  Both share the model policies and the trace-cache layout.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -106,7 +106,8 @@ __device__ __forceinline__ R bm_right(const StageArgs& a, int m) {
 
 // One element's packed geometry record: dsdx (4 P^2 values, as two planes of
 // P^2 pairs: (dsdx11, dsdx21) of every node, then (dsdx12, dsdx22)), nHat
-// (8 P), nScale (4 P), a J slot (P^2 doubles), sideInfo (20 ints).  Four kinds:
+// (8 P), nScale (4 P), a J slot (P^2 doubles), sideInfo (20 ints), padded to a
+// multiple of 16 bytes (odd P).  Four kinds:
 //   GEO_REF   FP64 metrics, J            (reference-rounding form)
 //   GEO_INVJ  FP64 metrics, 1/J          (production FP64 at P != 8)
 //   GEO_NOJ   FP64 metrics, no J slot    (production FP64 at P = 8: the stage
@@ -115,7 +116,6 @@ __device__ __forceinline__ R bm_right(const StageArgs& a, int m) {
 //   GEO_F32   FP32 metrics, FP64 1/J     (FP32 bulk: its stage rounds dsdx,
 //             nHat and nScale to FP32 before every use, so the record holds
 //             them rounded once; 1/J stays FP64)
-// Every kind is a multiple of 16 bytes for even P.
 enum GeoKind { GEO_REF = 0, GEO_INVJ = 1, GEO_NOJ = 2, GEO_F32 = 3 };
 struct GeoRec {
   int wm;                                // bytes per metric value (8 or 4)
@@ -125,7 +125,7 @@ __host__ __device__ constexpr GeoRec geo_rec(int P, int kind) {
   const int wm = kind == GEO_F32 ? 4 : 8;
   const int oNhat = 4 * P * P * wm, oNs = oNhat + 8 * P * wm, oJ = oNs + 4 * P * wm;
   const int oSi = oJ + (kind == GEO_NOJ ? 0 : 8 * P * P);
-  return GeoRec{wm, oNhat, oNs, oJ, oSi, oSi + 80};
+  return GeoRec{wm, oNhat, oNs, oJ, oSi, (oSi + 80 + 15) / 16 * 16};
 }
 
 // Trace-cache block size (values of the bulk type) of one (element, side).

@@ -19,9 +19,9 @@
 // an error word, waits (again bounded) for its other copy in flight and
 // returns; the host reports SELFGPU_ERR_TIMEOUT.
 //
-// Requires an even P (all per-element block sizes are then multiples of 16
-// bytes) and 16-byte aligned base pointers; the engine falls back to
-// k_fused_stage otherwise.
+// Requires 16-byte aligned base pointers; the engine falls back to
+// k_fused_stage otherwise.  (Tiles of odd P hold an even number of elements,
+// so that their pieces are multiples of 16 bytes.)
 #pragma once
 
 #include "fused_stage.cuh"
@@ -134,7 +134,15 @@ struct TmaTraits {
   // idle: four per five-warp group (144 of 160 lanes), measured 1.14x faster
   // for ShallowWater FP64, 1.12x for CompressibleIdealGas2D FP32 and, with
   // three 128-register groups (below), 1.27x for CompressibleIdealGas2D FP64.
-  static constexpr int EPG = (P == 4) ? 2 : ((P == 6) ? 4 : 1);
+  // Odd P takes an even number of elements, so that every piece of a tile is a
+  // multiple of 16 bytes (bulk copies): two at P = 7 and 5 (98 of 128 and 50
+  // of 64 lanes live), eight at P = 3 (72 of 96; its 96 face nodes fill the
+  // lanes).  On 256x256 meshes, us per stage, against the per-element kernel
+  // that ran odd P before: CompressibleIdealGas2D FP64 N = 6 491 -> 195, N = 4
+  // 248 -> 123, N = 2 136 -> 65; ShallowWater 364 -> 157, 173 -> 97, 75 -> 46.
+  // Four elements at P = 7, four or six at P = 5 and two or four at P = 3
+  // measured 1-60 % slower in FP64 CompressibleIdealGas2D.
+  static constexpr int EPG = (P == 4) ? 2 : ((P == 6) ? 4 : (P == 3) ? 8 : (P == 5 || P == 7) ? 2 : 1);
   static constexpr int TPE = (EPG * PP + 31) / 32 * 32;  // threads per group
   static_assert(TPE >= EPG * 4 * P, "the face phase gives each of the 4P face nodes its own thread");
   // 640 threads (five warps per scheduler at 96 registers) for P = 6 (ten
@@ -159,8 +167,15 @@ struct TmaTraits {
   // ShallowWater and LinearShallowWater kernels (80 registers without spills;
   // CompressibleIdealGas2D FP64 would spill and its shared memory holds ten
   // groups, the reference-rounding build would spill).
-  static constexpr int kMaxGroups =
-      (P <= 4) ? (((NV == 4 && sizeof(R) == 8) || ref_rounding<R>()) ? 15 : (sizeof(R) == 4 ? 24 : 20))
+  // Odd P: 512 threads in FP64 (128 registers; at 96 the kernels spill:
+  // CompressibleIdealGas2D N = 6 195 against 229 us), 640 for
+  // LinearShallowWater at P = 7, which does not spill there (140 against 150),
+  // and 768 in FP32 (896 and 640 measured within 4 %).
+  static constexpr int kOddThreads =
+      sizeof(R) == 4 ? 768 : (P == 7 && NV == 3 && !Phys::kLaggedVelocity) ? 640 : 512;
+  static constexpr int kMaxGroups = (P % 2)
+      ? (TPE > 32 && kOddThreads / TPE > 15 ? 15 : kOddThreads / TPE)
+      : (P <= 4) ? (((NV == 4 && sizeof(R) == 8) || ref_rounding<R>()) ? 15 : (sizeof(R) == 4 ? 24 : 20))
                : (P == 6 ? ((EPG == 4 && (Phys::kLaggedVelocity || NV == 4) && sizeof(R) == 8) ? 3 : 640 / TPE)
                          : ((sizeof(R) == 4) ? 14 : (NV == 3 && !ref_rounding<R>()) ? 12 : 10));
   static constexpr int kThreadsMax = kMaxGroups * TPE;
@@ -180,26 +195,55 @@ struct TmaTraits {
   // apart), and the divergence sums go to a separate array (NV P^2 per
   // element) instead of replacing the xi flux, since one element's
   // divergence threads may then span two warps.
+  static constexpr bool kOdd = (P % 2) != 0;  // rows of an odd length need no padding
   static constexpr bool kSwz = (P == 8);
-  static constexpr int RS = kSwz ? P : P + 1;
+  static constexpr int RS = (kSwz || kOdd) ? P : P + 1;
   static constexpr int FS = kSwz ? PP + 8 : P * RS;
   static constexpr int kU = (NF * FS > 2 * NV * PP) ? NF * FS : 2 * NV * PP;  // node fields alias the fluxes
   static constexpr int SS = side_stride(NV * P, (int)sizeof(R));
   static constexpr int EB = kU + 4 * SS;
-  static constexpr int kDiv = EPG > 1 ? NV * PP : 0;  // separate divergence sums per element
+  static constexpr int kDiv = (EPG > 1 && !kOdd) ? NV * PP : 0;  // separate divergence sums per element
   static constexpr int groupBytes = (int)(((EPG * (EB + kDiv)) * sizeof(R) + 127) / 128 * 128);
   // Weak-divergence volume sums: one thread per 2x2 block of nodes and pair
   // of variables.  The xi flux rows are stored with their value pairs
   // XOR-swizzled per row pair (P/2 a power of two), so that the paired loads
   // of a quarter-warp fall into distinct banks.
   static constexpr int HB = P / 2, NVP = (NV + 1) / 2, NB = HB * HB * NVP;
-  static_assert(EPG > 1 || NB <= 32, "one element's divergence blocks fit one warp");
-  static_assert(EPG * NB <= TPE, "every divergence block has its own thread");
-  static constexpr bool kSwzF = (HB & (HB - 1)) == 0;
+  static_assert(kOdd || EPG > 1 || NB <= 32, "one element's divergence blocks fit one warp");
+  static_assert(kOdd || EPG * NB <= TPE, "every divergence block has its own thread");
+  static constexpr bool kSwzF = !kOdd && (HB & (HB - 1)) == 0;
   // position of value m in row j of the xi flux
   __device__ __forceinline__ static int f0pos(int m, int j) {
     if constexpr (kSwzF) return 2 * ((m >> 1) ^ ((j >> 1) & (HB - 1))) + (m & 1);
     else return m;
+  }
+  // Divergence sums as FP64 tensor-core products: production and FP32-bulk
+  // forms at P = 8 and 6 (one element per warp) and 4 (two), production FP64
+  // at P = 7 (229 against 257 us per stage with sums in registers; at P = 5
+  // they are slower, 140 against 123)
+  static constexpr bool kDmma =
+      ((P == 8 && EPG == 1) || P == 6 || (P == 7 && sizeof(R) == 8)) && !ref_rounding<R>();
+  static constexpr bool kDmma4 = (P == 4 && EPG == 2 && TPE == 32) && !ref_rounding<R>();
+  // odd P otherwise: each node's thread forms its sums in registers, in the
+  // reference's order
+  static constexpr bool kRegDiv = kOdd && !kDmma;
+  // At P = 8 the products' operand loads read, per half-warp, four rows of
+  // the xi flux, the eta flux and the transposed dgMatrix at four columns
+  // each; rows two apart would share banks, so these three arrays keep the
+  // column index XOR 4 in row pairs 2-3 and 6-7 (the per-node stores of
+  // phase A stay conflict-free, as a half-warp stores two whole rows).
+  static constexpr bool kSw8 = (P == 8) && kDmma;
+  __device__ __forceinline__ static int cswz(int c, int r) { return kSw8 ? (c ^ (4 * ((r >> 1) & 1))) : c; }
+  // positions of F0(m, j), F1(i, j) and dgM(m, i)
+  __device__ __forceinline__ static int f0at(int m, int j) { return kSw8 ? P * j + cswz(m, j) : P * j + f0pos(m, j); }
+  __device__ __forceinline__ static int f1at(int i, int j) { return P * j + cswz(i, j); }
+  __device__ __forceinline__ static int dgat(int m, int i) { return P * m + cswz(i, m); }
+  // The auxiliaries of the volume flux.  FP32 bulk at odd P forms the full node
+  // state, as its per-element kernel does (the compiler contracts the pressure
+  // of the shorter form differently, in the last bit).
+  __device__ __forceinline__ static void flux_fields(R* f, const StageArgs& a) {
+    if constexpr (kOdd && sizeof(R) == 4) Phys::template node<R>(f, a);
+    else Phys::template node_flux<R>(f, a);
   }
   // offset of node (i, j) in field f's block of the node-field array
   __device__ __forceinline__ static int nf(int f, int i, int j) {
@@ -207,6 +251,233 @@ struct TmaTraits {
     else return RS * j + i;
   }
 };
+
+// Weak-divergence volume sums of a tile whose contravariant fluxes are in
+// shared memory (phase B, alongside the face phase; gBase is the group's array
+// of EB values per element), the
+// reference's order per node and variable (VectorDGDivergence_2D,
+// src/SELF_Lagrange.f90):
+//   d = 0;  for m ascending: d = (d + dgM(m,i) F0(m,j)) + dgM(m,j) F1(i,m).
+// A thread sums a 2x2 block of nodes for two variables, so every loaded
+// flux pair and dgMatrix pair serves two nodes.  One-element groups write
+// the sums over the xi flux ([NV][P^2], node-major) once the warp has read
+// it; two-element groups write them to their separate array.
+// Production FP64 and FP32-bulk forms at P = 8 and P = 6: the same sums
+// as FP64 tensor-core products (mma.sync m8n8k4 f64), D(j,i) = sum_m
+// F0(m,j) dgM(m,i) + dgM(m,j) F1(i,m), four chained products per variable
+// over one warp per element (a P = 6 element is padded with zeros to the
+// 8x8 shape; FP32-bulk fluxes are widened exactly to FP64 and the sums
+// rounded back once).  The order of the additions inside a product is the
+// hardware's, so only the forms without the reference's rounding use it.
+// At P = 4 one product covers both elements of a tile: rows and columns
+// 0-3 belong to the first element, 4-7 to the second; the xi product's
+// A rows and the eta product's B columns carry the element's flux, the
+// dgMatrix operand is the same for both, and the two diagonal 4x4 blocks
+// of the sum are the two elements' sums (the off-diagonal ones mix the
+// elements and are dropped).
+template <int P, class Phys, typename R>
+__device__ __forceinline__ void tile_volume_sums(R* gBase, const double* sdg, int t, int faceWarp, int nLive) {
+  using T = TmaTraits<P, Phys, R>;
+  constexpr int NV = T::NV, PP = T::PP, EPG = T::EPG, EB = T::EB, TPE = T::TPE;
+  if constexpr (T::kDmma4) {
+    const int lane = t & 31, gq = lane >> 2, kq = lane & 3;
+    const int eR = gq >> 2, jr = gq & 3;   // the element and node row of this lane's A row / B column
+    const R* bU = gBase + eR * EB;
+    const R* bF1 = bU + NV * PP;
+    const double dg = sdg[T::dgat(kq, jr)];    // dgM(m = kq, jr): B of the xi product, A of the eta product
+    // this lane's sums: row gq, columns 2 kq, 2 kq + 1 -> element kq >> 1
+    const bool diag = (eR == (kq >> 1)) && eR < nLive;
+    R* bD = gBase + EPG * EB + eR * NV * PP;
+    using R2 = typename std::conditional<sizeof(R) == 8, double2, float2>::type;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      double c0 = 0.0, c1 = 0.0;
+      const double aF0 = (double)bU[v * PP + T::f0at(kq, jr)];  // F0 at (m = kq, j = jr)
+      const double bF = (double)bF1[v * PP + T::f1at(jr, kq)];   // F1 at (i = jr, m = kq)
+      asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                   : "+d"(c0), "+d"(c1)
+                   : "d"(aF0), "d"(dg));
+      asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                   : "+d"(c0), "+d"(c1)
+                   : "d"(dg), "d"(bF));
+      if (diag) {  // D(j = jr, i = 2 (kq & 1)), D(jr, 2 (kq & 1) + 1)
+        R2 x;
+        x.x = (R)c0;
+        x.y = (R)c1;
+        reinterpret_cast<R2*>(bD + v * PP + P * jr)[kq & 1] = x;
+      }
+    }
+  } else if constexpr (T::kDmma) {
+    // the warps a tile's face threads leave free take its elements in turn
+    // (a one-element group: the warp that is not the face warp)
+    constexpr int kDW = (EPG == 1) ? 1 : ((TPE - EPG * 4 * P) / 32 > 0 ? (TPE - EPG * 4 * P) / 32 : 1);
+    const int w = t >> 5;
+    const bool run = (EPG == 1) ? (w != faceWarp) : (w < kDW);
+    for (int eB = (EPG == 1) ? 0 : w; run && eB < nLive; eB += kDW) {  // uniform over the warp
+      const R* bU = gBase + eB * EB;
+      const R* bF1 = bU + NV * PP;
+      R* bD = T::kDiv ? gBase + EPG * EB + eB * NV * PP : gBase + eB * EB;
+      const int lane = t & 31, gq = lane >> 2, kq = lane & 3;
+      double dv[NV][2];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        double c0 = 0.0, c1 = 0.0;
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk) {
+          const int m = 4 * kk + kq;
+          const bool in = (P == 8) || (gq < P && m < P);  // the zero padding of P = 6
+          const double aF0 = in ? (double)bU[v * PP + T::f0at(m, gq)] : 0.0;  // F0 at (m, j = gq)
+          const double dg = in ? sdg[T::dgat(m, gq)] : 0.0;                    // dgM(m, gq)
+          const double bF = in ? (double)bF1[v * PP + T::f1at(gq, m)] : 0.0;   // F1 at (i = gq, m)
+          asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                       : "+d"(c0), "+d"(c1)
+                       : "d"(aF0), "d"(dg));
+          asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                       : "+d"(c0), "+d"(c1)
+                       : "d"(dg), "d"(bF));
+        }
+        dv[v][0] = c0;  // D(j = gq, i = 2 kq), D(gq, 2 kq + 1)
+        dv[v][1] = c1;
+      }
+      if constexpr (T::kDiv == 0) __syncwarp();  // the warp has read the xi flux it overwrites
+      using R2 = typename std::conditional<sizeof(R) == 8, double2, float2>::type;
+      if constexpr (T::kOdd) {
+        if (gq < P) {
+#pragma unroll
+          for (int v = 0; v < NV; ++v) {
+            if (2 * kq < P) bD[v * PP + P * gq + 2 * kq] = (R)dv[v][0];
+            if (2 * kq + 1 < P) bD[v * PP + P * gq + 2 * kq + 1] = (R)dv[v][1];
+          }
+        }
+      } else if (gq < P && 2 * kq + 1 < P) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          R2 x;
+          x.x = (R)dv[v][0];
+          x.y = (R)dv[v][1];
+          reinterpret_cast<R2*>(bD + v * PP + P * gq)[kq] = x;
+        }
+      }
+    }
+  } else if constexpr (!T::kRegDiv) {
+    const bool mine = (EPG == 1) ? (TPE < 64 || (t >> 5) != faceWarp) : (t < EPG * T::NB);
+    if (mine) {
+      using R2 = typename std::conditional<sizeof(R) == 8, double2, float2>::type;
+      constexpr int HB = T::HB;
+      const int eB = (EPG == 1) ? 0 : t / T::NB;
+      const int tb = (EPG == 1) ? (t & 31) : t - eB * T::NB;
+      const bool on = (EPG == 1) ? (tb < T::NB) : (eB < nLive);
+      const R* bU = gBase + eB * EB;
+      const R* bF1 = bU + NV * PP;
+      R* bD = (EPG > 1) ? gBase + EPG * EB + eB * NV * PP : gBase;
+      const int vp = tb / (HB * HB), rem = tb - vp * (HB * HB), bj = rem / HB, bi = rem - bj * HB;
+      const int v0 = 2 * vp;
+      const bool two = v0 + 1 < NV;
+      R acc[2][2][2];  // [variable of the pair][row offset r (j)][column offset c (i)]
+#pragma unroll
+      for (int vv = 0; vv < 2; ++vv)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) acc[vv][r][0] = acc[vv][r][1] = (R)0;
+      if (on) {
+        const double2* sdg2 = reinterpret_cast<const double2*>(sdg);
+#pragma unroll
+        for (int mp = 0; mp < HB; ++mp) {
+          R f0[2][2][2];  // [vv][r][k]: F0(2 mp + k, 2 bj + r)
+          R f1[2][2][2];  // [vv][k][c]: F1(2 bi + c, 2 mp + k)
+#pragma unroll
+          for (int vv = 0; vv < 2; ++vv) {
+            const int v = (vv == 0 || two) ? v0 + vv : v0;
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              const int row = 2 * bj + r;
+              const R2 x = reinterpret_cast<const R2*>(bU + v * PP + P * row)[T::f0pos(2 * mp, row) >> 1];
+              f0[vv][r][0] = x.x;
+              f0[vv][r][1] = x.y;
+            }
+#pragma unroll
+            for (int kq = 0; kq < 2; ++kq) {
+              const R2 x = reinterpret_cast<const R2*>(bF1 + v * PP + P * (2 * mp + kq))[bi];
+              f1[vv][kq][0] = x.x;
+              f1[vv][kq][1] = x.y;
+            }
+          }
+#pragma unroll
+          for (int kq = 0; kq < 2; ++kq) {
+            const int m = 2 * mp + kq;
+            const double2 dI = sdg2[bi + HB * m], dJ = sdg2[bj + HB * m];
+            const R gi[2] = {(R)dI.x, (R)dI.y}, gj[2] = {(R)dJ.x, (R)dJ.y};
+#pragma unroll
+            for (int vv = 0; vv < 2; ++vv)
+#pragma unroll
+              for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+                  acc[vv][r][c] = acc[vv][r][c] + gi[c] * f0[vv][r][kq] + gj[r] * f1[vv][kq][c];
+          }
+        }
+      }
+      if constexpr (EPG == 1) __syncwarp();  // the warp has read the xi flux it overwrites
+      if (on) {
+#pragma unroll
+        for (int vv = 0; vv < 2; ++vv)
+          if (vv == 0 || two)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              R2 x;
+              x.x = acc[vv][r][0];
+              x.y = acc[vv][r][1];
+              reinterpret_cast<R2*>(bD + (v0 + vv) * PP + P * (2 * bj + r))[bi] = x;
+            }
+      }
+    }
+  }
+}
+
+// End traces of the node fields of a tile of `elems` elements (`live` of them
+// real), whose field arrays lie `stride` values apart: BoundaryInterp
+// (src/SELF_Lagrange.f90:2241-2270).  One task per (element, field, line,
+// orientation) reads the line's P values once and forms both of its end
+// traces: column l gives S (side 0) and N (side 2), row l gives W (3) and E
+// (1).  This thread takes the tasks k0, k0 + step, ... and passes each result
+// to emit(element, field, line, row, lo, hi).  P = 8 numbers the tasks by
+// field pair, orientation, field, line (an odd NT leaves the last pair's
+// second half idle), so that a half-warp reads the column lines (or the row
+// lines) of two fields; the padded layouts of the other P number them by
+// orientation, field, line, with no idle tasks.
+template <int P, class Phys, typename R, class Emit>
+__device__ __forceinline__ void tile_traces(const R* fields, int stride, int elems, int live, int k0, int step,
+                                            const StageArgs& a, Emit emit) {
+  using T = TmaTraits<P, Phys, R>;
+  constexpr int NT = T::NT;
+  constexpr int NTp = T::kSwz ? (NT + 1) / 2 * 2 : NT;
+  constexpr int TPEl = 2 * NTp * P;  // tasks per element
+  for (int kk = k0; kk < elems * TPEl; kk += step) {
+    const int eE = kk / TPEl, ks = kk - eE * TPEl;
+    if (eE >= live) continue;
+    int row, fi, l;
+    if constexpr (T::kSwz) {
+      const int fp = ks / (4 * P), r = ks - fp * 4 * P, r2 = r - (r / (2 * P)) * 2 * P, fs = r2 / P;
+      row = r / (2 * P);
+      l = r2 - fs * P;
+      fi = 2 * fp + fs;
+      if (fi >= NT) continue;
+    } else {
+      row = ks / (NT * P);
+      const int r = ks - row * NT * P;
+      fi = r / P;
+      l = r - fi * P;
+    }
+    const R* fv = fields + eE * stride + fi * T::FS;
+    R lo = (R)0, hi = (R)0;
+#pragma unroll
+    for (int m = 0; m < P; ++m) {
+      const R x = fv[row ? T::nf(fi, m, l) : T::nf(fi, l, m)];
+      lo = lo + bm_left<R>(a, m) * x;  // kernel-parameter constants (m is unrolled)
+      hi = hi + bm_right<R, P>(a, m) * x;
+    }
+    emit(eE, fi, l, row != 0, lo, hi);
+  }
+}
 
 template <int P, class Phys, typename R, bool kMulti = false>
 __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
@@ -223,20 +494,9 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
   // at P = 6, every model at P = 4)
   constexpr bool kNbrEarly =
       (P == 8) ? !(NV == 4 && ref_rounding<R>()) : (P == 6 && kSW && sizeof(R) == 8);
-  // divergence sums as FP64 tensor-core products (phase B): production and
-  // FP32-bulk forms at P = 8 and 6 (one element per warp) and 4 (two)
-  constexpr bool kDmma = ((P == 8 && EPG == 1) || P == 6) && !ref_rounding<R>();
-  constexpr bool kDmma4 = (P == 4 && EPG == 2 && TPE == 32) && !ref_rounding<R>();
-  // At P = 8 the products' operand loads read, per half-warp, four rows of
-  // the xi flux, the eta flux and the transposed dgMatrix at four columns
-  // each; rows two apart would share banks, so these three arrays keep the
-  // column index XOR 4 in row pairs 2-3 and 6-7 (the per-node stores of
-  // phase A stay conflict-free, as a half-warp stores two whole rows).
-  constexpr bool kSw8 = (P == 8) && kDmma;
-  auto cswz = [](int c, int r) { return kSw8 ? (c ^ (4 * ((r >> 1) & 1))) : c; };
-  auto f0at = [&](int m, int j) { return kSw8 ? P * j + cswz(m, j) : P * j + T::f0pos(m, j); };  // F0(m, j)
-  auto f1at = [&](int i, int j) { return P * j + cswz(i, j); };                                  // F1(i, j)
-  auto dgat = [&](int m, int i) { return P * m + cswz(i, m); };                                  // dgM(m, i)
+  auto f0at = [](int m, int j) { return T::f0at(m, j); };
+  auto f1at = [](int i, int j) { return T::f1at(i, j); };
+  auto dgat = [](int m, int i) { return T::dgat(m, i); };
   extern __shared__ __align__(128) unsigned char smem[];
   const int C = pl.groups;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);
@@ -317,7 +577,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
     xb[1] = a.fld[1] ? 2 * PP * 8 : 0;
   } else {
     xb[0] = a.fld[0] ? 2 * PP * 8 : 0;
-    xb[1] = a.fld[1] ? PP * 8 : 0;
+    xb[1] = a.fld[1] ? (T::kOdd ? 2 : 1) * PP * 8 : 0;
     xb[2] = xb[3] = xb[4] = a.fld[2] ? 16 * P * 8 : 0;
   }
   auto tile_live = [&](long long k) -> int {  // live elements of the CTA's local tile k
@@ -334,11 +594,23 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
     const uint32_t nl = (EPG == 1) ? 1u : (uint32_t)tile_live(k);
     unsigned char* sl = slots + (size_t)(2 * g + buf) * pl.slotBytes;
     uint64_t* bar = &full[2 * g + buf];
-    const uint32_t bytes = nl * (qb + gb + ob + vb + xb[0] + xb[1] + xb[2] + xb[3] + xb[4]);
+    // An odd number of elements of odd P (the last tile of a mesh) leaves a
+    // piece 8 bytes short of a multiple of 16: this thread, which also waits
+    // for the copies, then moves the last value itself.
+    auto whole = [&](uint32_t n) { return T::kOdd ? n & ~15u : n; };
+    auto copy = [&](unsigned char* dst, const void* src, uint32_t n) {
+      bulk_g2s(dst, src, whole(n), bar);
+      if (T::kOdd && (n & 8))
+        *reinterpret_cast<double*>(dst + whole(n)) =
+            *reinterpret_cast<const double*>(reinterpret_cast<const unsigned char*>(src) + whole(n));
+    };
+    uint32_t bytes = nl * (gb + ob + vb) + whole(nl * qb);
+#pragma unroll
+    for (int x = 0; x < 5; ++x) bytes += whole(nl * xb[x]);
     mbar_arrive_expect_tx(bar, bytes);
     if (a.debugStarve == 1 && blockIdx.x == 0 && k == 0) return;
     const R* trIn = reinterpret_cast<const R*>(cache_of(ms.tr, ms.cur0, st, a.trIn));
-    bulk_g2s(sl + pl.oQ, a.q + (size_t)e * NV * PP, nl * qb, bar);
+    copy(sl + pl.oQ, a.q + (size_t)e * NV * PP, nl * qb);
     bulk_g2s(sl + pl.oDsdx, reinterpret_cast<const unsigned char*>(a.geo) + (size_t)e * gb, nl * gb, bar);
     bulk_g2s(sl + pl.oOwn, trIn + (size_t)4 * TS * e, nl * ob, bar);
     if constexpr (kSW)
@@ -346,9 +618,9 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
                reinterpret_cast<const R*>(cache_of(ms.vel, ms.vcur0, st, a.velIn)) + (size_t)e * 8 * P, nl * vb,
                bar);
     if constexpr (kLSW) {
-      bulk_g2s(sl + pl.oX[0], a.fld[0] + (size_t)e * PP, nl * xb[0], bar);
-      bulk_g2s(sl + pl.oX[1], a.fld[1] + (size_t)e * 4 * P, nl * xb[1], bar);
-      if (xb[2]) bulk_g2s(sl + pl.oX[2], a.fld[2] + (size_t)e * PP, nl * xb[2], bar);
+      copy(sl + pl.oX[0], a.fld[0] + (size_t)e * PP, nl * xb[0]);
+      copy(sl + pl.oX[1], a.fld[1] + (size_t)e * 4 * P, nl * xb[1]);
+      if (xb[2]) copy(sl + pl.oX[2], a.fld[2] + (size_t)e * PP, nl * xb[2]);
     } else if constexpr (kSW) {
       if (xb[0]) bulk_g2s(sl + pl.oX[0], a.fld[0] + (size_t)e * 4 * P, nl * xb[0], bar);
       if (xb[1]) bulk_g2s(sl + pl.oX[1], a.fld[1] + (size_t)e * 2 * PP, nl * xb[1], bar);
@@ -357,8 +629,10 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
       if (xb[0])
         for (uint32_t x = 0; x < nl; ++x)
           bulk_g2s(sl + pl.oX[0] + x * xb[0], a.fld[0] + (size_t)(e + x) * 4 * PP, xb[0], bar);
-      // environmentals (P,P,2,nEl): variable 2 (drag) of each element
-      if (xb[1])
+      // environmentals (P,P,2,nEl): variable 2 (drag) of each element; both
+      // variables where P is odd (the second alone is not 16-byte aligned)
+      if (xb[1] && T::kOdd) bulk_g2s(sl + pl.oX[1], a.fld[1] + (size_t)e * 2 * PP, nl * xb[1], bar);
+      else if (xb[1])
         for (uint32_t x = 0; x < nl; ++x)
           bulk_g2s(sl + pl.oX[1] + x * xb[1], a.fld[1] + (size_t)(e + x) * 2 * PP + PP, xb[1], bar);
       if (xb[2])
@@ -391,7 +665,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
   R* gU = gBase + ee * EB;      // this thread's element: fluxes, later node fields
   R* gF1 = gU + NV * PP;        // eta flux [NV][P][P]
   R* gfb = gU + T::kU;          // [4][SS]: [NV][P] per side
-  R* gD = (EPG > 1) ? gBase + EPG * EB + ee * NV * PP : gU;  // divergence sums
+  R* gD = T::kDiv ? gBase + EPG * EB + ee * NV * PP : gU;  // divergence sums
   constexpr int rNhat = kRec.oNhat, rNs = kRec.oNs, rJ = kRec.oJ, rSi = kRec.oSi;
 
   int st = 0;        // stage of item w
@@ -456,7 +730,8 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
           na[0] = gg[2 * n];
           na[1] = gg[2 * n + 1];
         }
-        if (pl.oX[1] >= 0) na[2] = reinterpret_cast<const double*>(sl + pl.oX[1] + ee * xb[1])[n];
+        if (pl.oX[1] >= 0)
+          na[2] = reinterpret_cast<const double*>(sl + pl.oX[1] + ee * xb[1])[n + (T::kOdd ? PP : 0)];
       }
     };
 
@@ -502,7 +777,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
     if (active) {
 #pragma unroll
       for (int v = 0; v < NV; ++v) f[v] = (R)sq[n + PP * v];
-      Phys::template node_flux<R>(f, a);
+      T::flux_fields(f, a);
       double na[3];
       node_aux(na);
       R Fx[NV], Fy[NV];
@@ -534,174 +809,26 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
     }
     group_bar();  // contravariant fluxes ready
 
-    // ---- B (alongside the face phase C): weak-divergence volume sums, the
-    // reference's order per node and variable (VectorDGDivergence_2D,
-    // src/SELF_Lagrange.f90):
-    //   d = 0;  for m ascending: d = (d + dgM(m,i) F0(m,j)) + dgM(m,j) F1(i,m).
-    // A thread sums a 2x2 block of nodes for two variables, so every loaded
-    // flux pair and dgMatrix pair serves two nodes.  One-element groups write
-    // the sums over the xi flux ([NV][P^2], node-major) once the warp has read
-    // it; two-element groups write them to their separate array.
-    // Production FP64 and FP32-bulk forms at P = 8 and P = 6: the same sums
-    // as FP64 tensor-core products (mma.sync m8n8k4 f64), D(j,i) = sum_m
-    // F0(m,j) dgM(m,i) + dgM(m,j) F1(i,m), four chained products per variable
-    // over one warp per element (a P = 6 element is padded with zeros to the
-    // 8x8 shape; FP32-bulk fluxes are widened exactly to FP64 and the sums
-    // rounded back once).  The order of the additions inside a product is the
-    // hardware's, so only the forms without the reference's rounding use it.
-    // At P = 4 one product covers both elements of a tile: rows and columns
-    // 0-3 belong to the first element, 4-7 to the second; the xi product's
-    // A rows and the eta product's B columns carry the element's flux, the
-    // dgMatrix operand is the same for both, and the two diagonal 4x4 blocks
-    // of the sum are the two elements' sums (the off-diagonal ones mix the
-    // elements and are dropped).
-    if constexpr (kDmma4) {
-      const int lane = t & 31, gq = lane >> 2, kq = lane & 3;
-      const int eR = gq >> 2, jr = gq & 3;   // the element and node row of this lane's A row / B column
-      const R* bU = gBase + eR * EB;
-      const R* bF1 = bU + NV * PP;
-      const double dg = sdg[dgat(kq, jr)];    // dgM(m = kq, jr): B of the xi product, A of the eta product
-      // this lane's sums: row gq, columns 2 kq, 2 kq + 1 -> element kq >> 1
-      const bool diag = (eR == (kq >> 1)) && eR < nLive;
-      R* bD = gBase + EPG * EB + eR * NV * PP;
-      using R2 = typename std::conditional<sizeof(R) == 8, double2, float2>::type;
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        double c0 = 0.0, c1 = 0.0;
-        const double aF0 = (double)bU[v * PP + f0at(kq, jr)];  // F0 at (m = kq, j = jr)
-        const double bF = (double)bF1[v * PP + f1at(jr, kq)];   // F1 at (i = jr, m = kq)
-        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                     : "+d"(c0), "+d"(c1)
-                     : "d"(aF0), "d"(dg));
-        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                     : "+d"(c0), "+d"(c1)
-                     : "d"(dg), "d"(bF));
-        if (diag) {  // D(j = jr, i = 2 (kq & 1)), D(jr, 2 (kq & 1) + 1)
-          R2 x;
-          x.x = (R)c0;
-          x.y = (R)c1;
-          reinterpret_cast<R2*>(bD + v * PP + P * jr)[kq & 1] = x;
-        }
-      }
-    } else if constexpr (kDmma) {
-      // the warps a tile's face threads leave free take its elements in turn
-      // (a one-element group: the warp that is not the face warp)
-      constexpr int kDW = (EPG == 1) ? 1 : ((TPE - EPG * 4 * P) / 32 > 0 ? (TPE - EPG * 4 * P) / 32 : 1);
-      const int w = t >> 5;
-      const bool run = (EPG == 1) ? (w != faceWarp) : (w < kDW);
-      for (int eB = (EPG == 1) ? 0 : w; run && eB < nLive; eB += kDW) {  // uniform over the warp
-        const R* bU = gBase + eB * EB;
-        const R* bF1 = bU + NV * PP;
-        R* bD = (EPG > 1) ? gBase + EPG * EB + eB * NV * PP : gBase;
-        const int lane = t & 31, gq = lane >> 2, kq = lane & 3;
-        double dv[NV][2];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-          double c0 = 0.0, c1 = 0.0;
-#pragma unroll
-          for (int kk = 0; kk < 2; ++kk) {
-            const int m = 4 * kk + kq;
-            const bool in = (P == 8) || (gq < P && m < P);  // the zero padding of P = 6
-            const double aF0 = in ? (double)bU[v * PP + f0at(m, gq)] : 0.0;  // F0 at (m, j = gq)
-            const double dg = in ? sdg[dgat(m, gq)] : 0.0;                    // dgM(m, gq)
-            const double bF = in ? (double)bF1[v * PP + f1at(gq, m)] : 0.0;   // F1 at (i = gq, m)
-            asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                         : "+d"(c0), "+d"(c1)
-                         : "d"(aF0), "d"(dg));
-            asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                         : "+d"(c0), "+d"(c1)
-                         : "d"(dg), "d"(bF));
-          }
-          dv[v][0] = c0;  // D(j = gq, i = 2 kq), D(gq, 2 kq + 1)
-          dv[v][1] = c1;
-        }
-        if constexpr (EPG == 1) __syncwarp();  // the warp has read the xi flux it overwrites
-        using R2 = typename std::conditional<sizeof(R) == 8, double2, float2>::type;
-        if (gq < P && 2 * kq + 1 < P) {
-#pragma unroll
-          for (int v = 0; v < NV; ++v) {
-            R2 x;
-            x.x = (R)dv[v][0];
-            x.y = (R)dv[v][1];
-            reinterpret_cast<R2*>(bD + v * PP + P * gq)[kq] = x;
-          }
-        }
-      }
-    } else {
-      const bool mine = (EPG == 1) ? (TPE < 64 || (t >> 5) != faceWarp) : (t < EPG * T::NB);
-      if (mine) {
-        using R2 = typename std::conditional<sizeof(R) == 8, double2, float2>::type;
-        constexpr int HB = T::HB;
-        const int eB = (EPG == 1) ? 0 : t / T::NB;
-        const int tb = (EPG == 1) ? (t & 31) : t - eB * T::NB;
-        const bool on = (EPG == 1) ? (tb < T::NB) : (eB < nLive);
-        const R* bU = gBase + eB * EB;
-        const R* bF1 = bU + NV * PP;
-        R* bD = (EPG > 1) ? gBase + EPG * EB + eB * NV * PP : gBase;
-        const int vp = tb / (HB * HB), rem = tb - vp * (HB * HB), bj = rem / HB, bi = rem - bj * HB;
-        const int v0 = 2 * vp;
-        const bool two = v0 + 1 < NV;
-        R acc[2][2][2];  // [variable of the pair][row offset r (j)][column offset c (i)]
-#pragma unroll
-        for (int vv = 0; vv < 2; ++vv)
-#pragma unroll
-          for (int r = 0; r < 2; ++r) acc[vv][r][0] = acc[vv][r][1] = (R)0;
-        if (on) {
-          const double2* sdg2 = reinterpret_cast<const double2*>(sdg);
-#pragma unroll
-          for (int mp = 0; mp < HB; ++mp) {
-            R f0[2][2][2];  // [vv][r][k]: F0(2 mp + k, 2 bj + r)
-            R f1[2][2][2];  // [vv][k][c]: F1(2 bi + c, 2 mp + k)
-#pragma unroll
-            for (int vv = 0; vv < 2; ++vv) {
-              const int v = (vv == 0 || two) ? v0 + vv : v0;
-#pragma unroll
-              for (int r = 0; r < 2; ++r) {
-                const int row = 2 * bj + r;
-                const R2 x = reinterpret_cast<const R2*>(bU + v * PP + P * row)[T::f0pos(2 * mp, row) >> 1];
-                f0[vv][r][0] = x.x;
-                f0[vv][r][1] = x.y;
-              }
-#pragma unroll
-              for (int kq = 0; kq < 2; ++kq) {
-                const R2 x = reinterpret_cast<const R2*>(bF1 + v * PP + P * (2 * mp + kq))[bi];
-                f1[vv][kq][0] = x.x;
-                f1[vv][kq][1] = x.y;
-              }
-            }
-#pragma unroll
-            for (int kq = 0; kq < 2; ++kq) {
-              const int m = 2 * mp + kq;
-              const double2 dI = sdg2[bi + HB * m], dJ = sdg2[bj + HB * m];
-              const R gi[2] = {(R)dI.x, (R)dI.y}, gj[2] = {(R)dJ.x, (R)dJ.y};
-#pragma unroll
-              for (int vv = 0; vv < 2; ++vv)
-#pragma unroll
-                for (int r = 0; r < 2; ++r)
-#pragma unroll
-                  for (int c = 0; c < 2; ++c)
-                    acc[vv][r][c] = acc[vv][r][c] + gi[c] * f0[vv][r][kq] + gj[r] * f1[vv][kq][c];
-            }
-          }
-        }
-        if constexpr (EPG == 1) __syncwarp();  // the warp has read the xi flux it overwrites
-        if (on) {
-#pragma unroll
-          for (int vv = 0; vv < 2; ++vv)
-            if (vv == 0 || two)
-#pragma unroll
-              for (int r = 0; r < 2; ++r) {
-                R2 x;
-                x.x = acc[vv][r][0];
-                x.y = acc[vv][r][1];
-                reinterpret_cast<R2*>(bD + (v0 + vv) * PP + P * (2 * bj + r))[bi] = x;
-              }
-        }
-      }
-    }
+    // ---- B (alongside the face phase C): weak-divergence volume sums
+    tile_volume_sums<P, Phys, R>(gBase, sdg, t, faceWarp, nLive);
 
     // ---- C: faces; own traces of this stage's solution come from the cache,
     // the neighbour's were loaded before phase A
+    R dreg[NV];
+    if constexpr (T::kRegDiv) {
+      if (faceOn && !kNbrEarly) load_neighbour();  // in flight during the sums
+      if (active) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) dreg[v] = (R)0;
+#pragma unroll
+        for (int m = 0; m < P; ++m) {
+          const R gi = (R)sdg[dgat(m, i)], gj = (R)sdg[dgat(m, j)];
+#pragma unroll
+          for (int v = 0; v < NV; ++v)
+            dreg[v] = dreg[v] + gi * gU[v * PP + f0at(m, j)] + gj * gF1[v * PP + f1at(i, m)];
+        }
+      }
+    }
     {
       if (faceOn) {
         if (gridWait) {
@@ -711,7 +838,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
             gflag[g] = 0;  // checked after phase C
           __syncwarp();
         }
-        if (!kNbrEarly || gridWait) load_neighbour();
+        if ((!kNbrEarly && !T::kRegDiv) || gridWait) load_neighbour();
         const long long eF = e0 + eC;
         const int bcid = ssi[4];
         const bool physical = (bcid != 0) && (ssi[2] == 0);
@@ -755,7 +882,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
           velL[0] = vo[ii + P * (0 + 2 * s1)];
           velL[1] = vo[ii + P * (1 + 2 * s1)];
           R* vOut = velOut;
-          if constexpr (ref_rounding<R>()) {
+          if constexpr (ref_rounding<R>() || T::kOdd) {
             vOut[ii + P * (0 + 2 * (s1 + 4 * eF))] = L[0] / L[2];
             vOut[ii + P * (1 + 2 * (s1 + 4 * eF))] = L[1] / L[2];
           } else {
@@ -811,7 +938,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
       Phys::template source<double>(qv, na, a, Src);
       R d[NV];  // volume sums from phase B
 #pragma unroll
-      for (int v = 0; v < NV; ++v) d[v] = gD[v * PP + n];
+      for (int v = 0; v < NV; ++v) d[v] = T::kRegDiv ? dreg[v] : gD[v * PP + n];
       if constexpr (ref_rounding<R>()) {
         // the reference's divisions, rounded as it rounds them (bit-exact form)
         const R wi = (R)sqw[i], wj = (R)sqw[j];
@@ -865,50 +992,16 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
     }
     group_bar();
 
-    // ---- E: traces of the updated solution -> trace cache.  One task per
-    // (element, field, line, orientation) reads the line's P values once and
-    // forms both of its end traces (BoundaryInterp, src/SELF_Lagrange.f90:
-    // 2241-2270): column l gives S (side 0) and N (side 2), row l gives W (3)
-    // and E (1).  Tasks are numbered by field pair, orientation, field, line,
-    // so that for P = 8 a half-warp reads the column lines (or the row lines)
-    // of two fields.
+    // ---- E: traces of the updated solution -> trace cache.  (A one-element
+    // group's face warp starts one warp later, so the other warp takes the
+    // last, partial round.)
     {
-      // P = 8 numbers the tasks by field pair (an odd NT leaves the last
-      // pair's second half idle); the padded layouts of the other P number
-      // them by orientation, field, line, with no idle tasks
-      constexpr int NTp = T::kSwz ? (NT + 1) / 2 * 2 : NT;
-      constexpr int TPEl = 2 * NTp * P;  // tasks per element
-      // a one-element group's face warp starts one warp later, so the other
-      // warp takes the last, partial round
       const int k0 = (EPG == 1) ? (faceWarp ? t : (t + 32) % TPE) : t;
-      for (int kk = k0; kk < EPG * TPEl; kk += TPE) {
-        const int eE = kk / TPEl, ks = kk - eE * TPEl;
-        if (eE >= nLive) continue;
-        int row, fi, l;
-        if constexpr (T::kSwz) {
-          const int fp = ks / (4 * P), r = ks - fp * 4 * P, r2 = r - (r / (2 * P)) * 2 * P, fs = r2 / P;
-          row = r / (2 * P);
-          l = r2 - fs * P;
-          fi = 2 * fp + fs;
-          if (fi >= NT) continue;
-        } else {
-          row = ks / (NT * P);
-          const int r = ks - row * NT * P;
-          fi = r / P;
-          l = r - fi * P;
-        }
-        const R* fv = gBase + eE * EB + fi * FS;
-        R lo = (R)0, hi = (R)0;
-#pragma unroll
-        for (int m = 0; m < P; ++m) {
-          const R x = fv[row ? T::nf(fi, m, l) : T::nf(fi, l, m)];
-          lo = lo + bm_left<R>(a, m) * x;  // kernel-parameter constants (m is unrolled)
-          hi = hi + bm_right<R, P>(a, m) * x;
-        }
+      tile_traces<P, Phys, R>(gBase, EB, EPG, nLive, k0, TPE, a, [&](int eE, int fi, int l, bool row, R lo, R hi) {
         R* o = trOut + (size_t)4 * TS * (e0 + eE);
         o[l + P * fi + TS * (row ? 3 : 0)] = lo;
         o[l + P * fi + TS * (row ? 1 : 2)] = hi;
-      }
+      });
     }
     // no barrier here: the next tile's post-wait barrier orders the reuse of the arrays
     if constexpr (kMulti) {
@@ -936,7 +1029,6 @@ inline bool make_tma_plan(const StageArgs& a, int smemLimit, TmaPlan& pl, int ma
   constexpr int PP = T::PP, NV = T::NV, TS = T::TS, EPG = T::EPG;
   constexpr bool kLSW = (NV == 3 && !Phys::kLaggedVelocity);
   constexpr bool kSW = Phys::kLaggedVelocity;
-  if (P % 2 != 0) return false;
   int o = 0;
   auto put = [&](int bytes) {  // one piece of a tile: EPG elements' blocks back to back
     int at = o;
@@ -964,7 +1056,7 @@ inline bool make_tma_plan(const StageArgs& a, int smemLimit, TmaPlan& pl, int ma
     pl.oVelOwn = put(8 * P * (int)sizeof(R));
   } else {
     if (a.fld[0]) pl.oX[0] = put(2 * PP * 8);
-    if (a.fld[1]) pl.oX[1] = put(PP * 8);
+    if (a.fld[1]) pl.oX[1] = put((P % 2 ? 2 : 1) * PP * 8);
     if (a.fld[2])
       for (int x = 2; x < 5; ++x) pl.oX[x] = put(16 * P * 8);
   }

@@ -30,46 +30,44 @@ inline bool aligned16(const void* p) { return ((uintptr_t)p % 16) == 0; }
 template <int P, class Phys, typename R>
 cudaError_t launch_one(const StageArgs& a, const StageLaunch& L, cudaStream_t st, int* usedTma) {
   *usedTma = 0;
-  if constexpr (P % 2 == 0) {
-    bool ok = L.allowTma && a.mode != MODE_TRACES && a.geo != nullptr && aligned16(a.geo) && aligned16(a.q) &&
-              aligned16(sizeof(R) == 4 ? (const void*)a.Gf : (const void*)a.G) && aligned16(a.trIn) &&
-              (a.velIn == nullptr || aligned16(a.velIn));
-    for (int k = 0; k < 5; ++k) ok = ok && (a.fld[k] == nullptr || aligned16(a.fld[k]));
-    TmaPlan pl{};
-    if (ok && make_tma_plan<P, Phys, R>(a, L.smemOptin, pl, L.maxGroups)) {
-      // the shared-memory opt-in is per device: one bit per device that has it
-      static std::atomic<unsigned long long> attrSet{0};  // one instantiation per (P, Phys, R)
-      int dev = 0;
-      cudaError_t e = cudaGetDevice(&dev);
+  bool ok = L.allowTma && a.mode != MODE_TRACES && a.geo != nullptr && aligned16(a.geo) && aligned16(a.q) &&
+            aligned16(sizeof(R) == 4 ? (const void*)a.Gf : (const void*)a.G) && aligned16(a.trIn) &&
+            (a.velIn == nullptr || aligned16(a.velIn));
+  for (int k = 0; k < 5; ++k) ok = ok && (a.fld[k] == nullptr || aligned16(a.fld[k]));
+  TmaPlan pl{};
+  if (ok && make_tma_plan<P, Phys, R>(a, L.smemOptin, pl, L.maxGroups)) {
+    // the shared-memory opt-in is per device: one bit per device that has it
+    static std::atomic<unsigned long long> attrSet{0};  // one instantiation per (P, Phys, R)
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+    if (!(attrSet.load() & bit)) {
+      e = cudaFuncSetAttribute(k_fused_stage_tma<P, Phys, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               L.smemOptin);
       if (e != cudaSuccess) return e;
-      const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
-      if (!(attrSet.load() & bit)) {
-        e = cudaFuncSetAttribute(k_fused_stage_tma<P, Phys, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 L.smemOptin);
-        if (e != cudaSuccess) return e;
-        attrSet.fetch_or(bit);
-      }
-      using T = TmaTraits<P, Phys, R>;
-      const int tiles = (a.nEl + T::EPG - 1) / T::EPG;  // work items of EPG consecutive elements
-      const int grid = tiles < L.numSMs ? tiles : L.numSMs;
-      // Programmatic dependent launch: the launch and the kernel's prologue
-      // overlap the end of the previous kernel on the stream; the kernel waits
-      // for that kernel's completion (griddepcontrol.wait) before it touches
-      // any data the previous kernel may write or read.
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(grid);
-      cfg.blockDim = dim3(pl.groups * T::TPE);
-      cfg.dynamicSmemBytes = pl.smemBytes;
-      cfg.stream = st;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr[0].val.programmaticStreamSerializationAllowed = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      *usedTma = 1;
-      const TmaSteps none{};
-      return cudaLaunchKernelEx(&cfg, k_fused_stage_tma<P, Phys, R>, a, pl, none);
+      attrSet.fetch_or(bit);
     }
+    using T = TmaTraits<P, Phys, R>;
+    const int tiles = (a.nEl + T::EPG - 1) / T::EPG;  // work items of EPG consecutive elements
+    const int grid = tiles < L.numSMs ? tiles : L.numSMs;
+    // Programmatic dependent launch: the launch and the kernel's prologue
+    // overlap the end of the previous kernel on the stream; the kernel waits
+    // for that kernel's completion (griddepcontrol.wait) before it touches
+    // any data the previous kernel may write or read.
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(pl.groups * T::TPE);
+    cfg.dynamicSmemBytes = pl.smemBytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    *usedTma = 1;
+    const TmaSteps none{};
+    return cudaLaunchKernelEx(&cfg, k_fused_stage_tma<P, Phys, R>, a, pl, none);
   }
   constexpr int EPB = elems_per_block<P, Phys, R>();
   const int grid = (a.nEl + EPB - 1) / EPB;
