@@ -80,8 +80,7 @@ class ClosureMLP:
         n = features.shape[0]
         f = features.contiguous()
         y = labels.contiguous().to(torch.float32)
-        self.fmin = f.min(dim=0).values.cpu().numpy().astype(np.float32)
-        self.fmax = f.max(dim=0).values.cpu().numpy().astype(np.float32)
+        self.fmin, self.fmax = torch.stack(torch.aminmax(f, dim=0)).cpu().numpy().astype(np.float32)
         loss = np.zeros(epochs, dtype=np.float32)
         torch.cuda.synchronize()
         check(lib().selfgpu_mlp_train(f.data_ptr(), y.data_ptr(), int(n), int(epochs), int(batch), float(lr),

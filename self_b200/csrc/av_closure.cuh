@@ -103,52 +103,14 @@ __device__ __forceinline__ R av_sqrt(R x) {
   else return sqrtf(x);
 }
 
-// Modal decay activation from one variable's modes c[k + P l] (one thread).
-template <int P, typename R>
-__device__ R modal_activation(const R* c, double s0, double kappa) {
-  constexpr int N = P - 1;
-  R top = (R)0, total = (R)0;
-  for (int l = 0; l < P; ++l)
-    for (int k = 0; k < P; ++k) {
-      const R e = c[k + P * l] * c[k + P * l];
-      total = total + e;
-      if (k == N || l == N) top = top + e;
-    }
+// Modal decay activation from the energies of the top shell and of all modes.
+template <typename R>
+__device__ R activation_of(R top, R total, double s0, double kappa) {
   if (!(top > (R)0) || !(total > (R)0)) return (R)0;
   const R sv = av_log10<R>(top / total);
   if (sv < (R)s0 - (R)kappa) return (R)0;
   if (sv > (R)s0 + (R)kappa) return (R)1;
   return (R)0.5 * ((R)1 + av_sin<R>((R)kAvPi * (sv - (R)s0) / ((R)2 * (R)kappa)));
-}
-
-// The 18 features of one variable's modes (one thread); requires P >= 6.
-template <int P, typename R>
-__device__ void modal_features(const R* c, float* f) {
-  constexpr int N = P - 1;
-  R total = (R)0, sh[P], ex[P], ey[P];
-#pragma unroll
-  for (int k = 0; k < P; ++k) sh[k] = ex[k] = ey[k] = (R)0;
-  for (int l = 0; l < P; ++l)
-#pragma unroll
-    for (int k = 0; k < P; ++k) {
-      const R e = c[k + P * l] * c[k + P * l];
-      total = total + e;
-      const int m = k > l ? k : l;
-      sh[m] = sh[m] + e;
-      ex[k] = ex[k] + e;
-      ey[l] = ey[l] + e;
-    }
-#pragma unroll
-  for (int r = 0; r < 6; ++r) {
-    const int m = N - 5 + r;
-    const R fr[3] = {sh[m], ex[m], ey[m]};
-#pragma unroll
-    for (int g = 0; g < 3; ++g) {
-      R q = total > (R)0 ? fr[g] / total : (R)0;
-      if (q < (R)1e-16) q = (R)1e-16;
-      f[r + 6 * g] = (float)((av_log10<R>(q) + (R)8) / (R)8);
-    }
-  }
 }
 
 // ------------------------------------------------------ viscosity kernel
@@ -578,36 +540,82 @@ __global__ void __launch_bounds__(EPB* P* P, 4) k_av_grad(const AvArgs a) {
 }
 
 // Closure features of a stored FP64 state (training-data harvest): per element
-// the indicator activation and the 36 features.
+// the indicator activation and the 36 features, one warp per element.  Both
+// modal transforms are FP64 tensor-core products (m8n8k4, a P x P field padded
+// with zeros), the matrix held in registers as both products' operand, the
+// first product's result moved into the second's operand layout by shuffles;
+// then one lane per feature.  (A block per element whose first two threads
+// summed and took the logarithms alone: 115 us for 16 384 elements at P = 8.)
 template <int P>
-__global__ void __launch_bounds__(P* P) k_closure_features(const double* __restrict__ q, int nEl, AvArgs a,
-                                                            float* __restrict__ act, float* __restrict__ feat) {
-  constexpr int PP = P * P;
-  __shared__ double sq[2][PP], tt[2][PP], cc[2][PP], sT[PP];
-  const int t = threadIdx.x, i = t % P, j = t / P;
-  const long long e = blockIdx.x;
-  if (e >= nEl) return;
-  sT[t] = a.T[t];
-  sq[0][t] = q[t + (long long)PP * (2 + 4 * e)];
-  sq[1][t] = q[t + (long long)PP * (3 + 4 * e)];
-  __syncthreads();
+__global__ void __launch_bounds__(32 * kNuWarps) k_closure_features(const double* __restrict__ q, int nEl,
+                                                                    const AvArgs a, float* __restrict__ act,
+                                                                    float* __restrict__ feat) {
+  constexpr int PP = P * P, N = P - 1, KK = (P + 3) / 4;
+  __shared__ double cc[kNuWarps][2][PP];
+  const int w = threadIdx.x / 32, lane = threadIdx.x % 32, row = lane >> 2, col = lane & 3;
+  // T(row, col + 4 kk): rows of T as the first product's A, columns of T^T as the second's B
+  double T[KK];
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    double acc = 0.0;
-    for (int m = 0; m < P; ++m) acc = acc + sT[i + P * m] * sq[r][m + P * j];
-    tt[r][i + P * j] = acc;
-  }
-  __syncthreads();
+  for (int kk = 0; kk < KK; ++kk) T[kk] = row < P && col + 4 * kk < P ? a.T[row + P * (col + 4 * kk)] : 0.0;
+  auto mma = [](double& c0, double& c1, double x, double y) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(c0), "+d"(c1)
+                 : "d"(x), "d"(y));
+  };
+  for (long long e = (long long)blockIdx.x * kNuWarps + w; e < nEl; e += (long long)gridDim.x * kNuWarps) {
+    double total[2] = {0.0, 0.0};
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    double acc = 0.0;
-    for (int m = 0; m < P; ++m) acc = acc + sT[j + P * m] * tt[r][i + P * m];
-    cc[r][i + P * j] = acc;
-  }
-  __syncthreads();
-  if (t == 0 && act) act[e] = (float)modal_activation<P, double>(cc[0], a.s0, a.kappa);
-  if constexpr (P >= 6) {
-    if (t < 2 && feat) modal_features<P, double>(cc[t], feat + kMlpIn * e + 18 * t);
+    for (int r = 0; r < 2; ++r) {  // density, total energy
+      if (r == 1 && (P < 6 || !feat)) break;
+      const double* qe = q + (long long)PP * (2 + r + 4 * e);
+      double t0 = 0.0, t1 = 0.0;  // sum_m T(k, m) q(m, jj) at k = row, jj = 2 col, 2 col + 1
+#pragma unroll
+      for (int kk = 0; kk < KK; ++kk) {
+        const int m = col + 4 * kk;
+        mma(t0, t1, T[kk], row < P && m < P ? qe[m + P * row] : 0.0);
+      }
+      double c0 = 0.0, c1 = 0.0;  // sum_m (..)(k, m) T(l, m) at k = row, l = 2 col, 2 col + 1
+#pragma unroll
+      for (int kk = 0; kk < KK; ++kk) {
+        const int src = (lane & 28) + ((col + 4 * kk) >> 1);
+        const double x0 = __shfl_sync(0xffffffffu, t0, src), x1 = __shfl_sync(0xffffffffu, t1, src);
+        mma(c0, c1, (col & 1) ? x1 : x0, T[kk]);
+      }
+      c0 = c0 * c0;
+      c1 = c1 * c1;
+      if (row < P && 2 * col < P) cc[w][r][row + P * 2 * col] = c0;
+      if (row < P && 2 * col + 1 < P) cc[w][r][row + P * (2 * col + 1)] = c1;
+      double s = c0 + c1;  // (the padding's are zero)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      total[r] = s;
+    }
+    __syncwarp();
+    // lane tasks: the features, then (task kMlpIn) the activation
+    const int f0 = (P >= 6 && feat) ? lane : (lane == 0 ? kMlpIn : kMlpIn + 1);
+    for (int f = f0; f <= kMlpIn; f += 32) {
+      const bool top = f == kMlpIn;
+      const int r = top ? 0 : f / 18, grp = top ? 0 : (f % 18) / 6, m = top ? N : N - 5 + f % 6;
+      const double* e2 = cc[w][r];
+      double sum = 0.0;
+      if (grp == 0) {
+        for (int l = 0; l < m; ++l) sum = sum + e2[m + P * l];
+        for (int k = 0; k <= m; ++k) sum = sum + e2[k + P * m];
+      } else if (grp == 1) {
+        for (int l = 0; l < P; ++l) sum = sum + e2[m + P * l];
+      } else {
+        for (int k = 0; k < P; ++k) sum = sum + e2[k + P * m];
+      }
+      const double t = r ? total[1] : total[0];
+      if (top) {
+        if (act) act[e] = (float)activation_of<double>(sum, t, a.s0, a.kappa);
+      } else {
+        double x = t > 0.0 ? sum / t : 0.0;
+        if (x < 1e-16) x = 1e-16;
+        feat[kMlpIn * e + f] = (float)((log10(x) + 8.0) / 8.0);
+      }
+    }
+    __syncwarp();
   }
 }
 

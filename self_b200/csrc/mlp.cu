@@ -1,13 +1,17 @@
 // Training and standalone inference kernels of the closure MLP
 // (36 -> 32 -> 32 -> 1, ReLU, output clamped to [0, 1]; see av_closure.cuh).
 //
-// Training: minibatch Adam on float32 master weights.  Each step rounds the
-// weights to bfloat16 for the forward pass (the precision the closure runs
-// in), runs forward + backward with one thread per sample, reduces the
-// per-sample gradients across each warp with shuffles, accumulates warp sums
-// in shared memory and adds each block's sums to the global gradient once.
+// Training: minibatch Adam on float32 master weights, two kernels per step:
+//   k_grad  rounds the weights to bfloat16 for the forward pass (the precision
+//           the closure runs in) and takes the batch in tiles of 32 samples; a
+//           block keeps its tiles' activations and deltas in shared memory and
+//           every thread sums its own few parameters' gradients over the tile's
+//           samples in registers (dW = delta^T activation, an outer-product
+//           contraction), so the block writes each partial sum once;
+//   k_adam  adds the blocks' partial sums in a fixed order and updates.
 // Samples are drawn with replacement by a counter-based hash of
-// (seed, step, lane), so a run is reproducible for a given seed.
+// (seed, step, lane) and every sum has a fixed order, so a run is reproducible
+// bit for bit for a given seed.
 //
 // Loss: (clamp(z) - y)^2 with the gradient passed straight through the clamp
 // when z lies on the wrong side of it (z < 0 < y or z > 1 > y); a clamped
@@ -15,8 +19,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <cstring>
 #include <string>
-#include <vector>
 
 #include "av_closure.cuh"
 #include "selfgpu_internal.h"
@@ -42,153 +46,245 @@ __device__ __forceinline__ bool is_weight(int k) {
   return (k >= oW1 && k < oB1) || (k >= oW2 && k < oB2) || (k >= oW3 && k < oB3);
 }
 
-__global__ void k_round_weights(const float* __restrict__ master, float* __restrict__ fw) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < NP; k += gridDim.x * blockDim.x)
-    fw[k] = is_weight(k) ? __bfloat162float(__float2bfloat16_rn(master[k])) : master[k];
-}
-
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
-// accumulate one parameter's per-sample gradient: warp sum, then lane 0 adds to shared
-__device__ __forceinline__ void acc_grad(float* sg, int k, float v, int lane) {
-  v = warp_sum(v);
-  if (lane == 0) atomicAdd(&sg[k], v);
-}
+constexpr int kTile = 32;            // samples per tile, one per lane
+constexpr int kGradThreads = 256;
+constexpr int NPP = (NP + 31) / 32 * 32;  // stride of a block's partial sums
+constexpr int kMaxGradBlocks = 296;  // two blocks per SM; larger batches loop over tiles
 
-__global__ void __launch_bounds__(256) k_grad(const float* __restrict__ feat, const float* __restrict__ label,
-                                              int n, const float* __restrict__ fw, float* __restrict__ grad,
-                                              float* __restrict__ loss, unsigned long long seed, long long step,
-                                              int batch) {
-  __shared__ float sw[NP], sg[NP];
-  __shared__ float sloss;
-  for (int k = threadIdx.x; k < NP; k += blockDim.x) {
-    sw[k] = fw[k];
-    sg[k] = 0.f;
+// Latency bounds a step (a 4096-sample batch is 54 MFLOP): 128 tiles on as
+// many SMs.  Adding each sample's gradient to shared memory by warp shuffles
+// (2 273 five-step sums per warp, a block per 256 samples) took 390 us for a
+// 4096-sample step; this kernel and k_adam together are launch-bound.
+__global__ void __launch_bounds__(kGradThreads) k_grad(const float* feat, const float* label, int n,
+                                                       const float* master, float* part, float* lossPart,
+                                                       unsigned long long seed, long long step, int batch) {
+  // activations and deltas [sample][unit]; the odd strides keep the lanes'
+  // (one sample each) accesses to one unit in distinct banks
+  __shared__ float sw[NP], F[kTile][IN + 1], H1[kTile][H + 1], H2[kTile][H + 1], D1[kTile][H + 1], D2[kTile][H + 1];
+  __shared__ float sz[kTile], sg[kTile];
+  __shared__ long long sidx[kTile];
+  const int t = threadIdx.x, s = t & 31, w = t >> 5;
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the previous step's weights
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  for (int k = t; k < NP; k += kGradThreads) {
+    const float m = master[k];
+    sw[k] = is_weight(k) ? __bfloat162float(__float2bfloat16_rn(m)) : m;
   }
-  if (threadIdx.x == 0) sloss = 0.f;
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool live = b < batch;  // dead lanes contribute zero gradients (warp sums stay uniform)
-  long long idx = 0;
-  if (live) idx = (long long)(mix64(seed ^ mix64((unsigned long long)step * 0x100000001ull + (unsigned long long)b)) %
-                              (unsigned long long)n);
-  float f[IN], h1[H], h2[H];
+  // this thread's parameters: 9 of W1 (threads 0-127) or 8 of W2 (128-255),
+  // one row's consecutive columns; threads 0-96 also one of b1, b2, w3, b3
+  const int half = t >> 7, row = (t & 127) >> 2, col = (t & 3) * (half ? 8 : 9);
+  float acc[9], accB = 0.f, lsum = 0.f;
 #pragma unroll
-  for (int k = 0; k < IN; ++k) f[k] = live ? feat[k + (long long)IN * idx] : 0.f;
-#pragma unroll
-  for (int j = 0; j < H; ++j) {
-    float acc = 0.f;
-#pragma unroll
-    for (int k = 0; k < IN; ++k) acc = fmaf(sw[oW1 + j * IN + k], f[k], acc);
-    acc = acc + sw[oB1 + j];
-    h1[j] = acc > 0.f ? acc : 0.f;
-  }
-#pragma unroll
-  for (int j = 0; j < H; ++j) {
-    float acc = 0.f;
-#pragma unroll
-    for (int k = 0; k < H; ++k) acc = fmaf(sw[oW2 + j * H + k], h1[k], acc);
-    acc = acc + sw[oB2 + j];
-    h2[j] = acc > 0.f ? acc : 0.f;
-  }
-  float z = 0.f;
-#pragma unroll
-  for (int k = 0; k < H; ++k) z = fmaf(sw[oW3 + k], h2[k], z);
-  z = z + sw[oB3];
-  const float y = live ? label[idx] : 0.f;
-  const float a = z < 0.f ? 0.f : (z > 1.f ? 1.f : z);
-  float d = a - y;
-  if ((z < 0.f && y > 0.f) || (z > 1.f && y < 1.f)) d = z - y;  // straight through the clamp
-  if (!live) d = 0.f;
-  const float l = live ? (a - y) * (a - y) : 0.f;
-  const float ls = warp_sum(l);
-  if (lane == 0) atomicAdd(&sloss, ls);
-  const float g = 2.f * d / (float)batch;
-  // output layer
-  float dh2[H];
-#pragma unroll
-  for (int j = 0; j < H; ++j) {
-    acc_grad(sg, oW3 + j, g * h2[j], lane);
-    dh2[j] = h2[j] > 0.f ? g * sw[oW3 + j] : 0.f;
-  }
-  acc_grad(sg, oB3, g, lane);
-  // hidden layer 2
-  float dh1[H];
-#pragma unroll
-  for (int k = 0; k < H; ++k) dh1[k] = 0.f;
-#pragma unroll
-  for (int j = 0; j < H; ++j) {
-    acc_grad(sg, oB2 + j, dh2[j], lane);
-#pragma unroll
-    for (int k = 0; k < H; ++k) {
-      acc_grad(sg, oW2 + j * H + k, dh2[j] * h1[k], lane);
-      dh1[k] = fmaf(sw[oW2 + j * H + k], dh2[j], dh1[k]);
+  for (int k = 0; k < 9; ++k) acc[k] = 0.f;
+  const int tiles = (batch + kTile - 1) / kTile;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    __syncthreads();  // the weights, or the previous tile's arrays
+    if (t < kTile) {
+      const long long b = (long long)tile * kTile + t;
+      sidx[t] = b < batch ? (long long)(mix64(seed ^ mix64((unsigned long long)step * 0x100000001ull +
+                                                           (unsigned long long)b)) %
+                                        (unsigned long long)n)
+                          : -1;
     }
-  }
-  // hidden layer 1
+    __syncthreads();
+    for (int k = t; k < kTile * IN; k += kGradThreads) {
+      const int r = k / IN, c = k - r * IN;
+      const long long idx = sidx[r];
+      F[r][c] = idx >= 0 ? feat[c + (long long)IN * idx] : 0.f;
+    }
+    __syncthreads();
 #pragma unroll
-  for (int j = 0; j < H; ++j) {
-    const float dj = h1[j] > 0.f ? dh1[j] : 0.f;
-    acc_grad(sg, oB1 + j, dj, lane);
+    for (int u = 0; u < 4; ++u) {  // lane = sample, warp = 4 hidden units
+      const int j = 4 * w + u;
+      float a = 0.f;
 #pragma unroll
-    for (int k = 0; k < IN; ++k) acc_grad(sg, oW1 + j * IN + k, dj * f[k], lane);
+      for (int k = 0; k < IN; ++k) a = fmaf(sw[oW1 + j * IN + k], F[s][k], a);
+      a = a + sw[oB1 + j];
+      H1[s][j] = a > 0.f ? a : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int j = 4 * w + u;
+      float a = 0.f;
+#pragma unroll
+      for (int k = 0; k < H; ++k) a = fmaf(sw[oW2 + j * H + k], H1[s][k], a);
+      a = a + sw[oB2 + j];
+      H2[s][j] = a > 0.f ? a : 0.f;
+    }
+    __syncthreads();
+    if (w == 0) {
+      float z = 0.f;
+#pragma unroll
+      for (int k = 0; k < H; ++k) z = fmaf(sw[oW3 + k], H2[s][k], z);
+      z = z + sw[oB3];
+      const long long idx = sidx[s];
+      const float y = idx >= 0 ? label[idx] : 0.f;
+      const float a = z < 0.f ? 0.f : (z > 1.f ? 1.f : z);
+      float d = a - y;
+      if ((z < 0.f && y > 0.f) || (z > 1.f && y < 1.f)) d = z - y;  // straight through the clamp
+      sg[s] = idx >= 0 ? 2.f * d / (float)batch : 0.f;  // lanes beyond the batch carry no gradient
+      lsum += warp_sum(idx >= 0 ? (a - y) * (a - y) : 0.f);
+    }
+    __syncthreads();
+    const float g = sg[s];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int j = 4 * w + u;
+      D2[s][j] = H2[s][j] > 0.f ? g * sw[oW3 + j] : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = 4 * w + u;
+      float a = 0.f;
+#pragma unroll
+      for (int j = 0; j < H; ++j) a = fmaf(sw[oW2 + j * H + k], D2[s][j], a);
+      D1[s][k] = H1[s][k] > 0.f ? a : 0.f;
+    }
+    __syncthreads();
+    if (half == 0) {
+#pragma unroll 4
+      for (int r = 0; r < kTile; ++r) {
+        const float d = D1[r][row];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) acc[k] = fmaf(d, F[r][col + k], acc[k]);
+      }
+    } else {
+#pragma unroll 4
+      for (int r = 0; r < kTile; ++r) {
+        const float d = D2[r][row];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[k] = fmaf(d, H1[r][col + k], acc[k]);
+      }
+    }
+    if (t < 3 * H + 1)
+      for (int r = 0; r < kTile; ++r)
+        accB = accB + (t < H ? D1[r][t] : t < 2 * H ? D2[r][t - H] : t < 3 * H ? sg[r] * H2[r][t - 2 * H] : sg[r]);
   }
-  __syncthreads();
-  for (int k = threadIdx.x; k < NP; k += blockDim.x) atomicAdd(&grad[k], sg[k]);
-  if (threadIdx.x == 0) atomicAdd(loss, sloss);
+  float* o = part + (size_t)NPP * blockIdx.x;
+#pragma unroll
+  for (int k = 0; k < 9; ++k)
+    if (half == 0) o[oW1 + row * IN + col + k] = acc[k];
+    else if (k < 8) o[oW2 + row * H + col + k] = acc[k];
+  if (t < 3 * H + 1) o[t < H ? oB1 + t : t < 2 * H ? oB2 + t - H : t < 3 * H ? oW3 + t - 2 * H : oB3] = accB;
+  if (t == 0) lossPart[blockIdx.x] = lsum;
 }
 
-__global__ void k_adam(float* __restrict__ master, float* __restrict__ grad, float* __restrict__ m1,
-                       float* __restrict__ m2, float lr, float c1, float c2) {
+// 32 parameters per block: lane = parameter, warp = every eighth block's
+// partial sum, then the eight strips in order.
+__global__ void __launch_bounds__(256) k_adam(float* master, const float* part, const float* lossPart, int blocks,
+                                              float* m1, float* m2, float* loss, float lr, float c1, float c2) {
+  __shared__ float strip[8][32];
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < NP; k += gridDim.x * blockDim.x) {
-    const float gk = grad[k];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int k = blockIdx.x * 32 + lane;
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // this step's partial sums
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  float s = 0.f;
+  if (k < NP)
+    for (int r = w; r < blocks; r += 8) s += part[(size_t)NPP * r + k];
+  strip[w][lane] = s;
+  __syncthreads();
+  if (w == 0 && k < NP) {
+    float gk = 0.f;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) gk += strip[r][lane];
     m1[k] = b1 * m1[k] + (1.f - b1) * gk;
     m2[k] = b2 * m2[k] + (1.f - b2) * gk * gk;
     const float mh = m1[k] / c1, vh = m2[k] / c2;
     master[k] -= lr * mh / (sqrtf(vh) + eps);
-    grad[k] = 0.f;
+  }
+  if (blockIdx.x == 0 && w == 1) {
+    float l = 0.f;
+    for (int r = lane; r < blocks; r += 32) l += lossPart[r];
+    l = warp_sum(l);
+    if (lane == 0) *loss += l;
   }
 }
 
-// One thread per sample; the arithmetic of the in-stage MLP (av_closure.cuh).
-__global__ void __launch_bounds__(256) k_infer(const float* __restrict__ feat, int n,
-                                               const __nv_bfloat16* __restrict__ w, const float* __restrict__ p,
-                                               float* __restrict__ out) {
-  __shared__ float sW1[H * IN], sW2[H * H], sw3[H], sB[kMlpFloats];
-  for (int k = threadIdx.x; k < H * IN; k += blockDim.x) sW1[k] = __bfloat162float(w[k]);
-  for (int k = threadIdx.x; k < H * H; k += blockDim.x) sW2[k] = __bfloat162float(w[H * IN + k]);
-  for (int k = threadIdx.x; k < H; k += blockDim.x) sw3[k] = __bfloat162float(w[H * IN + H * H + k]);
-  for (int k = threadIdx.x; k < kMlpFloats; k += blockDim.x) sB[k] = p[k];
-  __syncthreads();
-  const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  float f[IN], h1[H];
-#pragma unroll
-  for (int k = 0; k < IN; ++k) f[k] = feat[k + (long long)IN * s];
-#pragma unroll
-  for (int j = 0; j < H; ++j) {
-    float acc = 0.f;
-#pragma unroll 4
-    for (int k = 0; k < IN; ++k) acc = fmaf(sW1[j * IN + k], f[k], acc);
-    acc = acc + sB[j];
-    h1[j] = acc > 0.f ? acc : 0.f;
+// A launch that may overlap the end of the previous kernel on the stream; the
+// kernel waits for that kernel's completion itself (griddepcontrol.wait).
+template <class... KArgs, class... Args>
+cudaError_t launch_dependent(void (*kernel)(KArgs...), int grid, int block, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
+// Weights (bfloat16 pairs) and parameters, passed by value: no device buffer
+// and no copy per call.
+struct MlpArgs {
+  uint32_t w[kMlpWeights / 2];
+  float p[kMlpFloats];
+};
+static_assert(kMlpWeights % 2 == 0, "weights travel as pairs");
+
+// The arithmetic of the in-stage MLP (av_closure.cuh).  Tiles of 32 samples as
+// in k_grad: lane = sample, warp = four hidden units.  (One thread per sample
+// evaluated its 2 208 products alone on at most one block per 256 samples:
+// 28 us for 16 384 samples.)
+__global__ void __launch_bounds__(kGradThreads) k_infer(const float* __restrict__ feat, int n,
+                                                        const __grid_constant__ MlpArgs args,
+                                                        float* __restrict__ out) {
+  __shared__ float sw[kMlpWeights], sB[2 * H + 1], F[kTile][IN + 1], H1[kTile][H + 1], H2[kTile][H + 1];
+  const int t = threadIdx.x, s = t & 31, w = t >> 5;
+  for (int k = t; k < kMlpWeights / 2; k += kGradThreads) {
+    const uint32_t x = args.w[k];
+    sw[2 * k] = __uint_as_float(x << 16);
+    sw[2 * k + 1] = __uint_as_float(x & 0xffff0000u);
   }
-  float z = 0.f;
-  for (int j = 0; j < H; ++j) {
-    float acc = 0.f;
-#pragma unroll 4
-    for (int k = 0; k < H; ++k) acc = fmaf(sW2[j * H + k], h1[k], acc);
-    acc = acc + sB[H + j];
-    z = fmaf(sw3[j], acc > 0.f ? acc : 0.f, z);
+  for (int k = t; k < 2 * H + 1; k += kGradThreads) sB[k] = args.p[k];
+  const float *sW1 = sw, *sW2 = sw + H * IN, *sw3 = sW2 + H * H;
+  for (long long s0 = (long long)blockIdx.x * kTile; s0 < n; s0 += (long long)gridDim.x * kTile) {
+    const int live = n - s0 < kTile ? (int)(n - s0) : kTile;
+    __syncthreads();
+    for (int k = t; k < kTile * IN; k += kGradThreads) {
+      const int r = k / IN;
+      F[r][k - r * IN] = r < live ? feat[IN * s0 + k] : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int j = 4 * w + u;
+      float acc = 0.f;
+#pragma unroll
+      for (int k = 0; k < IN; ++k) acc = fmaf(sW1[j * IN + k], F[s][k], acc);
+      acc = acc + sB[j];
+      H1[s][j] = acc > 0.f ? acc : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int j = 4 * w + u;
+      float acc = 0.f;
+#pragma unroll
+      for (int k = 0; k < H; ++k) acc = fmaf(sW2[j * H + k], H1[s][k], acc);
+      acc = acc + sB[H + j];
+      H2[s][j] = acc > 0.f ? acc : 0.f;
+    }
+    __syncthreads();
+    if (w == 0 && s < live) {
+      float z = 0.f;
+#pragma unroll
+      for (int j = 0; j < H; ++j) z = fmaf(sw3[j], H2[s][j], z);
+      z = z + sB[2 * H];
+      out[s0 + s] = z < 0.f ? 0.f : (z > 1.f ? 1.f : z);
+    }
   }
-  z = z + sB[2 * H];
-  out[s] = z < 0.f ? 0.f : (z > 1.f ? 1.f : z);
 }
 
 int fail(const char* where, cudaError_t e) {
@@ -204,37 +300,38 @@ int selfgpu_mlp_train(const float* features, const float* labels, int n, int epo
   if (!features || !labels || n < 1 || epochs < 0 || batch < 1 || batch > (1 << 22) || !(lr > 0.f) || !params)
     return set_error(SELFGPU_ERR_ARG, "selfgpu_mlp_train: bad arguments");
   cudaStream_t st = (cudaStream_t)stream;
-  float* buf = nullptr;  // master, forward, grad, m1, m2, loss
-  cudaError_t e = cudaMalloc(&buf, (5 * NP + 1) * sizeof(float));
+  const int tiles = (batch + kTile - 1) / kTile;
+  const int blocks = tiles < kMaxGradBlocks ? tiles : kMaxGradBlocks;
+  // master, m1, m2, the per-epoch losses (zeroed) and the blocks' partial sums
+  const size_t fixed = 3 * (size_t)NP + epochs, total = fixed + (size_t)blocks * (NPP + 1);
+  float* buf = nullptr;
+  cudaError_t e = cudaMalloc(&buf, total * sizeof(float));
   if (e != cudaSuccess) return fail("selfgpu_mlp_train", e);
-  float *master = buf, *fw = buf + NP, *grad = buf + 2 * NP, *m1 = buf + 3 * NP, *m2 = buf + 4 * NP,
-        *loss = buf + 5 * NP;
-  e = cudaMemsetAsync(buf, 0, (5 * NP + 1) * sizeof(float), st);
+  float *master = buf, *m1 = buf + NP, *m2 = buf + 2 * NP, *loss = buf + 3 * NP, *part = buf + fixed,
+        *lossPart = part + (size_t)blocks * NPP;
+  e = cudaMemsetAsync(buf, 0, fixed * sizeof(float), st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(master, params, NP * sizeof(float), cudaMemcpyHostToDevice, st);
   const long long stepsPerEpoch = ((long long)n + batch - 1) / batch;
   long long t = 0;
   float c1 = 1.f, c2 = 1.f;
   for (int ep = 0; ep < epochs && e == cudaSuccess; ++ep) {
-    e = cudaMemsetAsync(loss, 0, sizeof(float), st);
     for (long long s = 0; s < stepsPerEpoch && e == cudaSuccess; ++s, ++t) {
-      k_round_weights<<<(NP + 255) / 256, 256, 0, st>>>(master, fw);
-      k_grad<<<(batch + 255) / 256, 256, 0, st>>>(features, labels, n, fw, grad, loss, seed, t, batch);
+      e = launch_dependent(k_grad, blocks, kGradThreads, st, features, labels, n, master, part, lossPart, seed, t, batch);
       c1 *= 0.9f;
       c2 *= 0.999f;
-      k_adam<<<(NP + 255) / 256, 256, 0, st>>>(master, grad, m1, m2, lr, 1.f - c1, 1.f - c2);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess && lossPerEpoch) {
-      float h = 0.f;
-      e = cudaMemcpyAsync(&h, loss, sizeof(float), cudaMemcpyDeviceToHost, st);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-      lossPerEpoch[ep] = h / (float)(stepsPerEpoch * batch);
+      if (e == cudaSuccess)
+        e = launch_dependent(k_adam, (NP + 31) / 32, 256, st, master, part, lossPart, blocks, m1, m2, loss + ep, lr,
+                             1.f - c1, 1.f - c2);
     }
   }
+  if (e == cudaSuccess && lossPerEpoch && epochs > 0)
+    e = cudaMemcpyAsync(lossPerEpoch, loss, epochs * sizeof(float), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(params, master, NP * sizeof(float), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   cudaFree(buf);
   if (e != cudaSuccess) return fail("selfgpu_mlp_train", e);
+  if (lossPerEpoch)
+    for (int ep = 0; ep < epochs; ++ep) lossPerEpoch[ep] /= (float)(stepsPerEpoch * batch);
   return SELFGPU_OK;
 }
 
@@ -243,19 +340,14 @@ int selfgpu_mlp_infer(const float* features, int n, const uint16_t* weights, con
   if (!features || n < 1 || !weights || !params || !out)
     return set_error(SELFGPU_ERR_ARG, "selfgpu_mlp_infer: bad arguments");
   cudaStream_t st = (cudaStream_t)stream;
-  void* buf = nullptr;
-  cudaError_t e = cudaMalloc(&buf, kMlpWeights * sizeof(uint16_t) + kMlpFloats * sizeof(float) + 16);
-  if (e != cudaSuccess) return fail("selfgpu_mlp_infer", e);
-  __nv_bfloat16* w = reinterpret_cast<__nv_bfloat16*>(buf);
-  float* p = reinterpret_cast<float*>(reinterpret_cast<char*>(buf) + ((kMlpWeights * sizeof(uint16_t) + 15) / 16 * 16));
-  e = cudaMemcpyAsync(w, weights, kMlpWeights * sizeof(uint16_t), cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(p, params, kMlpFloats * sizeof(float), cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) {
-    k_infer<<<(n + 255) / 256, 256, 0, st>>>(features, n, w, p, out);
-    e = cudaGetLastError();
-  }
+  MlpArgs args;
+  std::memcpy(args.w, weights, sizeof(args.w));
+  std::memcpy(args.p, params, sizeof(args.p));
+  const long long tiles = ((long long)n + kTile - 1) / kTile;
+  k_infer<<<(int)(tiles < 4 * kMaxGradBlocks ? tiles : 4 * kMaxGradBlocks), kGradThreads, 0, st>>>(features, n, args,
+                                                                                               out);
+  cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cudaFree(buf);
   if (e != cudaSuccess) return fail("selfgpu_mlp_infer", e);
   return SELFGPU_OK;
 }

@@ -35,10 +35,11 @@ cudaError_t launch_element_size(const double* J, const double* qw, int P, int nE
 
 cudaError_t launch_closure_features(const double* q, int P, int nEl, const AvArgs& a, float* act, float* feat,
                                     cudaStream_t st) {
+  const int blocks = (nEl + kNuWarps - 1) / kNuWarps < 148 * 8 ? (nEl + kNuWarps - 1) / kNuWarps : 148 * 8;
   switch (P) {
 #define SG_FEAT_CASE(PV)                                                  \
   case PV:                                                                \
-    k_closure_features<PV><<<nEl, PV * PV, 0, st>>>(q, nEl, a, act, feat); \
+    k_closure_features<PV><<<blocks, 32 * kNuWarps, 0, st>>>(q, nEl, a, act, feat);  \
     return cudaGetLastError();
     SG_FEAT_CASE(2)
     SG_FEAT_CASE(3)

@@ -67,3 +67,69 @@ def test_odd_node_counts_run_the_persistent_kernel(model, N, nx, ny, form):
     assert S.lib().selfgpu_model2d_persistent_launch_count(mod._h) - l0 == 15
     ref.rk3(5, 1e-3)
     _check(S.to_host(mod.solution).reshape(q.shape, order="F"), ref.get("solution", q.shape), form)
+
+
+def _mix64(x):
+    x = (x + np.uint64(0x9E3779B97F4A7C15)).astype(np.uint64)
+    x = (x ^ (x >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
+    x = (x ^ (x >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
+    return x ^ (x >> np.uint64(31))
+
+
+@pytest.mark.parametrize("n,batch", [(40, 1), (100, 31), (100, 33), (3000, 9473)])  # tiles of 32, 296 blocks
+def test_training_steps_match_float64(n, batch):
+    """Two epochs of Adam against the same steps in float64: the losses to 1e-4 (float32 sums; 1e-2 over 80 steps, in
+    which a weight near a bfloat16 midpoint may round the other way for the forward pass), and a second run bit for
+    bit the first."""
+    from self_b200 import closure as CL
+    r = np.random.default_rng(n)
+    feat = r.uniform(0, 1, (n, 36)).astype(np.float32)
+    y = np.clip(2.0 * feat[:, 5] - 0.5, 0, 1).astype(np.float32)
+    F, Y = torch.from_numpy(feat).cuda(), torch.from_numpy(y).cuda()
+    m = CL.ClosureMLP(seed=2)
+    p0 = m.params.copy()
+    loss = m.train(F, Y, epochs=2, batch=batch, lr=1e-3, seed=9)
+    m2 = CL.ClosureMLP(params=p0.copy())
+    loss2 = m2.train(F, Y, epochs=2, batch=batch, lr=1e-3, seed=9)
+    np.testing.assert_array_equal(m.params, m2.params)
+    np.testing.assert_array_equal(loss, loss2)
+    p = p0.astype(np.float64)
+    m1, v1 = np.zeros_like(p), np.zeros_like(p)
+    cuts = np.cumsum([1152, 32, 1024, 32, 32])
+    steps, ref, t = -(-n // batch), [], 0
+    with np.errstate(over="ignore"):
+        for _ in range(2):
+            tot = 0.0
+            for _ in range(steps):
+                k = np.uint64(t) * np.uint64(0x100000001) + np.arange(batch, dtype=np.uint64)
+                idx = (_mix64(np.uint64(9) ^ _mix64(k)) % np.uint64(n)).astype(np.int64)
+                W1, b1, W2, b2, w3, b3 = np.split(p, cuts)
+                rnd = lambda a: O.bf16_round(a.astype(np.float32)).astype(np.float64)  # noqa: E731
+                W1, W2, w3 = rnd(W1).reshape(32, 36), rnd(W2).reshape(32, 32), rnd(w3)
+                x, lab = feat[idx].astype(np.float64), y[idx].astype(np.float64)
+                h1 = np.maximum(x @ W1.T + b1, 0)
+                h2 = np.maximum(h1 @ W2.T + b2, 0)
+                z = h2 @ w3 + b3
+                a = np.clip(z, 0, 1)
+                d = np.where(((z < 0) & (lab > 0)) | ((z > 1) & (lab < 1)), z - lab, a - lab)
+                tot += ((a - lab) ** 2).sum()
+                gz = 2 * d / batch
+                d2 = gz[:, None] * w3 * (h2 > 0)
+                d1 = (d2 @ W2) * (h1 > 0)
+                g = np.concatenate([(d1.T @ x).ravel(), d1.sum(0), (d2.T @ h1).ravel(), d2.sum(0), h2.T @ gz,
+                                    [gz.sum()]])
+                t += 1
+                m1, v1 = 0.9 * m1 + 0.1 * g, 0.999 * v1 + 0.001 * g * g
+                p = p - 1e-3 * (m1 / (1 - 0.9 ** t)) / (np.sqrt(v1 / (1 - 0.999 ** t)) + 1e-8)
+            ref.append(tot / (steps * batch))
+    np.testing.assert_allclose(loss, ref, rtol=1e-2 if steps > 4 else 1e-4)
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 37921])  # a short tile; more tiles than blocks
+def test_inference_tiles(n):
+    """The clamped output against the restatement, to 1e-5 (float32 sums of 36 and 32 products of order one)."""
+    from self_b200 import closure as CL
+    m = CL.ClosureMLP(seed=5)
+    f = np.random.default_rng(n).uniform(-1, 1, (n, 36)).astype(np.float32)
+    got = m.infer(torch.from_numpy(f).cuda()).cpu().numpy()
+    assert np.abs(got - O.mlp_forward(f.T, *m.unpack())).max() < 1e-5
