@@ -6,10 +6,12 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "av_closure.cuh"
@@ -89,56 +91,138 @@ __global__ void k_move_blocks(const uint32_t* __restrict__ src, const int* __res
   }
 }
 
-// Entropy integrands (CalculateEntropy of the three models), summed per
-// element in the reference's node order (j outer, i inner):
+// Sums over the nodes of a mesh: one grid, every thread a strided subset of
+// the nodes (coalesced), block sums by warp shuffles, and the last block adds
+// the block sums -- all in an order that depends on the sizes only, so the
+// result is reproducible.  Four blocks per SM: the gas entropy's logarithms
+// and divisions need the warps.  (One thread per element, then one block over
+// the elements: 47 us for 1 008 and for 10 560 elements at P = 8, and 137 us
+// for the one-block integral of 7 500 elements at P = 4.)
+constexpr int kSumBlocks = 592, kSumThreads = 256;
+struct SumScratch {
+  double result;
+  unsigned done;  // zero between launches
+  double part[kSumBlocks];
+};
+
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Every thread's s summed into x->result by the last block to finish.
+__device__ void sum_grid(double s, SumScratch* x) {
+  __shared__ double ws[kSumThreads / 32];
+  __shared__ bool last;
+  const int t = threadIdx.x, w = t >> 5;
+  auto block_sum = [&](double v) {  // on thread 0
+    v = warp_sum(v);
+    if ((t & 31) == 0) ws[w] = v;
+    __syncthreads();
+    v = 0.0;
+    if (t == 0)
+      for (int k = 0; k < kSumThreads / 32; ++k) v += ws[k];
+    __syncthreads();
+    return v;
+  };
+  s = block_sum(s);
+  if (t == 0) {
+    x->part[blockIdx.x] = s;
+    __threadfence();
+    last = atomicAdd(&x->done, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  double v = 0.0;
+  for (int k = t; k < (int)gridDim.x; k += kSumThreads) v += __ldcg(&x->part[k]);
+  v = block_sum(v);
+  if (t == 0) {
+    x->result = v;
+    x->done = 0;
+  }
+}
+
+int sum_blocks(long long nodes) {
+  return (int)std::min<long long>((nodes + kSumThreads - 1) / kSumThreads, kSumBlocks);
+}
+
+// node k of the mesh: its element and its index within the element
+__device__ __forceinline__ long long element_of(long long k, int PP, int& n) {
+  const long long e = k < (1LL << 32) ? (long long)((unsigned)k / (unsigned)PP) : k / PP;
+  n = (int)(k - e * PP);
+  return e;
+}
+
+// Entropy integrands (CalculateEntropy of the three models):
 //   LSW  0.5 (H (u^2 + v^2) + g eta^2) J w_i w_j  (src/models/SELF_LinearShallowWater.f90:171-216)
 //   SW   (0.5 (Hu^2/H + Hv^2/H) + 0.5 g H^2 - g H b) J w_i w_j  (src/models/SELF_ShallowWater.f90:149-188)
 //   CIG  rho (log p - gamma log rho) / (gamma - 1) w_i w_j J, p from the
 //        solution as ConservativeToPrimitive forms it (src/models/SELF_CompressibleIdealGas2D.f90:782-823)
 // `aux` is H (LSW) or the topography b (SW), (P,P,1,nEl).
-__global__ void k_entropy_elements(int model, const double* __restrict__ q, const double* __restrict__ J,
-                                   const double* __restrict__ aux, QwArr qw, int P, int nEl, double g, double gamma,
-                                   double* __restrict__ out) {
-  const int PP = P * P;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nEl; e += (long long)gridDim.x * blockDim.x) {
-    const int nv = model == SELFGPU_MODEL_CIG ? 4 : 3;
-    const double* qe = q + (size_t)nv * PP * e;
-    double s = 0.0;
-    for (int j = 0; j < P; ++j)
-      for (int i = 0; i < P; ++i) {
-        const int n = i + P * j;
-        const double Jac = J[n + (size_t)PP * e], wi = qw.w[i], wj = qw.w[j];
-        if (model == SELFGPU_MODEL_LSW) {
-          const double u = qe[n], v = qe[n + PP], eta = qe[n + 2 * PP], H = aux[n + (size_t)PP * e];
-          s = s + 0.5 * (H * (u * u + v * v) + g * eta * eta) * Jac * wi * wj;
-        } else if (model == SELFGPU_MODEL_SW) {
-          const double Hu = qe[n], Hv = qe[n + PP], H = qe[n + 2 * PP];
-          const double b = aux ? aux[n + (size_t)PP * e] : 0.0;
-          s = s + (0.5 * (Hu * Hu / H + Hv * Hv / H) + 0.5 * g * H * H - g * H * b) * Jac * wi * wj;
-        } else {
-          const double rhoU = qe[n], rhoV = qe[n + PP], rho = qe[n + 2 * PP], rhoE = qe[n + 3 * PP];
-          const double u = rhoU / rho, v = rhoV / rho;
-          const double p = (gamma - 1.0) * (rhoE - 0.5 * (rhoU * u + rhoV * v));
-          s = s + rho * (log(p) - gamma * log(rho)) / (gamma - 1.0) * wi * wj * Jac;
-        }
-      }
-    out[e] = s;
+__global__ void __launch_bounds__(kSumThreads) k_entropy(int model, const double* __restrict__ q,
+                                                         const double* __restrict__ J, const double* __restrict__ aux,
+                                                         QwArr qw, int P, int nEl, double g, double gamma,
+                                                         SumScratch* x) {
+  const int PP = P * P, nv = model == SELFGPU_MODEL_CIG ? 4 : 3;
+  const long long nodes = (long long)PP * nEl;
+  double s = 0.0;
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nodes; k += (long long)gridDim.x * blockDim.x) {
+    int n;
+    const long long e = element_of(k, PP, n);
+    const double* qe = q + nv * PP * e + n;
+    const double wt = qw.w[n % P] * qw.w[n / P] * J[k];
+    if (model == SELFGPU_MODEL_LSW) {
+      const double u = qe[0], v = qe[PP], eta = qe[2 * PP], H = aux[k];
+      s += 0.5 * (H * (u * u + v * v) + g * eta * eta) * wt;
+    } else if (model == SELFGPU_MODEL_SW) {
+      const double Hu = qe[0], Hv = qe[PP], H = qe[2 * PP];
+      const double b = aux ? aux[k] : 0.0;
+      s += (0.5 * (Hu * Hu / H + Hv * Hv / H) + 0.5 * g * H * H - g * H * b) * wt;
+    } else {
+      const double rhoU = qe[0], rhoV = qe[PP], rho = qe[2 * PP], rhoE = qe[3 * PP];
+      const double p = (gamma - 1.0) * (rhoE - 0.5 * (rhoU * rhoU + rhoV * rhoV) / rho);
+      s += rho * (log(p) - gamma * log(rho)) * wt;
+    }
+  }
+  if (model == SELFGPU_MODEL_CIG) s = s / (gamma - 1.0);
+  sum_grid(s, x);
+}
+
+// Scratch of selfgpu_integral_mapped_scalar2d, which belongs to no handle: a
+// few slots of static device memory (a stream-ordered allocation per call went
+// back to the system at every synchronisation).  A call owns a slot from its
+// launch until it has read the result.
+constexpr int kSumSlots = 32;
+__device__ SumScratch g_sumSlots[kSumSlots];
+std::atomic<unsigned> g_sumSlotsUsed{0};
+
+int acquire_sum_slot() {
+  while (true) {
+    unsigned used = g_sumSlotsUsed.load();
+    if (used == 0xffffffffu) {  // all in use: their owners are waiting for the device
+      std::this_thread::yield();
+      continue;
+    }
+    int k = 0;
+    while (used >> k & 1u) ++k;
+    if (g_sumSlotsUsed.compare_exchange_weak(used, used | 1u << k)) return k;
   }
 }
 
-// Deterministic sum of n values by one block: strided partial sums, then a
-// shared-memory tree.  The result lands in out[0].
-__global__ void __launch_bounds__(1024) k_sum_block(const double* __restrict__ x, long long n, double* out) {
-  __shared__ double part[1024];
+__global__ void __launch_bounds__(kSumThreads) k_integral(const double* __restrict__ f, int var, int nVar,
+                                                          const double* __restrict__ J, QwArr qw, int P, int nEl,
+                                                          int slot) {
+  const int PP = P * P;
+  const long long nodes = (long long)PP * nEl;
   double s = 0.0;
-  for (long long k = threadIdx.x; k < n; k += blockDim.x) s += x[k];
-  part[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
-    __syncthreads();
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nodes; k += (long long)gridDim.x * blockDim.x) {
+    int n;
+    const long long e = element_of(k, PP, n);
+    s += f[n + (size_t)PP * (var + (size_t)nVar * e)] * qw.w[n % P] * qw.w[n / P] * J[k];
   }
-  if (threadIdx.x == 0) out[0] = part[0];
+  sum_grid(s, &g_sumSlots[slot]);
 }
 
 int nt_of(int model) { return model == SELFGPU_MODEL_CIG ? 9 : 3; }
@@ -181,7 +265,7 @@ struct selfgpu_model2d {
   float* mlpB = nullptr;
   double* geo = nullptr;  // packed geometry records (persistent kernel)
   float* gf = nullptr;    // RK register of the FP32-bulk form (P,P,NV,nEl); workSol is unused then
-  double* entropyBuf = nullptr;  // per-element entropy sums (nEl) and the total
+  SumScratch* sums = nullptr;  // entropy reduction
   bool multistep = false;         // rk3 as one cooperative launch where the mesh fits one wave
   bool multistage = false;        // rk3 as one launch of the persistent kernel over all stages
   unsigned* stepBar = nullptr;    // grid-barrier / stage-end counter of the one-launch paths
@@ -437,13 +521,15 @@ int selfgpu_model2d_create(selfgpu_model2d** out, int model, int N, int nEl, int
     selfgpu_model2d_destroy(m);
     return fail_cuda("selfgpu_model2d_create: trace cache", e);
   }
-  e = cudaMalloc(&m->dflag, 2 * sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(m->dflag, 0, 2 * sizeof(int));
+  // flags (the first 16 bytes) and the scratch of reductions
+  e = cudaMalloc(&m->dflag, 16 + sizeof(SumScratch));
+  if (e == cudaSuccess) e = cudaMemset(m->dflag, 0, 16 + sizeof(SumScratch));
   if (e != cudaSuccess) {
     selfgpu_model2d_destroy(m);
     return fail_cuda("selfgpu_model2d_create", e);
   }
   m->derr = m->dflag + 1;
+  m->sums = reinterpret_cast<SumScratch*>(m->dflag + 4);
   cudaDeviceGetAttribute(&m->cfg.smemOptin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   cudaDeviceGetAttribute(&m->cfg.numSMs, cudaDevAttrMultiProcessorCount, dev);
   m->base.err = m->derr;
@@ -465,7 +551,7 @@ int selfgpu_model2d_destroy(selfgpu_model2d* m) {
     if (m->vel[k]) cudaFree(m->vel[k]);
   }
   for (void* p : {(void*)m->avNu, (void*)m->avAct, (void*)m->avFallbacks, (void*)m->avH, m->avVisc, m->avVtr,
-                  (void*)m->mlpW, (void*)m->mlpB, (void*)m->geo, (void*)m->entropyBuf, (void*)m->stepBar,
+                  (void*)m->mlpW, (void*)m->mlpB, (void*)m->geo, (void*)m->stepBar,
                   (void*)m->gf})
     if (p) cudaFree(p);
   if (m->dflag) cudaFree(m->dflag);
@@ -1096,45 +1182,19 @@ int selfgpu_model2d_entropy(selfgpu_model2d* m, double* entropy) {
   else if (m->model == SELFGPU_MODEL_SW) aux = m->base.fld[2];
   if (!m->haveInterp) return set_error(SELFGPU_ERR_STATE, "selfgpu_model2d_entropy: no interpolant");
   cudaError_t e = cudaSuccess;
-  if (!m->entropyBuf) e = cudaMalloc(&m->entropyBuf, ((size_t)m->nEl + 1) * sizeof(double));
-  if (e != cudaSuccess) return fail_cuda("selfgpu_model2d_entropy", e);
   QwArr w{};
   for (int k = 0; k < m->P; ++k) w.w[k] = m->base.qw[k];
-  const int blocks = (m->nEl + 127) / 128 < 1184 ? (m->nEl + 127) / 128 : 1184;
-  k_entropy_elements<<<blocks, 128, 0, m->stream>>>(m->model, m->base.q, m->base.J, aux, w, m->P, m->nEl, m->base.g,
-                                                    m->base.gamma, m->entropyBuf);
-  k_sum_block<<<1, 1024, 0, m->stream>>>(m->entropyBuf, m->nEl, m->entropyBuf + m->nEl);
-  m->launches += 2;
+  k_entropy<<<sum_blocks((long long)m->P * m->P * m->nEl), kSumThreads, 0, m->stream>>>(
+      m->model, m->base.q, m->base.J, aux, w, m->P, m->nEl, m->base.g, m->base.gamma, m->sums);
+  e = cudaGetLastError();
+  ++m->launches;
   double h = 0.0;
-  e = cudaMemcpyAsync(&h, m->entropyBuf + m->nEl, sizeof(double), cudaMemcpyDeviceToHost, m->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(&h, &m->sums->result, sizeof(double), cudaMemcpyDeviceToHost, m->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
   if (e != cudaSuccess) return fail_cuda("selfgpu_model2d_entropy", e);
   *entropy = h;
   return SELFGPU_OK;
-}
-
-// One block: every thread sums a strided subset of the elements, each element
-// in the reference's node order, then a shared-memory tree (fixed order).
-__global__ void __launch_bounds__(1024) k_integral_block(const double* __restrict__ f, int var, int nVar,
-                                                         const double* __restrict__ J, QwArr qw, int P, int nEl,
-                                                         double* out) {
-  __shared__ double part[1024];
-  const int PP = P * P;
-  double s = 0.0;
-  for (long long e = threadIdx.x; e < nEl; e += blockDim.x) {
-    const double* fe = f + (size_t)PP * (var + (size_t)nVar * e);
-    double se = 0.0;
-    for (int j = 0; j < P; ++j)
-      for (int i = 0; i < P; ++i) se = se + fe[i + P * j] * qw.w[i] * qw.w[j] * J[i + P * j + (size_t)PP * e];
-    s += se;
-  }
-  part[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[0] = part[0];
 }
 
 int selfgpu_integral_mapped_scalar2d(const double* interior, int iVar, int nVar, const double* J,
@@ -1144,16 +1204,16 @@ int selfgpu_integral_mapped_scalar2d(const double* interior, int iVar, int nVar,
     return set_error(SELFGPU_ERR_ARG, "selfgpu_integral_mapped_scalar2d: bad arguments");
   QwArr w{};
   for (int k = 0; k <= N; ++k) w.w[k] = qWeights[k];
-  double* d = nullptr;
   cudaStream_t st = (cudaStream_t)stream;
-  cudaError_t e = cudaMallocAsync(&d, sizeof(double), st);
-  if (e != cudaSuccess) return fail_cuda("selfgpu_integral_mapped_scalar2d", e);
-  k_integral_block<<<1, 1024, 0, st>>>(interior, iVar - 1, nVar, J, w, N + 1, nEl, d);
-  e = cudaGetLastError();
+  const int slot = acquire_sum_slot();
+  k_integral<<<sum_blocks((long long)(N + 1) * (N + 1) * nEl), kSumThreads, 0, st>>>(interior, iVar - 1, nVar, J, w,
+                                                                                 N + 1, nEl, slot);
+  cudaError_t e = cudaGetLastError();
   double h = 0.0;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d, sizeof(double), cudaMemcpyDeviceToHost, st);
-  cudaFreeAsync(d, st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyFromSymbolAsync(&h, g_sumSlots, sizeof(double), slot * sizeof(SumScratch), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  g_sumSlotsUsed.fetch_and(~(1u << slot));
   if (e != cudaSuccess) return fail_cuda("selfgpu_integral_mapped_scalar2d", e);
   *result = h;
   return SELFGPU_OK;

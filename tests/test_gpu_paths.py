@@ -69,6 +69,25 @@ def test_odd_node_counts_run_the_persistent_kernel(model, N, nx, ny, form):
     _check(S.to_host(mod.solution).reshape(q.shape, order="F"), ref.get("solution", q.shape), form)
 
 
+@pytest.mark.parametrize("N,nx,ny", [(2, 1, 1), (3, 17, 5), (7, 40, 37)])  # one block; several; more than one sweep
+def test_integral_and_entropy_sums(N, nx, ny):
+    """The reductions against their defining sums in long double; 1e-13 relative to the sum of magnitudes (a pairwise
+    sum of n <= 1e5 terms rounds to far below n eps)."""
+    import self_b200 as S
+    ref, mod, q = _pair("CIG", dict(nx=nx, ny=ny, bcid=O.BC_NONORMALFLOW, amp=0.0), N, S.FP64)
+    wJ = S.to_host(mod._wJ()).astype(np.longdouble)  # (P, P, nEl)
+    f = S.MappedScalar2D(mod.interp, 4, mod.nElem)
+    f.interior.copy_(mod.solution)
+    for v in range(4):
+        terms = q[:, :, v].astype(np.longdouble) * wJ
+        assert abs(f.Integral(mod.geometry, v + 1) - float(terms.sum())) <= 1e-13 * float(np.abs(terms).sum())
+    ru, rv, r, e = (q[:, :, k].astype(np.longdouble) for k in range(4))
+    p = 0.4 * (e - 0.5 * (ru * ru + rv * rv) / r)
+    terms = r * (np.log(p) - 1.4 * np.log(r)) / 0.4 * wJ
+    for _ in range(2):  # the scratch is left as it was found
+        assert abs(mod.CalculateEntropy() - float(terms.sum())) <= 1e-13 * float(np.abs(terms).sum())
+
+
 def _mix64(x):
     x = (x + np.uint64(0x9E3779B97F4A7C15)).astype(np.uint64)
     x = (x ^ (x >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
