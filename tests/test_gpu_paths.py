@@ -69,6 +69,53 @@ def test_odd_node_counts_run_the_persistent_kernel(model, N, nx, ny, form):
     _check(S.to_host(mod.solution).reshape(q.shape, order="F"), ref.get("solution", q.shape), form)
 
 
+@pytest.mark.parametrize("N", [2, 3, 6, 7, 8, 10])
+@pytest.mark.parametrize("nVar,nEl", [(1, 1), (3, 5), (2, 131)])
+def test_plane_operators_match_the_oracle(N, nVar, nEl):
+    """The operators that take several planes per block, at plane counts that leave the last block short, and the
+    degrees beyond the compiled ones: bit for bit the oracle's."""
+    import self_b200 as S
+    P, w = N + 1, S.lib()
+    Lo = O.Lagrange(N, O.GAUSS, 5, O.UNIFORM)
+    om = O.Mesh(nEl, 1, periodic=(True, False), bcid=O.BC_NONORMALFLOW)
+    g = O.Geometry(N, om)
+    r = np.random.default_rng(N + nEl)
+    f = np.asfortranarray(r.standard_normal((P, P, nVar, nEl)))
+    v = np.asfortranarray(r.standard_normal((2, P, P, nVar, nEl)))
+    avg = np.asfortranarray(r.standard_normal((P, nVar, 4, nEl)))
+    p = lambda t: S._lib.pp(t.data_ptr())  # noqa: E731
+    dev = {k: S.to_device(a) for k, a in dict(f=f, v=v, avg=avg, dsdx=g.dsdx, J=g.J, nHat=g.nHat, nScale=g.nScale,
+                                               **{m: getattr(Lo, m) for m in ("iMatrix", "dMatrix", "dgMatrix",
+                                                                              "bMatrix", "qWeights")}).items()}
+    a = {k: p(t) for k, t in dev.items()}
+
+    def run(call, shape, *args):
+        out = S.to_device(np.zeros(shape, order="F"))
+        call(*[p(out) if x is None else x for x in args])
+        torch.cuda.synchronize()
+        return S.to_host(out).reshape(shape, order="F")
+
+    n = (N, nVar, nEl)
+    eq = np.testing.assert_array_equal
+    eq(run(w.ScalarGridInterp_2D_gpu_wrapper, (6, 6, nVar, nEl), a["iMatrix"], a["f"], None, N, 5, nVar, nEl),
+       O.scalar_grid_interp(Lo, f))
+    eq(run(w.VectorGridInterp_2D_gpu_wrapper, (2, 6, 6, nVar, nEl), a["iMatrix"], a["v"], None, N, 5, nVar, nEl),
+       O.vector_grid_interp(Lo, v))
+    eq(run(w.ScalarBoundaryInterp_2D_gpu_wrapper, (P, nVar, 4, nEl), a["bMatrix"], a["f"], None, *n),
+       O.scalar_boundary_interp(Lo, f))
+    eq(run(w.VectorBoundaryInterp_2D_gpu_wrapper, (2, P, nVar, 4, nEl), a["bMatrix"], a["v"], None, *n),
+       O.vector_boundary_interp(Lo, v))
+    eq(run(w.VectorGradient_2D_gpu_wrapper, (2, 2, P, P, nVar, nEl), a["dMatrix"], a["v"], None, *n),
+       O.vector_gradient(Lo, v))
+    eq(run(w.VectorDGDivergence_2D_gpu_wrapper, (P, P, nVar, nEl), a["dgMatrix"], a["bMatrix"], a["qWeights"], a["v"],
+           a["avg"], None, *n), O.vector_dg_divergence(Lo, v, avg))
+    eq(run(w.GradientSF_MappedScalar2D_gpu_wrapper, (2, P, P, nVar, nEl), a["f"], a["dsdx"], a["J"], None,
+           a["dMatrix"], *n), O.gradient_sf(Lo, f, g.dsdx, g.J))
+    eq(run(w.GradientBR_MappedScalar2D_gpu_wrapper, (2, P, P, nVar, nEl), a["f"], a["avg"], a["dsdx"], a["J"],
+           a["nHat"], a["nScale"], None, a["dgMatrix"], a["bMatrix"], a["qWeights"], *n),
+       O.gradient_br(Lo, f, avg, g.dsdx, g.J, g.nHat, g.nScale))
+
+
 @pytest.mark.parametrize("N,nx,ny", [(2, 1, 1), (3, 17, 5), (7, 40, 37)])  # one block; several; more than one sweep
 def test_integral_and_entropy_sums(N, nx, ny):
     """The reductions against their defining sums in long double; 1e-13 relative to the sum of magnitudes (a pairwise
