@@ -47,6 +47,9 @@
 namespace selfgpu {
 
 constexpr int kMlpIn = 36, kMlpHidden = 32;
+// row strides of the weight matrices in shared memory: odd, so that the lanes'
+// (one unit each) reads of a column fall into distinct banks
+constexpr int kW1Stride = kMlpIn + 1, kW2Stride = kMlpHidden + 1;
 constexpr int kMlpWeights = kMlpHidden * kMlpIn + kMlpHidden * kMlpHidden + kMlpHidden;  // bf16 values
 constexpr int kMlpFloats = kMlpHidden + kMlpHidden + 1 + 2 * kMlpIn;                    // b1 b2 b3 fmin fmax
 constexpr double kAvPi = 3.141592653589793;                                             // 4 atan(1)
@@ -114,11 +117,11 @@ __device__ R activation_of(R top, R total, double s0, double kappa) {
 }
 
 // ------------------------------------------------------ viscosity kernel
-// One lane per element: density modes, activation and screening; then, warp
-// wide (warp-level synchronisation only) and only for the warp's elements
-// that need them, the MLP where the indicator does not screen the element
-// out, and the wave speed where the activation is not zero; the viscosity and
-// an entry in the list of active elements.
+// Density modes, activation and screening by a group of lanes per element;
+// then, warp wide (warp-level synchronisation only) and only for the warp's
+// elements that need them, the MLP where the indicator does not screen the
+// element out, and the wave speed where the activation is not zero; the
+// viscosity and an entry in the list of active elements.
 template <int P, typename R>
 struct NuWarpSmem {
   static constexpr int PP = P * P;
@@ -126,7 +129,7 @@ struct NuWarpSmem {
   R tt[PP];
   R c[2][PP];  // modal energies c^2
   R part[3][P];
-  R act[32], lam[32];  // per lane's element
+  R act[32], lam[32];  // per element of the warp
   float feat[kMlpIn];
   float h1[kMlpHidden];
 };
@@ -209,8 +212,8 @@ __device__ R warp_mlp_act(const AvArgs& a, const R* sT, NuWarpSmem<P, R>& s, con
   __syncwarp();
   {
     float acc = 0.f;  // lane = hidden unit
-#pragma unroll 4
-    for (int k = 0; k < kMlpIn; ++k) acc = fmaf(sW1[lane * kMlpIn + k], s.feat[k], acc);
+#pragma unroll 12
+    for (int k = 0; k < kMlpIn; ++k) acc = fmaf(sW1[lane * kW1Stride + k], s.feat[k], acc);
     acc = acc + sB[lane];
     s.h1[lane] = acc > 0.f ? acc : 0.f;
   }
@@ -218,23 +221,24 @@ __device__ R warp_mlp_act(const AvArgs& a, const R* sT, NuWarpSmem<P, R>& s, con
   float h2;
   {
     float acc = 0.f;
-#pragma unroll 4
-    for (int k = 0; k < kMlpHidden; ++k) acc = fmaf(sW2[lane * kMlpHidden + k], s.h1[k], acc);
+#pragma unroll 16
+    for (int k = 0; k < kMlpHidden; ++k) acc = fmaf(sW2[lane * kW2Stride + k], s.h1[k], acc);
     acc = acc + sB[kMlpHidden + lane];
     h2 = acc > 0.f ? acc : 0.f;
   }
   __syncwarp();
   s.h1[lane] = h2;  // the second hidden layer reuses the first's array
   __syncwarp();
+  const float *fmin = sB + 2 * kMlpHidden + 1, *fmax = fmin + kMlpIn;
+  bool mine = true;  // this lane's features lie in the training range
+  for (int k = lane; k < kMlpIn; k += 32)
+    mine = mine && s.feat[k] >= fmin[k] - kMlpRangeMargin && s.feat[k] <= fmax[k] + kMlpRangeMargin;
+  const bool inRange = __all_sync(0xffffffffu, mine);
   if (lane == 0) {
     if (a.fallbacks) atomicAdd(a.fallbacks + 1, 1);
-    bool inRange = true;
-    const float* fmin = sB + 2 * kMlpHidden + 1;
-    const float* fmax = fmin + kMlpIn;
-    for (int k = 0; k < kMlpIn; ++k)
-      inRange = inRange && s.feat[k] >= fmin[k] - kMlpRangeMargin && s.feat[k] <= fmax[k] + kMlpRangeMargin;
     if (inRange) {
       float z = 0.f;
+#pragma unroll
       for (int k = 0; k < kMlpHidden; ++k) z = fmaf(sw3[k], s.h1[k], z);
       z = z + sB[2 * kMlpHidden];
       act = (R)(z < 0.f ? 0.f : (z > 1.f ? 1.f : z));
@@ -287,114 +291,120 @@ __device__ __forceinline__ void indicator_act(const AvArgs& a, R total, R top, b
   }
 }
 
+// One group of kNuLanes lanes per element, lane j holding row j of the density:
+// the xi transform is the lane's own, the eta transform reads the group's rows
+// from shared memory, and lane l sums eta-degree l -- the operations and
+// summation orders of one thread that does it all.  (One lane per element held
+// 64 densities, left 4 of 5 resident warps idle on a mesh of 10 560 elements
+// and took 15 us there in FP64 at P = 8, each lane's chain of 1 024
+// multiply-adds and 64 uncoalesced loads being the time.)
+template <int P>
+constexpr int nu_lanes() {
+  return P <= 2 ? 2 : (P <= 4 ? 4 : 8);
+}
+
 template <int P, typename R>
 __global__ void __launch_bounds__(32 * kNuWarps) k_av_nu(const AvArgs a) {
-  constexpr int PP = P * P, N = P - 1;
+  constexpr int PP = P * P, N = P - 1, GL = nu_lanes<P>(), GE = 32 / GL;  // elements per warp
   __shared__ NuWarpSmem<P, R> ws[kNuWarps];
+  __shared__ R sTt[kNuWarps][GE][PP + 1];  // xi transforms (k, jj) at [jj + P k]
   __shared__ R sT[PP];
-  __shared__ float sW1[kMlpHidden * kMlpIn], sW2[kMlpHidden * kMlpHidden], sw3[kMlpHidden], sB[kMlpFloats];
+  __shared__ float sW1[kMlpHidden * kW1Stride], sW2[kMlpHidden * kW2Stride], sw3[kMlpHidden], sB[kMlpFloats];
   const bool mlp = (a.mode == AV_MLP) && (P >= 6);
   for (int k = threadIdx.x; k < PP; k += blockDim.x) sT[k] = (R)a.T[k];
   if (mlp) {
-    for (int k = threadIdx.x; k < kMlpHidden * kMlpIn; k += blockDim.x) sW1[k] = __bfloat162float(a.mlpW[k]);
+    for (int k = threadIdx.x; k < kMlpHidden * kMlpIn; k += blockDim.x)
+      sW1[k / kMlpIn * kW1Stride + k % kMlpIn] = __bfloat162float(a.mlpW[k]);
     for (int k = threadIdx.x; k < kMlpHidden * kMlpHidden; k += blockDim.x)
-      sW2[k] = __bfloat162float(a.mlpW[kMlpHidden * kMlpIn + k]);
+      sW2[k / kMlpHidden * kW2Stride + k % kMlpHidden] = __bfloat162float(a.mlpW[kMlpHidden * kMlpIn + k]);
     for (int k = threadIdx.x; k < kMlpHidden; k += blockDim.x)
       sw3[k] = __bfloat162float(a.mlpW[kMlpHidden * kMlpIn + kMlpHidden * kMlpHidden + k]);
     for (int k = threadIdx.x; k < kMlpFloats; k += blockDim.x) sB[k] = a.mlpB[k];
   }
   __syncthreads();
   const int w = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int grp = lane / GL, r = lane % GL;  // the lane's element of the warp's GE, and its row / eta-degree
+  const int leader = grp * GL;
   NuWarpSmem<P, R>& s = ws[w];
-  {
-    // One lane per element for the indicator (the warp's 32 elements are
-    // spread over the mesh, so that the few that need the MLP or the wave
-    // speed, done warp-wide, are spread over the warps too).  FP64 at P = 8
-    // holds 64 densities per lane and spills a little; still measured 7 %
-    // faster per C5 step than one warp per element.
-    const long long nW = (long long)gridDim.x * kNuWarps;
-    for (long long base = (long long)blockIdx.x * kNuWarps + w; base < a.nEl; base += 32 * nW) {
-      const long long e = base + (long long)lane * nW;
-      R actInd = (R)0;
-      int need = 0;
-      if (e < a.nEl) {
-        // density modes: the operations and summation orders of warp_modal_energy
-        // and of the per-eta-degree sums
-        R q[PP];
-        const double2* qg = reinterpret_cast<const double2*>(a.q + (long long)PP * (2 + 4 * e));
+  R* tt = sTt[w][grp];
+  // a warp's elements are spread over the mesh, so that the few that need the
+  // MLP or the wave speed, done warp-wide, are spread over the warps too
+  const long long nW = (long long)gridDim.x * kNuWarps;
+  for (long long base = (long long)blockIdx.x * kNuWarps + w; base < a.nEl; base += GE * nW) {
+    const long long e = base + (long long)grp * nW;
+    const bool live = e < a.nEl;
+    if (live && r < P) {
+      R q[P];
+      const double* qg = a.q + (long long)PP * (2 + 4 * e) + P * r;
 #pragma unroll
-        for (int k = 0; k < PP / 2; ++k) {
-          const double2 x = qg[k];
-          q[2 * k] = (R)x.x;
-          q[2 * k + 1] = (R)x.y;
-        }
-        if constexpr (PP % 2) q[PP - 1] = (R)a.q[(long long)PP * (2 + 4 * e) + PP - 1];
-        R tot[P], top[P];
+      for (int m = 0; m < P; ++m) q[m] = (R)qg[m];
 #pragma unroll
-        for (int l = 0; l < P; ++l) tot[l] = top[l] = (R)0;
+      for (int k = 0; k < P; ++k) {
+        R acc = (R)0;
 #pragma unroll
-        for (int k = 0; k < P; ++k) {
-          R tt[P];
-#pragma unroll
-          for (int jj = 0; jj < P; ++jj) {
-            R acc = (R)0;
-#pragma unroll
-            for (int m = 0; m < P; ++m) acc = acc + sT[k + P * m] * q[m + P * jj];
-            tt[jj] = acc;
-          }
-#pragma unroll
-          for (int l = 0; l < P; ++l) {
-            R acc = (R)0;
-#pragma unroll
-            for (int m = 0; m < P; ++m) acc = acc + sT[l + P * m] * tt[m];
-            const R c = acc * acc;
-            tot[l] = tot[l] + c;
-            if (k == N) top[l] = c;
-          }
-        }
-        top[N] = tot[N];
-        R total = (R)0, topS = (R)0;
-#pragma unroll
-        for (int l = 0; l < P; ++l) {
-          total = total + tot[l];
-          topS = topS + top[l];
-        }
-        indicator_act<R>(a, total, topS, mlp, actInd, need);
+        for (int m = 0; m < P; ++m) acc = acc + sT[k + P * m] * q[m];
+        tt[r + P * k] = acc;
       }
-      s.act[lane] = actInd;
-      const unsigned needMask = __ballot_sync(0xffffffffu, need);
-      __syncwarp();
-      for (unsigned mk = needMask; mk; mk &= mk - 1) {
-        const int b = __ffs(mk) - 1;
-        const R act = warp_mlp_act<P, R>(a, sT, s, sW1, sW2, sw3, sB, base + (long long)b * nW, lane,
-                                         __shfl_sync(0xffffffffu, actInd, b));
-        if (lane == 0) s.act[b] = act;
-        __syncwarp();
+    }
+    __syncwarp();
+    R tot = (R)0, topL = (R)0;  // eta-degree r: all xi-degrees, and xi-degree N
+    if (live && r < P) {
+#pragma unroll
+      for (int k = 0; k < P; ++k) {
+        R acc = (R)0;
+#pragma unroll
+        for (int m = 0; m < P; ++m) acc = acc + sT[r + P * m] * tt[m + P * k];
+        const R c = acc * acc;
+        tot = tot + c;
+        if (k == N) topL = c;
       }
-      const R act = s.act[lane];
-      const unsigned actMask = __ballot_sync(0xffffffffu, e < a.nEl && act != (R)0);
-      for (unsigned mk = actMask; mk; mk &= mk - 1) {
-        const int b = __ffs(mk) - 1;
-        const R lam = warp_wave_speed<P, R>(a, base + (long long)b * nW, lane);
-        if (lane == 0) s.lam[b] = lam;
-      }
-      __syncwarp();
-      double nu = 0.0;
-      if (e < a.nEl) {
-        if (act != (R)0) nu = (double)act * a.avC * a.hEl[e] / (double)N * (double)s.lam[lane];
-        a.nu[e] = nu;
-        a.act[e] = (float)act;
-        if (mlp && a.actInd) a.actInd[e] = (float)actInd;
-      }
-      const unsigned nzMask = __ballot_sync(0xffffffffu, nu != 0.0);
-      if (nzMask) {
-        int b0 = 0;
-        if (lane == 0) b0 = atomicAdd(a.activeCount, __popc(nzMask));
-        b0 = __shfl_sync(0xffffffffu, b0, 0);
-        if (nu != 0.0) a.activeList[b0 + __popc(nzMask & ((1u << lane) - 1u))] = (int)e;
-      }
+      if (r == N) topL = tot;
+    }
+    R total = (R)0, topS = (R)0;
+#pragma unroll
+    for (int l = 0; l < P; ++l) {
+      total = total + __shfl_sync(0xffffffffu, tot, leader + l);
+      topS = topS + __shfl_sync(0xffffffffu, topL, leader + l);
+    }
+    R actInd = (R)0;
+    int need = 0;
+    if (live && r == 0) {
+      indicator_act<R>(a, total, topS, mlp, actInd, need);
+      s.act[grp] = actInd;
+    }
+    const unsigned needMask = __ballot_sync(0xffffffffu, need);
+    __syncwarp();
+    for (unsigned mk = needMask; mk; mk &= mk - 1) {
+      const int ln = __ffs(mk) - 1, b = ln / GL;
+      const R act = warp_mlp_act<P, R>(a, sT, s, sW1, sW2, sw3, sB, base + (long long)b * nW, lane,
+                                       __shfl_sync(0xffffffffu, actInd, ln));
+      if (lane == 0) s.act[b] = act;
       __syncwarp();
     }
+    const bool mine = live && r == 0;  // the element's lane
+    const R act = mine ? s.act[grp] : (R)0;
+    const unsigned actMask = __ballot_sync(0xffffffffu, act != (R)0);
+    for (unsigned mk = actMask; mk; mk &= mk - 1) {
+      const int b = (__ffs(mk) - 1) / GL;
+      const R lam = warp_wave_speed<P, R>(a, base + (long long)b * nW, lane);
+      if (lane == 0) s.lam[b] = lam;
+    }
+    __syncwarp();
+    double nu = 0.0;
+    if (mine) {
+      if (act != (R)0) nu = (double)act * a.avC * a.hEl[e] / (double)N * (double)s.lam[grp];
+      a.nu[e] = nu;
+      a.act[e] = (float)act;
+      if (mlp && a.actInd) a.actInd[e] = (float)actInd;
+    }
+    const unsigned nzMask = __ballot_sync(0xffffffffu, nu != 0.0);
+    if (nzMask) {
+      int b0 = 0;
+      if (lane == 0) b0 = atomicAdd(a.activeCount, __popc(nzMask));
+      b0 = __shfl_sync(0xffffffffu, b0, 0);
+      if (nu != 0.0) a.activeList[b0 + __popc(nzMask & ((1u << lane) - 1u))] = (int)e;
+    }
+    __syncwarp();
   }
 }
 
@@ -407,26 +417,36 @@ struct GradSmem {
   R q[4][PP];
   R dsdx[4][PP];  // (dsdx11, dsdx21, dsdx12, dsdx22) per node
   R avg[4][4][P];
+  R nh[4][P][2], ns[4][P];
   R g[2][4][PP];  // nu grad q
 };
 
+// elements per block: one thread per node and variable
 template <int P, typename R>
 constexpr int av_elems_per_block() {
-  int e = 128 / (P * P);
+  int e = 256 / (4 * P * P);
   if (e < 1) e = 1;
-  while (e > 1 && (size_t)e * sizeof(GradSmem<P, R>) > 30 * 1024) --e;
+  while (e > 1 && (size_t)e * sizeof(GradSmem<P, R>) > 44 * 1024) --e;
   return e;
 }
 
+// A shocked region is a few hundred elements, so the kernel's time is the
+// latency of one element's chain (loads, sums, ten divisions per node and
+// variable, traces): a thread per (node, variable) and the face metrics in
+// shared memory.  (One thread per node doing its four variables in turn, the
+// metrics read from global memory for each: 12 us for the 5 % of 10 560
+// elements at P = 8 in FP64 that a shock band activates.)
 template <int P, typename R, int EPB>
-__global__ void __launch_bounds__(EPB* P* P, 4) k_av_grad(const AvArgs a) {
-  constexpr int PP = P * P, N = P - 1, VS = visc_side_stride<P>();
+__global__ void __launch_bounds__(EPB * 4 * P * P) k_av_grad(const AvArgs a) {
+  constexpr int PP = P * P, N = P - 1, VS = visc_side_stride<P>(), TPE = 4 * PP;
   constexpr int TS = trace_side_stride<P, 9, R>();
   __shared__ GradSmem<P, R> sm_all[EPB];
   __shared__ double sdg[PP], sb[2 * P], sw[P];
   const int tid = threadIdx.x;
-  const int slot = tid / PP;
-  const int t = tid - slot * PP;
+  const int slot = tid / TPE;
+  const int u = tid - slot * TPE;  // thread of the element
+  const int v = u / PP;            // variable (and metric component)
+  const int t = u - v * PP;        // node
   const int i = t % P, j = t / P;
   GradSmem<P, R>& sm = sm_all[slot];
   for (int k = tid; k < PP; k += blockDim.x) sdg[k] = a.dgM[k];
@@ -437,102 +457,95 @@ __global__ void __launch_bounds__(EPB* P* P, 4) k_av_grad(const AvArgs a) {
   const int count = *a.activeCount;
   // every block runs the same number of rounds (block-uniform barriers)
   for (int base = blockIdx.x * EPB; base < count; base += gridDim.x * EPB) {
-    const bool live = base + slot < count && t < PP;
+    const bool live = base + slot < count;
     const long long e = live ? a.activeList[base + slot] : 0;
+    R nu = (R)0, Jij = (R)1;
     if (live) {
-#pragma unroll
-      for (int v = 0; v < 4; ++v) sm.q[v][t] = (R)a.q[t + (long long)PP * (v + 4 * e)];
-      const double* gd = a.dsdx + 4 * (t + (long long)PP * e);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) sm.dsdx[k][t] = (R)gd[k];
-      // averaged conservative traces (BassiRebaySides) with the stage's exterior states
-      for (int k = t; k < 4 * P; k += PP) {
+      sm.q[v][t] = (R)a.q[t + (long long)PP * (v + 4 * e)];
+      sm.dsdx[v][t] = (R)a.dsdx[v + 4 * (t + (long long)PP * e)];
+      nu = (R)a.nu[e];
+      Jij = (R)a.J[t + (long long)PP * e];
+      for (int k = u; k < 4 * P; k += TPE) {
         const int s1 = k / P, ii = k % P;
+        sm.nh[s1][ii][0] = (R)a.nHat[2 * (k + (long long)P * 4 * e)];
+        sm.nh[s1][ii][1] = (R)a.nHat[2 * (k + (long long)P * 4 * e) + 1];
+        sm.ns[s1][ii] = (R)a.nScale[k + (long long)P * 4 * e];
+      }
+      // averaged conservative traces (BassiRebaySides) with the stage's exterior states
+      for (int k = u; k < 16 * P; k += TPE) {
+        const int w = k / (4 * P), c = k - w * 4 * P, s1 = c / P, ii = c % P;
         const int* si = a.sideInfo + 5 * (s1 + 4 * e);
-        const R* own = trIn + (long long)TS * (s1 + 4 * e);
-        R L[4], X[4];
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-          L[w] = own[ii + P * w];
-          X[w] = (R)0;
-        }
+        const R* own = trIn + (long long)TS * (s1 + 4 * e) + ii;
+        const R L = own[P * w];
+        R X = (R)0;
         const int bcid = si[4];
         if (bcid == 0) {
           const long long e2 = si[2] - 1;
           const int s2 = si[3] / 10 - 1, flip = si[3] % 10;
-          const R* nb = trIn + (long long)TS * (s2 + 4 * e2);
-          const int i2 = flip ? N - ii : ii;
-#pragma unroll
-          for (int w = 0; w < 4; ++w) X[w] = nb[i2 + P * w];
+          X = trIn[(long long)TS * (s2 + 4 * e2) + (flip ? N - ii : ii) + P * w];
         } else if (si[2] == 0) {  // physical side: the boundary condition's exterior state
           if (bcid == SG_BC_NONORMALFLOW) {
-            const double2 nh = reinterpret_cast<const double2*>(a.nHat)[ii + (long long)P * (s1 + 4 * e)];
-            reflect<R>(L[0], L[1], nh.x, nh.y, X[0], X[1]);
-            X[2] = L[2];
-            X[3] = L[3];
+            if (w < 2) {
+              const double* nh = a.nHat + 2 * (ii + (long long)P * (s1 + 4 * e));
+              R x0, x1;
+              reflect<R>(own[0], own[P], nh[0], nh[1], x0, x1);
+              X = w == 0 ? x0 : x1;
+            } else {
+              X = L;
+            }
           } else if ((bcid == SG_BC_PRESCRIBED || bcid == SG_BC_RADIATION) && a.presc) {
-#pragma unroll
-            for (int w = 0; w < 4; ++w) X[w] = (R)a.presc[ii + (long long)P * (w + 4 * (s1 + 4 * e))];
+            X = (R)a.presc[ii + (long long)P * (w + 4 * (s1 + 4 * e))];
           }
         }
-#pragma unroll
-        for (int w = 0; w < 4; ++w) sm.avg[s1][w][ii] = (R)0.5 * (L[w] + X[w]);
+        sm.avg[s1][w][ii] = (R)0.5 * (L + X);
       }
     }
     __syncthreads();
     // BR1 gradient (GradientBR_MappedScalar2D, src/SELF_MappedData.f90:990-1074) scaled by nu,
     // and the contravariant viscous flux (src/models/hip/SELF_Advection2D.cpp:66-95)
     if (live) {
-      const R nu = (R)a.nu[e];
-      const double* nH = a.nHat + 2 * (long long)P * 4 * e;
-      const double* nS = a.nScale + (long long)P * 4 * e;
-      const R Jij = (R)a.J[t + (long long)PP * e];
       R* visc = reinterpret_cast<R*>(a.visc);
-#pragma unroll 1
-      for (int v = 0; v < 4; ++v) {
-        R gx = (R)0, gy = (R)0;
+      R gx = (R)0, gy = (R)0;
 #pragma unroll
-        for (int ii = 0; ii < P; ++ii) {
-          const R qa = sm.q[v][ii + P * j], qb = sm.q[v][i + P * ii];
-          R f1 = qa * sm.dsdx[0][ii + P * j];
-          R f2 = qb * sm.dsdx[2][i + P * ii];
-          gx = gx + (R)sdg[ii + P * i] * f1 + (R)sdg[ii + P * j] * f2;
-          f1 = qa * sm.dsdx[1][ii + P * j];
-          f2 = qb * sm.dsdx[3][i + P * ii];
-          gy = gy + (R)sdg[ii + P * i] * f1 + (R)sdg[ii + P * j] * f2;
-        }
-        // nHat(d, k, side) at nH[d + 2 (k + P side)], nScale(k, side) at nS[k + P side]
-        R f1 = sm.avg[1][v][j] * (R)nH[0 + 2 * (j + P * 1)] * (R)nS[j + P * 1];
-        R f2 = sm.avg[3][v][j] * (R)nH[0 + 2 * (j + P * 3)] * (R)nS[j + P * 3];
-        gx = gx + (f1 * (R)sb[i + P] + f2 * (R)sb[i]) / (R)sw[i];
-        f1 = sm.avg[2][v][i] * (R)nH[0 + 2 * (i + P * 2)] * (R)nS[i + P * 2];
-        f2 = sm.avg[0][v][i] * (R)nH[0 + 2 * (i + P * 0)] * (R)nS[i + P * 0];
-        gx = gx + (f1 * (R)sb[j + P] + f2 * (R)sb[j]) / (R)sw[j];
-        f1 = sm.avg[1][v][j] * (R)nH[1 + 2 * (j + P * 1)] * (R)nS[j + P * 1];
-        f2 = sm.avg[3][v][j] * (R)nH[1 + 2 * (j + P * 3)] * (R)nS[j + P * 3];
-        gy = gy + (f1 * (R)sb[i + P] + f2 * (R)sb[i]) / (R)sw[i];
-        f1 = sm.avg[2][v][i] * (R)nH[1 + 2 * (i + P * 2)] * (R)nS[i + P * 2];
-        f2 = sm.avg[0][v][i] * (R)nH[1 + 2 * (i + P * 0)] * (R)nS[i + P * 0];
-        gy = gy + (f1 * (R)sb[j + P] + f2 * (R)sb[j]) / (R)sw[j];
-        gx = gx / Jij;
-        gy = gy / Jij;
-        gx = gx * nu;
-        gy = gy * nu;
-        sm.g[0][v][t] = gx;
-        sm.g[1][v][t] = gy;
-        const R c1 = -(sm.dsdx[0][t] * gx + sm.dsdx[1][t] * gy);
-        const R c2 = -(sm.dsdx[2][t] * gx + sm.dsdx[3][t] * gy);
-        visc[t + (long long)PP * (0 + 2 * (v + 4 * e))] = c1;
-        visc[t + (long long)PP * (1 + 2 * (v + 4 * e))] = c2;
+      for (int ii = 0; ii < P; ++ii) {
+        const R qa = sm.q[v][ii + P * j], qb = sm.q[v][i + P * ii];
+        R f1 = qa * sm.dsdx[0][ii + P * j];
+        R f2 = qb * sm.dsdx[2][i + P * ii];
+        gx = gx + (R)sdg[ii + P * i] * f1 + (R)sdg[ii + P * j] * f2;
+        f1 = qa * sm.dsdx[1][ii + P * j];
+        f2 = qb * sm.dsdx[3][i + P * ii];
+        gy = gy + (R)sdg[ii + P * i] * f1 + (R)sdg[ii + P * j] * f2;
       }
+      R f1 = sm.avg[1][v][j] * sm.nh[1][j][0] * sm.ns[1][j];
+      R f2 = sm.avg[3][v][j] * sm.nh[3][j][0] * sm.ns[3][j];
+      gx = gx + (f1 * (R)sb[i + P] + f2 * (R)sb[i]) / (R)sw[i];
+      f1 = sm.avg[2][v][i] * sm.nh[2][i][0] * sm.ns[2][i];
+      f2 = sm.avg[0][v][i] * sm.nh[0][i][0] * sm.ns[0][i];
+      gx = gx + (f1 * (R)sb[j + P] + f2 * (R)sb[j]) / (R)sw[j];
+      f1 = sm.avg[1][v][j] * sm.nh[1][j][1] * sm.ns[1][j];
+      f2 = sm.avg[3][v][j] * sm.nh[3][j][1] * sm.ns[3][j];
+      gy = gy + (f1 * (R)sb[i + P] + f2 * (R)sb[i]) / (R)sw[i];
+      f1 = sm.avg[2][v][i] * sm.nh[2][i][1] * sm.ns[2][i];
+      f2 = sm.avg[0][v][i] * sm.nh[0][i][1] * sm.ns[0][i];
+      gy = gy + (f1 * (R)sb[j + P] + f2 * (R)sb[j]) / (R)sw[j];
+      gx = gx / Jij;
+      gy = gy / Jij;
+      gx = gx * nu;
+      gy = gy * nu;
+      sm.g[0][v][t] = gx;
+      sm.g[1][v][t] = gy;
+      const R c1 = -(sm.dsdx[0][t] * gx + sm.dsdx[1][t] * gy);
+      const R c2 = -(sm.dsdx[2][t] * gx + sm.dsdx[3][t] * gy);
+      visc[t + (long long)PP * (0 + 2 * (v + 4 * e))] = c1;
+      visc[t + (long long)PP * (1 + 2 * (v + 4 * e))] = c2;
     }
     __syncthreads();
     // face traces of nu grad q (VectorBoundaryInterp_2D, src/SELF_Lagrange.f90:2284-2316)
     if (live) {
       R* vo = reinterpret_cast<R*>(a.vtr) + (long long)4 * VS * e;
-      for (int k = t; k < 4 * 8 * P; k += PP) {
-        const int ii = k % P, d = (k / P) % 2, v = (k / (2 * P)) % 4, s1 = k / (8 * P);
-        vo[s1 * VS + ii + P * (d + 2 * v)] = face_trace<P, R>(sm.g[d][v], sb, s1, ii);
+      for (int k = u; k < 4 * 8 * P; k += TPE) {
+        const int ii = k % P, d = (k / P) % 2, vv = (k / (2 * P)) % 4, s1 = k / (8 * P);
+        vo[s1 * VS + ii + P * (d + 2 * vv)] = face_trace<P, R>(sm.g[d][vv], sb, s1, ii);
       }
     }
     __syncthreads();  // the slot's arrays are reused by the next round
@@ -630,7 +643,7 @@ template <int P, typename R>
 cudaError_t launch_av_pair(const AvArgs& a, cudaStream_t st, int numSMs, bool formNu) {
   constexpr int EPB = av_elems_per_block<P, R>();
   if (!formNu) {
-    k_av_grad<P, R, EPB><<<4 * numSMs, EPB * P * P, 0, st>>>(a);
+    k_av_grad<P, R, EPB><<<4 * numSMs, EPB * 4 * P * P, 0, st>>>(a);
     return cudaGetLastError();
   }
   cudaError_t e = cudaMemsetAsync(a.activeCount, 0, sizeof(int), st);
@@ -644,11 +657,12 @@ cudaError_t launch_av_pair(const AvArgs& a, cudaStream_t st, int numSMs, bool fo
       nb = 4;
     nuPerSM.store(nb);
   }
-  const long long nuBlocks = (a.nEl + kNuWarps - 1) / kNuWarps;
+  const int perBlock = kNuWarps * 32 / nu_lanes<P>();  // elements
+  const long long nuBlocks = ((long long)a.nEl + perBlock - 1) / perBlock;
   const long long cap = (long long)nuPerSM.load() * numSMs;
   const int g1 = (int)(nuBlocks < cap ? nuBlocks : cap);
   k_av_nu<P, R><<<g1, 32 * kNuWarps, 0, st>>>(a);
-  k_av_grad<P, R, EPB><<<4 * numSMs, EPB * P * P, 0, st>>>(a);
+  k_av_grad<P, R, EPB><<<4 * numSMs, EPB * 4 * P * P, 0, st>>>(a);
   return cudaGetLastError();
 }
 

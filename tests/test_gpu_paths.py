@@ -199,3 +199,22 @@ def test_inference_tiles(n):
     f = np.random.default_rng(n).uniform(-1, 1, (n, 36)).astype(np.float32)
     got = m.infer(torch.from_numpy(f).cuda()).cpu().numpy()
     assert np.abs(got - O.mlp_forward(f.T, *m.unpack())).max() < 1e-5
+
+
+@pytest.mark.parametrize("N", [2, 4, 6])
+@pytest.mark.parametrize("nx,ny", [(1, 1), (7, 5), (131, 41)])  # less than a warp's elements; a short one; several blocks
+def test_closure_lane_groups(N, nx, ny):
+    """Eight lanes per element: groups without an element, and fewer node rows than lanes, against the oracle."""
+    import self_b200 as S
+    kw = dict(nx=nx, ny=ny, periodic=(False, False), bcid=O.BC_NONORMALFLOW, amp=0.02 if nx > 1 else 0.0)
+    ref, mod, _ = _pair("CIG", kw, N, S.FP64)
+    q = C.shock_state(O.Geometry(N, C.oracle_mesh(kw)).x, 1)
+    ref.set("solution", q)
+    mod.SetSolution(q)
+    ref.set_closure(1, c=1.0)
+    mod.SetClosure(S.CLOSURE_INDICATOR, c=1.0)
+    t = ref.tendency()
+    got = S.to_host(mod.CalculateTendency()).reshape(t.shape, order="F")
+    nu = ref.get("avNu")
+    assert np.abs(mod.ClosureState()[0].cpu().numpy() - nu).max() <= 1e-13 * nu.max()
+    _check(got, t, S.FP64)
