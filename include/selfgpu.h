@@ -328,17 +328,20 @@ long long selfgpu_model2d_persistent_launch_count(const selfgpu_model2d* m);
 
 /* Kernel choice: persistent = 1 (default) uses the warp-specialised kernel
  * that streams elements through shared memory with bulk asynchronous copies
- * wherever it applies (even P, 16-byte aligned buffers); 0 forces the
- * one-CTA-per-element-group kernel. */
+ * wherever it applies (16-byte aligned buffers); 0 forces the
+ * one-CTA-per-element-group kernel.  Either way rk3 then runs stage launches
+ * (see set_multistep). */
 int selfgpu_model2d_set_kernel(selfgpu_model2d* m, int persistent);
 
-/* Opt-in (enable = 1): selfgpu_model2d_rk3 runs all 3 nSteps RK stages as
- * ONE cooperative launch (k_fused_steps: the per-element stage body, then a
- * grid barrier before the next stage reads the traces other CTAs wrote) when
- * the mesh's element groups fit one wave of resident CTAs -- small,
- * launch-latency bound meshes such as the 10x10 gravity-wave release.  Larger
- * meshes, a bound closure or halo fall back to graph-replayed steps.  The
- * barrier waits are bounded like the persistent kernel's (set_wait_limit;
+/* selfgpu_model2d_rk3 runs all 3 nSteps RK stages as ONE cooperative launch
+ * that keeps the state on chip (k_fused_resident) where the mesh's tiles of
+ * elements all fit resident CTAs: up to 4 736 elements at N = 7, 7 104 at
+ * N = 5, 18 944 at N = 3 (148 SMs; three quarters of that with the reference's
+ * roundings), without a closure or halo and with neighbour records that name
+ * each other.  That is the default until set_kernel, set_launch or
+ * set_multistage chooses among the stage launches; enable = 1 keeps it on
+ * after those, 0 turns it off.  Results equal the stage launches bit for bit.
+ * The waits for neighbours' traces are bounded (set_wait_limit;
  * SELFGPU_ERR_TIMEOUT from sync). */
 int selfgpu_model2d_set_multistep(selfgpu_model2d* m, int enable);
 
@@ -390,7 +393,8 @@ int selfgpu_model2d_autotune(selfgpu_model2d* m, int* persistent, int* groups, f
  * one element's copies without issuing them, so its consumers' wait runs
  * out; with enable = 2 one group of a multi-stage launch (set_multistage)
  * never announces the end of its stages, so the others' stage-end waits run
- * out. */
+ * out, and one CTA of an on-chip launch (set_multistep) publishes no traces,
+ * so its neighbours' waits do. */
 int selfgpu_model2d_set_wait_limit(selfgpu_model2d* m, long long cycles);
 int selfgpu_model2d_inject_stall(selfgpu_model2d* m, int enable);
 

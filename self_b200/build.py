@@ -19,7 +19,7 @@ BUILD_DIR = os.path.join(HERE, "_build")
 SOURCES = [("setup_host.cpp", []), ("legacy_ops.cu", ["-fmad=false"]), ("stage_fp64.cu", ["-fmad=false"]),
            ("stage_fp64_prod.cu", []), ("stage_fp32.cu", []), ("engine.cu", []), ("noalloc.cu", ["-fmad=false"]),
            ("mlp.cu", []), ("checkpoint.cpp", []), ("decomp.cpp", []), ("hip_shim.cpp", [])]
-HEADERS = ["selfgpu_internal.h", "physics.cuh", "fused_stage.cuh", "fused_stage_tma.cuh", "stage_dispatch.cuh",
+HEADERS = ["selfgpu_internal.h", "physics.cuh", "fused_stage.cuh", "fused_stage_tma.cuh", "fused_resident.cuh", "stage_dispatch.cuh",
            "av_closure.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O3", "--expt-relaxed-constexpr",

@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "av_closure.cuh"
+#include "fused_resident.cuh"
 #include "fused_stage.cuh"
 #include "fused_stage_tma.cuh"
 #include "selfgpu_internal.h"
@@ -266,9 +267,18 @@ struct selfgpu_model2d {
   double* geo = nullptr;  // packed geometry records (persistent kernel)
   float* gf = nullptr;    // RK register of the FP32-bulk form (P,P,NV,nEl); workSol is unused then
   SumScratch* sums = nullptr;  // entropy reduction
-  bool multistep = false;         // rk3 as one cooperative launch where the mesh fits one wave
+  // rk3 as one launch of k_fused_resident where the mesh fits: on or off by
+  // set_multistep, else wherever the caller has not chosen among the stage
+  // launches (set_kernel, set_launch, set_multistage)
+  enum { RESIDENT_AUTO, RESIDENT_OFF, RESIDENT_ON };
+  int resident = RESIDENT_AUTO;
+  bool stagesChosen = false;
+  int residentTiles = 0;          // tiles per CTA; 0 where the mesh does not fit
+  bool symmetric = false;         // every exchanged side's neighbour exchanges with that side
+  void* xch = nullptr;            // k_fused_resident's published traces and set counter
+  void* caches = nullptr;         // the allocation that holds tr, vel and xch
   bool multistage = false;        // rk3 as one launch of the persistent kernel over all stages
-  unsigned* stepBar = nullptr;    // grid-barrier / stage-end counter of the one-launch paths
+  unsigned* stepBar = nullptr;    // stage-end counter of the multi-stage launch
 
   size_t elemBytes() const { return form == SELFGPU_FP32_BULK ? sizeof(float) : sizeof(double); }
 
@@ -315,40 +325,53 @@ struct selfgpu_model2d {
     return e;
   }
 
-  // nSteps RK3 steps as one cooperative launch of k_fused_steps from the
-  // current parities; cudaErrorCooperativeLaunchTooLarge when the element
-  // groups do not fit one wave of resident CTAs (the caller falls back).
-  cudaError_t launch_steps(double dt, int nSteps) {
-    cudaError_t e = cudaSuccess;
-    if (!stepBar) e = cudaMalloc(&stepBar, sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMemsetAsync(stepBar, 0, sizeof(unsigned), stream);
-    if (e != cudaSuccess) return e;
-    StepsArgs sa{};
-    sa.nSteps = nSteps;
-    sa.dt = dt;
-    for (int k = 0; k < 3; ++k) {
-      sa.rkA[k] = kRK3a[k];
-      sa.rkG[k] = kRK3g[k];
+  cudaError_t launch_resident_form(const StageArgs& a, ResidentArgs& ra) {
+    switch (form) {
+      case SELFGPU_FP64: return launch_resident_fp64(model, P, a, ra, cfg, stream);
+      case SELFGPU_FP64_REF: return launch_resident_fp64_ref(model, P, a, ra, cfg, stream);
+      default: return launch_resident_fp32(model, P, a, ra, cfg, stream);
     }
-    sa.tr[0] = tr[0];
-    sa.tr[1] = tr[1];
-    sa.vel[0] = vel[0];
-    sa.vel[1] = vel[1];
-    sa.cur = cur;
-    sa.vcur = vcur;
-    sa.bar = stepBar;
+  }
+
+  // nSteps RK3 steps as one launch of k_fused_resident (it forms stale traces
+  // itself: no prologue); cudaErrorCooperativeLaunchTooLarge when the mesh
+  // does not fit resident CTAs (the caller falls back).
+  cudaError_t launch_resident(double dt, int nSteps) {
+    ResidentArgs ra{};
     StageArgs a = base;
     a.mode = MODE_RK;
-    switch (form) {
-      case SELFGPU_FP64: e = launch_steps_fp64(model, P, a, sa, cfg.numSMs, stream); break;
-      case SELFGPU_FP64_REF: e = launch_steps_fp64_ref(model, P, a, sa, cfg.numSMs, stream); break;
-      default: e = launch_steps_fp32(model, P, a, sa, cfg.numSMs, stream); break;
-    }
-    if (e != cudaSuccess) return e;
-    ++launches;
-    if ((3LL * nSteps) & 1) {  // three cache swaps per step
-      cur = 1 - cur;
-      if (model == SELFGPU_MODEL_SW) vcur = 1 - vcur;
+    if (!xch) return cudaErrorCooperativeLaunchTooLarge;
+    ra.tiles = residentTiles;
+    const size_t pub = publish_bytes();
+    cudaError_t e = cudaSuccess;
+    constexpr int kChunk = 100000;  // steps per launch
+    for (int done = 0; done < nSteps;) {
+      const int k = (nSteps - done) < kChunk ? (nSteps - done) : kChunk;
+      ra.nStages = 3 * k;
+      ra.fresh = valid ? 0 : 1;
+      ra.dt = dt;
+      for (int m = 0; m < 3; ++m) {
+        ra.rkA[m] = kRK3a[m];
+        ra.rkG[m] = kRK3g[m];
+      }
+      // the parities that as many stage launches leave; one pair may serve as
+      // input and output, since a CTA writes its final traces only after its
+      // neighbours have read the initial ones
+      const int odd = ra.nStages & 1;
+      ra.trIn = tr[cur];
+      ra.velIn = vel[vcur];
+      ra.trOut = tr[cur ^ odd];
+      ra.velOut = vel[vcur ^ odd];
+      ra.xch[0] = xch;
+      ra.xch[1] = reinterpret_cast<char*>(xch) + pub;
+      ra.epoch = reinterpret_cast<ResidentEpoch*>(reinterpret_cast<char*>(xch) + 2 * pub);
+      e = launch_resident_form(a, ra);
+      if (e != cudaSuccess) return e;
+      ++launches;
+      valid = true;
+      cur ^= odd;
+      if (model == SELFGPU_MODEL_SW) vcur ^= odd;
+      done += k;
     }
     return cudaSuccess;
   }
@@ -456,19 +479,40 @@ struct selfgpu_model2d {
   }
   size_t vel_block_bytes() const { return (size_t)2 * P * elemBytes(); }
 
+  // one of k_fused_resident's two sets of published traces
+  size_t publish_bytes() const { return 2 * elemBytes() * nt_of(model) * P * 4 * (size_t)nEl; }
+
+  // The caches and, where the mesh fits k_fused_resident, its published traces
+  // (zeroed: no set number is 0) and set counter, in one allocation.
   cudaError_t alloc_caches() {
-    for (int k = 0; k < 2; ++k) {
-      if (tr[k]) cudaFree(tr[k]);
-      if (vel[k]) cudaFree(vel[k]);
-      tr[k] = vel[k] = nullptr;
+    if (caches) cudaFree(caches);
+    caches = nullptr;
+    for (int k = 0; k < 2; ++k) tr[k] = vel[k] = nullptr;
+    xch = nullptr;
+    ResidentArgs ra{};
+    StageArgs a{};
+    a.nEl = nEl;
+    residentTiles = nHalo == 0 && launch_resident_form(a, ra) == cudaSuccess ? ra.tiles : 0;
+    cudaGetLastError();
+    const size_t nb = 4 * (size_t)(nEl + nHalo), t = (trace_block_bytes() * nb + 255) / 256 * 256,
+                 v = model == SELFGPU_MODEL_SW ? (vel_block_bytes() * nb + 255) / 256 * 256 : 0;
+    size_t x = residentTiles ? 2 * publish_bytes() + sizeof(ResidentEpoch) : 0;
+    cudaError_t e = cudaMalloc(&caches, 2 * (t + v) + x);
+    if (e == cudaErrorMemoryAllocation && x) {  // without the published traces, then
+      cudaGetLastError();
+      residentTiles = 0;
+      x = 0;
+      e = cudaMalloc(&caches, 2 * (t + v));
     }
-    const size_t nb = 4 * (size_t)(nEl + nHalo);
+    if (e != cudaSuccess) return e;
+    char* c = reinterpret_cast<char*>(caches);
     for (int k = 0; k < 2; ++k) {
-      cudaError_t e = cudaMalloc(&tr[k], trace_block_bytes() * nb);
-      if (e == cudaSuccess && model == SELFGPU_MODEL_SW) e = cudaMalloc(&vel[k], vel_block_bytes() * nb);
-      if (e != cudaSuccess) return e;
+      tr[k] = c + k * t;
+      if (v) vel[k] = c + 2 * t + k * v;
     }
-    return cudaSuccess;
+    if (!x) return cudaSuccess;
+    xch = c + 2 * (t + v);
+    return cudaMemsetAsync(xch, 0, x, stream);
   }
 };
 
@@ -514,6 +558,8 @@ int selfgpu_model2d_create(selfgpu_model2d** out, int model, int N, int nEl, int
     }
     m->ownStream = true;
   }
+  cudaDeviceGetAttribute(&m->cfg.smemOptin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  cudaDeviceGetAttribute(&m->cfg.numSMs, cudaDevAttrMultiProcessorCount, dev);
   // one (element, side) block holds NT fields x P nodes, padded to 16 bytes
   // (trace_side_stride in fused_stage.cuh)
   e = m->alloc_caches();
@@ -530,8 +576,6 @@ int selfgpu_model2d_create(selfgpu_model2d** out, int model, int N, int nEl, int
   }
   m->derr = m->dflag + 1;
   m->sums = reinterpret_cast<SumScratch*>(m->dflag + 4);
-  cudaDeviceGetAttribute(&m->cfg.smemOptin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  cudaDeviceGetAttribute(&m->cfg.numSMs, cudaDevAttrMultiProcessorCount, dev);
   m->base.err = m->derr;
   m->base.waitCycles = 4000000000LL;  // about 2 s at the B200 boost clock
   m->base.nEl = nEl;
@@ -546,13 +590,9 @@ int selfgpu_model2d_destroy(selfgpu_model2d* m) {
   if (!m) return SELFGPU_OK;
   if (m->stream) cudaStreamSynchronize(m->stream);
   m->drop_graphs();
-  for (int k = 0; k < 2; ++k) {
-    if (m->tr[k]) cudaFree(m->tr[k]);
-    if (m->vel[k]) cudaFree(m->vel[k]);
-  }
   for (void* p : {(void*)m->avNu, (void*)m->avAct, (void*)m->avFallbacks, (void*)m->avH, m->avVisc, m->avVtr,
                   (void*)m->mlpW, (void*)m->mlpB, (void*)m->geo, (void*)m->stepBar,
-                  (void*)m->gf})
+                  (void*)m->gf, m->caches})
     if (p) cudaFree(p);
   if (m->dflag) cudaFree(m->dflag);
   if (m->ownStream) cudaStreamDestroy(m->stream);
@@ -581,6 +621,14 @@ int selfgpu_model2d_set_geometry(selfgpu_model2d* m, const double* dsdx, const d
     return set_error(SELFGPU_ERR_ARG, "selfgpu_model2d_set_geometry: dsdx and nHat must be 16-byte aligned");
   int rc = validate_side_info(sideInfo_h, m->nEl, m->nEl + m->nHalo);
   if (rc != SELFGPU_OK) return rc;
+  m->symmetric = true;
+  for (int b = 0; b < 4 * m->nEl && m->symmetric; ++b) {
+    const int* si = sideInfo_h + 5 * (size_t)b;
+    if (si[4] != 0) continue;
+    const int e2 = si[2] - 1, s2 = si[3] / 10 - 1;
+    const int* sn = sideInfo_h + 5 * (s2 + 4 * (size_t)e2);
+    m->symmetric = e2 < m->nEl && sn[4] == 0 && 4 * (sn[2] - 1) + sn[3] / 10 - 1 == b;
+  }
   m->base.dsdx = dsdx;
   m->base.J = J;
   m->base.nHat = nHat;
@@ -730,6 +778,15 @@ int selfgpu_model2d_rk3(selfgpu_model2d* m, double dt, int nSteps) {
   if (rc) return rc;
   if (nSteps < 0) return set_error(SELFGPU_ERR_ARG, "selfgpu_model2d_rk3: nSteps < 0");
   cudaError_t e = cudaSuccess;
+  if ((m->resident == m->RESIDENT_ON || (m->resident == m->RESIDENT_AUTO && !m->stagesChosen)) && nSteps > 0 &&
+      m->avMode == AV_OFF && m->nHalo == 0 && m->symmetric && m->base.debugStarve != 1) {
+    e = m->launch_resident(dt, nSteps);
+    if (e == cudaSuccess) return SELFGPU_OK;
+    cudaGetLastError();
+    if (e != cudaErrorCooperativeLaunchTooLarge)
+      return fail_cuda("selfgpu_model2d_rk3: resident launch", e);
+    // larger meshes: stage launches below
+  }
   if (m->multistage && nSteps > 0 && m->avMode == AV_OFF && m->nHalo == 0 && m->base.debugStarve != 1 &&
       m->cfg.allowTma) {
     e = m->valid ? cudaSuccess : m->prologue();
@@ -742,15 +799,6 @@ int selfgpu_model2d_rk3(selfgpu_model2d* m, double dt, int nSteps) {
       return fail_cuda("selfgpu_model2d_rk3: multi-stage launch", e);
     m->cur = c0;  // nothing was launched: stage launches below
     m->vcur = v0;
-  }
-  if (m->multistep && nSteps > 0 && m->avMode == AV_OFF && m->nHalo == 0 && !m->base.debugStarve) {
-    e = m->valid ? cudaSuccess : m->prologue();
-    if (e != cudaSuccess) return fail_cuda("selfgpu_model2d_rk3", e);
-    e = m->launch_steps(dt, nSteps);
-    if (e == cudaSuccess) return SELFGPU_OK;
-    cudaGetLastError();
-    if (e != cudaErrorCooperativeLaunchTooLarge) return fail_cuda("selfgpu_model2d_rk3: multi-step launch", e);
-    // the mesh does not fit one wave: graph-replayed steps below
   }
   if (!m->valid) {
     e = m->prologue();
@@ -836,13 +884,14 @@ int selfgpu_model2d_inject_stall(selfgpu_model2d* m, int enable) {
 
 int selfgpu_model2d_set_multistep(selfgpu_model2d* m, int enable) {
   if (!m) return set_error(SELFGPU_ERR_ARG, "selfgpu_model2d_set_multistep: null handle");
-  m->multistep = enable != 0;
+  m->resident = enable ? m->RESIDENT_ON : m->RESIDENT_OFF;
   return SELFGPU_OK;
 }
 
 int selfgpu_model2d_set_kernel(selfgpu_model2d* m, int persistent) {
   if (!m) return set_error(SELFGPU_ERR_ARG, "selfgpu_model2d_set_kernel: null handle");
   m->cfg.allowTma = persistent != 0;
+  m->stagesChosen = true;
   m->drop_graphs();
   return SELFGPU_OK;
 }
@@ -850,12 +899,14 @@ int selfgpu_model2d_set_kernel(selfgpu_model2d* m, int persistent) {
 int selfgpu_model2d_set_multistage(selfgpu_model2d* m, int enable) {
   if (!m) return set_error(SELFGPU_ERR_ARG, "selfgpu_model2d_set_multistage: null handle");
   m->multistage = enable != 0;
+  m->stagesChosen = true;
   return SELFGPU_OK;
 }
 
 int selfgpu_model2d_set_launch(selfgpu_model2d* m, int persistent, int groups) {
   if (!m || groups < 0) return set_error(SELFGPU_ERR_ARG, "selfgpu_model2d_set_launch: bad arguments");
   m->cfg.allowTma = persistent != 0;
+  m->stagesChosen = true;
   m->cfg.maxGroups = groups;
   m->drop_graphs();
   return SELFGPU_OK;

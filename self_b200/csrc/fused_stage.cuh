@@ -151,6 +151,8 @@ __host__ __device__ constexpr int geo_kind() {
          : (P == 8 ? GEO_NOJ : GEO_INVJ);
 }
 
+struct NoFaceK {};  // no constants of a face node
+
 struct PhysLSW {
   static constexpr int NV = 3, NT = 3, NF = 3;
   static constexpr bool kLaggedVelocity = false;
@@ -175,9 +177,16 @@ struct PhysLSW {
     S[1] = -fc * f[0];
     S[2] = (R)0;
   }
+  // constants of a face node (x as for face)
+  template <typename R>
+  using FaceK = LswFace<R>;
+  template <typename R>
+  __device__ static LswFace<R> face_constants(const double* x, const StageArgs& s) {
+    return lsw_face<R>((R)x[0], (R)s.g);
+  }
   template <typename R>
   __device__ static void face(int bcid, bool physical, const R* L, R* X, const R*, const R*, double n1, double n2,
-                              double nmag, const double* x, const StageArgs& s, R out[3]) {
+                              double nmag, const double*, const LswFace<R>& k, const StageArgs& s, R out[3]) {
     if (physical) {  // src/models/SELF_LinearShallowWater.f90:323-349
       if (bcid == SG_BC_NONORMALFLOW) {
         reflect<R>(L[0], L[1], n1, n2, X[0], X[1]);
@@ -186,7 +195,7 @@ struct PhysLSW {
         X[0] = X[1] = X[2] = (R)0;
       }
     }
-    lsw_riemann<R>(L[0], L[1], L[2], X[0], X[1], X[2], (R)x[0], (R)s.g, n1, n2, nmag, out);
+    lsw_riemann<R>(L[0], L[1], L[2], X[0], X[1], X[2], k, (R)s.g, n1, n2, nmag, out);
   }
 };
 
@@ -221,8 +230,14 @@ struct PhysSW {
     S[2] = (R)0;
   }
   template <typename R>
+  using FaceK = NoFaceK;
+  template <typename R>
+  __device__ static NoFaceK face_constants(const double*, const StageArgs&) {
+    return {};
+  }
+  template <typename R>
   __device__ static void face(int bcid, bool physical, const R* L, R* X, const R* velL, const R* velR, double n1,
-                              double n2, double nmag, const double* x, const StageArgs& s, R out[3]) {
+                              double n2, double nmag, const double* x, NoFaceK, const StageArgs& s, R out[3]) {
     if (physical) {  // src/models/SELF_ShallowWater.f90:305-338
       if (bcid == SG_BC_NONORMALFLOW) {
         reflect<R>(L[0], L[1], n1, n2, X[0], X[1]);
@@ -284,8 +299,14 @@ struct PhysCIG {
     S[3] = -f[0] * gx - f[0] * gy;
   }
   template <typename R>
+  using FaceK = NoFaceK;
+  template <typename R>
+  __device__ static NoFaceK face_constants(const double*, const StageArgs&) {
+    return {};
+  }
+  template <typename R>
   __device__ static void face(int bcid, bool physical, const R* L, R* X, const R*, const R*, double n1, double n2,
-                              double nmag, const double* x, const StageArgs& s, R out[4]) {
+                              double nmag, const double* x, NoFaceK, const StageArgs& s, R out[4]) {
     if (physical) {  // src/models/SELF_CompressibleIdealGas2D.f90:1256-1317
       if (bcid == SG_BC_NONORMALFLOW) {
         reflect<R>(L[0], L[1], n1, n2, X[0], X[1]);
@@ -427,35 +448,17 @@ struct Smem {
   R vel[Phys::kLaggedVelocity ? 2 : 1][4][2][P];
 };
 
-// The per-stage part of a launch (mode, RK coefficients, the trace-cache
-// halves read and written); everything else comes from StageArgs.
-struct StageVar {
-  int mode;
-  double rk_a, rk_gdt, rk_g;
-  const void* trIn;
-  void* trOut;
-  const void* velIn;
-  void* velOut;
-};
-
-// A load from the trace cache.  kCoherent = true (the multi-stage kernel,
-// where other CTAs of the same launch wrote the data a grid barrier ago)
-// reads through L2 only, never a possibly stale L1 line.
-template <bool kCoherent, typename R>
-__device__ __forceinline__ R ld_trace(const R* p) {
-  if constexpr (kCoherent) return __ldcg(p);
-  else return *p;
-}
-
-// One stage over the CTA's EPB element slots (one thread per node): the body
-// of k_fused_stage, shared with the multi-stage kernel k_fused_steps.  The
-// operator matrices are already in shared memory (sdg, sb, srw).
-template <int P, class Phys, typename R, int EPB, bool kCoherent>
-__device__ __forceinline__ void fused_stage_group(const StageArgs& a, const StageVar& sv, Smem<P, Phys, R>* sm_all,
-                                                  const double* sdg, const double* sb, const double* srw) {
+// One stage over the CTA's EPB element slots, one thread per node.
+template <int P, class Phys, typename R, int EPB>
+__global__ void __launch_bounds__(EPB* P* P) k_fused_stage(const StageArgs a) {
   constexpr int NV = Phys::NV, NT = Phys::NT, NF = Phys::NF, PP = P * P, N = P - 1;
   constexpr int TS = trace_side_stride<P, NT, R>();
   using S = Smem<P, Phys, R>;
+  __shared__ S sm_all[EPB];
+  __shared__ double sdg[PP], sb[2 * P], srw[P];
+  for (int k = threadIdx.x; k < PP; k += blockDim.x) sdg[k] = a.dgM[k];
+  for (int k = threadIdx.x; k < 2 * P; k += blockDim.x) sb[k] = a.bM[k];
+  for (int k = threadIdx.x; k < P; k += blockDim.x) srw[k] = a.qw[k];
 
   const int tid = threadIdx.x;
   const int slot = tid / PP;
@@ -465,8 +468,8 @@ __device__ __forceinline__ void fused_stage_group(const StageArgs& a, const Stag
 
   const long long e = (long long)blockIdx.x * EPB + slot;
   const bool live = e < a.nEl;
-  const R* trIn = reinterpret_cast<const R*>(sv.trIn);
-  R* trOut = reinterpret_cast<R*>(sv.trOut);
+  const R* trIn = reinterpret_cast<const R*>(a.trIn);
+  R* trOut = reinterpret_cast<R*>(a.trOut);
   const long long gnode = t + (long long)PP * e;
 
   if (live) {
@@ -476,155 +479,152 @@ __device__ __forceinline__ void fused_stage_group(const StageArgs& a, const Stag
     Phys::template node<R>(f, a);
 #pragma unroll
     for (int v = 0; v < NF; ++v) sm.fld[v][t] = f[v];
-    if (sv.mode != MODE_TRACES) {
-      double na[3];
-      node_aux_global<Phys>(a, t, e, PP, na);
-      R Fx[NV], Fy[NV];
-      Phys::template flux<R>(f, na, a, Fx, Fy);
-      const double2* gp = reinterpret_cast<const double2*>(a.dsdx + 4 * gnode);
-      const double2 c1 = gp[0], c2 = gp[1];  // (dsdx11, dsdx21), (dsdx12, dsdx22)
-      R F0[NV], F1[NV];
+    double na[3];
+    node_aux_global<Phys>(a, t, e, PP, na);
+    R Fx[NV], Fy[NV];
+    Phys::template flux<R>(f, na, a, Fx, Fy);
+    const double2* gp = reinterpret_cast<const double2*>(a.dsdx + 4 * gnode);
+    const double2 c1 = gp[0], c2 = gp[1];  // (dsdx11, dsdx21), (dsdx12, dsdx22)
+    R F0[NV], F1[NV];
 #pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        F0[v] = (R)c1.x * Fx[v] + (R)c1.y * Fy[v];
-        F1[v] = (R)c2.x * Fx[v] + (R)c2.y * Fy[v];
-      }
-      if constexpr (NV == 4)
-        if (a.av) av_volume_add<P, R>(a, t, e, F0, F1);
+    for (int v = 0; v < NV; ++v) {
+      F0[v] = (R)c1.x * Fx[v] + (R)c1.y * Fy[v];
+      F1[v] = (R)c2.x * Fx[v] + (R)c2.y * Fy[v];
+    }
+    if constexpr (NV == 4)
+      if (a.av) av_volume_add<P, R>(a, t, e, F0, F1);
 #pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        sm.Fc[0][v][t] = F0[v];
-        sm.Fc[1][v][t] = F1[v];
+    for (int v = 0; v < NV; ++v) {
+      sm.Fc[0][v][t] = F0[v];
+      sm.Fc[1][v][t] = F1[v];
+    }
+    for (int k = t; k < 4 * NT * P; k += PP) {
+      const int ii = k % P, fs = k / P, fi = fs % NT, s1 = fs / NT;
+      const int* si = a.sideInfo + 5 * (s1 + 4 * e);
+      R val = (R)0;
+      if (si[4] == 0) {
+        const long long e2 = si[2] - 1;
+        const int s2 = si[3] / 10 - 1, flip = si[3] % 10;
+        val = trIn[(flip ? N - ii : ii) + P * fi + (long long)TS * (s2 + 4 * e2)];
       }
-      for (int k = t; k < 4 * NT * P; k += PP) {
-        const int ii = k % P, fs = k / P, fi = fs % NT, s1 = fs / NT;
-        const int* si = a.sideInfo + 5 * (s1 + 4 * e);
+      sm.ext[s1][fi][ii] = val;
+      // own traces of this stage's solution: the trace cache holds them (the
+      // previous launch formed them from the same values with the same sums)
+      sm.own[s1][fi][ii] = trIn[ii + P * fi + (long long)TS * (s1 + 4 * e)];
+    }
+    if constexpr (Phys::kLaggedVelocity) {
+      const R* vIn = reinterpret_cast<const R*>(a.velIn);
+      for (int k = t; k < 16 * P; k += PP) {
+        const int ii = k % P, d = (k / P) % 2, s1 = (k / (2 * P)) % 4, which = k / (8 * P);
         R val = (R)0;
-        if (si[4] == 0) {
-          const long long e2 = si[2] - 1;
-          const int s2 = si[3] / 10 - 1, flip = si[3] % 10;
-          val = ld_trace<kCoherent>(trIn + (flip ? N - ii : ii) + P * fi + (long long)TS * (s2 + 4 * e2));
-        }
-        sm.ext[s1][fi][ii] = val;
-        // own traces of this stage's solution: the trace cache holds them (the
-        // previous launch formed them from the same values with the same sums)
-        sm.own[s1][fi][ii] = ld_trace<kCoherent>(trIn + ii + P * fi + (long long)TS * (s1 + 4 * e));
-      }
-      if constexpr (Phys::kLaggedVelocity) {
-        const R* vIn = reinterpret_cast<const R*>(sv.velIn);
-        for (int k = t; k < 16 * P; k += PP) {
-          const int ii = k % P, d = (k / P) % 2, s1 = (k / (2 * P)) % 4, which = k / (8 * P);
-          R val = (R)0;
-          if (which == 0) {
-            val = ld_trace<kCoherent>(vIn + ii + P * (d + 2 * (s1 + 4 * e)));
-          } else {
-            const int* si = a.sideInfo + 5 * (s1 + 4 * e);
-            if (si[4] == 0) {  // velocity%extBoundary is only ever set by the exchange (H8)
-              const long long e2 = si[2] - 1;
-              const int s2 = si[3] / 10 - 1, flip = si[3] % 10;
-              val = ld_trace<kCoherent>(vIn + (flip ? N - ii : ii) + P * (d + 2 * (s2 + 4 * e2)));
-            }
+        if (which == 0) {
+          val = vIn[ii + P * (d + 2 * (s1 + 4 * e))];
+        } else {
+          const int* si = a.sideInfo + 5 * (s1 + 4 * e);
+          if (si[4] == 0) {  // velocity%extBoundary is only ever set by the exchange (H8)
+            const long long e2 = si[2] - 1;
+            const int s2 = si[3] / 10 - 1, flip = si[3] % 10;
+            val = vIn[(flip ? N - ii : ii) + P * (d + 2 * (s2 + 4 * e2))];
           }
-          sm.vel[which][s1][d][ii] = val;
         }
+        sm.vel[which][s1][d][ii] = val;
       }
     }
   }
-  if (sv.mode != MODE_TRACES) {
-    __syncthreads();
-    // 4P face nodes per element; for P <= 3 there are fewer node threads (P*P)
-    if (live)
-      for (int k = t; k < 4 * P; k += PP) {
-        const int s1 = k / P, ii = k % P;
-        const int* si = a.sideInfo + 5 * (s1 + 4 * e);
-        const int bcid = si[4];
-        const bool physical = (bcid != 0) && (si[2] == 0);
-        R L[NT], X[NT];
+  __syncthreads();
+  // 4P face nodes per element; for P <= 3 there are fewer node threads (P*P)
+  if (live)
+    for (int k = t; k < 4 * P; k += PP) {
+      const int s1 = k / P, ii = k % P;
+      const int* si = a.sideInfo + 5 * (s1 + 4 * e);
+      const int bcid = si[4];
+      const bool physical = (bcid != 0) && (si[2] == 0);
+      R L[NT], X[NT];
 #pragma unroll
-        for (int m = 0; m < NT; ++m) {
-          L[m] = sm.own[s1][m][ii];
-          X[m] = (bcid == 0) ? sm.ext[s1][m][ii] : (R)0;
-        }
-        const long long gface = ii + (long long)P * (s1 + 4 * e);
-        const double2 nh = reinterpret_cast<const double2*>(a.nHat)[gface];
-        const double ns = a.nScale[gface];
-        double fx[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        if (physical) face_aux_global<Phys>(a, s1, ii, e, P, fx);
-        else if constexpr (Phys::NV == 3 && !Phys::kLaggedVelocity) face_aux_global<Phys>(a, s1, ii, e, P, fx);
-        R velL[2] = {(R)0, (R)0}, velR[2] = {(R)0, (R)0};
-        if constexpr (Phys::kLaggedVelocity) {
-          velL[0] = sm.vel[0][s1][0][ii];
-          velL[1] = sm.vel[0][s1][1][ii];
-          velR[0] = sm.vel[1][s1][0][ii];
-          velR[1] = sm.vel[1][s1][1][ii];
-          R* vOut = reinterpret_cast<R*>(sv.velOut);  // read by the next stage
-          vOut[ii + P * (0 + 2 * (s1 + 4 * e))] = L[0] / L[2];
-          vOut[ii + P * (1 + 2 * (s1 + 4 * e))] = L[1] / L[2];
-        }
-        R out[NV];
-        Phys::template face<R>(bcid, physical, L, X, velL, velR, nh.x, nh.y, ns, fx, a, out);
-        if constexpr (NV == 4)
-          if (a.av) av_face_add<P, R>(a, s1, ii, e, si, nh.x, nh.y, ns, out);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) sm.fb[s1][v][ii] = out[v];
+      for (int m = 0; m < NT; ++m) {
+        L[m] = sm.own[s1][m][ii];
+        X[m] = (bcid == 0) ? sm.ext[s1][m][ii] : (R)0;
       }
-    __syncthreads();
-    if (live) {
-      R f[NF];
-#pragma unroll
-      for (int v = 0; v < NF; ++v) f[v] = sm.fld[v][t];
-      double na[3];
-      node_aux_global<Phys>(a, t, e, PP, na);
-      // sources in FP64 in every form (well-balanced topography / gravity terms)
-      double qd[NV], Src[NV];
-#pragma unroll
-      for (int v = 0; v < NV; ++v) qd[v] = a.q[t + (long long)PP * (v + NV * e)];
-      Phys::template source<double>(qd, na, a, Src);
-      const double Jij = a.J[gnode];
-      const R wi = (R)srw[i], wj = (R)srw[j];
-      // FP32 bulk and production FP64: products with the reciprocals (the
-      // reference-rounding FP64 build divides as the reference does)
-      const R rwi = (R)(1.0 / srw[i]), rwj = (R)(1.0 / srw[j]);
-      const double rJ = 1.0 / Jij;
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        R d = (R)0;
-#pragma unroll
-        for (int m = 0; m < P; ++m)
-          d = d + (R)sdg[m + P * i] * sm.Fc[0][v][m + P * j] + (R)sdg[m + P * j] * sm.Fc[1][v][i + P * m];
-        const R lx = (R)sb[i + P] * sm.fb[1][v][j] + (R)sb[i] * sm.fb[3][v][j];
-        const R ly = (R)sb[j + P] * sm.fb[2][v][i] + (R)sb[j] * sm.fb[0][v][i];
-        double dsdt;
-        if constexpr (ref_rounding<R>()) {
-          d = d + lx / wi + ly / wj;
-          dsdt = Src[v] - (double)d / Jij;
-        } else {
-          d = d + lx * rwi + ly * rwj;
-          dsdt = Src[v] - (double)d * rJ;
-        }
-        const long long gi = t + (long long)PP * (v + NV * e);
-        if (sv.mode == MODE_TENDENCY) {
-          a.dSdt[gi] = dsdt;
-        } else {
-          // the FP32-bulk form carries the RK register in FP32; the solution
-          // update below uses this stage's unrounded FP64 value
-          const double Gn = sv.rk_a * (sizeof(R) == 4 ? (double)a.Gf[gi] : a.G[gi]) + dsdt;
-          if constexpr (sizeof(R) == 4) a.Gf[gi] = (float)Gn;
-          else a.G[gi] = Gn;
-          const double qn = qd[v] + (a.dtElem ? sv.rk_g * a.dtElem[e] : sv.rk_gdt) * Gn;
-          a.q[gi] = qn;
-          f[v] = (R)qn;
-        }
+      const long long gface = ii + (long long)P * (s1 + 4 * e);
+      const double2 nh = reinterpret_cast<const double2*>(a.nHat)[gface];
+      const double ns = a.nScale[gface];
+      double fx[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+      if (physical) face_aux_global<Phys>(a, s1, ii, e, P, fx);
+      else if constexpr (Phys::NV == 3 && !Phys::kLaggedVelocity) face_aux_global<Phys>(a, s1, ii, e, P, fx);
+      R velL[2] = {(R)0, (R)0}, velR[2] = {(R)0, (R)0};
+      if constexpr (Phys::kLaggedVelocity) {
+        velL[0] = sm.vel[0][s1][0][ii];
+        velL[1] = sm.vel[0][s1][1][ii];
+        velR[0] = sm.vel[1][s1][0][ii];
+        velR[1] = sm.vel[1][s1][1][ii];
+        R* vOut = reinterpret_cast<R*>(a.velOut);  // read by the next stage
+        vOut[ii + P * (0 + 2 * (s1 + 4 * e))] = L[0] / L[2];
+        vOut[ii + P * (1 + 2 * (s1 + 4 * e))] = L[1] / L[2];
       }
-      if (sv.mode == MODE_RK) {
-        // only this thread reads node t of fld in this phase, so it may overwrite it
-        Phys::template node<R>(f, a);
+      R out[NV];
+      Phys::template face<R>(bcid, physical, L, X, velL, velR, nh.x, nh.y, ns, fx,
+                                Phys::template face_constants<R>(fx, a), a, out);
+      if constexpr (NV == 4)
+        if (a.av) av_face_add<P, R>(a, s1, ii, e, si, nh.x, nh.y, ns, out);
 #pragma unroll
-        for (int v = 0; v < NF; ++v) sm.fld[v][t] = f[v];
+      for (int v = 0; v < NV; ++v) sm.fb[s1][v][ii] = out[v];
+    }
+  __syncthreads();
+  if (live) {
+    R f[NF];
+#pragma unroll
+    for (int v = 0; v < NF; ++v) f[v] = sm.fld[v][t];
+    double na[3];
+    node_aux_global<Phys>(a, t, e, PP, na);
+    // sources in FP64 in every form (well-balanced topography / gravity terms)
+    double qd[NV], Src[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) qd[v] = a.q[t + (long long)PP * (v + NV * e)];
+    Phys::template source<double>(qd, na, a, Src);
+    const double Jij = a.J[gnode];
+    const R wi = (R)srw[i], wj = (R)srw[j];
+    // FP32 bulk and production FP64: products with the reciprocals (the
+    // reference-rounding FP64 build divides as the reference does)
+    const R rwi = (R)(1.0 / srw[i]), rwj = (R)(1.0 / srw[j]);
+    const double rJ = 1.0 / Jij;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      R d = (R)0;
+#pragma unroll
+      for (int m = 0; m < P; ++m)
+        d = d + (R)sdg[m + P * i] * sm.Fc[0][v][m + P * j] + (R)sdg[m + P * j] * sm.Fc[1][v][i + P * m];
+      const R lx = (R)sb[i + P] * sm.fb[1][v][j] + (R)sb[i] * sm.fb[3][v][j];
+      const R ly = (R)sb[j + P] * sm.fb[2][v][i] + (R)sb[j] * sm.fb[0][v][i];
+      double dsdt;
+      if constexpr (ref_rounding<R>()) {
+        d = d + lx / wi + ly / wj;
+        dsdt = Src[v] - (double)d / Jij;
+      } else {
+        d = d + lx * rwi + ly * rwj;
+        dsdt = fma(-(double)d, rJ, Src[v]);
+      }
+      const long long gi = t + (long long)PP * (v + NV * e);
+      if (a.mode == MODE_TENDENCY) {
+        a.dSdt[gi] = dsdt;
+      } else {
+        // the FP32-bulk form carries the RK register in FP32; the solution
+        // update below uses this stage's unrounded FP64 value
+        const double Gn = a.rk_a * (sizeof(R) == 4 ? (double)a.Gf[gi] : a.G[gi]) + dsdt;
+        if constexpr (sizeof(R) == 4) a.Gf[gi] = (float)Gn;
+        else a.G[gi] = Gn;
+        const double qn = qd[v] + (a.dtElem ? a.rk_g * a.dtElem[e] : a.rk_gdt) * Gn;
+        a.q[gi] = qn;
+        f[v] = (R)qn;
       }
     }
-    if (sv.mode == MODE_TENDENCY) return;
+    if (a.mode == MODE_RK) {
+      // only this thread reads node t of fld in this phase, so it may overwrite it
+      Phys::template node<R>(f, a);
+#pragma unroll
+      for (int v = 0; v < NF; ++v) sm.fld[v][t] = f[v];
+    }
   }
+  if (a.mode == MODE_TENDENCY) return;
   __syncthreads();
   // traces of the (updated) solution -> trace cache: one task per (field,
   // line, orientation) forms both end traces of the line (column l: S and N,
@@ -645,110 +645,7 @@ __device__ __forceinline__ void fused_stage_group(const StageArgs& a, const Stag
       o[l + P * fi + TS * (row ? 3 : 0)] = lo;
       o[l + P * fi + TS * (row ? 1 : 2)] = hi;
     }
-  if constexpr (Phys::kLaggedVelocity) {
-    // Start of a run: the stage-lagged velocity traces equal those of this
-    // solution (SetSolution leaves solution%boundary = BoundaryInterp(solution)).
-    if (sv.mode == MODE_TRACES && sv.velOut != nullptr) {
-      __syncthreads();
-      if (live)
-        for (int k = t; k < 4 * P; k += PP) {
-          const int s1 = k / P, ii = k % P;
-          R* vOut = reinterpret_cast<R*>(sv.velOut);
-          const R H = o[ii + P * 2 + TS * s1];
-          vOut[ii + P * (0 + 2 * (s1 + 4 * e))] = o[ii + P * 0 + TS * s1] / H;
-          vOut[ii + P * (1 + 2 * (s1 + 4 * e))] = o[ii + P * 1 + TS * s1] / H;
-        }
-    }
-  }
 }
 
-
-template <int P, class Phys, typename R, int EPB>
-__global__ void __launch_bounds__(EPB* P* P) k_fused_stage(const StageArgs a) {
-  constexpr int PP = P * P;
-  __shared__ Smem<P, Phys, R> sm_all[EPB];
-  __shared__ double sdg[PP], sb[2 * P], srw[P];
-  for (int k = threadIdx.x; k < PP; k += blockDim.x) sdg[k] = a.dgM[k];
-  for (int k = threadIdx.x; k < 2 * P; k += blockDim.x) sb[k] = a.bM[k];
-  for (int k = threadIdx.x; k < P; k += blockDim.x) srw[k] = a.qw[k];
-  const StageVar sv{a.mode, a.rk_a, a.rk_gdt, a.rk_g, a.trIn, a.trOut, a.velIn, a.velOut};
-  fused_stage_group<P, Phys, R, EPB, false>(a, sv, sm_all, sdg, sb, srw);
-}
-
-// ------------------------------------------------- multi-stage (one launch)
-// Arguments of k_fused_steps: nSteps Williamson RK3 steps of size dt from
-// the trace-cache halves cur / vcur, with a grid barrier counter.
-struct StepsArgs {
-  int nSteps;
-  double dt;
-  double rkA[3], rkG[3];
-  const void* tr[2];
-  const void* vel[2];
-  int cur, vcur;
-  unsigned* bar;  // zero at launch; counts CTA arrivals over all barriers
-};
-
-// Grid-wide barrier number k (1-based) of a launch whose CTAs are all
-// resident (cooperative launch).  Bounded: a CTA that waits longer than
-// `cycles` sets the error word and returns false (the launch then stops).
-__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned k, long long cycles, int* err) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(bar, 1u);
-    const unsigned target = k * gridDim.x;
-    int ok = 1;
-    const long long t0 = clock64();
-    while (true) {
-      unsigned v;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-      if (v >= target) break;
-      if (clock64() - t0 > cycles) {
-        ok = 0;
-        if (err) atomicExch(err, 1);
-        break;
-      }
-      __nanosleep(32);
-    }
-    __threadfence();
-    s_ok = ok;
-  }
-  __syncthreads();
-  return s_ok != 0;
-}
-
-// All RK stages of nSteps steps in one cooperative launch, for meshes whose
-// element groups fit one wave of resident CTAs (the small, launch-latency
-// bound cases): each stage is the k_fused_stage body over the CTA's elements,
-// then a grid barrier before the next stage reads the traces other CTAs
-// wrote.  Trace reads go through L2 (ld_trace<true>).
-template <int P, class Phys, typename R, int EPB>
-__global__ void __launch_bounds__(EPB* P* P) k_fused_steps(const StageArgs a, const StepsArgs sa) {
-  constexpr int PP = P * P;
-  __shared__ Smem<P, Phys, R> sm_all[EPB];
-  __shared__ double sdg[PP], sb[2 * P], srw[P];
-  for (int k = threadIdx.x; k < PP; k += blockDim.x) sdg[k] = a.dgM[k];
-  for (int k = threadIdx.x; k < 2 * P; k += blockDim.x) sb[k] = a.bM[k];
-  for (int k = threadIdx.x; k < P; k += blockDim.x) srw[k] = a.qw[k];
-  int cur = sa.cur, vcur = sa.vcur;
-  unsigned k = 0;
-  for (int s = 0; s < sa.nSteps; ++s)
-    for (int m = 0; m < 3; ++m) {
-      StageVar sv;
-      sv.mode = MODE_RK;
-      sv.rk_a = sa.rkA[m];
-      sv.rk_gdt = sa.rkG[m] * sa.dt;
-      sv.rk_g = sa.rkG[m];
-      sv.trIn = sa.tr[cur];
-      sv.trOut = const_cast<void*>(sa.tr[1 - cur]);
-      sv.velIn = sa.vel[vcur];
-      sv.velOut = const_cast<void*>(sa.vel[1 - vcur]);
-      fused_stage_group<P, Phys, R, EPB, true>(a, sv, sm_all, sdg, sb, srw);
-      cur ^= 1;
-      if constexpr (Phys::kLaggedVelocity) vcur ^= 1;
-      if (!grid_barrier(sa.bar, ++k, a.waitCycles, a.err)) return;
-    }
-}
 
 }  // namespace selfgpu

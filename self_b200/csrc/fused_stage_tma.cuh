@@ -479,6 +479,74 @@ __device__ __forceinline__ void tile_traces(const R* fields, int stride, int ele
   }
 }
 
+// PhysCIG::node in FP32 with every product rounded by itself, whatever the
+// compiler would contract: the traces of a state set from outside are the
+// first stage's input, and a last-bit difference there is visible in the
+// solution (2e-9 relative after twelve steps).
+__device__ __forceinline__ void cig_fields_rounded(float* f, float gamma) {
+  const float r = 1.0f / f[2];
+  f[4] = __fmul_rn(f[0], r);
+  f[5] = __fmul_rn(f[1], r);
+  const float ke = __fmul_rn(0.5f, __fadd_rn(__fmul_rn(f[0], f[4]), __fmul_rn(f[1], f[5])));
+  f[6] = __fmul_rn(gamma - 1.0f, __fsub_rn(f[3], ke));
+  f[7] = __fadd_rn(f[3], f[6]);
+  f[8] = sqrtf(__fmul_rn(__fmul_rn(gamma, f[6]), r));
+}
+
+// The trace cache (and, ShallowWater, the lagged velocity traces, which start
+// as those of this solution: SetSolution leaves solution%boundary =
+// BoundaryInterp(solution)) of a solution set from outside.  Bound by memory:
+// the solution read, the traces written.  Blocks of 256 threads, one node per
+// thread, with only the node fields in shared memory: 2 048 threads per SM.
+template <int P, class Phys, typename R>
+struct TraceBlock {
+  static constexpr int elems = 256 / (P * P), threads = elems * P * P;
+};
+template <int P, class Phys, typename R>
+__global__ void __launch_bounds__(TraceBlock<P, Phys, R>::threads) k_traces(const StageArgs a) {
+  using T = TmaTraits<P, Phys, R>;
+  constexpr int NV = T::NV, NF = T::NF, PP = T::PP, TS = T::TS, FS = T::FS;
+  constexpr int EPB = TraceBlock<P, Phys, R>::elems, NTH = TraceBlock<P, Phys, R>::threads;
+  __shared__ R sm[EPB * NF * FS];
+  const int t = threadIdx.x, slot = t / PP, n = t - slot * PP;
+  const long long e0 = (long long)blockIdx.x * EPB;
+  const int live = a.nEl - e0 < EPB ? (int)(a.nEl - e0) : EPB;
+  if (slot < live) {
+    R f[NF];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) f[v] = (R)a.q[n + (long long)PP * (v + NV * (e0 + slot))];
+    if constexpr (NV == 4 && sizeof(R) == 4) cig_fields_rounded(f, (float)a.gamma);
+    else Phys::template node<R>(f, a);
+#pragma unroll
+    for (int v = 0; v < NF; ++v) sm[(slot * NF + v) * FS + T::nf(v, n % P, n / P)] = f[v];
+  }
+  __syncthreads();
+  R* trOut = reinterpret_cast<R*>(a.trOut) + (size_t)4 * TS * e0;
+  tile_traces<P, Phys, R>(sm, NF * FS, EPB, live, t, NTH, a, [&](int eE, int fi, int l, bool row, R lo, R hi) {
+    R* o = trOut + 4 * TS * eE + l + P * fi;
+    o[TS * (row ? 3 : 0)] = lo;
+    o[TS * (row ? 1 : 2)] = hi;
+  });
+  if constexpr (Phys::kLaggedVelocity) {
+    __syncthreads();
+    R* vOut = reinterpret_cast<R*>(a.velOut) + (size_t)8 * P * e0;
+    for (int k = t; k < live * 4 * P; k += NTH) {
+      const int es = k / P, ii = k - es * P;  // (element, side)
+      const R* o = trOut + TS * es + ii;
+      const R H = o[2 * P];
+      vOut[2 * P * es + ii] = o[0] / H;
+      vOut[2 * P * es + ii + P] = o[P] / H;
+    }
+  }
+}
+
+template <int P, class Phys, typename R>
+cudaError_t launch_traces(const StageArgs& a, cudaStream_t st) {
+  using B = TraceBlock<P, Phys, R>;
+  k_traces<P, Phys, R><<<(a.nEl + B::elems - 1) / B::elems, B::threads, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
 template <int P, class Phys, typename R, bool kMulti = false>
 __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
     k_fused_stage_tma(const StageArgs a, const TmaPlan pl, const TmaSteps ms) {
@@ -892,7 +960,8 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
           }
         }
         R out[NV];
-        Phys::template face<R>(bcid, physical, L, X, velL, velR, nh.x, nh.y, ns, fx, a, out);
+        Phys::template face<R>(bcid, physical, L, X, velL, velR, nh.x, nh.y, ns, fx,
+                               Phys::template face_constants<R>(fx, a), a, out);
         if constexpr (NV == 4)
           if (a.av) av_face_add<P, R>(a, s1, ii, eF, ssi, nh.x, nh.y, ns, out);
         R* fb = gBase + eC * EB + T::kU;
@@ -958,7 +1027,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
         for (int v = 0; v < NV; ++v) {
           const R dv = d[v] + (bi1 * gfb[1 * SS + v * P + j] + bi0 * gfb[3 * SS + v * P + j]) * rwi +
                        (bj1 * gfb[2 * SS + v * P + i] + bj0 * gfb[0 * SS + v * P + i]) * rwj;
-          dsdt[v] = Src[v] - (double)dv * rJ;
+          dsdt[v] = fma(-(double)dv, rJ, Src[v]);  // (explicit: Src may be a product too)
         }
       }
     }

@@ -10,7 +10,7 @@
 // interpolation and derivative operators take whole planes or elements per
 // block, each input read once from memory; the arithmetic of each output
 // follows the CPU branch of the reference term by term.  The whole-stage
-// kernels (fused_stage_tma.cuh) are the fast path; these
+// kernels (fused_stage_tma.cuh, fused_resident.cuh) are the fast path; these
 // exist so an unmodified SELF caller can use the library operator by operator.
 #include <cuda_runtime.h>
 
@@ -778,7 +778,7 @@ __global__ void k_lsw_riemann(double* __restrict__ flux, const double* __restric
     const long long base = i + (long long)P * nVar * se;
     double out[3];
     lsw_riemann<double>(sol[base], sol[base + P], sol[base + 2 * P], ext[base], ext[base + P], ext[base + 2 * P],
-                        H[k], g, nHat[2 * k], nHat[2 * k + 1], nScale[k], out);
+                        lsw_face<double>(H[k], g), g, nHat[2 * k], nHat[2 * k + 1], nScale[k], out);
     flux[base] = out[0];
     flux[base + P] = out[1];
     flux[base + 2 * P] = out[2];

@@ -38,6 +38,7 @@
 #include <string>
 
 #include "fused_stage.cuh"
+#include "fused_stage_tma.cuh"
 #include "selfgpu_internal.h"
 
 namespace selfgpu {
@@ -83,8 +84,7 @@ cudaError_t launch_pair(StageArgs a, cudaStream_t st) {
   StageArgs t = a;
   t.mode = MODE_TRACES;
   t.trIn = nullptr;
-  k_fused_stage<P, PhysCIG, double, EPB><<<grid, EPB * P * P, 0, st>>>(t);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_traces<P, PhysCIG, double>(t, st);
   if (e != cudaSuccess) return e;
   a.mode = MODE_TENDENCY;
   a.trIn = a.trOut;

@@ -48,17 +48,49 @@ __device__ __forceinline__ void reflect(R u, R v, double n1, double n2, R& ue, R
   ve = (a * a - b * b) * v - (R)2 * a * b * u;
 }
 
+// a b + c d: each product rounded (reference roundings), or the first fused with
+// the rounded second.  Written out where the compiler's own choice of the fused
+// product differed between the kernels that share an expression.
+template <typename R>
+__device__ __forceinline__ R sum_of_products(R a, R b, R c, R d) {
+  if constexpr (ref_rounding<R>()) return a * b + c * d;
+  else if constexpr (sizeof(R) == 8) return __fma_rn(a, b, __dmul_rn(c, d));
+  else return __fmaf_rn(a, b, __fmul_rn(c, d));
+}
+
 // ------------------------------------------------------------ LinearShallowWater
 // Characteristic upwind flux, src/models/SELF_LinearShallowWater.f90:529-551.
+// The wave speed of a face node and, in production FP64, the reciprocals that
+// replace the divisions by g and c do not change from stage to stage.
 template <typename R>
-__device__ __forceinline__ void lsw_riemann(R uL, R vL, R etaL, R uR, R vR, R etaR, R Hb, R g, double n1,
-                                            double n2, double nmag, R out[3]) {
-  const R a = (R)n1, b = (R)n2, s = (R)nmag;
-  const R c = sqrt(g * Hb);
+struct LswFace {
+  R c, rg, rc;
+};
+template <typename R>
+__device__ __forceinline__ LswFace<R> lsw_face(R Hb, R g) {
+  LswFace<R> k;
+  k.c = sqrt(g * Hb);
+  k.rg = k.rc = (R)0;
+  if constexpr (sizeof(R) == 8 && !ref_rounding<R>()) {
+    k.rg = (R)1 / g;
+    k.rc = (R)1 / k.c;
+  }
+  return k;
+}
+template <typename R>
+__device__ __forceinline__ void lsw_riemann(R uL, R vL, R etaL, R uR, R vR, R etaR, const LswFace<R>& k, R g,
+                                            double n1, double n2, double nmag, R out[3]) {
+  const R a = (R)n1, b = (R)n2, s = (R)nmag, c = k.c;
   const R unL = uL * a + vL * b;
   const R unR = uR * a + vR * b;
-  const R wL = (R)0.5 * (unL / g + etaL / c);
-  const R wR = (R)0.5 * (unR / g - etaR / c);
+  R wL, wR;
+  if constexpr (sizeof(R) == 8 && !ref_rounding<R>()) {
+    wL = (R)0.5 * sum_of_products(unL, k.rg, etaL, k.rc);
+    wR = (R)0.5 * sum_of_products(unR, k.rg, -etaR, k.rc);
+  } else {
+    wL = (R)0.5 * (unL / g + etaL / c);
+    wR = (R)0.5 * (unR / g - etaR / c);
+  }
   out[0] = g * c * (wL - wR) * a * s;
   out[1] = g * c * (wL - wR) * b * s;
   out[2] = c * c * (wL + wR) * s;
@@ -71,16 +103,17 @@ template <typename R>
 __device__ __forceinline__ void sw_riemann(R HuL, R HvL, R HL, R HuR, R HvR, R HR, R uL, R vL, R uR, R vR, R g,
                                            double n1, double n2, double nmag, R out[3]) {
   const R a = (R)n1, b = (R)n2, s = (R)nmag;
-  const R unL = uL * a + vL * b;
-  const R unR = uR * a + vR * b;
+  const R unL = sum_of_products(uL, a, vL, b);
+  const R unR = sum_of_products(uR, a, vR, b);
   const R cL = sqrt(g * HL);
   const R cR = sqrt(g * HR);
-  const R fL1 = HuL * unL + g * HL * HL * (R)0.5 * a;
-  const R fL2 = HvL * unL + g * HL * HL * (R)0.5 * b;
-  const R fL3 = HuL * a + HvL * b;
-  const R fR1 = HuR * unR + g * HR * HR * (R)0.5 * a;
-  const R fR2 = HvR * unR + g * HR * HR * (R)0.5 * b;
-  const R fR3 = HuR * a + HvR * b;
+  const R pL = g * HL * HL * (R)0.5, pR = g * HR * HR * (R)0.5;
+  const R fL1 = sum_of_products(HuL, unL, pL, a);
+  const R fL2 = sum_of_products(HvL, unL, pL, b);
+  const R fL3 = sum_of_products(HuL, a, HvL, b);
+  const R fR1 = sum_of_products(HuR, unR, pR, a);
+  const R fR2 = sum_of_products(HvR, unR, pR, b);
+  const R fR3 = sum_of_products(HuR, a, HvR, b);
   const R alpha = fmax(fmax(fabs(unL + cL), fabs(unR + cR)), fmax(fabs(unL - cL), fabs(unR - cR)));
   out[0] = (R)0.5 * (fL1 + fR1 + alpha * (HuL - HuR)) * s;
   out[1] = (R)0.5 * (fL2 + fR2 + alpha * (HvL - HvR)) * s;
@@ -90,10 +123,11 @@ __device__ __forceinline__ void sw_riemann(R HuL, R HvL, R HL, R HuR, R HvR, R H
 // Volume flux, src/models/SELF_ShallowWater.f90:400-441.
 template <typename R>
 __device__ __forceinline__ void sw_flux(R Hu, R Hv, R H, R u, R v, R g, R Fx[3], R Fy[3]) {
-  Fx[0] = u * Hu + (R)0.5 * g * H * H;
+  const R gh = (R)0.5 * g * H;
+  Fx[0] = sum_of_products(u, Hu, gh, H);
   Fy[0] = v * Hu;
   Fx[1] = u * Hv;
-  Fy[1] = v * Hv + (R)0.5 * g * H * H;
+  Fy[1] = sum_of_products(v, Hv, gh, H);
   Fx[2] = Hu;
   Fy[2] = Hv;
 }

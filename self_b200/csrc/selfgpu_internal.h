@@ -45,12 +45,14 @@ cudaError_t launch_stage_fp64_ref(int model, int P, const StageArgs& a, const St
                                   int* usedTma);
 cudaError_t launch_stage_fp32(int model, int P, const StageArgs& a, const StageLaunch& L, cudaStream_t st,
                               int* usedTma);
-// nSteps RK3 steps in one cooperative launch (k_fused_steps), per form
-struct StepsArgs;
-cudaError_t launch_steps_fp64(int model, int P, const StageArgs& a, const StepsArgs& sa, int numSMs, cudaStream_t st);
-cudaError_t launch_steps_fp64_ref(int model, int P, const StageArgs& a, const StepsArgs& sa, int numSMs,
-                                  cudaStream_t st);
-cudaError_t launch_steps_fp32(int model, int P, const StageArgs& a, const StepsArgs& sa, int numSMs, cudaStream_t st);
+// all stages of an rk3 call in one cooperative launch of k_fused_resident, per form
+struct ResidentArgs;
+cudaError_t launch_resident_fp64(int model, int P, const StageArgs& a, ResidentArgs& ra, const StageLaunch& L,
+                                 cudaStream_t st);
+cudaError_t launch_resident_fp64_ref(int model, int P, const StageArgs& a, ResidentArgs& ra, const StageLaunch& L,
+                                     cudaStream_t st);
+cudaError_t launch_resident_fp32(int model, int P, const StageArgs& a, ResidentArgs& ra, const StageLaunch& L,
+                                 cudaStream_t st);
 // several RK stages in one cooperative launch of the persistent kernel
 // (k_fused_stage_tma<..., true>; cudaErrorNotSupported where it does not apply)
 struct TmaSteps;

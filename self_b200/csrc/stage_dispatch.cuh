@@ -12,6 +12,7 @@
 
 #include "fused_stage.cuh"
 #include "fused_stage_tma.cuh"
+#include "fused_resident.cuh"
 #include "selfgpu_internal.h"
 
 namespace selfgpu {
@@ -30,7 +31,8 @@ inline bool aligned16(const void* p) { return ((uintptr_t)p % 16) == 0; }
 template <int P, class Phys, typename R>
 cudaError_t launch_one(const StageArgs& a, const StageLaunch& L, cudaStream_t st, int* usedTma) {
   *usedTma = 0;
-  bool ok = L.allowTma && a.mode != MODE_TRACES && a.geo != nullptr && aligned16(a.geo) && aligned16(a.q) &&
+  if (a.mode == MODE_TRACES) return launch_traces<P, Phys, R>(a, st);
+  bool ok = L.allowTma && a.geo != nullptr && aligned16(a.geo) && aligned16(a.q) &&
             aligned16(sizeof(R) == 4 ? (const void*)a.Gf : (const void*)a.G) && aligned16(a.trIn) &&
             (a.velIn == nullptr || aligned16(a.velIn));
   for (int k = 0; k < 5; ++k) ok = ok && (a.fld[k] == nullptr || aligned16(a.fld[k]));
@@ -162,44 +164,69 @@ cudaError_t launch_P(int P, const StageArgs& a, const StageLaunch& L, cudaStream
   }
 }
 
-// One cooperative launch of k_fused_steps; cudaErrorCooperativeLaunchTooLarge
-// when the element groups do not fit one wave of resident CTAs.
+// All stages of an rk3 call in one cooperative launch of k_fused_resident with
+// ra.tiles tiles per CTA.  With ra.tiles = 0 nothing is launched: ra.tiles is
+// set to the fewest tiles per CTA with which the mesh fits resident CTAs, and
+// cudaErrorCooperativeLaunchTooLarge returned when there is none.
 template <int P, class Phys, typename R>
-cudaError_t launch_steps_one(const StageArgs& a, const StepsArgs& sa, int numSMs, cudaStream_t st) {
-  constexpr int EPB = elems_per_block<P, Phys, R>();
-  const int grid = (a.nEl + EPB - 1) / EPB;
-  int perSM = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_fused_steps<P, Phys, R, EPB>, EPB * P * P, 0);
-  if (e != cudaSuccess) return e;
-  if ((long long)perSM * numSMs < grid) return cudaErrorCooperativeLaunchTooLarge;
-  StageArgs aa = a;
-  StepsArgs ss = sa;
-  void* args[] = {&aa, &ss};
-  return cudaLaunchCooperativeKernel((const void*)k_fused_steps<P, Phys, R, EPB>, dim3(grid), dim3(EPB * P * P),
-                                     args, 0, st);
+cudaError_t launch_resident_one(const StageArgs& a, ResidentArgs& ra, const StageLaunch& L, cudaStream_t st) {
+  using T = TmaTraits<P, Phys, R>;
+  using X = ResTraits<P, Phys, R>;
+  const long long total = ((long long)a.nEl + T::EPG - 1) / T::EPG;
+  auto one = k_fused_resident<P, Phys, R, false>;
+  auto many = k_fused_resident<P, Phys, R, true>;
+  if (ra.tiles == 0) {
+    int nb = 0;
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, one, T::TPE, 0);
+    if (e != cudaSuccess) return e;
+    if (total <= (long long)nb * L.numSMs) {
+      ra.tiles = 1;
+      return cudaSuccess;
+    }
+    e = cudaFuncSetAttribute(many, cudaFuncAttributeMaxDynamicSharedMemorySize, resident_tiles<P, Phys, R>() * X::tileBytes);
+    for (int k = 2; k <= resident_tiles<P, Phys, R>() && e == cudaSuccess; ++k) {
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, many, T::TPE, (size_t)k * X::tileBytes);
+      if (e == cudaSuccess && (total + k - 1) / k <= (long long)nb * L.numSMs) {
+        ra.tiles = k;
+        return cudaSuccess;
+      }
+    }
+    return e != cudaSuccess ? e : cudaErrorCooperativeLaunchTooLarge;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((total + ra.tiles - 1) / ra.tiles));
+  cfg.blockDim = dim3(T::TPE);
+  cfg.dynamicSmemBytes = ra.tiles > 1 ? (size_t)ra.tiles * X::tileBytes : 0;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;  // all CTAs resident: the exchange waits need it
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, ra.tiles > 1 ? many : one, a, ra);
 }
 
 template <class Phys, typename R>
-cudaError_t launch_steps_P(int P, const StageArgs& a, const StepsArgs& sa, int numSMs, cudaStream_t st) {
+cudaError_t launch_resident_P(int P, const StageArgs& a, ResidentArgs& ra, const StageLaunch& L, cudaStream_t st) {
   switch (P) {
-    case 2: return launch_steps_one<2, Phys, R>(a, sa, numSMs, st);
-    case 3: return launch_steps_one<3, Phys, R>(a, sa, numSMs, st);
-    case 4: return launch_steps_one<4, Phys, R>(a, sa, numSMs, st);
-    case 5: return launch_steps_one<5, Phys, R>(a, sa, numSMs, st);
-    case 6: return launch_steps_one<6, Phys, R>(a, sa, numSMs, st);
-    case 7: return launch_steps_one<7, Phys, R>(a, sa, numSMs, st);
-    case 8: return launch_steps_one<8, Phys, R>(a, sa, numSMs, st);
+    case 2: return launch_resident_one<2, Phys, R>(a, ra, L, st);
+    case 3: return launch_resident_one<3, Phys, R>(a, ra, L, st);
+    case 4: return launch_resident_one<4, Phys, R>(a, ra, L, st);
+    case 5: return launch_resident_one<5, Phys, R>(a, ra, L, st);
+    case 6: return launch_resident_one<6, Phys, R>(a, ra, L, st);
+    case 7: return launch_resident_one<7, Phys, R>(a, ra, L, st);
+    case 8: return launch_resident_one<8, Phys, R>(a, ra, L, st);
     default: return cudaErrorInvalidValue;
   }
 }
 
 template <typename R>
-cudaError_t launch_steps_impl(int model, int P, const StageArgs& a, const StepsArgs& sa, int numSMs,
-                              cudaStream_t st) {
+cudaError_t launch_resident_impl(int model, int P, const StageArgs& a, ResidentArgs& ra, const StageLaunch& L,
+                                 cudaStream_t st) {
   switch (model) {
-    case SELFGPU_MODEL_LSW: return launch_steps_P<PhysLSW, R>(P, a, sa, numSMs, st);
-    case SELFGPU_MODEL_SW: return launch_steps_P<PhysSW, R>(P, a, sa, numSMs, st);
-    case SELFGPU_MODEL_CIG: return launch_steps_P<PhysCIG, R>(P, a, sa, numSMs, st);
+    case SELFGPU_MODEL_LSW: return launch_resident_P<PhysLSW, R>(P, a, ra, L, st);
+    case SELFGPU_MODEL_SW: return launch_resident_P<PhysSW, R>(P, a, ra, L, st);
+    case SELFGPU_MODEL_CIG: return launch_resident_P<PhysCIG, R>(P, a, ra, L, st);
     default: return cudaErrorInvalidValue;
   }
 }

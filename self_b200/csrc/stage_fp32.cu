@@ -12,8 +12,9 @@ cudaError_t launch_stage_fp32(int model, int P, const StageArgs& a, const StageL
 cudaError_t launch_av_prep_fp32(int P, const AvArgs& a, cudaStream_t st, int numSMs, bool formNu) {
   return launch_av_prep_impl<float>(P, a, st, numSMs, formNu);
 }
-cudaError_t launch_steps_fp32(int model, int P, const StageArgs& a, const StepsArgs& sa, int numSMs, cudaStream_t st) {
-  return launch_steps_impl<float>(model, P, a, sa, numSMs, st);
+cudaError_t launch_resident_fp32(int model, int P, const StageArgs& a, ResidentArgs& ra, const StageLaunch& L,
+                                 cudaStream_t st) {
+  return launch_resident_impl<float>(model, P, a, ra, L, st);
 }
 cudaError_t launch_stages_tma_fp32(int model, int P, const StageArgs& a, const StageLaunch& L, const TmaSteps& ms,
                                   cudaStream_t st) {

@@ -12,8 +12,9 @@ cudaError_t launch_stage_fp64(int model, int P, const StageArgs& a, const StageL
                               int* usedTma) {
   return launch_stage_impl<double>(model, P, a, L, st, usedTma);
 }
-cudaError_t launch_steps_fp64(int model, int P, const StageArgs& a, const StepsArgs& sa, int numSMs, cudaStream_t st) {
-  return launch_steps_impl<double>(model, P, a, sa, numSMs, st);
+cudaError_t launch_resident_fp64(int model, int P, const StageArgs& a, ResidentArgs& ra, const StageLaunch& L,
+                                 cudaStream_t st) {
+  return launch_resident_impl<double>(model, P, a, ra, L, st);
 }
 cudaError_t launch_stages_tma_fp64(int model, int P, const StageArgs& a, const StageLaunch& L, const TmaSteps& ms,
                                   cudaStream_t st) {

@@ -69,6 +69,91 @@ def test_odd_node_counts_run_the_persistent_kernel(model, N, nx, ny, form):
     _check(S.to_host(mod.solution).reshape(q.shape, order="F"), ref.get("solution", q.shape), form)
 
 
+@pytest.mark.parametrize("form", [0, 2])
+@pytest.mark.parametrize("model", ["LSW", "SW", "CIG"])
+@pytest.mark.parametrize("N", [2, 3, 4, 5, 6, 7])
+@pytest.mark.parametrize("kind", ["single", "torus", "flipped", "ring", "radiation"])
+def test_resident_launch_matches_the_oracle(model, N, kind, form):
+    """An rk3 call of a small mesh is one launch; over calls of several lengths (odd and even stage counts, stale and
+    cached traces) it equals the oracle."""
+    import self_b200 as S
+    if kind == "radiation" and model == "CIG":
+        pytest.skip("zero exterior density")
+    ref, mod, q = _pair(model, C.mesh_kwargs(kind), N, form)
+    dt = 2e-4
+    for n in (1, 2, 3):
+        l0 = mod.LaunchCount()
+        mod.ForwardStep(n, dt)
+        assert mod.LaunchCount() - l0 == 1
+        ref.rk3(n, dt)
+    mod.Sync()
+    _check(S.to_host(mod.solution).reshape(q.shape, order="F"), ref.get("solution", q.shape), form)
+
+
+@pytest.mark.parametrize("form_name", ["FP64", "FP64_REF", "FP32_BULK"])
+@pytest.mark.parametrize("model,N,nx", [("CIG", 7, 33), ("CIG", 7, 52), ("SW", 7, 52), ("LSW", 5, 61), ("SW", 3, 70),
+                                        ("CIG", 4, 60), ("SW", 6, 45)])
+def test_resident_launch_equals_stage_launches(model, N, nx, form_name):
+    """One and several tiles per CTA: the solution and the register of the stage launches bit for bit, with a common
+    and with per-element time steps, a tendency between the calls."""
+    import self_b200 as S
+    out = []
+    for pinned in (False, True):
+        _, mod, q = _pair(model, dict(nx=nx, ny=nx - 2, periodic=(True, False), bcid=O.BC_NONORMALFLOW, amp=0.02), N,
+                          getattr(S, form_name))
+        if pinned:
+            S.check(S.lib().selfgpu_model2d_set_launch(mod._h, 1, 0))
+            S.check(S.lib().selfgpu_model2d_set_multistage(mod._h, 0))
+        l0 = mod.LaunchCount()
+        mod.ForwardStep(2, 1e-5)
+        assert pinned or mod.LaunchCount() - l0 == 1
+        mod.CalculateTendency()
+        mod._set_field("elementDt", 1e-5 * (1.0 + 0.5 * torch.sin(torch.arange(mod.nElem, device="cuda").double())))
+        mod.ForwardStep(3, 0.0)
+        mod.Sync()
+        out.append((mod.solution.clone(), mod.workSol.clone(), mod.CalculateTendency().clone()))
+    assert torch.isfinite(out[0][0]).all()
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
+
+
+def test_resident_exchange_wait_is_bounded():
+    """One CTA publishes no traces: its neighbours' waits run out, sync reports it, and the handle then runs again."""
+    import self_b200 as S
+    L = S.lib()
+    _, mod, q = _pair("CIG", C.mesh_kwargs("periodic"), 7, S.FP64)
+    assert L.selfgpu_model2d_set_wait_limit(mod._h, 20_000_000) == 0  # ~10 ms
+    assert L.selfgpu_model2d_inject_stall(mod._h, 2) == 0
+    mod.ForwardStep(2, 1e-4)
+    with pytest.raises(S.SelfGpuError) as ei:
+        mod.Sync()
+    assert ei.value.code == 6
+    assert L.selfgpu_model2d_inject_stall(mod._h, 0) == 0
+    ref, _, _ = _pair("CIG", C.mesh_kwargs("periodic"), 7, S.FP64)
+    mod.SetSolution(q)
+    mod.ForwardStep(3, 1e-4)
+    mod.Sync()
+    ref.rk3(3, 1e-4)
+    _check(S.to_host(mod.solution).reshape(q.shape, order="F"), ref.get("solution", q.shape), S.FP64)
+
+
+def test_one_sided_neighbours_keep_stage_launches():
+    """A mesh whose sideInfo names a neighbour that does not name it back: no exchange of published traces."""
+    import self_b200 as S
+    m = S.Mesh2D(4, 3, periodic=(True, True))
+    si = m.sideInfo.copy(order="F")
+    si[2, 1, 0], si[3, 1, 0] = 7, 41  # east side of element 1: the west side of element 7 (not its true neighbour)
+    mesh = S.Mesh2D.from_arrays(m.nodeCoords, si)
+    mod = S.CompressibleIdealGas2D(mesh, S.SEMQuad(S.Lagrange(5, S.GAUSS, 5, S.UNIFORM), mesh))
+    q = torch.ones_like(mod.solution)
+    q[:, 3] = 3.0
+    mod.SetSolution(q)
+    l0 = mod.LaunchCount()
+    mod.ForwardStep(2, 1e-5)
+    mod.Sync()
+    assert mod.LaunchCount() - l0 == 1 + 6
+
+
 @pytest.mark.parametrize("N", [2, 3, 6, 7, 8, 10])
 @pytest.mark.parametrize("nVar,nEl", [(1, 1), (3, 5), (2, 131)])
 def test_plane_operators_match_the_oracle(N, nVar, nEl):
