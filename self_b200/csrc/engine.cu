@@ -247,7 +247,7 @@ struct selfgpu_model2d {
   int* derr = nullptr;  // error word of the persistent kernel's bounded waits
   long long launches = 0;
   long long tmaLaunches = 0;
-  StageLaunch cfg{true, 0, 148, 0};
+  StageLaunch cfg{true, 0, 148, 0, 0};
   // graph cache: one captured RK step per starting buffer parity
   cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
   long long graphTma[2][2] = {{0, 0}, {0, 0}};
@@ -560,6 +560,7 @@ int selfgpu_model2d_create(selfgpu_model2d** out, int model, int N, int nEl, int
   }
   cudaDeviceGetAttribute(&m->cfg.smemOptin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   cudaDeviceGetAttribute(&m->cfg.numSMs, cudaDevAttrMultiProcessorCount, dev);
+  cudaDeviceGetAttribute(&m->cfg.l2Bytes, cudaDevAttrL2CacheSize, dev);
   // one (element, side) block holds NT fields x P nodes, padded to 16 bytes
   // (trace_side_stride in fused_stage.cuh)
   e = m->alloc_caches();

@@ -61,6 +61,9 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
       "l"(src), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
 }
+__device__ __forceinline__ void prefetch_l2(const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void named_bar(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
@@ -84,6 +87,7 @@ __device__ __forceinline__ bool wait_at_least(const unsigned* p, unsigned v, lon
 // of the CTA's shared memory.  Built on the host by make_tma_plan().
 struct TmaPlan {
   int groups;      // consumer groups per CTA
+  int prefetch;    // fetch each tile's RK register into L2 with its copies
   int slotBytes;   // bytes of one element buffer
   int oQ, oDsdx, oNhat, oNs, oJ, oSi, oOwn;  // oDsdx..oSi lie in the packed geometry record
   int oX[5];       // model fields: LSW (H, Hb, fC), SW (topoB, grad), CIG (envG, drag, presc x3 -> oX[2..4])
@@ -562,6 +566,16 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
   // at P = 6, every model at P = 4)
   constexpr bool kNbrEarly =
       (P == 8) ? !(NV == 4 && ref_rounding<R>()) : (P == 6 && kSW && sizeof(R) == 8);
+  // The RK register's tile requested into L2 two tiles ahead of its use, so
+  // that phase D's loads wait for L2 and not for HBM.  At P = 8 and 6 in the
+  // production and FP32-bulk forms, and only where the stage's data exceed L2
+  // (us per stage, without -> with: 256x256 CompressibleIdealGas2D P = 8 FP64
+  // 175.9 -> 172.5, FP32 133.6 -> 129.4, ShallowWater P = 8 FP32 111.7 ->
+  // 105.4, P = 6 FP32 90.5 -> 83.4; on 96x96, where they fit, 1-4 % slower;
+  // P = 4 within 1 %; the reference-rounding kernels 3 % slower).  Loading the
+  // register into the node threads' registers before the face phase instead was
+  // slower (ShallowWater P = 8 FP32 117.6 us).
+  constexpr bool kPrefetch = (P == 8 || P == 6) && !ref_rounding<R>();
   auto f0at = [](int m, int j) { return T::f0at(m, j); };
   auto f1at = [](int i, int j) { return T::f1at(i, j); };
   auto dgat = [](int m, int i) { return T::dgat(m, i); };
@@ -679,6 +693,11 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
     if (a.debugStarve == 1 && blockIdx.x == 0 && k == 0) return;
     const R* trIn = reinterpret_cast<const R*>(cache_of(ms.tr, ms.cur0, st, a.trIn));
     copy(sl + pl.oQ, a.q + (size_t)e * NV * PP, nl * qb);
+    if constexpr (kPrefetch)
+      if (pl.prefetch && rk) {  // the register, which the node threads load themselves in phase D
+        if constexpr (sizeof(R) == 4) prefetch_l2(a.Gf + (size_t)e * NV * PP, nl * NV * PP * 4);
+        else prefetch_l2(a.G + (size_t)e * NV * PP, nl * NV * PP * 8);
+      }
     bulk_g2s(sl + pl.oDsdx, reinterpret_cast<const unsigned char*>(a.geo) + (size_t)e * gb, nl * gb, bar);
     bulk_g2s(sl + pl.oOwn, trIn + (size_t)4 * TS * e, nl * ob, bar);
     if constexpr (kSW)
@@ -1093,7 +1112,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
 
 // Host-side plan for k_fused_stage_tma given the smem budget.
 template <int P, class Phys, typename R>
-inline bool make_tma_plan(const StageArgs& a, int smemLimit, TmaPlan& pl, int maxGroups = 0) {
+inline bool make_tma_plan(const StageArgs& a, int smemLimit, long long l2Bytes, TmaPlan& pl, int maxGroups = 0) {
   using T = TmaTraits<P, Phys, R>;
   constexpr int PP = T::PP, NV = T::NV, TS = T::TS, EPG = T::EPG;
   constexpr bool kLSW = (NV == 3 && !Phys::kLaggedVelocity);
@@ -1129,6 +1148,9 @@ inline bool make_tma_plan(const StageArgs& a, int smemLimit, TmaPlan& pl, int ma
     if (a.fld[2])
       for (int x = 2; x < 5; ++x) pl.oX[x] = put(16 * P * 8);
   }
+  // one stage's data: the tiles' copies, the register, and the traces written
+  pl.prefetch =
+      (long long)a.nEl * (o / EPG + NV * PP * (int)sizeof(R) + 4 * TS * (int)sizeof(R)) > l2Bytes ? 1 : 0;
   pl.slotBytes = (o + 127) / 128 * 128;
   pl.groupBytes = T::groupBytes;
   const int cMax = (maxGroups > 0 && maxGroups < T::kMaxGroups) ? maxGroups : T::kMaxGroups;

@@ -32,6 +32,7 @@ struct StageLaunch {
   int smemOptin;   // opt-in shared memory per block (bytes)
   int numSMs;
   int maxGroups;   // cap on the persistent kernel's consumer groups (0 = as many as fit)
+  int l2Bytes;     // the device's L2
 };
 }  // namespace selfgpu
 

@@ -37,7 +37,7 @@ cudaError_t launch_one(const StageArgs& a, const StageLaunch& L, cudaStream_t st
             (a.velIn == nullptr || aligned16(a.velIn));
   for (int k = 0; k < 5; ++k) ok = ok && (a.fld[k] == nullptr || aligned16(a.fld[k]));
   TmaPlan pl{};
-  if (ok && make_tma_plan<P, Phys, R>(a, L.smemOptin, pl, L.maxGroups)) {
+  if (ok && make_tma_plan<P, Phys, R>(a, L.smemOptin, L.l2Bytes, pl, L.maxGroups)) {
     // the shared-memory opt-in is per device: one bit per device that has it
     static std::atomic<unsigned long long> attrSet{0};  // one instantiation per (P, Phys, R)
     int dev = 0;
@@ -93,7 +93,7 @@ cudaError_t launch_stages_tma_one(const StageArgs& a, const StageLaunch& L, TmaS
               (ms.vel[1] == nullptr || aligned16(ms.vel[1])) && a.av == 0 && a.debugStarve != 1;
     for (int k = 0; k < 5; ++k) ok = ok && (a.fld[k] == nullptr || aligned16(a.fld[k]));
     TmaPlan pl{};
-    if (!ok || !make_tma_plan<P, Phys, R>(a, L.smemOptin, pl, L.maxGroups)) return cudaErrorNotSupported;
+    if (!ok || !make_tma_plan<P, Phys, R>(a, L.smemOptin, L.l2Bytes, pl, L.maxGroups)) return cudaErrorNotSupported;
     using T = TmaTraits<P, Phys, R>;
     const long long tiles = ((long long)a.nEl + T::EPG - 1) / T::EPG;
     const int grid = tiles < L.numSMs ? (int)tiles : L.numSMs;
