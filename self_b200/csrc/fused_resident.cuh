@@ -115,10 +115,12 @@ struct ResTraits {
   using T = TmaTraits<P, Phys, R>;
   using Pub = typename std::conditional<sizeof(R) == 8, Pub64, Pub32>::type;
   // node fields apart from the fluxes (a thread writes its next flux while
-  // others still form traces), then (one tile per CTA) the tile's own traces
-  static constexpr int oFields = T::EPG * (T::EB + T::kDiv);
-  static constexpr int FB = T::NF * T::FS, OB = 4 * T::NT * P;  // per element
-  static constexpr int oOwn = oFields + T::EPG * FB;
+  // others still form traces; within the element's arrays where TmaTraits keeps
+  // them apart already), then (one tile per CTA) the tile's own traces
+  static constexpr int arrays = T::EPG * (T::EB + T::kDiv);
+  static constexpr int oFields = T::kSep ? T::oN : arrays;
+  static constexpr int FB = T::kSep ? T::EB : T::NF * T::FS, OB = 4 * T::NT * P;  // per element
+  static constexpr int oOwn = arrays + (T::kSep ? 0 : T::EPG * FB);
   static constexpr int values(bool many) { return oOwn + (many ? 0 : T::EPG * OB); }
   // 128 registers per thread: the node state of a tile is about 50
   static constexpr int kMinCtas = 65536 / (128 * T::TPE) > 1 ? 65536 / (128 * T::TPE) : 1;

@@ -203,9 +203,33 @@ struct TmaTraits {
   static constexpr bool kSwz = (P == 8);
   static constexpr int RS = (kSwz || kOdd) ? P : P + 1;
   static constexpr int FS = kSwz ? PP + 8 : P * RS;
-  static constexpr int kU = (NF * FS > 2 * NV * PP) ? NF * FS : 2 * NV * PP;  // node fields alias the fluxes
+  // Node fields: over the fluxes, or (kSep) in an array of their own.  Apart,
+  // a thread may write its node's fields while others still read the fluxes and
+  // its next fluxes while others still form traces, which saves two of a tile's
+  // five group barriers; the larger elements leave room for fewer groups.
+  // us per stage on 256x256, together -> apart: P = 6 CompressibleIdealGas2D
+  // FP64 141 -> 135.5, FP32 113.6 -> 109, reference rounding 150 -> 137,
+  // ShallowWater FP64 103 -> 97, LinearShallowWater 94.4 -> 92.7; P = 7 FP32
+  // 177 -> 165, reference 280 -> 265, LinearShallowWater FP64 144 -> 134, but
+  // production ShallowWater 158 -> 170 and CompressibleIdealGas2D 195 -> 197;
+  // P = 5 FP32 102 -> 96, reference 145 -> 137, production FP64 96x96 17.9 ->
+  // 19.8; P = 3 within 2 % but for FP32 CompressibleIdealGas2D (48 -> 45); P = 8
+  // loses more groups than the barriers cost.
+  static constexpr bool kProd = sizeof(R) == 8 && !ref_rounding<R>();
+  static constexpr bool kSep = P == 6 || (P == 5 && !kProd) ||
+                               (P == 7 && (!kProd || (NV == 3 && !Phys::kLaggedVelocity)));
+  static constexpr int kU = (!kSep && NF * FS > 2 * NV * PP) ? NF * FS : 2 * NV * PP;
   static constexpr int SS = side_stride(NV * P, (int)sizeof(R));
-  static constexpr int EB = kU + 4 * SS;
+  static constexpr int EB = kU + 4 * SS + (kSep ? NF * FS : 0);
+  static constexpr int oN = kSep ? kU + 4 * SS : 0;  // node fields within an element's arrays
+  // Every thread waits for the tile's copies itself (instead of thread 0 for
+  // the group): with kSep there is no barrier to wait at, and at P = 4 a
+  // one-warp group that one lane waited for ran its lanes apart afterwards
+  // (256x256, one -> all: reference rounding CompressibleIdealGas2D 185 -> 95,
+  // ShallowWater 125 -> 65, LinearShallowWater 112 -> 60 us; production FP64
+  // 74.3 -> 72.9, 54.3 -> 54.0, 47.7 -> 47.6; FP32 CompressibleIdealGas2D
+  // 55.0 -> 57.4, so one lane there).
+  static constexpr bool kAllWait = kSep || (P == 4 && sizeof(R) == 8);
   static constexpr int kDiv = (EPG > 1 && !kOdd) ? NV * PP : 0;  // separate divergence sums per element
   static constexpr int groupBytes = (int)(((EPG * (EB + kDiv)) * sizeof(R) + 127) / 128 * 128);
   // Weak-divergence volume sums: one thread per 2x2 block of nodes and pair
@@ -604,6 +628,8 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
     sb[k] = a.bM[k];
     if constexpr (sizeof(R) == 4) sbR[k] = a.bMf[k];
   }
+  if (T::kAllWait)
+    for (int k = threadIdx.x; k < C; k += blockDim.x) gflag[k] = 1;
   for (int k = threadIdx.x; k < P; k += blockDim.x) {
     sqw[k] = a.qw[k];
     sqwr[k] = 1.0 / a.qw[k];
@@ -677,15 +703,20 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
     unsigned char* sl = slots + (size_t)(2 * g + buf) * pl.slotBytes;
     uint64_t* bar = &full[2 * g + buf];
     // An odd number of elements of odd P (the last tile of a mesh) leaves a
-    // piece 8 bytes short of a multiple of 16: this thread, which also waits
-    // for the copies, then moves the last value itself.
+    // piece 8 bytes short of a multiple of 16: this thread then moves the last
+    // value itself.
     auto whole = [&](uint32_t n) { return T::kOdd ? n & ~15u : n; };
-    auto copy = [&](unsigned char* dst, const void* src, uint32_t n) {
-      bulk_g2s(dst, src, whole(n), bar);
-      if (T::kOdd && (n & 8))
-        *reinterpret_cast<double*>(dst + whole(n)) =
-            *reinterpret_cast<const double*>(reinterpret_cast<const unsigned char*>(src) + whole(n));
-    };
+    auto copy = [&](unsigned char* dst, const void* src, uint32_t n) { bulk_g2s(dst, src, whole(n), bar); };
+    if (T::kOdd && (nl & 1)) {  // before the arrival on the barrier, which releases the stores
+      auto tail = [&](unsigned char* dst, const double* src, uint32_t n) {
+        if (n & 8) *reinterpret_cast<double*>(dst + whole(n)) = src[n / 8 - 1];
+      };
+      tail(sl + pl.oQ, a.q + (size_t)e * NV * PP, nl * qb);
+      if constexpr (kLSW) {
+        tail(sl + pl.oX[0], a.fld[0] + (size_t)e * PP, nl * xb[0]);
+        if (xb[2]) tail(sl + pl.oX[2], a.fld[2] + (size_t)e * PP, nl * xb[2]);
+      }
+    }
     uint32_t bytes = nl * (gb + ob + vb) + whole(nl * qb);
 #pragma unroll
     for (int x = 0; x < 5; ++x) bytes += whole(nl * xb[x]);
@@ -706,7 +737,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
                bar);
     if constexpr (kLSW) {
       copy(sl + pl.oX[0], a.fld[0] + (size_t)e * PP, nl * xb[0]);
-      copy(sl + pl.oX[1], a.fld[1] + (size_t)e * 4 * P, nl * xb[1]);
+      bulk_g2s(sl + pl.oX[1], a.fld[1] + (size_t)e * 4 * P, nl * xb[1], bar);
       if (xb[2]) copy(sl + pl.oX[2], a.fld[2] + (size_t)e * PP, nl * xb[2]);
     } else if constexpr (kSW) {
       if (xb[0]) bulk_g2s(sl + pl.oX[0], a.fld[0] + (size_t)e * 4 * P, nl * xb[0], bar);
@@ -750,6 +781,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
   const int faceWarp = (EPG == 1 && TPE >= 64) ? ((g >> 1) & 1) : 0;
   R* gBase = reinterpret_cast<R*>(smem + pl.oGroups + (size_t)g * pl.groupBytes);
   R* gU = gBase + ee * EB;      // this thread's element: fluxes, later node fields
+  R* gN = gU + T::oN;           // node fields
   R* gF1 = gU + NV * PP;        // eta flux [NV][P][P]
   R* gfb = gU + T::kU;          // [4][SS]: [NV][P] per side
   R* gD = T::kDiv ? gBase + EPG * EB + ee * NV * PP : gU;  // divergence sums
@@ -785,9 +817,16 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
     const int buf = (int)(w & 1);
     const uint32_t par = (uint32_t)((w >> 1) & 1);
     const unsigned char* sl = slots + (size_t)(2 * g + buf) * pl.slotBytes;
-    if (t == 0) gflag[g] = mbar_wait(&full[2 * g + buf], par, a.waitCycles) ? 1 : 0;
-    group_bar();
-    if (!gflag[g]) {
+    bool copied = true;  // (kAllWait: as this thread saw it; the group agrees at its next barrier)
+    if constexpr (T::kAllWait) {
+      copied = mbar_wait(&full[2 * g + buf], par, a.waitCycles);
+      if (!copied) gflag[g] = 0;
+      if constexpr (!T::kSep) group_bar();
+    } else {
+      if (t == 0) gflag[g] = mbar_wait(&full[2 * g + buf], par, a.waitCycles) ? 1 : 0;
+      group_bar();
+    }
+    auto give_up = [&]() {
       if (t == 0) {
         if (a.err) atomicExch(a.err, 1);
         // Wait (bounded) once more for this buffer's copies and for those of
@@ -795,6 +834,9 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
         mbar_wait(&full[2 * g + buf], par, a.waitCycles);
         if (w + 1 < nItems) mbar_wait(&full[2 * g + (buf ^ 1)], (uint32_t)(((w + 1) >> 1) & 1), a.waitCycles);
       }
+    };
+    if (!T::kSep && !gflag[g]) {
+      give_up();
       break;
     }
     const unsigned char* rec = sl + pl.oDsdx + (size_t)ee * gb;  // this thread's element's geometry record
@@ -854,14 +896,14 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
         }
     };
     if constexpr (kNbrEarly)
-      if (faceOn && !gridWait) load_neighbour();
+      if (faceOn && !gridWait && copied) load_neighbour();
 
     // ---- A: flux auxiliaries, contravariant flux.  The buffer stays valid
     // until the end of phase D, so the solution, J and the node auxiliaries
     // are read again where they are needed instead of living in registers
     // across the face phase.
     R f[NF];
-    if (active) {
+    if (active && copied) {
 #pragma unroll
       for (int v = 0; v < NV; ++v) f[v] = (R)sq[n + PP * v];
       T::flux_fields(f, a);
@@ -895,6 +937,10 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
       }
     }
     group_bar();  // contravariant fluxes ready
+    if (T::kSep && !gflag[g]) {
+      give_up();
+      break;
+    }
 
     // ---- B (alongside the face phase C): weak-divergence volume sums
     tile_volume_sums<P, Phys, R>(gBase, sdg, t, faceWarp, nLive);
@@ -1050,11 +1096,15 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
         }
       }
     }
-    group_bar();  // every thread is done reading the flux arrays and the buffer
-    if (t == 0) {  // refill the buffer: generic-proxy reads before the async-proxy writes
+    auto refill = [&]() {  // the buffer: generic-proxy reads before the async-proxy writes
+      if (t != 0) return;
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       if (!kMulti || jj + 2 < nMineG) issue(w + 2, st, jj + 2);
       else issue(w + 2, st + 1, jj + 2 - nMineG);
+    };
+    if (!T::kSep || !rk) {
+      group_bar();  // every thread is done reading the flux arrays and the buffer
+      refill();
     }
     if (!rk) {
       if (active)
@@ -1076,16 +1126,17 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
       }
       Phys::template node<R>(f, a);
 #pragma unroll
-      for (int v = 0; v < NF; ++v) gU[v * FS + T::nf(v, i, j)] = f[v];
+      for (int v = 0; v < NF; ++v) gN[v * FS + T::nf(v, i, j)] = f[v];
     }
     group_bar();
+    if constexpr (T::kSep) refill();
 
     // ---- E: traces of the updated solution -> trace cache.  (A one-element
     // group's face warp starts one warp later, so the other warp takes the
     // last, partial round.)
     {
       const int k0 = (EPG == 1) ? (faceWarp ? t : (t + 32) % TPE) : t;
-      tile_traces<P, Phys, R>(gBase, EB, EPG, nLive, k0, TPE, a, [&](int eE, int fi, int l, bool row, R lo, R hi) {
+      tile_traces<P, Phys, R>(gBase + T::oN, EB, EPG, nLive, k0, TPE, a, [&](int eE, int fi, int l, bool row, R lo, R hi) {
         R* o = trOut + (size_t)4 * TS * (e0 + eE);
         o[l + P * fi + TS * (row ? 3 : 0)] = lo;
         o[l + P * fi + TS * (row ? 1 : 2)] = hi;
