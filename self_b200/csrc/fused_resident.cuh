@@ -119,7 +119,7 @@ struct ResTraits {
   // them apart already), then (one tile per CTA) the tile's own traces
   static constexpr int arrays = T::EPG * (T::EB + T::kDiv);
   static constexpr int oFields = T::kSep ? T::oN : arrays;
-  static constexpr int FB = T::kSep ? T::EB : T::NF * T::FS, OB = 4 * T::NT * P;  // per element
+  static constexpr int FB = T::kSep ? T::EB : T::NT * T::FS, OB = 4 * T::NT * P;  // per element
   static constexpr int oOwn = arrays + (T::kSep ? 0 : T::EPG * FB);
   static constexpr int values(bool many) { return oOwn + (many ? 0 : T::EPG * OB); }
   // 128 registers per thread: the node state of a tile is about 50
@@ -274,17 +274,17 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::TPE, ResTraits<P, Phys,
   // node fields of the solution q -> shared memory (first: of a solution set
   // from outside, rounded as k_traces does)
   auto put_fields = [&](bool first) {
-    R f[NF];
+    R f[NT];
 #pragma unroll
     for (int v = 0; v < NV; ++v) f[v] = (R)q[v];
     if constexpr (NV == 4 && sizeof(R) == 4) {
       if (first) cig_fields_rounded(f, (float)a.gamma);
-      else Phys::template node<R>(f, a);
+      else T::trace_fields(f, a);
     } else {
-      Phys::template node<R>(f, a);
+      T::trace_fields(f, a);
     }
 #pragma unroll
-    for (int v = 0; v < NF; ++v) gN[v * FS + T::nf(v, i, j)] = f[v];
+    for (int v = 0; v < NT; ++v) gN[v * FS + T::nf(v, i, j)] = f[v];
   };
   // traces of the node fields: published as `set` (and, one tile per CTA, kept
   // for the tile's own faces), or (last) written to the trace cache
@@ -447,6 +447,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::TPE, ResTraits<P, Phys,
         if constexpr (kSW) {
           // the next stage's are this stage's traces' (and, after SetSolution,
           // the first stage's too); walls keep velR = 0
+          constexpr bool kDivide = ref_rounding<R>() || (T::kOdd && sizeof(R) == 4);  // as the stage launches
           auto velocity = [&](const R* tr, R v[2], bool divide) {
             if (divide) {
               v[0] = tr[0] / tr[2];
@@ -461,8 +462,8 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::TPE, ResTraits<P, Phys,
             velocity(L, vL, true);
             if (nbBlk >= 0) velocity(Xn, vR, true);
           }
-          velocity(L, velL, ref_rounding<R>() || T::kOdd);
-          if (nbBlk >= 0) velocity(Xn, velR, ref_rounding<R>() || T::kOdd);
+          velocity(L, velL, kDivide);
+          if (nbBlk >= 0) velocity(Xn, velR, kDivide);
           if constexpr (kMany) {
             R* sv = tile_vel(k);
             sv[0] = velL[0], sv[X::faces] = velL[1], sv[2 * X::faces] = velR[0], sv[3 * X::faces] = velR[1];

@@ -218,9 +218,9 @@ struct TmaTraits {
   static constexpr bool kProd = sizeof(R) == 8 && !ref_rounding<R>();
   static constexpr bool kSep = P == 6 || (P == 5 && !kProd) ||
                                (P == 7 && (!kProd || (NV == 3 && !Phys::kLaggedVelocity)));
-  static constexpr int kU = (!kSep && NF * FS > 2 * NV * PP) ? NF * FS : 2 * NV * PP;
+  static constexpr int kU = (!kSep && NT * FS > 2 * NV * PP) ? NT * FS : 2 * NV * PP;
   static constexpr int SS = side_stride(NV * P, (int)sizeof(R));
-  static constexpr int EB = kU + 4 * SS + (kSep ? NF * FS : 0);
+  static constexpr int EB = kU + 4 * SS + (kSep ? NT * FS : 0);
   static constexpr int oN = kSep ? kU + 4 * SS : 0;  // node fields within an element's arrays
   // Every thread waits for the tile's copies itself (instead of thread 0 for
   // the group): with kSep there is no barrier to wait at, and at P = 4 a
@@ -269,6 +269,12 @@ struct TmaTraits {
   // The auxiliaries of the volume flux.  FP32 bulk at odd P forms the full node
   // state, as its per-element kernel does (the compiler contracts the pressure
   // of the shorter form differently, in the last bit).
+  // The traced fields of a node's solution f[0..NV).  (ShallowWater's are the
+  // solution itself: with the velocities formed and stored along, as the flux
+  // needs them, its stages took 1-4 % longer.)
+  __device__ __forceinline__ static void trace_fields(R* f, const StageArgs& a) {
+    if constexpr (NT > NV) Phys::template node<R>(f, a);
+  }
   __device__ __forceinline__ static void flux_fields(R* f, const StageArgs& a) {
     if constexpr (kOdd && sizeof(R) == 4) Phys::template node<R>(f, a);
     else Phys::template node_flux<R>(f, a);
@@ -533,24 +539,24 @@ struct TraceBlock {
 template <int P, class Phys, typename R>
 __global__ void __launch_bounds__(TraceBlock<P, Phys, R>::threads) k_traces(const StageArgs a) {
   using T = TmaTraits<P, Phys, R>;
-  constexpr int NV = T::NV, NF = T::NF, PP = T::PP, TS = T::TS, FS = T::FS;
+  constexpr int NV = T::NV, NT = T::NT, PP = T::PP, TS = T::TS, FS = T::FS;
   constexpr int EPB = TraceBlock<P, Phys, R>::elems, NTH = TraceBlock<P, Phys, R>::threads;
-  __shared__ R sm[EPB * NF * FS];
+  __shared__ R sm[EPB * NT * FS];
   const int t = threadIdx.x, slot = t / PP, n = t - slot * PP;
   const long long e0 = (long long)blockIdx.x * EPB;
   const int live = a.nEl - e0 < EPB ? (int)(a.nEl - e0) : EPB;
   if (slot < live) {
-    R f[NF];
+    R f[NT];
 #pragma unroll
     for (int v = 0; v < NV; ++v) f[v] = (R)a.q[n + (long long)PP * (v + NV * (e0 + slot))];
     if constexpr (NV == 4 && sizeof(R) == 4) cig_fields_rounded(f, (float)a.gamma);
-    else Phys::template node<R>(f, a);
+    else T::trace_fields(f, a);
 #pragma unroll
-    for (int v = 0; v < NF; ++v) sm[(slot * NF + v) * FS + T::nf(v, n % P, n / P)] = f[v];
+    for (int v = 0; v < NT; ++v) sm[(slot * NT + v) * FS + T::nf(v, n % P, n / P)] = f[v];
   }
   __syncthreads();
   R* trOut = reinterpret_cast<R*>(a.trOut) + (size_t)4 * TS * e0;
-  tile_traces<P, Phys, R>(sm, NF * FS, EPB, live, t, NTH, a, [&](int eE, int fi, int l, bool row, R lo, R hi) {
+  tile_traces<P, Phys, R>(sm, NT * FS, EPB, live, t, NTH, a, [&](int eE, int fi, int l, bool row, R lo, R hi) {
     R* o = trOut + 4 * TS * eE + l + P * fi;
     o[TS * (row ? 3 : 0)] = lo;
     o[TS * (row ? 1 : 2)] = hi;
@@ -1015,7 +1021,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
           velL[0] = vo[ii + P * (0 + 2 * s1)];
           velL[1] = vo[ii + P * (1 + 2 * s1)];
           R* vOut = velOut;
-          if constexpr (ref_rounding<R>() || T::kOdd) {
+          if constexpr (ref_rounding<R>() || (T::kOdd && sizeof(R) == 4)) {
             vOut[ii + P * (0 + 2 * (s1 + 4 * eF))] = L[0] / L[2];
             vOut[ii + P * (1 + 2 * (s1 + 4 * eF))] = L[1] / L[2];
           } else {
@@ -1124,9 +1130,9 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
         a.q[gi] = qn;
         f[v] = (R)qn;
       }
-      Phys::template node<R>(f, a);
+      T::trace_fields(f, a);
 #pragma unroll
-      for (int v = 0; v < NF; ++v) gN[v * FS + T::nf(v, i, j)] = f[v];
+      for (int v = 0; v < NT; ++v) gN[v * FS + T::nf(v, i, j)] = f[v];
     }
     group_bar();
     if constexpr (T::kSep) refill();

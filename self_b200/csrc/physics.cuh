@@ -114,7 +114,8 @@ __device__ __forceinline__ void sw_riemann(R HuL, R HvL, R HL, R HuR, R HvR, R H
   const R fR1 = sum_of_products(HuR, unR, pR, a);
   const R fR2 = sum_of_products(HvR, unR, pR, b);
   const R fR3 = sum_of_products(HuR, a, HvR, b);
-  const R alpha = fmax(fmax(fabs(unL + cL), fabs(unR + cR)), fmax(fabs(unL - cL), fabs(unR - cR)));
+  // max(|u + c|, |u - c|) = |u| + c, with the same rounding
+  const R alpha = fmax(fabs(unL) + cL, fabs(unR) + cR);
   out[0] = (R)0.5 * (fL1 + fR1 + alpha * (HuL - HuR)) * s;
   out[1] = (R)0.5 * (fL2 + fR2 + alpha * (HvL - HvR)) * s;
   out[2] = (R)0.5 * (fL3 + fR3 + alpha * (HL - HR)) * s;
