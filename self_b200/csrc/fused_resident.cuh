@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::TPE, ResTraits<P, Phys,
       __syncthreads();  // fluxes and own traces
 
       // volume sums, alongside the face threads' exchange and Riemann flux
-      tile_volume_sums<P, Phys, R>(gBase, sdg, t, faceWarp, nLive);
+      tile_volume_sums<P, Phys, R>(gBase, sdg, t, faceWarp, nLive, a);
       R dreg[NV];
       if constexpr (T::kRegDiv) {
         if (active) {
@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::TPE, ResTraits<P, Phys,
         Phys::template source<double>(q, na, a, Src);
         R d[NV];
 #pragma unroll
-        for (int v = 0; v < NV; ++v) d[v] = T::kRegDiv ? dreg[v] : gD[v * PP + n];
+        for (int v = 0; v < NV; ++v) d[v] = T::kRegDiv ? dreg[v] : T::kLines ? gU[v * PP + n] + gF1[v * PP + T::f1at(i, j)] : gD[v * PP + n];
         const double gdt = a.dtElem ? rkG * gdtE : rkGdt;
         const R bi0 = sb[i], bi1 = sb[i + P], bj0 = sb[j], bj1 = sb[j + P], wi = sw[i], wj = sw[j];
 #pragma unroll

@@ -254,7 +254,16 @@ struct TmaTraits {
   static constexpr bool kDmma4 = (P == 4 && EPG == 2 && TPE == 32) && !ref_rounding<R>();
   // odd P otherwise: each node's thread forms its sums in registers, in the
   // reference's order
-  static constexpr bool kRegDiv = kOdd && !kDmma;
+  // production FP64 at P = 3 and 5: a thread per line of a variable, its sums
+  // along the line in registers with the matrix as kernel-parameter constants,
+  // written over the line.  A line's P values are read once for its P nodes
+  // (10 shared accesses instead of 40 per thread at P = 5, where the L1 pipe ran
+  // at 70 %): us per stage on 256x256, a sum per node -> lines, P = 5
+  // ShallowWater 98 -> 88, CompressibleIdealGas2D 123 -> 112, LinearShallowWater
+  // 81 -> 76; P = 3 46.5 -> 44.7, 64.7 -> 63.5, 39.2 -> 39.0; at P = 7 192
+  // against the products' 195, but ShallowWater 184 against 158.
+  static constexpr bool kLines = kOdd && kProd && !kDmma;
+  static constexpr bool kRegDiv = kOdd && !kDmma && !kLines;
   // At P = 8 the products' operand loads read, per half-warp, four rows of
   // the xi flux, the eta flux and the transposed dgMatrix at four columns
   // each; rows two apart would share banks, so these three arrays keep the
@@ -264,7 +273,7 @@ struct TmaTraits {
   __device__ __forceinline__ static int cswz(int c, int r) { return kSw8 ? (c ^ (4 * ((r >> 1) & 1))) : c; }
   // positions of F0(m, j), F1(i, j) and dgM(m, i)
   __device__ __forceinline__ static int f0at(int m, int j) { return kSw8 ? P * j + cswz(m, j) : P * j + f0pos(m, j); }
-  __device__ __forceinline__ static int f1at(int i, int j) { return P * j + cswz(i, j); }
+  __device__ __forceinline__ static int f1at(int i, int j) { return kLines ? P * i + j : P * j + cswz(i, j); }
   __device__ __forceinline__ static int dgat(int m, int i) { return P * m + cswz(i, m); }
   // The auxiliaries of the volume flux.  FP32 bulk at odd P forms the full node
   // state, as its per-element kernel does (the compiler contracts the pressure
@@ -310,10 +319,28 @@ struct TmaTraits {
 // of the sum are the two elements' sums (the off-diagonal ones mix the
 // elements and are dropped).
 template <int P, class Phys, typename R>
-__device__ __forceinline__ void tile_volume_sums(R* gBase, const double* sdg, int t, int faceWarp, int nLive) {
+__device__ __forceinline__ void tile_volume_sums(R* gBase, const double* sdg, int t, int faceWarp, int nLive,
+                                                 const StageArgs& a) {
   using T = TmaTraits<P, Phys, R>;
   constexpr int NV = T::NV, PP = T::PP, EPG = T::EPG, EB = T::EB, TPE = T::TPE;
-  if constexpr (T::kDmma4) {
+  if constexpr (T::kLines) {
+    constexpr int LE = 2 * NV * P;  // lines of an element: xi lines of the xi flux, eta lines of the eta flux
+    for (int k = t; k < EPG * LE; k += TPE) {
+      const int eE = k / LE;
+      if (eE >= nLive) break;
+      R* line = gBase + eE * EB + P * (k - eE * LE);
+      R x[P];
+#pragma unroll
+      for (int m = 0; m < P; ++m) x[m] = line[m];
+#pragma unroll
+      for (int l = 0; l < P; ++l) {
+        R s = a.dgM[P * l] * x[0];  // (kernel-parameter constants)
+#pragma unroll
+        for (int m = 1; m < P; ++m) s = s + a.dgM[m + P * l] * x[m];
+        line[l] = s;
+      }
+    }
+  } else if constexpr (T::kDmma4) {
     const int lane = t & 31, gq = lane >> 2, kq = lane & 3;
     const int eR = gq >> 2, jr = gq & 3;   // the element and node row of this lane's A row / B column
     const R* bU = gBase + eR * EB;
@@ -949,13 +976,14 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
     }
 
     // ---- B (alongside the face phase C): weak-divergence volume sums
-    tile_volume_sums<P, Phys, R>(gBase, sdg, t, faceWarp, nLive);
+    if constexpr (T::kRegDiv || T::kLines)
+      if (faceOn && !kNbrEarly) load_neighbour();  // in flight during the sums
+    tile_volume_sums<P, Phys, R>(gBase, sdg, t, faceWarp, nLive, a);
 
     // ---- C: faces; own traces of this stage's solution come from the cache,
     // the neighbour's were loaded before phase A
     R dreg[NV];
     if constexpr (T::kRegDiv) {
-      if (faceOn && !kNbrEarly) load_neighbour();  // in flight during the sums
       if (active) {
 #pragma unroll
         for (int v = 0; v < NV; ++v) dreg[v] = (R)0;
@@ -977,7 +1005,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
             gflag[g] = 0;  // checked after phase C
           __syncwarp();
         }
-        if ((!kNbrEarly && !T::kRegDiv) || gridWait) load_neighbour();
+        if ((!kNbrEarly && !T::kRegDiv && !T::kLines) || gridWait) load_neighbour();
         const long long eF = e0 + eC;
         const int bcid = ssi[4];
         const bool physical = (bcid != 0) && (ssi[2] == 0);
@@ -1078,7 +1106,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
       Phys::template source<double>(qv, na, a, Src);
       R d[NV];  // volume sums from phase B
 #pragma unroll
-      for (int v = 0; v < NV; ++v) d[v] = T::kRegDiv ? dreg[v] : gD[v * PP + n];
+      for (int v = 0; v < NV; ++v) d[v] = T::kRegDiv ? dreg[v] : T::kLines ? gU[v * PP + n] + gF1[v * PP + f1at(i, j)] : gD[v * PP + n];
       if constexpr (ref_rounding<R>()) {
         // the reference's divisions, rounded as it rounds them (bit-exact form)
         const R wi = (R)sqw[i], wj = (R)sqw[j];
