@@ -146,6 +146,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::TPE, ResTraits<P, Phys,
   constexpr int kWm = kRec.wm, rBytes = kRec.bytes, rNhat = kRec.oNhat, rNs = kRec.oNs, rJ = kRec.oJ, rSi = kRec.oSi;
   __shared__ __align__(16) R sm[X::values(kMany)];
   __shared__ __align__(16) double sdg[PP];
+  __shared__ R sdgR[T::kRegDiv ? PP : 1];
   // bMatrix, and the quadrature weights (reference roundings) or their
   // reciprocals, in the bulk type
   __shared__ R sb[2 * P], sw[P];
@@ -153,7 +154,11 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::TPE, ResTraits<P, Phys,
   __shared__ int sOk;
   extern __shared__ __align__(16) unsigned char state[];  // kMany: the tiles' state
   const int t = threadIdx.x;
-  for (int k = t; k < PP; k += TPE) sdg[T::dgat(k / P, k % P)] = a.dgM[k / P + P * (k % P)];
+  for (int k = t; k < PP; k += TPE) {
+    const double d = a.dgM[k / P + P * (k % P)];
+    sdg[T::dgat(k / P, k % P)] = d;
+    if constexpr (T::kRegDiv) sdgR[T::dgat(k / P, k % P)] = (R)d;
+  }
   for (int k = t; k < 2 * P; k += TPE) sb[k] = k < P ? bm_left<R>(a, k) : bm_right<R, P>(a, k - P);
   for (int k = t; k < P; k += TPE) sw[k] = ref_rounding<R>() ? (R)a.qw[k] : (R)(1.0 / a.qw[k]);
   if (t == 0) {
@@ -395,7 +400,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::TPE, ResTraits<P, Phys,
           for (int v = 0; v < NV; ++v) dreg[v] = (R)0;
 #pragma unroll
           for (int m = 0; m < P; ++m) {
-            const R gi = (R)sdg[T::dgat(m, i)], gj = (R)sdg[T::dgat(m, j)];
+            const R gi = sdgR[T::dgat(m, i)], gj = sdgR[T::dgat(m, j)];
 #pragma unroll
             for (int v = 0; v < NV; ++v)
               dreg[v] = dreg[v] + gi * gU[v * PP + T::f0at(m, j)] + gj * gF1[v * PP + T::f1at(i, m)];

@@ -213,11 +213,16 @@ struct TmaTraits {
   // 177 -> 165, reference 280 -> 265, LinearShallowWater FP64 144 -> 134, but
   // production ShallowWater 158 -> 170 and CompressibleIdealGas2D 195 -> 197;
   // P = 5 FP32 102 -> 96, reference 145 -> 137, production FP64 96x96 17.9 ->
-  // 19.8; P = 3 within 2 % but for FP32 CompressibleIdealGas2D (48 -> 45); P = 8
-  // loses more groups than the barriers cost.
+  // 19.8; P = 4 FP32 ShallowWater 44.2 -> 42.1, LinearShallowWater 40.0 -> 38.4,
+  // CompressibleIdealGas2D 55 -> 58, its reference roundings 95 -> 87.6, the
+  // other FP64 forms within 2 %; P = 3 CompressibleIdealGas2D FP32 47.8 -> 45.1,
+  // production FP64 119x119 14.3 -> 13.7, the others within 2 %; P = 8 loses
+  // more groups than the barriers cost.
   static constexpr bool kProd = sizeof(R) == 8 && !ref_rounding<R>();
   static constexpr bool kSep = P == 6 || (P == 5 && !kProd) ||
-                               (P == 7 && (!kProd || (NV == 3 && !Phys::kLaggedVelocity)));
+                               (P == 7 && (!kProd || (NV == 3 && !Phys::kLaggedVelocity))) ||
+                               (P == 4 && (sizeof(R) == 4 ? NV == 3 : NV == 4 && !kProd)) ||
+                               (P == 3 && NV == 4 && (kProd || sizeof(R) == 4));
   static constexpr int kU = (!kSep && NT * FS > 2 * NV * PP) ? NT * FS : 2 * NV * PP;
   static constexpr int SS = side_stride(NV * P, (int)sizeof(R));
   static constexpr int EB = kU + 4 * SS + (kSep ? NT * FS : 0);
@@ -646,6 +651,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
   // bMatrix and 1/w in the bulk type (FP32-bulk form: rounded copies after 1/w)
   R* sbR = sizeof(R) == 8 ? reinterpret_cast<R*>(sb) : reinterpret_cast<R*>(sqwr + P);
   R* sqwrR = sizeof(R) == 8 ? reinterpret_cast<R*>(sqwr) : sbR + 2 * P;
+  R* sdgR = sizeof(R) == 8 ? reinterpret_cast<R*>(sdg) : sqwrR + P;  // (kRegDiv)
   volatile int* gflag = reinterpret_cast<volatile int*>(smem + pl.oFlags);
   unsigned char* slots = smem + pl.oSlots;
 
@@ -656,7 +662,11 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
   // dgMatrix transposed (sdg[i + P m] = dgM(m, i), the column index swizzled
   // where kSw8): a warp's reads of the columns of its nodes' i (or j) are then
   // consecutive
-  for (int k = threadIdx.x; k < PP; k += blockDim.x) sdg[dgat(k / P, k % P)] = a.dgM[k / P + P * (k % P)];
+  for (int k = threadIdx.x; k < PP; k += blockDim.x) {
+    const double d = a.dgM[k / P + P * (k % P)];
+    sdg[dgat(k / P, k % P)] = d;
+    if constexpr (T::kRegDiv && sizeof(R) == 4) sdgR[dgat(k / P, k % P)] = (R)d;
+  }
   for (int k = threadIdx.x; k < 2 * P; k += blockDim.x) {
     sb[k] = a.bM[k];
     if constexpr (sizeof(R) == 4) sbR[k] = a.bMf[k];
@@ -989,7 +999,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
         for (int v = 0; v < NV; ++v) dreg[v] = (R)0;
 #pragma unroll
         for (int m = 0; m < P; ++m) {
-          const R gi = (R)sdg[dgat(m, i)], gj = (R)sdg[dgat(m, j)];
+          const R gi = sdgR[dgat(m, i)], gj = sdgR[dgat(m, j)];
 #pragma unroll
           for (int v = 0; v < NV; ++v)
             dreg[v] = dreg[v] + gi * gU[v * PP + f0at(m, j)] + gj * gF1[v * PP + f1at(i, m)];
@@ -1245,7 +1255,7 @@ inline bool make_tma_plan(const StageArgs& a, int smemLimit, long long l2Bytes, 
     s = (s + 15) / 16 * 16;
     const int oMats = s;
     s += (PP + 4 * P) * 8;  // dgMatrix, bMatrix, weights, reciprocal weights
-    if (sizeof(R) == 4) s += (3 * P * 4 + 15) / 16 * 16;  // their FP32 copies
+    if (sizeof(R) == 4) s += ((3 * P + (T::kRegDiv ? PP : 0)) * 4 + 15) / 16 * 16;  // their FP32 copies
     const int oFlags = s;
     s += C * 4;  // group flags
     s = (s + 127) / 128 * 128;
