@@ -141,6 +141,11 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::TPE, ResTraits<P, Phys,
   constexpr int FS = T::FS, SS = T::SS, EPG = T::EPG, EB = T::EB;
   constexpr bool kLSW = (NV == 3 && !Phys::kLaggedVelocity);
   constexpr bool kSW = Phys::kLaggedVelocity;
+  // an orientation per warp (tile_traces), us per stage, tasks in common -> per
+  // warp: LinearShallowWater FP64 34x34 1.63 -> 1.54, 64x64 7.70 -> 7.43,
+  // CompressibleIdealGas2D FP64 64x64 12.5 -> 11.9, FP32 34x34 2.43 -> 2.35 but
+  // 64x64 9.39 -> 9.85; reference roundings 3.34 -> 3.46
+  constexpr bool kWarpTraces = T::kSwz && !ref_rounding<R>() && !(kMany && NV == 4 && sizeof(R) == 4);
   constexpr int kGeo = geo_kind<P, R>();
   constexpr GeoRec kRec = geo_rec(P, kGeo);
   constexpr int kWm = kRec.wm, rBytes = kRec.bytes, rNhat = kRec.oNhat, rNs = kRec.oNs, rJ = kRec.oJ, rSi = kRec.oSi;
@@ -296,8 +301,8 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::TPE, ResTraits<P, Phys,
   auto put_traces = [&](unsigned long long set, bool last) {
     Pub* out = reinterpret_cast<Pub*>(ra.xch[set & 1]);
     const bool stall = a.debugStarve == 2 && blockIdx.x == 0;  // (test hook: CTA 0 publishes nothing)
-    tile_traces<P, Phys, R>(sm + X::oFields, X::FB, EPG, nLive, t, TPE, a,
-                            [&](int eE, int fi, int l, bool row, R lo, R hi) {
+    tile_traces<P, Phys, R, kWarpTraces>(sm + X::oFields, X::FB, EPG, nLive, t, TPE, a,
+                                         [&](int eE, int fi, int l, bool row, R lo, R hi) {
       const int sl = row ? 3 : 0, sh = row ? 1 : 2;
       if (last) {
         R* o = reinterpret_cast<R*>(ra.trOut) + (size_t)4 * TS * (e0 + eE);

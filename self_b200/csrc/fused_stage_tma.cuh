@@ -93,6 +93,7 @@ struct TmaPlan {
   int oX[5];       // model fields: LSW (H, Hb, fC), SW (topoB, grad), CIG (envG, drag, presc x3 -> oX[2..4])
   int oVelOwn;
   int oMats, oFlags, oSlots, oGroups, groupBytes, smemBytes;
+  int oTasks;
 };
 
 // Several RK stages in one launch of k_fused_stage_tma<..., true>: stage s
@@ -252,8 +253,8 @@ struct TmaTraits {
   }
   // Divergence sums as FP64 tensor-core products: production and FP32-bulk
   // forms at P = 8 and 6 (one element per warp) and 4 (two), production FP64
-  // at P = 7 (229 against 257 us per stage with sums in registers; at P = 5
-  // they are slower, 140 against 123)
+  // at P = 7 (229 against 257 us per stage with a sum per node; at P = 5 they
+  // are slower, 140 against 123)
   static constexpr bool kDmma =
       ((P == 8 && EPG == 1) || P == 6 || (P == 7 && sizeof(R) == 8)) && !ref_rounding<R>();
   static constexpr bool kDmma4 = (P == 4 && EPG == 2 && TPE == 32) && !ref_rounding<R>();
@@ -293,6 +294,27 @@ struct TmaTraits {
     if constexpr (kOdd && sizeof(R) == 4) Phys::template node<R>(f, a);
     else Phys::template node_flux<R>(f, a);
   }
+  // Trace tasks of a tile, one per (element, direction, field, line), in rounds
+  // of a task per thread.  Where a thread has several, it reads each one's
+  // offsets from a table made once per CTA: working them out (divisions by 2 NT
+  // P, NT P and P) cost as much as the sums.  us per stage on 256x256, without
+  // -> with: CompressibleIdealGas2D P = 6 FP32 109 -> 101.5, FP64 135 -> 129,
+  // reference roundings 183 -> 171; P = 4 FP32 54.8 -> 49.4; P = 5 FP32 96.2 ->
+  // 89.5; P = 3 FP32 47.8 -> 43.2; P = 7 FP32 165 -> 160; ShallowWater FP32 P =
+  // 4 44.2 -> 41.0.  With one round (ShallowWater and LinearShallowWater at P =
+  // 5 to 7) the table's load is one more step before the tile's end, 1-7 %
+  // slower but for FP32 at P = 7 (134 -> 129), and ShallowWater at P = 3 lost
+  // 2-3 % too.
+  static constexpr int kTasks = EPG * 2 * NT * P, kRounds = (kTasks + TPE - 1) / TPE;
+  static constexpr int kTaskTab = !kSwz && (kRounds > 1 ? !(P == 3 && Phys::kLaggedVelocity) : P == 7 && sizeof(R) == 4)
+                                      ? kRounds * TPE
+                                      : 0;
+  // P = 8: an orientation per warp (tile_traces).  us per stage, tasks in
+  // common -> per warp: CompressibleIdealGas2D FP64 128x128 47.7 -> 46.9, 256x256
+  // 171.9 -> 170.4, FP32 37.4 -> 36.2 and 128.9 -> 127.3, ShallowWater FP32 32.1
+  // -> 31.5; but LinearShallowWater FP64 122.4 -> 124.7, reference roundings 222
+  // -> 226, ShallowWater FP64 134.5 -> 135.3.
+  static constexpr bool kWarpTraces = kSwz && (sizeof(R) == 4 || (kProd && NV == 4));
   // offset of node (i, j) in field f's block of the node-field array
   __device__ __forceinline__ static int nf(int f, int i, int j) {
     if constexpr (kSwz) return P * j + (i ^ (((j >> 1) ^ (4 * (f & 1))) & (P - 1)));
@@ -509,39 +531,105 @@ __device__ __forceinline__ void tile_volume_sums(R* gBase, const double* sdg, in
 // field pair, orientation, field, line (an odd NT leaves the last pair's
 // second half idle), so that a half-warp reads the column lines (or the row
 // lines) of two fields; the padded layouts of the other P number them by
-// orientation, field, line, with no idle tasks.
-template <int P, class Phys, typename R, class Emit>
+// orientation, field, line, with no idle tasks.  With kWarp (P = 8) each warp
+// has one orientation instead, so that no address depends on the task: fewer
+// instructions, but an uneven last round is not shared out.
+template <int P, class Phys, typename R, bool kWarp, class Emit>
 __device__ __forceinline__ void tile_traces(const R* fields, int stride, int elems, int live, int k0, int step,
                                             const StageArgs& a, Emit emit) {
   using T = TmaTraits<P, Phys, R>;
   constexpr int NT = T::NT;
-  constexpr int NTp = T::kSwz ? (NT + 1) / 2 * 2 : NT;
-  constexpr int TPEl = 2 * NTp * P;  // tasks per element
-  for (int kk = k0; kk < elems * TPEl; kk += step) {
-    const int eE = kk / TPEl, ks = kk - eE * TPEl;
-    if (eE >= live) continue;
-    int row, fi, l;
-    if constexpr (T::kSwz) {
-      const int fp = ks / (4 * P), r = ks - fp * 4 * P, r2 = r - (r / (2 * P)) * 2 * P, fs = r2 / P;
-      row = r / (2 * P);
-      l = r2 - fs * P;
-      fi = 2 * fp + fs;
-      if (fi >= NT) continue;
-    } else {
-      row = ks / (NT * P);
-      const int r = ks - row * NT * P;
-      fi = r / P;
-      l = r - fi * P;
+  if constexpr (kWarp) {
+    static_assert(P == 8, "64 threads per element");
+    // lane l + 8 f takes line l of fields f, f + 4, ..., whose swizzle is the
+    // same, so that a lane's eight offsets serve all its tasks
+    const int l = k0 & 7, f0 = (k0 & 31) >> 3;
+    const bool row = (k0 >> 5) & 1;
+    for (int eE = k0 >> 6; eE < live; eE += step >> 6) {
+      const R* fv = fields + eE * stride + f0 * T::FS;
+      int at[P];
+#pragma unroll
+      for (int m = 0; m < P; ++m) at[m] = row ? T::nf(f0, m, l) : T::nf(f0, l, m);
+#pragma unroll
+      for (int f = 0; f < NT; f += 4) {
+        if (f0 + f >= NT) break;
+        R lo = (R)0, hi = (R)0;
+#pragma unroll
+        for (int m = 0; m < P; ++m) {
+          const R x = fv[f * T::FS + at[m]];
+          lo = lo + bm_left<R>(a, m) * x;  // kernel-parameter constants (m is unrolled)
+          hi = hi + bm_right<R, P>(a, m) * x;
+        }
+        emit(eE, f0 + f, l, row, lo, hi);
+      }
     }
-    const R* fv = fields + eE * stride + fi * T::FS;
+  } else {
+    constexpr int NTp = T::kSwz ? (NT + 1) / 2 * 2 : NT;
+    constexpr int TPEl = 2 * NTp * P;  // tasks per element
+    for (int kk = k0; kk < elems * TPEl; kk += step) {
+      const int eE = kk / TPEl, ks = kk - eE * TPEl;
+      if (eE >= live) continue;
+      int row, fi, l;
+      if constexpr (T::kSwz) {
+        const int fp = ks / (4 * P), r = ks - fp * 4 * P, r2 = r - (r / (2 * P)) * 2 * P, fs = r2 / P;
+        row = r / (2 * P);
+        l = r2 - fs * P;
+        fi = 2 * fp + fs;
+        if (fi >= NT) continue;
+      } else {
+        row = ks / (NT * P);
+        const int r = ks - row * NT * P;
+        fi = r / P;
+        l = r - fi * P;
+      }
+      const R* fv = fields + eE * stride + fi * T::FS;
+      R lo = (R)0, hi = (R)0;
+#pragma unroll
+      for (int m = 0; m < P; ++m) {
+        const R x = fv[row ? T::nf(fi, m, l) : T::nf(fi, l, m)];
+        lo = lo + bm_left<R>(a, m) * x;  // kernel-parameter constants (m is unrolled)
+        hi = hi + bm_right<R, P>(a, m) * x;
+      }
+      emit(eE, fi, l, row != 0, lo, hi);
+    }
+  }
+}
+
+// The same from a table of tasks: line's first node (17 bits up), its direction
+// (bit 16) and the offset of its value in the tile's trace blocks (16 bits;
+// 0xffff: no task).
+template <int P, class Phys, typename R>
+__device__ __forceinline__ uint32_t trace_task(int k) {
+  using T = TmaTraits<P, Phys, R>;
+  constexpr int NT = T::NT;
+  if (k >= T::kTasks) return 0xffffu;
+  const int eE = k / (2 * NT * P), ks = k - eE * 2 * NT * P, row = ks / (NT * P), r = ks - row * NT * P;
+  const int fi = r / P, l = r - fi * P;
+  const uint32_t src = eE * T::EB + fi * T::FS + (row ? T::RS * l : l);
+  return src << 17 | (uint32_t)row << 16 | (uint32_t)(4 * T::TS * eE + l + P * fi);
+}
+template <int P, class Phys, typename R>
+__device__ __forceinline__ void table_traces(const R* fields, const uint32_t* tasks, int live, int t,
+                                             const StageArgs& a, R* out) {
+  using T = TmaTraits<P, Phys, R>;
+  static_assert(T::EPG * T::EB < (1 << 15) && 4 * T::TS * T::EPG < 0xffff, "a task fits its table entry");
+#pragma unroll
+  for (int r = 0; r < T::kRounds; ++r) {
+    const uint32_t k = tasks[r * T::TPE + t];
+    const int o = k & 0xffffu;
+    if (o >= 4 * T::TS * live) continue;
+    const bool row = k & 0x10000u;
+    const R* fv = fields + (k >> 17);
+    const int step = row ? 1 : T::RS;
     R lo = (R)0, hi = (R)0;
 #pragma unroll
     for (int m = 0; m < P; ++m) {
-      const R x = fv[row ? T::nf(fi, m, l) : T::nf(fi, l, m)];
+      const R x = fv[m * step];
       lo = lo + bm_left<R>(a, m) * x;  // kernel-parameter constants (m is unrolled)
       hi = hi + bm_right<R, P>(a, m) * x;
     }
-    emit(eE, fi, l, row != 0, lo, hi);
+    out[o + T::TS * (row ? 3 : 0)] = lo;
+    out[o + T::TS * (row ? 1 : 2)] = hi;
   }
 }
 
@@ -588,7 +676,7 @@ __global__ void __launch_bounds__(TraceBlock<P, Phys, R>::threads) k_traces(cons
   }
   __syncthreads();
   R* trOut = reinterpret_cast<R*>(a.trOut) + (size_t)4 * TS * e0;
-  tile_traces<P, Phys, R>(sm, NT * FS, EPB, live, t, NTH, a, [&](int eE, int fi, int l, bool row, R lo, R hi) {
+  tile_traces<P, Phys, R, false>(sm, NT * FS, EPB, live, t, NTH, a, [&](int eE, int fi, int l, bool row, R lo, R hi) {
     R* o = trOut + 4 * TS * eE + l + P * fi;
     o[TS * (row ? 3 : 0)] = lo;
     o[TS * (row ? 1 : 2)] = hi;
@@ -671,6 +759,8 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
     sb[k] = a.bM[k];
     if constexpr (sizeof(R) == 4) sbR[k] = a.bMf[k];
   }
+  uint32_t* tasks = reinterpret_cast<uint32_t*>(smem + pl.oTasks);
+  for (int k = threadIdx.x; k < T::kTaskTab; k += blockDim.x) tasks[k] = trace_task<P, Phys, R>(k);
   if (T::kAllWait)
     for (int k = threadIdx.x; k < C; k += blockDim.x) gflag[k] = 1;
   for (int k = threadIdx.x; k < P; k += blockDim.x) {
@@ -1175,12 +1265,15 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::kThreadsMax, 1)
     group_bar();
     if constexpr (T::kSep) refill();
 
-    // ---- E: traces of the updated solution -> trace cache.  (A one-element
-    // group's face warp starts one warp later, so the other warp takes the
-    // last, partial round.)
-    {
-      const int k0 = (EPG == 1) ? (faceWarp ? t : (t + 32) % TPE) : t;
-      tile_traces<P, Phys, R>(gBase + T::oN, EB, EPG, nLive, k0, TPE, a, [&](int eE, int fi, int l, bool row, R lo, R hi) {
+    // ---- E: traces of the updated solution -> trace cache.  (Without kWarp a
+    // one-element group's face warp starts one warp later, so the other warp
+    // takes the last, partial round.)
+    if constexpr (T::kTaskTab > 0) {
+      table_traces<P, Phys, R>(gBase + T::oN, tasks, nLive, t, a, trOut + (size_t)4 * TS * e0);
+    } else {
+      const int k0 = (EPG == 1 && !T::kWarpTraces) ? (faceWarp ? t : (t + 32) % TPE) : t;
+      tile_traces<P, Phys, R, T::kWarpTraces>(gBase + T::oN, EB, EPG, nLive, k0, TPE, a,
+                                              [&](int eE, int fi, int l, bool row, R lo, R hi) {
         R* o = trOut + (size_t)4 * TS * (e0 + eE);
         o[l + P * fi + TS * (row ? 3 : 0)] = lo;
         o[l + P * fi + TS * (row ? 1 : 2)] = hi;
@@ -1256,6 +1349,8 @@ inline bool make_tma_plan(const StageArgs& a, int smemLimit, long long l2Bytes, 
     const int oMats = s;
     s += (PP + 4 * P) * 8;  // dgMatrix, bMatrix, weights, reciprocal weights
     if (sizeof(R) == 4) s += ((3 * P + (T::kRegDiv ? PP : 0)) * 4 + 15) / 16 * 16;  // their FP32 copies
+    const int oTasks = s;
+    s += T::kTaskTab * 4;
     const int oFlags = s;
     s += C * 4;  // group flags
     s = (s + 127) / 128 * 128;
@@ -1266,6 +1361,7 @@ inline bool make_tma_plan(const StageArgs& a, int smemLimit, long long l2Bytes, 
     if (s <= smemLimit) {
       pl.groups = C;
       pl.oMats = oMats;
+      pl.oTasks = oTasks;
       pl.oFlags = oFlags;
       pl.oSlots = oSlots;
       pl.oGroups = oGroups;
