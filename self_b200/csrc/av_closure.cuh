@@ -78,7 +78,8 @@ struct AvArgs {
   float* act;          // activation applied (nEl)
   float* actInd;       // indicator activation (nEl), written in AV_MLP mode
   int* fallbacks;      // AV_MLP counters: [0] features outside the training range, [1] MLP evaluations
-  int* activeCount;    // elements with nu > 0 in this stage (reset before the viscosity kernel)
+  int* activeCount;    // elements with nu > 0, written by the viscosity kernel's last block
+  int* nuState;        // its running count and the blocks that have finished, zero between launches
   int* activeList;     // their ids (nEl capacity)
   void* visc;          // contravariant viscous volume flux (P*P, 2, 4, nEl), bulk type
   void* vtr;           // per (element, side): nu grad q traces at [i + P (d + 2 v)], bulk type
@@ -310,6 +311,9 @@ __global__ void __launch_bounds__(32 * kNuWarps) k_av_nu(const AvArgs a) {
   __shared__ R sTt[kNuWarps][GE][PP + 1];  // xi transforms (k, jj) at [jj + P k]
   __shared__ R sT[PP];
   __shared__ float sW1[kMlpHidden * kW1Stride], sW2[kMlpHidden * kW2Stride], sw3[kMlpHidden], sB[kMlpFloats];
+  // (see k_av_grad)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const bool mlp = (a.mode == AV_MLP) && (P >= 6);
   for (int k = threadIdx.x; k < PP; k += blockDim.x) sT[k] = (R)a.T[k];
   if (mlp) {
@@ -400,11 +404,22 @@ __global__ void __launch_bounds__(32 * kNuWarps) k_av_nu(const AvArgs a) {
     const unsigned nzMask = __ballot_sync(0xffffffffu, nu != 0.0);
     if (nzMask) {
       int b0 = 0;
-      if (lane == 0) b0 = atomicAdd(a.activeCount, __popc(nzMask));
+      if (lane == 0) b0 = atomicAdd(&a.nuState[0], __popc(nzMask));
       b0 = __shfl_sync(0xffffffffu, b0, 0);
       if (nu != 0.0) a.activeList[b0 + __popc(nzMask & ((1u << lane) - 1u))] = (int)e;
     }
     __syncwarp();
+  }
+  // the last block publishes the count and leaves the state zero for the next
+  // launch (a memset before each launch cost a gap of its own)
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&a.nuState[1], 1) == (int)gridDim.x - 1) {
+      __threadfence();
+      *a.activeCount = atomicExch(&a.nuState[0], 0);
+      a.nuState[1] = 0;
+    }
   }
 }
 
@@ -453,6 +468,11 @@ __global__ void __launch_bounds__(EPB * 4 * P * P) k_av_grad(const AvArgs a) {
   for (int k = tid; k < 2 * P; k += blockDim.x) sb[k] = a.bM[k];
   for (int k = tid; k < P; k += blockDim.x) sw[k] = a.qw[k];
   __syncthreads();
+  // A programmatic dependent launch, as the stage kernel's: what precedes the
+  // wait reads kernel parameters only, and the next kernel of the stage may
+  // start while this one runs.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const R* trIn = reinterpret_cast<const R*>(a.trIn);
   const int count = *a.activeCount;
   // every block runs the same number of rounds (block-uniform barriers)
@@ -642,12 +662,8 @@ struct QwArr {
 template <int P, typename R>
 cudaError_t launch_av_pair(const AvArgs& a, cudaStream_t st, int numSMs, bool formNu) {
   constexpr int EPB = av_elems_per_block<P, R>();
-  if (!formNu) {
-    k_av_grad<P, R, EPB><<<4 * numSMs, EPB * 4 * P * P, 0, st>>>(a);
-    return cudaGetLastError();
-  }
-  cudaError_t e = cudaMemsetAsync(a.activeCount, 0, sizeof(int), st);
-  if (e != cudaSuccess) return e;
+  auto grad = [&]() { return launch_dependent(k_av_grad<P, R, EPB>, 4 * numSMs, EPB * 4 * P * P, st, a); };
+  if (!formNu) return grad();
   // one wave of resident blocks, each warp striding over its share of the
   // elements (a partial second wave would run at low occupancy)
   static std::atomic<int> nuPerSM{0};  // resident blocks per SM, one instantiation per (P, R)
@@ -661,9 +677,8 @@ cudaError_t launch_av_pair(const AvArgs& a, cudaStream_t st, int numSMs, bool fo
   const long long nuBlocks = ((long long)a.nEl + perBlock - 1) / perBlock;
   const long long cap = (long long)nuPerSM.load() * numSMs;
   const int g1 = (int)(nuBlocks < cap ? nuBlocks : cap);
-  k_av_nu<P, R><<<g1, 32 * kNuWarps, 0, st>>>(a);
-  k_av_grad<P, R, EPB><<<4 * numSMs, EPB * 4 * P * P, 0, st>>>(a);
-  return cudaGetLastError();
+  cudaError_t e = launch_dependent(k_av_nu<P, R>, g1, 32 * kNuWarps, st, a);
+  return e == cudaSuccess ? grad() : e;
 }
 
 template <typename R>

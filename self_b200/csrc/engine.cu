@@ -258,7 +258,8 @@ struct selfgpu_model2d {
   AvArgs av{};
   double* avNu = nullptr;
   float* avAct = nullptr;  // [0, nEl): activation applied, [nEl, 2 nEl): indicator activation
-  int* avFallbacks = nullptr;  // [0] MLP fallbacks, [1] MLP evaluations, [2] active count, then the active list
+  int* avFallbacks = nullptr;  // [0] MLP fallbacks, [1] MLP evaluations, [2] active count, [3..4] AvArgs::nuState, then
+                               // the active list
   double* avH = nullptr;
   void* avVisc = nullptr;
   void* avVtr = nullptr;
@@ -1047,11 +1048,11 @@ int selfgpu_model2d_set_closure(selfgpu_model2d* m, int mode, double c, double s
   if (!m->avNu) {
     e = cudaMalloc(&m->avNu, nEl * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&m->avAct, 2 * nEl * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&m->avFallbacks, (3 + nEl) * sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc(&m->avFallbacks, (5 + nEl) * sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&m->avH, nEl * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&m->avVisc, 8 * PP * nEl * m->elemBytes());
     if (e == cudaSuccess) e = cudaMalloc(&m->avVtr, 4 * 8 * (size_t)m->P * nEl * m->elemBytes());
-    if (e == cudaSuccess) e = cudaMemsetAsync(m->avFallbacks, 0, 2 * sizeof(int), m->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(m->avFallbacks, 0, 5 * sizeof(int), m->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(m->avAct, 0, 2 * nEl * sizeof(float), m->stream);
     if (e != cudaSuccess) return fail_cuda("selfgpu_model2d_set_closure", e);
   }
@@ -1070,7 +1071,8 @@ int selfgpu_model2d_set_closure(selfgpu_model2d* m, int mode, double c, double s
   x.actInd = m->avAct + nEl;
   x.fallbacks = m->avFallbacks;
   x.activeCount = m->avFallbacks + 2;
-  x.activeList = m->avFallbacks + 3;
+  x.nuState = m->avFallbacks + 3;
+  x.activeList = m->avFallbacks + 5;
   x.visc = m->avVisc;
   x.vtr = m->avVtr;
   x.mlpW = m->mlpW;

@@ -662,6 +662,7 @@ __global__ void __launch_bounds__(TraceBlock<P, Phys, R>::threads) k_traces(cons
   constexpr int NV = T::NV, NT = T::NT, PP = T::PP, TS = T::TS, FS = T::FS;
   constexpr int EPB = TraceBlock<P, Phys, R>::elems, NTH = TraceBlock<P, Phys, R>::threads;
   __shared__ R sm[EPB * NT * FS];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // (the stage kernel waits itself)
   const int t = threadIdx.x, slot = t / PP, n = t - slot * PP;
   const long long e0 = (long long)blockIdx.x * EPB;
   const int live = a.nEl - e0 < EPB ? (int)(a.nEl - e0) : EPB;

@@ -209,22 +209,6 @@ __global__ void __launch_bounds__(256) k_adam(float* master, const float* part, 
   }
 }
 
-// A launch that may overlap the end of the previous kernel on the stream; the
-// kernel waits for that kernel's completion itself (griddepcontrol.wait).
-template <class... KArgs, class... Args>
-cudaError_t launch_dependent(void (*kernel)(KArgs...), int grid, int block, cudaStream_t st, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
-}
-
 // Weights (bfloat16 pairs) and parameters, passed by value: no device buffer
 // and no copy per call.
 struct MlpArgs {

@@ -39,6 +39,27 @@ struct StageLaunch {
 #include <cuda_runtime.h>
 
 namespace selfgpu {
+// A launch that may overlap the end of the previous kernel on the stream; the
+// kernel waits for that kernel's completion itself (griddepcontrol.wait).
+template <class... KArgs, class... Args>
+inline cudaError_t launch_dependent_smem(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t st,
+                                         Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+template <class... KArgs, class... Args>
+inline cudaError_t launch_dependent(void (*kernel)(KArgs...), int grid, int block, cudaStream_t st, Args... args) {
+  return launch_dependent_smem(kernel, grid, block, 0, st, args...);
+}
 // production FP64 (stage_fp64_prod.cu), reference roundings (stage_fp64.cu), FP32 bulk
 cudaError_t launch_stage_fp64(int model, int P, const StageArgs& a, const StageLaunch& L, cudaStream_t st,
                               int* usedTma);
