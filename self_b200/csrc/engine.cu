@@ -112,8 +112,9 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// Every thread's s summed into x->result by the last block to finish.
-__device__ void sum_grid(double s, SumScratch* x) {
+// Every thread's s summed into x->result, or into *out (host memory) where
+// there is one, by the last block to finish.
+__device__ void sum_grid(double s, SumScratch* x, double* out) {
   __shared__ double ws[kSumThreads / 32];
   __shared__ bool last;
   const int t = threadIdx.x, w = t >> 5;
@@ -140,7 +141,12 @@ __device__ void sum_grid(double s, SumScratch* x) {
   for (int k = t; k < (int)gridDim.x; k += kSumThreads) v += __ldcg(&x->part[k]);
   v = block_sum(v);
   if (t == 0) {
-    x->result = v;
+    if (out) {
+      *out = v;
+      __threadfence_system();
+    } else {
+      x->result = v;
+    }
     x->done = 0;
   }
 }
@@ -156,6 +162,57 @@ __device__ __forceinline__ long long element_of(long long k, int PP, int& n) {
   return e;
 }
 
+// Scratch of the sums: a few slots of static device memory (a stream-ordered
+// allocation per call went back to the system at every synchronisation).  A
+// call owns a slot from its launch until it has read the result.
+constexpr int kSumSlots = 32;
+__device__ SumScratch g_sumSlots[kSumSlots];
+std::atomic<unsigned> g_sumSlotsUsed{0};
+
+int acquire_sum_slot() {
+  while (true) {
+    unsigned used = g_sumSlotsUsed.load();
+    if (used == 0xffffffffu) {  // all in use: their owners are waiting for the device
+      std::this_thread::yield();
+      continue;
+    }
+    int k = 0;
+    while (used >> k & 1u) ++k;
+    if (g_sumSlotsUsed.compare_exchange_weak(used, used | 1u << k)) return k;
+  }
+}
+
+void release_sum_slot(int k) { g_sumSlotsUsed.fetch_and(~(1u << k)); }
+
+// The slots' results in host memory that the device writes, so that a call ends
+// with one synchronisation (a copy of the result after the kernel took 5 us
+// more); null where that memory cannot be had.
+double* sum_results() {
+  static double* const page = [] {
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, kSumSlots * sizeof(double), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+    return (double*)p;
+  }();
+  return page;
+}
+
+// The sum of a launch in `slot`, when the stream has got there.
+cudaError_t read_sum(int slot, double* result, cudaStream_t st) {
+  const double* page = sum_results();
+  cudaError_t e = cudaSuccess;
+  if (!page)
+    e = cudaMemcpyFromSymbolAsync(result, g_sumSlots, sizeof(double), slot * sizeof(SumScratch), cudaMemcpyDeviceToHost,
+                                  st);
+  const cudaError_t e2 = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = e2;
+  if (e == cudaSuccess && page) *result = *reinterpret_cast<const volatile double*>(page + slot);
+  return e;
+}
+double* sum_target(int slot) { return sum_results() ? sum_results() + slot : nullptr; }
+
 // Entropy integrands (CalculateEntropy of the three models):
 //   LSW  0.5 (H (u^2 + v^2) + g eta^2) J w_i w_j  (src/models/SELF_LinearShallowWater.f90:171-216)
 //   SW   (0.5 (Hu^2/H + Hv^2/H) + 0.5 g H^2 - g H b) J w_i w_j  (src/models/SELF_ShallowWater.f90:149-188)
@@ -165,7 +222,8 @@ __device__ __forceinline__ long long element_of(long long k, int PP, int& n) {
 __global__ void __launch_bounds__(kSumThreads) k_entropy(int model, const double* __restrict__ q,
                                                          const double* __restrict__ J, const double* __restrict__ aux,
                                                          QwArr qw, int P, int nEl, double g, double gamma,
-                                                         SumScratch* x) {
+                                                         int slot, double* out) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the stage that forms q
   const int PP = P * P, nv = model == SELFGPU_MODEL_CIG ? 4 : 3;
   const long long nodes = (long long)PP * nEl;
   double s = 0.0;
@@ -188,33 +246,12 @@ __global__ void __launch_bounds__(kSumThreads) k_entropy(int model, const double
     }
   }
   if (model == SELFGPU_MODEL_CIG) s = s / (gamma - 1.0);
-  sum_grid(s, x);
-}
-
-// Scratch of selfgpu_integral_mapped_scalar2d, which belongs to no handle: a
-// few slots of static device memory (a stream-ordered allocation per call went
-// back to the system at every synchronisation).  A call owns a slot from its
-// launch until it has read the result.
-constexpr int kSumSlots = 32;
-__device__ SumScratch g_sumSlots[kSumSlots];
-std::atomic<unsigned> g_sumSlotsUsed{0};
-
-int acquire_sum_slot() {
-  while (true) {
-    unsigned used = g_sumSlotsUsed.load();
-    if (used == 0xffffffffu) {  // all in use: their owners are waiting for the device
-      std::this_thread::yield();
-      continue;
-    }
-    int k = 0;
-    while (used >> k & 1u) ++k;
-    if (g_sumSlotsUsed.compare_exchange_weak(used, used | 1u << k)) return k;
-  }
+  sum_grid(s, &g_sumSlots[slot], out);
 }
 
 __global__ void __launch_bounds__(kSumThreads) k_integral(const double* __restrict__ f, int var, int nVar,
                                                           const double* __restrict__ J, QwArr qw, int P, int nEl,
-                                                          int slot) {
+                                                          int slot, double* out) {
   const int PP = P * P;
   const long long nodes = (long long)PP * nEl;
   double s = 0.0;
@@ -223,7 +260,7 @@ __global__ void __launch_bounds__(kSumThreads) k_integral(const double* __restri
     const long long e = element_of(k, PP, n);
     s += f[n + (size_t)PP * (var + (size_t)nVar * e)] * qw.w[n % P] * qw.w[n / P] * J[k];
   }
-  sum_grid(s, &g_sumSlots[slot]);
+  sum_grid(s, &g_sumSlots[slot], out);
 }
 
 int nt_of(int model) { return model == SELFGPU_MODEL_CIG ? 9 : 3; }
@@ -267,7 +304,6 @@ struct selfgpu_model2d {
   float* mlpB = nullptr;
   double* geo = nullptr;  // packed geometry records (persistent kernel)
   float* gf = nullptr;    // RK register of the FP32-bulk form (P,P,NV,nEl); workSol is unused then
-  SumScratch* sums = nullptr;  // entropy reduction
   // rk3 as one launch of k_fused_resident where the mesh fits: on or off by
   // set_multistep, else wherever the caller has not chosen among the stage
   // launches (set_kernel, set_launch, set_multistage)
@@ -569,15 +605,13 @@ int selfgpu_model2d_create(selfgpu_model2d** out, int model, int N, int nEl, int
     selfgpu_model2d_destroy(m);
     return fail_cuda("selfgpu_model2d_create: trace cache", e);
   }
-  // flags (the first 16 bytes) and the scratch of reductions
-  e = cudaMalloc(&m->dflag, 16 + sizeof(SumScratch));
-  if (e == cudaSuccess) e = cudaMemset(m->dflag, 0, 16 + sizeof(SumScratch));
+  e = cudaMalloc(&m->dflag, 2 * sizeof(int));
+  if (e == cudaSuccess) e = cudaMemset(m->dflag, 0, 2 * sizeof(int));
   if (e != cudaSuccess) {
     selfgpu_model2d_destroy(m);
     return fail_cuda("selfgpu_model2d_create", e);
   }
   m->derr = m->dflag + 1;
-  m->sums = reinterpret_cast<SumScratch*>(m->dflag + 4);
   m->base.err = m->derr;
   m->base.waitCycles = 4000000000LL;  // about 2 s at the B200 boost clock
   m->base.nEl = nEl;
@@ -1238,14 +1272,13 @@ int selfgpu_model2d_entropy(selfgpu_model2d* m, double* entropy) {
   cudaError_t e = cudaSuccess;
   QwArr w{};
   for (int k = 0; k < m->P; ++k) w.w[k] = m->base.qw[k];
-  k_entropy<<<sum_blocks((long long)m->P * m->P * m->nEl), kSumThreads, 0, m->stream>>>(
-      m->model, m->base.q, m->base.J, aux, w, m->P, m->nEl, m->base.g, m->base.gamma, m->sums);
-  e = cudaGetLastError();
+  const int slot = acquire_sum_slot();
+  e = launch_dependent(k_entropy, sum_blocks((long long)m->P * m->P * m->nEl), kSumThreads, m->stream, m->model,
+                       m->base.q, m->base.J, aux, w, m->P, m->nEl, m->base.g, m->base.gamma, slot, sum_target(slot));
   ++m->launches;
   double h = 0.0;
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&h, &m->sums->result, sizeof(double), cudaMemcpyDeviceToHost, m->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
+  if (e == cudaSuccess) e = read_sum(slot, &h, m->stream);
+  release_sum_slot(slot);
   if (e != cudaSuccess) return fail_cuda("selfgpu_model2d_entropy", e);
   *entropy = h;
   return SELFGPU_OK;
@@ -1261,13 +1294,11 @@ int selfgpu_integral_mapped_scalar2d(const double* interior, int iVar, int nVar,
   cudaStream_t st = (cudaStream_t)stream;
   const int slot = acquire_sum_slot();
   k_integral<<<sum_blocks((long long)(N + 1) * (N + 1) * nEl), kSumThreads, 0, st>>>(interior, iVar - 1, nVar, J, w,
-                                                                                 N + 1, nEl, slot);
+                                                                                 N + 1, nEl, slot, sum_target(slot));
   cudaError_t e = cudaGetLastError();
   double h = 0.0;
-  if (e == cudaSuccess)
-    e = cudaMemcpyFromSymbolAsync(&h, g_sumSlots, sizeof(double), slot * sizeof(SumScratch), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  g_sumSlotsUsed.fetch_and(~(1u << slot));
+  if (e == cudaSuccess) e = read_sum(slot, &h, st);
+  release_sum_slot(slot);
   if (e != cudaSuccess) return fail_cuda("selfgpu_integral_mapped_scalar2d", e);
   *result = h;
   return SELFGPU_OK;
