@@ -488,6 +488,12 @@ int selfgpu_cig2d_closure_features(const double* solution, int N, int nEl, const
 int selfgpu_mlp_train(const float* features, const float* labels, int n, int epochs, int batch, float lr,
                       unsigned long long seed, float* params, float* lossPerEpoch, void* stream);
 
+/* The same, and the features' range over the samples: range (host, 72 floats,
+ * may be NULL) receives the 36 minima, then the 36 maxima (NaN for a feature
+ * with a NaN), as set_mlp's parameters hold them. */
+int selfgpu_mlp_train_range(const float* features, const float* labels, int n, int epochs, int batch, float lr,
+                            unsigned long long seed, float* params, float* lossPerEpoch, float* range, void* stream);
+
 /* Inference of the closure MLP over n device feature vectors (36, n) into
  * out (n floats), with the device-side weights layout of set_mlp (host arrays). */
 int selfgpu_mlp_infer(const float* features, int n, const uint16_t* weights, const float* params, float* out,

@@ -65,6 +65,8 @@ _SIGS = {
                                                c_void_p, c_void_p, c_void_p]),
     "selfgpu_mlp_train": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, ctypes.c_float, ctypes.c_ulonglong,
                                   c_void_p, c_void_p, c_void_p]),
+    "selfgpu_mlp_train_range": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, ctypes.c_float, ctypes.c_ulonglong,
+                                        c_void_p, c_void_p, c_void_p, c_void_p]),
     "selfgpu_mlp_infer": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "selfgpu_ckpt_open": (c_int, [ctypes.POINTER(c_void_p), ctypes.c_char_p, c_int]),
     "selfgpu_ckpt_put": (c_int, [c_void_p, ctypes.c_char_p, c_void_p, c_int, c_int, c_void_p, c_int]),

@@ -80,11 +80,12 @@ class ClosureMLP:
         n = features.shape[0]
         f = features.contiguous()
         y = labels.contiguous().to(torch.float32)
-        self.fmin, self.fmax = torch.stack(torch.aminmax(f, dim=0)).cpu().numpy().astype(np.float32)
         loss = np.zeros(epochs, dtype=np.float32)
+        fmin_fmax = np.empty((2, N_IN), dtype=np.float32)
         torch.cuda.synchronize()
-        check(lib().selfgpu_mlp_train(f.data_ptr(), y.data_ptr(), int(n), int(epochs), int(batch), float(lr),
-                                      int(seed), _vp(self.params), _vp(loss), stream))
+        check(lib().selfgpu_mlp_train_range(f.data_ptr(), y.data_ptr(), int(n), int(epochs), int(batch), float(lr),
+                                            int(seed), _vp(self.params), _vp(loss), _vp(fmin_fmax), stream))
+        self.fmin, self.fmax = fmin_fmax
         return loss
 
     def infer(self, features, stream=None):

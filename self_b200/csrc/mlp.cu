@@ -21,6 +21,7 @@
 
 #include <cstring>
 #include <string>
+#include <vector>
 
 #include "av_closure.cuh"
 #include "selfgpu_internal.h"
@@ -209,6 +210,65 @@ __global__ void __launch_bounds__(256) k_adam(float* master, const float* part, 
   }
 }
 
+// Minimum and maximum of each feature over the samples (NaN where one is NaN),
+// by the last of the blocks to finish.  Consecutive threads read consecutive
+// values; a thread's values all belong to its own feature.  (Two reductions by
+// the caller's tensor library with a copy each: 79 us for 16 384 samples; this
+// kernel's result comes back with the trained weights.)
+constexpr int kRangeBlocks = 148, kRangeRows = 8, kRangeThreads = kRangeRows * IN;
+struct RangeScratch {
+  float result[2 * IN];  // minima, maxima
+  unsigned done;         // zero before the launch
+  float part[kRangeBlocks][2 * IN];
+};
+__device__ __forceinline__ float min_nan(float a, float b) { return a != a ? a : (b < a || b != b ? b : a); }
+__device__ __forceinline__ float max_nan(float a, float b) { return a != a ? a : (b > a || b != b ? b : a); }
+__global__ void __launch_bounds__(kRangeThreads) k_range(const float* __restrict__ feat, int n, RangeScratch* x) {
+  __shared__ float slo[kRangeRows][IN], shi[kRangeRows][IN];
+  __shared__ bool last;
+  const int t = threadIdx.x, r = t / IN, c = t - r * IN;
+  const float first = feat[c];
+  float lo = first, hi = first;
+  for (long long row = (long long)blockIdx.x * kRangeRows + r; row < n; row += (long long)gridDim.x * kRangeRows) {
+    const float v = feat[row * IN + c];
+    lo = min_nan(lo, v);
+    hi = max_nan(hi, v);
+  }
+  auto block_range = [&]() {  // over the rows of threads, on the first
+    slo[r][c] = lo;
+    shi[r][c] = hi;
+    __syncthreads();
+    if (r == 0)
+      for (int k = 1; k < kRangeRows; ++k) {
+        lo = min_nan(lo, slo[k][c]);
+        hi = max_nan(hi, shi[k][c]);
+      }
+  };
+  block_range();
+  if (r == 0) {
+    x->part[blockIdx.x][c] = lo;
+    x->part[blockIdx.x][IN + c] = hi;
+    __threadfence();
+  }
+  __syncthreads();
+  if (t == 0) {
+    last = atomicAdd(&x->done, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  lo = hi = first;
+  for (int b = r; b < (int)gridDim.x; b += kRangeRows) {
+    lo = min_nan(lo, __ldcg(&x->part[b][c]));
+    hi = max_nan(hi, __ldcg(&x->part[b][IN + c]));
+  }
+  block_range();
+  if (r == 0) {
+    x->result[c] = lo;
+    x->result[IN + c] = hi;
+  }
+}
+
 // Weights (bfloat16 pairs) and parameters, passed by value: no device buffer
 // and no copy per call.
 struct MlpArgs {
@@ -281,20 +341,33 @@ extern "C" {
 
 int selfgpu_mlp_train(const float* features, const float* labels, int n, int epochs, int batch, float lr,
                       unsigned long long seed, float* params, float* lossPerEpoch, void* stream) {
+  return selfgpu_mlp_train_range(features, labels, n, epochs, batch, lr, seed, params, lossPerEpoch, nullptr, stream);
+}
+
+int selfgpu_mlp_train_range(const float* features, const float* labels, int n, int epochs, int batch, float lr,
+                            unsigned long long seed, float* params, float* lossPerEpoch, float* range, void* stream) {
   if (!features || !labels || n < 1 || epochs < 0 || batch < 1 || batch > (1 << 22) || !(lr > 0.f) || !params)
     return set_error(SELFGPU_ERR_ARG, "selfgpu_mlp_train: bad arguments");
   cudaStream_t st = (cudaStream_t)stream;
   const int tiles = (batch + kTile - 1) / kTile;
   const int blocks = tiles < kMaxGradBlocks ? tiles : kMaxGradBlocks;
-  // master, m1, m2, the per-epoch losses (zeroed) and the blocks' partial sums
-  const size_t fixed = 3 * (size_t)NP + epochs, total = fixed + (size_t)blocks * (NPP + 1);
+  // master and the per-epoch losses, which come back in one copy with the
+  // features' range, m1 and m2 (all zeroed), and the blocks' partial sums
+  const size_t rangeAt = NP + (size_t)epochs, back = rangeAt + (range ? 2 * IN : 0);
+  const size_t scratch = range ? sizeof(RangeScratch) / sizeof(float) : 0;
+  const size_t fixed = rangeAt + scratch + 2 * (size_t)NP, total = fixed + (size_t)blocks * (NPP + 1);
+  std::vector<float> host(back);
   float* buf = nullptr;
   cudaError_t e = cudaMalloc(&buf, total * sizeof(float));
   if (e != cudaSuccess) return fail("selfgpu_mlp_train", e);
-  float *master = buf, *m1 = buf + NP, *m2 = buf + 2 * NP, *loss = buf + 3 * NP, *part = buf + fixed,
+  float *master = buf, *loss = buf + NP, *m1 = buf + rangeAt + scratch, *m2 = m1 + NP, *part = buf + fixed,
         *lossPart = part + (size_t)blocks * NPP;
   e = cudaMemsetAsync(buf, 0, fixed * sizeof(float), st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(master, params, NP * sizeof(float), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess && range) {
+    k_range<<<kRangeBlocks, kRangeThreads, 0, st>>>(features, n, reinterpret_cast<RangeScratch*>(buf + rangeAt));
+    e = cudaGetLastError();
+  }
   const long long stepsPerEpoch = ((long long)n + batch - 1) / batch;
   long long t = 0;
   float c1 = 1.f, c2 = 1.f;
@@ -308,14 +381,14 @@ int selfgpu_mlp_train(const float* features, const float* labels, int n, int epo
                              1.f - c1, 1.f - c2);
     }
   }
-  if (e == cudaSuccess && lossPerEpoch && epochs > 0)
-    e = cudaMemcpyAsync(lossPerEpoch, loss, epochs * sizeof(float), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(params, master, NP * sizeof(float), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(host.data(), buf, back * sizeof(float), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   cudaFree(buf);
   if (e != cudaSuccess) return fail("selfgpu_mlp_train", e);
+  std::memcpy(params, host.data(), NP * sizeof(float));
   if (lossPerEpoch)
-    for (int ep = 0; ep < epochs; ++ep) lossPerEpoch[ep] /= (float)(stepsPerEpoch * batch);
+    for (int ep = 0; ep < epochs; ++ep) lossPerEpoch[ep] = host[NP + ep] / (float)(stepsPerEpoch * batch);
+  if (range) std::memcpy(range, host.data() + rangeAt, 2 * IN * sizeof(float));
   return SELFGPU_OK;
 }
 

@@ -276,6 +276,19 @@ def test_training_steps_match_float64(n, batch):
     np.testing.assert_allclose(loss, ref, rtol=1e-2 if steps > 4 else 1e-4)
 
 
+@pytest.mark.parametrize("n", [1, 7, 1185, 30001])  # fewer rows than a block's; one row more than a sweep; several
+@pytest.mark.parametrize("nan", [False, True])
+def test_feature_range_of_a_training_set(n, nan):
+    from self_b200 import closure as CL
+    f = np.random.default_rng(n).standard_normal((n, 36)).astype(np.float32)
+    if nan:
+        f[n // 2, 5] = np.nan
+    m = CL.ClosureMLP(seed=0)
+    m.train(torch.from_numpy(f).cuda(), torch.zeros(n, device="cuda"), epochs=0, batch=8)
+    np.testing.assert_array_equal(m.fmin, f.min(axis=0))
+    np.testing.assert_array_equal(m.fmax, f.max(axis=0))
+
+
 @pytest.mark.parametrize("n", [1, 31, 33, 37921])  # a short tile; more tiles than blocks
 def test_inference_tiles(n):
     """The clamped output against the restatement, to 1e-5 (float32 sums of 36 and 32 products of order one)."""
