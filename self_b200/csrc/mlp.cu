@@ -68,9 +68,28 @@ __global__ void __launch_bounds__(kGradThreads) k_grad(const float* feat, const 
   // activations and deltas [sample][unit]; the odd strides keep the lanes'
   // (one sample each) accesses to one unit in distinct banks
   __shared__ float sw[NP], F[kTile][IN + 1], H1[kTile][H + 1], H2[kTile][H + 1], D1[kTile][H + 1], D2[kTile][H + 1];
-  __shared__ float sz[kTile], sg[kTile];
+  __shared__ float sy[kTile], sg[kTile];
   __shared__ long long sidx[kTile];
   const int t = threadIdx.x, s = t & 31, w = t >> 5;
+  auto gather = [&](int tile) {  // the tile's samples
+    if (t < kTile) {
+      const long long b = (long long)tile * kTile + t;
+      const long long idx = b < batch ? (long long)(mix64(seed ^ mix64((unsigned long long)step * 0x100000001ull +
+                                                                       (unsigned long long)b)) %
+                                                    (unsigned long long)n)
+                                      : -1;
+      sidx[t] = idx;
+      sy[t] = idx >= 0 ? label[idx] : 0.f;
+    }
+    __syncthreads();
+    for (int k = t; k < kTile * IN; k += kGradThreads) {
+      const int r = k / IN, c = k - r * IN;
+      const long long idx = sidx[r];
+      F[r][c] = idx >= 0 ? feat[c + (long long)IN * idx] : 0.f;
+    }
+  };
+  // the first tile's samples, which no step changes, before the wait
+  gather(blockIdx.x);
   asm volatile("griddepcontrol.wait;" ::: "memory");  // the previous step's weights
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   for (int k = t; k < NP; k += kGradThreads) {
@@ -85,21 +104,11 @@ __global__ void __launch_bounds__(kGradThreads) k_grad(const float* feat, const 
   for (int k = 0; k < 9; ++k) acc[k] = 0.f;
   const int tiles = (batch + kTile - 1) / kTile;
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    __syncthreads();  // the weights, or the previous tile's arrays
-    if (t < kTile) {
-      const long long b = (long long)tile * kTile + t;
-      sidx[t] = b < batch ? (long long)(mix64(seed ^ mix64((unsigned long long)step * 0x100000001ull +
-                                                           (unsigned long long)b)) %
-                                        (unsigned long long)n)
-                          : -1;
+    __syncthreads();  // the weights and the first tile, or the previous tile's arrays
+    if (tile != (int)blockIdx.x) {
+      gather(tile);
+      __syncthreads();
     }
-    __syncthreads();
-    for (int k = t; k < kTile * IN; k += kGradThreads) {
-      const int r = k / IN, c = k - r * IN;
-      const long long idx = sidx[r];
-      F[r][c] = idx >= 0 ? feat[c + (long long)IN * idx] : 0.f;
-    }
-    __syncthreads();
 #pragma unroll
     for (int u = 0; u < 4; ++u) {  // lane = sample, warp = 4 hidden units
       const int j = 4 * w + u;
@@ -126,7 +135,7 @@ __global__ void __launch_bounds__(kGradThreads) k_grad(const float* feat, const 
       for (int k = 0; k < H; ++k) z = fmaf(sw[oW3 + k], H2[s][k], z);
       z = z + sw[oB3];
       const long long idx = sidx[s];
-      const float y = idx >= 0 ? label[idx] : 0.f;
+      const float y = sy[s];
       const float a = z < 0.f ? 0.f : (z > 1.f ? 1.f : z);
       float d = a - y;
       if ((z < 0.f && y > 0.f) || (z > 1.f && y < 1.f)) d = z - y;  // straight through the clamp
@@ -186,6 +195,10 @@ __global__ void __launch_bounds__(256) k_adam(float* master, const float* part, 
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int k = blockIdx.x * 32 + lane;
+  // what the previous step's k_adam wrote is complete: k_grad lets this kernel
+  // start only after its own wait for it
+  float m1k = 0.f, m2k = 0.f, mk = 0.f;
+  if (w == 0 && k < NP) m1k = m1[k], m2k = m2[k], mk = master[k];
   asm volatile("griddepcontrol.wait;" ::: "memory");  // this step's partial sums
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   float s = 0.f;
@@ -197,10 +210,10 @@ __global__ void __launch_bounds__(256) k_adam(float* master, const float* part, 
     float gk = 0.f;
 #pragma unroll
     for (int r = 0; r < 8; ++r) gk += strip[r][lane];
-    m1[k] = b1 * m1[k] + (1.f - b1) * gk;
-    m2[k] = b2 * m2[k] + (1.f - b2) * gk * gk;
-    const float mh = m1[k] / c1, vh = m2[k] / c2;
-    master[k] -= lr * mh / (sqrtf(vh) + eps);
+    m1[k] = m1k = b1 * m1k + (1.f - b1) * gk;
+    m2[k] = m2k = b2 * m2k + (1.f - b2) * gk * gk;
+    const float mh = m1k / c1, vh = m2k / c2;
+    master[k] = mk - lr * mh / (sqrtf(vh) + eps);
   }
   if (blockIdx.x == 0 && w == 1) {
     float l = 0.f;
