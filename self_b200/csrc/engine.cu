@@ -1,8 +1,9 @@
 // The fused tendency engine behind selfgpu_model2d_*: binds the caller's
 // (Fortran-owned) device buffers, owns the ping-pong face-trace cache, and
-// drives the fused stage kernel through Williamson RK3 steps.  One RK step is
-// three launches; after the first step of a given dt the step is replayed from
-// a captured CUDA graph.
+// drives the stage kernels through Williamson RK3 steps: all steps of a call in
+// one launch on small meshes (fused_resident.cuh) and on some at degree 7, else
+// three launches per step, which after the first step of a given dt are
+// replayed from a captured CUDA graph.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -21,10 +21,12 @@
 // one face exchange: solution and G read+write, metric terms read once, own
 // traces written once, neighbour traces read once.
 //
-// Two kernels implement this: k_fused_stage (below; one CTA of P*P-thread
-// element groups, plain loads; any degree) and k_fused_stage_tma
-// (fused_stage_tma.cuh; persistent, bulk-async copies into a shared-memory
-// ring).  Both share the model policies and the trace-cache layout.
+// Three kernels implement this: k_fused_stage_tma (fused_stage_tma.cuh;
+// persistent, bulk-async copies into a shared-memory ring), k_fused_resident
+// (fused_resident.cuh; all stages of a call with the state on chip, for small
+// meshes) and k_fused_stage (below; one CTA of P*P-thread element groups, plain
+// loads; any degree and alignment, the fallback).  They share the model
+// policies; the first and the last share the trace-cache layout.
 #pragma once
 
 #include <cuda_runtime.h>

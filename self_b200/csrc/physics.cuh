@@ -1,6 +1,6 @@
 // Point-wise physics of the three 2-D models, shared by the drop-in
-// per-operator kernels (legacy_ops.cu) and the fused stage kernel
-// (fused_stage.cu).  Each function restates one CPU branch of the reference
+// per-operator kernels (legacy_ops.cu) and the stage kernels (fused_stage*.cuh,
+// fused_resident.cuh).  Each function restates one CPU branch of the reference
 // with the same left-to-right evaluation order; `R` is the bulk arithmetic
 // type (double for the parity form, float for the FP32-bulk form) and normals
 // and face scales always arrive in double.
