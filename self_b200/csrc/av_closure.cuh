@@ -450,7 +450,9 @@ constexpr int av_elems_per_block() {
 // variable, traces): a thread per (node, variable) and the face metrics in
 // shared memory.  (One thread per node doing its four variables in turn, the
 // metrics read from global memory for each: 12 us for the 5 % of 10 560
-// elements at P = 8 in FP64 that a shock band activates.)
+// elements at P = 8 in FP64 that a shock band activates.  Each value stored to
+// shared memory as it came, so that the loads waited for one another: 9.1 us on
+// the 256x256 Riemann problem at P = 6 in FP32, now 8.1.)
 template <int P, typename R, int EPB>
 __global__ void __launch_bounds__(EPB * 4 * P * P) k_av_grad(const AvArgs a) {
   constexpr int PP = P * P, N = P - 1, VS = visc_side_stride<P>(), TPE = 4 * PP;
@@ -474,36 +476,29 @@ __global__ void __launch_bounds__(EPB * 4 * P * P) k_av_grad(const AvArgs a) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const R* trIn = reinterpret_cast<const R*>(a.trIn);
+  // this thread's entry of the list, read along with the count
+  long long base = (long long)blockIdx.x * EPB;
+  int first = base + slot < a.nEl ? a.activeList[base + slot] : 0;
   const int count = *a.activeCount;
   // every block runs the same number of rounds (block-uniform barriers)
-  for (int base = blockIdx.x * EPB; base < count; base += gridDim.x * EPB) {
+  for (; base < count; base += (long long)gridDim.x * EPB) {
     const bool live = base + slot < count;
-    const long long e = live ? a.activeList[base + slot] : 0;
+    const long long e = live ? first : 0;
+    first = base + slot + (long long)gridDim.x * EPB < a.nEl ? a.activeList[base + slot + (long long)gridDim.x * EPB] : 0;
     R nu = (R)0, Jij = (R)1;
     if (live) {
-      sm.q[v][t] = (R)a.q[t + (long long)PP * (v + 4 * e)];
-      sm.dsdx[v][t] = (R)a.dsdx[v + 4 * (t + (long long)PP * e)];
-      nu = (R)a.nu[e];
-      Jij = (R)a.J[t + (long long)PP * e];
-      for (int k = u; k < 4 * P; k += TPE) {
-        const int s1 = k / P, ii = k % P;
-        sm.nh[s1][ii][0] = (R)a.nHat[2 * (k + (long long)P * 4 * e)];
-        sm.nh[s1][ii][1] = (R)a.nHat[2 * (k + (long long)P * 4 * e) + 1];
-        sm.ns[s1][ii] = (R)a.nScale[k + (long long)P * 4 * e];
-      }
-      // averaged conservative traces (BassiRebaySides) with the stage's exterior states
-      for (int k = u; k < 16 * P; k += TPE) {
+      // averaged conservative traces (BassiRebaySides) with the stage's
+      // exterior states; the first task's connectivity, then all the element's
+      // values, are requested before any is used
+      auto trace_average = [&](int k, int si2, int si3, int bcid, R L) {
         const int w = k / (4 * P), c = k - w * 4 * P, s1 = c / P, ii = c % P;
-        const int* si = a.sideInfo + 5 * (s1 + 4 * e);
         const R* own = trIn + (long long)TS * (s1 + 4 * e) + ii;
-        const R L = own[P * w];
         R X = (R)0;
-        const int bcid = si[4];
         if (bcid == 0) {
-          const long long e2 = si[2] - 1;
-          const int s2 = si[3] / 10 - 1, flip = si[3] % 10;
+          const long long e2 = si2 - 1;
+          const int s2 = si3 / 10 - 1, flip = si3 % 10;
           X = trIn[(long long)TS * (s2 + 4 * e2) + (flip ? N - ii : ii) + P * w];
-        } else if (si[2] == 0) {  // physical side: the boundary condition's exterior state
+        } else if (si2 == 0) {  // physical side: the boundary condition's exterior state
           if (bcid == SG_BC_NONORMALFLOW) {
             if (w < 2) {
               const double* nh = a.nHat + 2 * (ii + (long long)P * (s1 + 4 * e));
@@ -517,7 +512,40 @@ __global__ void __launch_bounds__(EPB * 4 * P * P) k_av_grad(const AvArgs a) {
             X = (R)a.presc[ii + (long long)P * (w + 4 * (s1 + 4 * e))];
           }
         }
-        sm.avg[s1][w][ii] = (R)0.5 * (L + X);
+        return (R)0.5 * (L + X);
+      };
+      int si2 = 0, si3 = 0, si4 = 1;
+      R L = (R)0, X = (R)0;
+      const int tw = u / (4 * P), tc = u - tw * 4 * P, ts = tc / P, ti = tc % P;
+      if (u < 16 * P) {
+        const int* si = a.sideInfo + 5 * (ts + 4 * e);
+        si2 = si[2], si3 = si[3], si4 = si[4];
+        L = trIn[(long long)TS * (ts + 4 * e) + ti + P * tw];
+      }
+      const double qv = a.q[t + (long long)PP * (v + 4 * e)], dv = a.dsdx[v + 4 * (t + (long long)PP * e)];
+      const double nuE = a.nu[e], Jv = a.J[t + (long long)PP * e];
+      double n1 = 0.0, n2 = 0.0, ns = 0.0;
+      if (u < 4 * P) {
+        n1 = a.nHat[2 * (u + (long long)P * 4 * e)];
+        n2 = a.nHat[2 * (u + (long long)P * 4 * e) + 1];
+        ns = a.nScale[u + (long long)P * 4 * e];
+      }
+      if (u < 16 * P) X = trace_average(u, si2, si3, si4, L);
+      nu = (R)nuE;
+      Jij = (R)Jv;
+      sm.q[v][t] = (R)qv;
+      sm.dsdx[v][t] = (R)dv;
+      if (u < 4 * P) {
+        sm.nh[u / P][u % P][0] = (R)n1;
+        sm.nh[u / P][u % P][1] = (R)n2;
+        sm.ns[u / P][u % P] = (R)ns;
+      }
+      if (u < 16 * P) sm.avg[ts][tw][ti] = X;
+      for (int k = u + TPE; k < 16 * P; k += TPE) {  // (P = 2 and 3)
+        const int w = k / (4 * P), c = k - w * 4 * P, s1 = c / P, ii = c % P;
+        const int* si = a.sideInfo + 5 * (s1 + 4 * e);
+        const R Lk = trIn[(long long)TS * (s1 + 4 * e) + ii + P * w];
+        sm.avg[s1][w][ii] = trace_average(k, si[2], si[3], si[4], Lk);
       }
     }
     __syncthreads();
