@@ -652,6 +652,10 @@ __device__ __forceinline__ void cig_fields_rounded(float* f, float gamma) {
 // BoundaryInterp(solution)) of a solution set from outside.  Bound by memory:
 // the solution read, the traces written.  Blocks of 256 threads, one node per
 // thread, with only the node fields in shared memory: 2 048 threads per SM.
+// At P = 8 CompressibleIdealGas2D's sums take an orientation per warp (FP32
+// 256x256 77.9 -> 71.8 us, FP64 128x128 19.7 -> 18.6; ShallowWater 25.8 -> 26.8).
+// Persistent blocks that load the next elements during the sums were slower
+// (FP64 128x128 24.7-26.7 us).
 template <int P, class Phys, typename R>
 struct TraceBlock {
   static constexpr int elems = 256 / (P * P), threads = elems * P * P;
@@ -677,7 +681,8 @@ __global__ void __launch_bounds__(TraceBlock<P, Phys, R>::threads) k_traces(cons
   }
   __syncthreads();
   R* trOut = reinterpret_cast<R*>(a.trOut) + (size_t)4 * TS * e0;
-  tile_traces<P, Phys, R, false>(sm, NT * FS, EPB, live, t, NTH, a, [&](int eE, int fi, int l, bool row, R lo, R hi) {
+  tile_traces<P, Phys, R, P == 8 && NV == 4>(sm, NT * FS, EPB, live, t, NTH, a,
+                                             [&](int eE, int fi, int l, bool row, R lo, R hi) {
     R* o = trOut + 4 * TS * eE + l + P * fi;
     o[TS * (row ? 3 : 0)] = lo;
     o[TS * (row ? 1 : 2)] = hi;
