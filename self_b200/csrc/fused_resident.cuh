@@ -412,8 +412,28 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::TPE, ResTraits<P, Phys,
           }
         }
       }
+      // ShallowWater: the next stage's lagged velocities are those of this stage's
+      // traces (and, after SetSolution, the first stage's too); walls keep velR =
+      // 0.  With kAhead the side's own is formed before the neighbour's traces are
+      // waited for and the neighbour's after the barrier: at P = 8 with one tile
+      // per CTA a stage on 10x10 / 34x34 takes 1.59 / 2.09 us instead of 1.72 /
+      // 2.28 in FP64, 2.39 / 3.50 instead of 2.68 / 3.89 with the reference's
+      // roundings, 1.39 / 1.72 instead of 1.48 / 1.79 in FP32; with several tiles
+      // 2-10 % slower, at P = 4 to 6 between 8 % faster and 7 % slower.
+      constexpr bool kAhead = kSW && !kMany && P == 8;
+      constexpr bool kDivide = ref_rounding<R>() || (T::kOdd && sizeof(R) == 4);  // as the stage launches
+      auto velocity = [&](const R* tr, R v[2], bool divide) {
+        if (divide) {
+          v[0] = tr[0] / tr[2];
+          v[1] = tr[1] / tr[2];
+        } else {
+          const R rH = (R)1 / tr[2];
+          v[0] = tr[0] * rH;
+          v[1] = tr[1] * rH;
+        }
+      };
+      R L[NT], Xn[NT], nextL[2] = {(R)0, (R)0};
       if (faceOn) {
-        R L[NT], Xn[NT];
         if (cached) {
           const R* tr = reinterpret_cast<const R*>(ra.trIn);
 #pragma unroll
@@ -433,6 +453,7 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::TPE, ResTraits<P, Phys,
 #pragma unroll
             for (int f = 0; f < NT; ++f) L[f] = own[P * f];
           }
+          if constexpr (kAhead) velocity(L, nextL, kDivide);
 #pragma unroll
           for (int f = 0; f < NT; ++f) Xn[f] = (R)0;
           if (nbBlk >= 0) {
@@ -455,33 +476,23 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::TPE, ResTraits<P, Phys,
           if (physical) face_aux_global<Phys>(a, s1, ii, eF, P, fx);
         R vL[2] = {velL[0], velL[1]}, vR[2] = {velR[0], velR[1]};  // this stage's lagged velocities
         if constexpr (kSW) {
-          // the next stage's are this stage's traces' (and, after SetSolution,
-          // the first stage's too); walls keep velR = 0
-          constexpr bool kDivide = ref_rounding<R>() || (T::kOdd && sizeof(R) == 4);  // as the stage launches
-          auto velocity = [&](const R* tr, R v[2], bool divide) {
-            if (divide) {
-              v[0] = tr[0] / tr[2];
-              v[1] = tr[1] / tr[2];
-            } else {
-              const R rH = (R)1 / tr[2];
-              v[0] = tr[0] * rH;
-              v[1] = tr[1] * rH;
-            }
-          };
-          if (s == 0 && ra.fresh) {
-            velocity(L, vL, true);
-            if (nbBlk >= 0) velocity(Xn, vR, true);
+          if (cached || !kAhead) velocity(L, nextL, kDivide);
+          if constexpr (!kAhead) {
+            velL[0] = nextL[0], velL[1] = nextL[1];
+            if (nbBlk >= 0) velocity(Xn, velR, kDivide);
           }
-          velocity(L, velL, kDivide);
-          if (nbBlk >= 0) velocity(Xn, velR, kDivide);
           if constexpr (kMany) {
             R* sv = tile_vel(k);
             sv[0] = velL[0], sv[X::faces] = velL[1], sv[2 * X::faces] = velR[0], sv[3 * X::faces] = velR[1];
           }
+          if (s == 0 && ra.fresh) {
+            velocity(L, vL, true);
+            if (nbBlk >= 0) velocity(Xn, vR, true);
+          }
           if (last) {
             R* vo = reinterpret_cast<R*>(ra.velOut);
-            vo[ii + P * (0 + 2 * (s1 + 4 * eF))] = velL[0];
-            vo[ii + P * (1 + 2 * (s1 + 4 * eF))] = velL[1];
+            vo[ii + P * (0 + 2 * (s1 + 4 * eF))] = nextL[0];
+            vo[ii + P * (1 + 2 * (s1 + 4 * eF))] = nextL[1];
           }
         }
         R out[NV];
@@ -492,6 +503,11 @@ __global__ void __launch_bounds__(TmaTraits<P, Phys, R>::TPE, ResTraits<P, Phys,
       __syncthreads();  // volume sums and face fluxes
       if (!sOk) break;
 
+      if constexpr (kAhead)
+        if (faceOn) {
+          velL[0] = nextL[0], velL[1] = nextL[1];
+          if (nbBlk >= 0) velocity(Xn, velR, kDivide);
+        }
       if (active) {
         double Src[NV];
         Phys::template source<double>(q, na, a, Src);
