@@ -195,12 +195,12 @@ __global__ void __launch_bounds__(256) k_adam(float* master, const float* part, 
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int k = blockIdx.x * 32 + lane;
-  // what the previous step's k_adam wrote is complete: k_grad lets this kernel
-  // start only after its own wait for it
-  float m1k = 0.f, m2k = 0.f, mk = 0.f;
-  if (w == 0 && k < NP) m1k = m1[k], m2k = m2[k], mk = master[k];
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // this step's partial sums
+  // Only this wait makes earlier grids' writes visible here: this step's partial
+  // sums, and the moments and weights of the previous step's k_adam.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  float m1k = 0.f, m2k = 0.f, mk = 0.f;  // in flight during the sums
+  if (w == 0 && k < NP) m1k = m1[k], m2k = m2[k], mk = master[k];
   float s = 0.f;
   if (k < NP)
     for (int r = w; r < blocks; r += 8) s += part[(size_t)NPP * r + k];
