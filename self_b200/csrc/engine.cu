@@ -220,10 +220,9 @@ double* sum_target(int slot) { return sum_results() ? sum_results() + slot : nul
 //   CIG  rho (log p - gamma log rho) / (gamma - 1) w_i w_j J, p from the
 //        solution as ConservativeToPrimitive forms it (src/models/SELF_CompressibleIdealGas2D.f90:782-823)
 // `aux` is H (LSW) or the topography b (SW), (P,P,1,nEl).
-__global__ void __launch_bounds__(kSumThreads) k_entropy(int model, const double* __restrict__ q,
-                                                         const double* __restrict__ J, const double* __restrict__ aux,
-                                                         QwArr qw, int P, int nEl, double g, double gamma,
-                                                         int slot, double* out) {
+__global__ void __launch_bounds__(kSumThreads) k_entropy(int model, const double* q, const double* J,
+                                                         const double* aux, QwArr qw, int P, int nEl, double g,
+                                                         double gamma, int slot, double* out) {
   asm volatile("griddepcontrol.wait;" ::: "memory");  // the stage that forms q
   const int PP = P * P, nv = model == SELFGPU_MODEL_CIG ? 4 : 3;
   const long long nodes = (long long)PP * nEl;

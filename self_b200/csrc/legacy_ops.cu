@@ -43,7 +43,10 @@ inline void check_launch(const char* name) {
 // and its first blocks' start overlap that kernel's last wave.  The first thing
 // each does is to let its own successor start and to wait for the previous
 // kernel's completion, before it touches any data.  (64x64 elements, N = 7, the
-// operators of one right-hand side: 152 us without, 113 with.)
+// operators of one right-hand side: 152 us without, 113 with.)  No pointer is
+// __restrict__: the previous kernel may write what this one reads while this
+// one is already running, and the qualifier would let the compiler read it
+// through the non-coherent path or ahead of the wait.
 __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -76,8 +79,8 @@ __device__ __forceinline__ long long divide(long long k, int d, int& rem) {
 // Run-time degrees (N > 7) and target grids too large for a block's shared
 // memory: one thread per output, operands from global memory.
 // src/SELF_Lagrange.f90:741-789; iM(ii,m) at iM[ii + P*m]
-__global__ void k_scalar_grid_interp(const double* __restrict__ iM, const double* __restrict__ f,
-                                     double* __restrict__ fo, int N, int M, long long n) {
+__global__ void k_scalar_grid_interp(const double* iM, const double* f,
+                                     double* fo, int N, int M, long long n) {
   after_previous();
   const int P = N + 1, Q = M + 1;
   GRID_STRIDE(k, n) {
@@ -95,8 +98,8 @@ __global__ void k_scalar_grid_interp(const double* __restrict__ iM, const double
 }
 
 // src/SELF_Lagrange.f90:824-875
-__global__ void k_vector_grid_interp(const double* __restrict__ iM, const double* __restrict__ f,
-                                     double* __restrict__ fo, int N, int M, long long n) {
+__global__ void k_vector_grid_interp(const double* iM, const double* f,
+                                     double* fo, int N, int M, long long n) {
   after_previous();
   const int P = N + 1, Q = M + 1;
   GRID_STRIDE(k, n) {  // k enumerates (dir, i, j, var*el)
@@ -116,8 +119,8 @@ __global__ void k_vector_grid_interp(const double* __restrict__ iM, const double
 }
 
 // src/SELF_Lagrange.f90:2241-2270; one thread per (i, var, el) writes 4 sides
-__global__ void k_scalar_boundary_interp(const double* __restrict__ bM, const double* __restrict__ f,
-                                         double* __restrict__ fb, int N, int nVar, long long n) {
+__global__ void k_scalar_boundary_interp(const double* bM, const double* f,
+                                         double* fb, int N, int nVar, long long n) {
   after_previous();
   const int P = N + 1;
   GRID_STRIDE(k, n) {
@@ -144,8 +147,8 @@ __global__ void k_scalar_boundary_interp(const double* __restrict__ bM, const do
 
 // src/SELF_Lagrange.f90:2284-2316 (C = 2) and 2330-2366 (C = 4): components fastest
 template <int C>
-__global__ void k_multi_boundary_interp(const double* __restrict__ bM, const double* __restrict__ f,
-                                        double* __restrict__ fb, int N, int nVar, long long n) {
+__global__ void k_multi_boundary_interp(const double* bM, const double* f,
+                                        double* fb, int N, int nVar, long long n) {
   after_previous();
   const int P = N + 1;
   GRID_STRIDE(k, n) {  // k enumerates (comp, i, var, el)
@@ -172,8 +175,8 @@ __global__ void k_multi_boundary_interp(const double* __restrict__ bM, const dou
 }
 
 // src/SELF_Lagrange.f90:1424-1463
-__global__ void k_vector_gradient_any(const double* __restrict__ dM, const double* __restrict__ f,
-                                      double* __restrict__ gf, int N, long long n) {
+__global__ void k_vector_gradient_any(const double* dM, const double* f,
+                                      double* gf, int N, long long n) {
   after_previous();
   const int P = N + 1;
   GRID_STRIDE(k, n) {  // k enumerates (i, j, var*el)
@@ -196,9 +199,9 @@ __global__ void k_vector_gradient_any(const double* __restrict__ dM, const doubl
 }
 
 // src/SELF_Lagrange.f90:1589-1625
-__global__ void k_vector_dg_divergence_any(const double* __restrict__ dgM, const double* __restrict__ bM,
-                                       const double* __restrict__ qw, const double* __restrict__ f,
-                                       const double* __restrict__ bf, double* __restrict__ df, int N, int nVar,
+__global__ void k_vector_dg_divergence_any(const double* dgM, const double* bM,
+                                       const double* qw, const double* f,
+                                       const double* bf, double* df, int N, int nVar,
                                        long long n) {
   after_previous();
   const int P = N + 1;
@@ -230,8 +233,8 @@ __host__ __device__ constexpr int row_stride(int P) { return P | 1; }
 // iM[ii + P*m].  The xi sums of a row are formed once for all eta targets (the
 // reference's order per value).
 template <int P, int C>
-__global__ void __launch_bounds__(kThreads) k_grid_interp(const double* __restrict__ iM,
-                                                          const double* __restrict__ f, double* __restrict__ fo, int M,
+__global__ void __launch_bounds__(kThreads) k_grid_interp(const double* iM,
+                                                          const double* f, double* fo, int M,
                                                           int planes, long long nPlanes) {
   after_previous();
   extern __shared__ double sm[];
@@ -271,8 +274,8 @@ __global__ void __launch_bounds__(kThreads) k_grid_interp(const double* __restri
 // src/SELF_Lagrange.f90:2241-2270 (C = 1), 2284-2316 (C = 2) and 2330-2366
 // (C = 4): components fastest; one task per (component, node, side, plane)
 template <int P, int C>
-__global__ void __launch_bounds__(kThreads) k_boundary_interp(const double* __restrict__ bM,
-                                                              const double* __restrict__ f, double* __restrict__ fb,
+__global__ void __launch_bounds__(kThreads) k_boundary_interp(const double* bM,
+                                                              const double* f, double* fb,
                                                               int nVar, int planes, long long nPlanes) {
   after_previous();
   extern __shared__ double sm[];
@@ -321,16 +324,16 @@ struct NodeBlock {
 
 // column i of a P x P matrix at m[ii + P i]
 template <int P>
-__device__ __forceinline__ void load_column(const double* __restrict__ m, int i, double c[P]) {
+__device__ __forceinline__ void load_column(const double* m, int i, double c[P]) {
 #pragma unroll
   for (int ii = 0; ii < P; ++ii) c[ii] = m[ii + P * i];
 }
 
 // src/SELF_Lagrange.f90:1424-1463
 template <int P>
-__global__ void __launch_bounds__(NodeBlock<P>::threads, 3) k_vector_gradient(const double* __restrict__ dM,
-                                                                           const double* __restrict__ f,
-                                                                           double* __restrict__ gf,
+__global__ void __launch_bounds__(NodeBlock<P>::threads, 3) k_vector_gradient(const double* dM,
+                                                                           const double* f,
+                                                                           double* gf,
                                                                            long long nPlanes) {
   after_previous();
   using B = NodeBlock<P>;
@@ -377,8 +380,8 @@ __global__ void __launch_bounds__(NodeBlock<P>::threads, 3) k_vector_gradient(co
 // src/SELF_Lagrange.f90:1589-1625
 template <int P>
 __global__ void __launch_bounds__(NodeBlock<P>::threads, 3) k_vector_dg_divergence(
-    const double* __restrict__ dgM, const double* __restrict__ bM, const double* __restrict__ qw,
-    const double* __restrict__ f, const double* __restrict__ bf, double* __restrict__ df, int nVar,
+    const double* dgM, const double* bM, const double* qw,
+    const double* f, const double* bf, double* df, int nVar,
     long long nPlanes) {
   after_previous();
   using B = NodeBlock<P>;
@@ -421,7 +424,7 @@ __global__ void __launch_bounds__(NodeBlock<P>::threads, 3) k_vector_dg_divergen
 }
 
 // src/SELF_Data.f90:1570-1607
-__global__ void k_determinant(const double* __restrict__ t, double* __restrict__ det, long long n) {
+__global__ void k_determinant(const double* t, double* det, long long n) {
   after_previous();
   GRID_STRIDE(k, n) {
     const double* a = t + 4 * k;
@@ -430,7 +433,7 @@ __global__ void k_determinant(const double* __restrict__ t, double* __restrict__
 }
 
 // src/SELF_Geometry.f90:448-457 (dsdx(:,1) = (dy/ds2, -dx/ds2), dsdx(:,2) = (-dy/ds1, dx/ds1))
-__global__ void k_contravariant_basis(const double* __restrict__ dxds, double* __restrict__ dsdx, long long n) {
+__global__ void k_contravariant_basis(const double* dxds, double* dsdx, long long n) {
   after_previous();
   GRID_STRIDE(k, n) {
     const double* a = dxds + 4 * k;
@@ -444,7 +447,7 @@ __global__ void k_contravariant_basis(const double* __restrict__ dxds, double* _
 
 // Sign adjustment of dsdx on the faces: outward on East/North for J > 0,
 // src/SELF_Geometry.f90:462-520 (fac), applied to all four components.
-__global__ void k_adjust_boundary_basis(double* __restrict__ dsdxB, const double* __restrict__ JB, int N,
+__global__ void k_adjust_boundary_basis(double* dsdxB, const double* JB, int N,
                                         long long n) {
   after_previous();
   const int P = N + 1;
@@ -460,8 +463,8 @@ __global__ void k_adjust_boundary_basis(double* __restrict__ dsdxB, const double
 // nHat and nScale from the (unsigned) face contravariant basis, then the sign
 // adjustment, as CalculateContravariantBasis_SEMQuad does on the host
 // (src/SELF_Geometry.f90:458-522).
-__global__ void k_face_normals(double* __restrict__ dsdxB, const double* __restrict__ JB, double* __restrict__ nHat,
-                               double* __restrict__ nScale, int N, long long n) {
+__global__ void k_face_normals(double* dsdxB, const double* JB, double* nHat,
+                               double* nScale, int N, long long n) {
   after_previous();
   const int P = N + 1;
   GRID_STRIDE(k, n) {
@@ -481,11 +484,11 @@ __global__ void k_face_normals(double* __restrict__ dsdxB, const double* __restr
 
 // ---------------------------------------------------------------- MappedData
 // src/SELF_MappedData.f90:955-1078 (BR1 gradient, weak form), N > 7
-__global__ void k_gradient_br(const double* __restrict__ f, const double* __restrict__ avgB,
-                              const double* __restrict__ dsdx, const double* __restrict__ J,
-                              const double* __restrict__ nHat, const double* __restrict__ nScale,
-                              double* __restrict__ gradF, const double* __restrict__ dgM,
-                              const double* __restrict__ bM, const double* __restrict__ qw, int N, int nVar,
+__global__ void k_gradient_br(const double* f, const double* avgB,
+                              const double* dsdx, const double* J,
+                              const double* nHat, const double* nScale,
+                              double* gradF, const double* dgM,
+                              const double* bM, const double* qw, int N, int nVar,
                               long long n) {
   after_previous();
   const int P = N + 1;
@@ -532,8 +535,8 @@ __global__ void k_gradient_br(const double* __restrict__ f, const double* __rest
 }
 
 // src/SELF_MappedData.f90:1080-1149 (strong form), N > 7
-__global__ void k_gradient_sf(const double* __restrict__ f, const double* __restrict__ dsdx,
-                              const double* __restrict__ J, double* __restrict__ gradF, const double* __restrict__ dM,
+__global__ void k_gradient_sf(const double* f, const double* dsdx,
+                              const double* J, double* gradF, const double* dM,
                               int N, int nVar, long long n) {
   after_previous();
   const int P = N + 1;
@@ -566,10 +569,10 @@ __global__ void k_gradient_sf(const double* __restrict__ f, const double* __rest
 // a face node's products with the normal by the nodes of its line.
 template <int P, bool kWeak>
 __global__ void __launch_bounds__(NodeBlock<P>::threads, 3) k_gradient(
-    const double* __restrict__ f, const double* __restrict__ avgB, const double* __restrict__ dsdx,
-    const double* __restrict__ J, const double* __restrict__ nHat, const double* __restrict__ nScale,
-    double* __restrict__ gradF, const double* __restrict__ D, const double* __restrict__ bM,
-    const double* __restrict__ qw, int nVar, long long nPlanes) {
+    const double* f, const double* avgB, const double* dsdx,
+    const double* J, const double* nHat, const double* nScale,
+    double* gradF, const double* D, const double* bM,
+    const double* qw, int nVar, long long nPlanes) {
   after_previous();
   using B = NodeBlock<P>;
   constexpr int PP = B::PP, RS = B::RS, FS = B::FS;
@@ -640,7 +643,7 @@ __global__ void __launch_bounds__(NodeBlock<P>::threads, 3) k_gradient(
 
 // src/SELF_MappedData.f90:1235-1268 (C = 1) and the vector analogue (C = 2)
 template <int PC, int C>
-__global__ void k_jacobian_weight(double* __restrict__ f, const double* __restrict__ J, int N, int nVar,
+__global__ void k_jacobian_weight(double* f, const double* J, int N, int nVar,
                                   long long n) {
   after_previous();
   const int P = nodes<PC>(N);
@@ -655,7 +658,7 @@ __global__ void k_jacobian_weight(double* __restrict__ f, const double* __restri
 
 // src/SELF_MappedData.f90:2220-2269
 template <int PC>
-__global__ void k_contravariant_projection(double* __restrict__ f, const double* __restrict__ dsdx, int N, int nVar,
+__global__ void k_contravariant_projection(double* f, const double* dsdx, int N, int nVar,
                                            long long n) {
   after_previous();
   const int P = nodes<PC>(N);
@@ -673,8 +676,8 @@ __global__ void k_contravariant_projection(double* __restrict__ f, const double*
 // src/SELF_MappedData.f90:834-917 (C = 1) and 1870-1958 (C = 2): one thread per
 // (component, node, var, side, element) output of extBoundary.
 template <int PC, int C>
-__global__ void k_side_exchange(double* __restrict__ ext, const double* __restrict__ bnd,
-                                const int* __restrict__ sideInfo, const int* __restrict__ elemToRank, int rankId,
+__global__ void k_side_exchange(double* ext, const double* bnd,
+                                const int* sideInfo, const int* elemToRank, int rankId,
                                 int offset, int N, int nVar, long long n) {
   after_previous();
   const int P = nodes<PC>(N);
@@ -704,8 +707,8 @@ __global__ void k_side_exchange(double* __restrict__ ext, const double* __restri
 }
 
 // src/SELF_MappedData.f90:919-953
-__global__ void k_bassi_rebay(double* __restrict__ avg, const double* __restrict__ bnd,
-                              const double* __restrict__ ext, long long n) {
+__global__ void k_bassi_rebay(double* avg, const double* bnd,
+                              const double* ext, long long n) {
   after_previous();
   GRID_STRIDE(k, n) avg[k] = 0.5 * (bnd[k] + ext[k]);
 }
@@ -713,7 +716,7 @@ __global__ void k_bassi_rebay(double* __restrict__ avg, const double* __restrict
 // ------------------------------------------------------------------- Model2D
 // src/SELF_Model2D.f90:734-748 (workSol may have nWork != nVar variables)
 template <int PC>
-__global__ void k_update_grk(double* __restrict__ grk, double* __restrict__ sol, const double* __restrict__ dSdt,
+__global__ void k_update_grk(double* grk, double* sol, const double* dSdt,
                              double a, double g, double dt, int nWork, int N, int nVar, long long n) {
   after_previous();
   const int P2 = nodes<PC>(N) * nodes<PC>(N);
@@ -729,13 +732,13 @@ __global__ void k_update_grk(double* __restrict__ grk, double* __restrict__ sol,
   }
 }
 
-__global__ void k_update_solution(double* __restrict__ sol, const double* __restrict__ dSdt, double dt, long long n) {
+__global__ void k_update_solution(double* sol, const double* dSdt, double dt, long long n) {
   after_previous();
   GRID_STRIDE(k, n) sol[k] = sol[k] + dt * dSdt[k];
 }
 
 // src/SELF_Model2D.f90:845-857
-__global__ void k_dsdt(const double* __restrict__ div, const double* __restrict__ src, double* __restrict__ dSdt,
+__global__ void k_dsdt(const double* div, const double* src, double* dSdt,
                        long long n) {
   after_previous();
   GRID_STRIDE(k, n) dSdt[k] = src[k] - div[k];
@@ -744,8 +747,8 @@ __global__ void k_dsdt(const double* __restrict__ div, const double* __restrict_
 // -------------------------------------------------------- LinearShallowWater
 // src/models/SELF_LinearShallowWater.f90:298-355; thread per (i, side, el)
 template <int PC>
-__global__ void k_lsw_bc(const double* __restrict__ sol, double* __restrict__ ext, const double* __restrict__ nHat,
-                         const int* __restrict__ sideInfo, int N, int nVar, long long n) {
+__global__ void k_lsw_bc(const double* sol, double* ext, const double* nHat,
+                         const int* sideInfo, int N, int nVar, long long n) {
   after_previous();
   const int P = nodes<PC>(N);
   GRID_STRIDE(k, n) {
@@ -770,7 +773,7 @@ __global__ void k_lsw_bc(const double* __restrict__ sol, double* __restrict__ ex
 }
 
 template <int PC>
-__global__ void k_lsw_source(double* __restrict__ src, const double* __restrict__ sol, const double* __restrict__ f,
+__global__ void k_lsw_source(double* src, const double* sol, const double* f,
                              int N, int nVar, long long n) {
   after_previous();
   const int P2 = nodes<PC>(N) * nodes<PC>(N);
@@ -786,7 +789,7 @@ __global__ void k_lsw_source(double* __restrict__ src, const double* __restrict_
 }
 
 template <int PC>
-__global__ void k_lsw_flux(double* __restrict__ flux, const double* __restrict__ sol, const double* __restrict__ H,
+__global__ void k_lsw_flux(double* flux, const double* sol, const double* H,
                            double g, int N, int nVar, long long n) {
   after_previous();
   const int P2 = nodes<PC>(N) * nodes<PC>(N);
@@ -805,9 +808,9 @@ __global__ void k_lsw_flux(double* __restrict__ flux, const double* __restrict__
 }
 
 template <int PC>
-__global__ void k_lsw_riemann(double* __restrict__ flux, const double* __restrict__ sol,
-                              const double* __restrict__ ext, const double* __restrict__ H,
-                              const double* __restrict__ nHat, const double* __restrict__ nScale, double g, int N,
+__global__ void k_lsw_riemann(double* flux, const double* sol,
+                              const double* ext, const double* H,
+                              const double* nHat, const double* nScale, double g, int N,
                               int nVar, long long n) {
   after_previous();
   const int P = nodes<PC>(N);
@@ -826,8 +829,8 @@ __global__ void k_lsw_riemann(double* __restrict__ flux, const double* __restric
 
 // -------------------------------------------------------------- ShallowWater
 template <int PC>
-__global__ void k_sw_bc(const double* __restrict__ sol, double* __restrict__ ext, const double* __restrict__ topoB,
-                        const double* __restrict__ nHat, const int* __restrict__ sideInfo, int N, int nVar,
+__global__ void k_sw_bc(const double* sol, double* ext, const double* topoB,
+                        const double* nHat, const int* sideInfo, int N, int nVar,
                         long long n) {
   after_previous();
   const int P = nodes<PC>(N);
@@ -852,7 +855,7 @@ __global__ void k_sw_bc(const double* __restrict__ sol, double* __restrict__ ext
 }
 
 template <int PC>
-__global__ void k_sw_source(double* __restrict__ src, const double* __restrict__ sol, const double* __restrict__ gH,
+__global__ void k_sw_source(double* src, const double* sol, const double* gH,
                             double fC, double g, int N, int nVar, long long n) {
   after_previous();
   const int P2 = nodes<PC>(N) * nodes<PC>(N);
@@ -867,7 +870,7 @@ __global__ void k_sw_source(double* __restrict__ src, const double* __restrict__
 }
 
 template <int PC>
-__global__ void k_sw_flux(double* __restrict__ flux, const double* __restrict__ sol, const double* __restrict__ vel,
+__global__ void k_sw_flux(double* flux, const double* sol, const double* vel,
                           double g, int N, int nVar, long long n) {
   after_previous();
   const int P2 = nodes<PC>(N) * nodes<PC>(N);
@@ -885,9 +888,9 @@ __global__ void k_sw_flux(double* __restrict__ flux, const double* __restrict__ 
 }
 
 template <int PC>
-__global__ void k_sw_riemann(double* __restrict__ flux, const double* __restrict__ sol, const double* __restrict__ ext,
-                             const double* __restrict__ vel, const double* __restrict__ velExt,
-                             const double* __restrict__ nHat, const double* __restrict__ nScale, double g, int N,
+__global__ void k_sw_riemann(double* flux, const double* sol, const double* ext,
+                             const double* vel, const double* velExt,
+                             const double* nHat, const double* nScale, double g, int N,
                              int nVar, long long n) {
   after_previous();
   const int P = nodes<PC>(N);
@@ -908,7 +911,7 @@ __global__ void k_sw_riemann(double* __restrict__ flux, const double* __restrict
 // velocity = (Hu, Hv)/H on interior nodes (first kernel) and on face nodes
 // (second), src/models/SELF_ShallowWater.f90:205-236
 template <int PC, bool kFace>
-__global__ void k_sw_velocity(const double* __restrict__ sol, double* __restrict__ vel, int N, int nVar,
+__global__ void k_sw_velocity(const double* sol, double* vel, int N, int nVar,
                               long long n) {
   after_previous();
   const int stride = kFace ? nodes<PC>(N) : nodes<PC>(N) * nodes<PC>(N);
@@ -924,8 +927,8 @@ __global__ void k_sw_velocity(const double* __restrict__ sol, double* __restrict
 
 // ---------------------------------------------------- CompressibleIdealGas2D
 template <int PC>
-__global__ void k_cig_source(double* __restrict__ src, const double* __restrict__ sol,
-                             const double* __restrict__ envGrad, int N, int nVar, long long n) {
+__global__ void k_cig_source(double* src, const double* sol,
+                             const double* envGrad, int N, int nVar, long long n) {
   after_previous();
   const int P2 = nodes<PC>(N) * nodes<PC>(N);
   GRID_STRIDE(k, n) {
@@ -944,8 +947,8 @@ __global__ void k_cig_source(double* __restrict__ src, const double* __restrict_
 }
 
 template <int PC>
-__global__ void k_cig_flux(double* __restrict__ flux, const double* __restrict__ sol, const double* __restrict__ prim,
-                           const double* __restrict__ diag, int N, int nVar, long long n) {
+__global__ void k_cig_flux(double* flux, const double* sol, const double* prim,
+                           const double* diag, int N, int nVar, long long n) {
   after_previous();
   const int P2 = nodes<PC>(N) * nodes<PC>(N);
   GRID_STRIDE(k, n) {
@@ -964,10 +967,10 @@ __global__ void k_cig_flux(double* __restrict__ flux, const double* __restrict__
 }
 
 template <int PC>
-__global__ void k_cig_llf(double* __restrict__ flux, const double* __restrict__ sol, const double* __restrict__ solE,
-                          const double* __restrict__ prim, const double* __restrict__ primE,
-                          const double* __restrict__ diag, const double* __restrict__ diagE,
-                          const double* __restrict__ nHat, const double* __restrict__ nScale, int N, int nVar,
+__global__ void k_cig_llf(double* flux, const double* sol, const double* solE,
+                          const double* prim, const double* primE,
+                          const double* diag, const double* diagE,
+                          const double* nHat, const double* nScale, int N, int nVar,
                           int nDiag, long long n) {
   after_previous();
   const int P = nodes<PC>(N);
@@ -997,8 +1000,8 @@ __global__ void k_cig_llf(double* __restrict__ flux, const double* __restrict__ 
 }
 
 template <int PC>
-__global__ void k_cig_bc(const double* __restrict__ in, double* __restrict__ ext, const double* __restrict__ presc,
-                         const double* __restrict__ nHat, const int* __restrict__ sideInfo, int N, int nv,
+__global__ void k_cig_bc(const double* in, double* ext, const double* presc,
+                         const double* nHat, const int* sideInfo, int N, int nv,
                          int reflectPair, long long n) {
   after_previous();
   const int P = nodes<PC>(N);
@@ -1025,7 +1028,7 @@ __global__ void k_cig_bc(const double* __restrict__ in, double* __restrict__ ext
 // CalculateDiagnostics (mode 0), ConservativeToPrimitive (mode 1),
 // ConservativeToEntropy (mode 2); src/models/SELF_CompressibleIdealGas2D.f90:1076-1215
 template <int PC>
-__global__ void k_cig_pointwise(const double* __restrict__ sol, double* __restrict__ out, double gamma, double Rg,
+__global__ void k_cig_pointwise(const double* sol, double* out, double gamma, double Rg,
                                 int mode, int N, int nVar, int nOut, long long n) {
   after_previous();
   const int P2 = nodes<PC>(N) * nodes<PC>(N);

@@ -49,3 +49,10 @@ def test_nothing_is_read_before_the_wait():
             assert (name, p) in INPUTS or not re.search(rf"\b{p}\b", before), (name, p)
         for s in re.findall(r"(?:StageArgs|AvArgs)\s+(\w+)", params):
             assert set(re.findall(rf"\b{s}\.(\w+)", before)) <= VALUES, name
+
+
+def test_no_pointer_of_a_dependent_kernel_is_restrict():
+    """__restrict__ promises that nobody else writes the data while the kernel runs, but its run overlaps the kernel
+    that writes it: the compiler could read it through the non-coherent path or move a read ahead of the wait."""
+    for name, params, _, body in dependent_kernels():
+        assert "__restrict__" not in params and "__restrict__" not in body, name
