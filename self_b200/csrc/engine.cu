@@ -371,9 +371,10 @@ struct selfgpu_model2d {
   }
 
   // nSteps RK3 steps as one launch of k_fused_resident (it forms stale traces
-  // itself: no prologue); cudaErrorCooperativeLaunchTooLarge when the mesh
-  // does not fit resident CTAs (the caller falls back).
-  cudaError_t launch_resident(double dt, int nSteps) {
+  // itself: no prologue).  Where the mesh does not fit resident CTAs
+  // (cudaErrorCooperativeLaunchTooLarge) or the launch is refused, `done` steps
+  // have been issued and the caller runs the others otherwise.
+  cudaError_t launch_resident(double dt, int nSteps, int& done) {
     ResidentArgs ra{};
     StageArgs a = base;
     a.mode = MODE_RK;
@@ -382,7 +383,7 @@ struct selfgpu_model2d {
     const size_t pub = publish_bytes();
     cudaError_t e = cudaSuccess;
     constexpr int kChunk = 100000;  // steps per launch
-    for (int done = 0; done < nSteps;) {
+    for (done = 0; done < nSteps;) {
       const int k = (nSteps - done) < kChunk ? (nSteps - done) : kChunk;
       ra.nStages = 3 * k;
       ra.fresh = valid ? 0 : 1;
@@ -416,17 +417,18 @@ struct selfgpu_model2d {
   unsigned long long gen = 0;  // bumped whenever captured work goes stale (ensemble graphs check it)
 
   // nSteps RK3 steps as launches of the persistent kernel that each run many
-  // stages (k_fused_stage_tma<..., true>), from the current parities;
-  // cudaErrorNotSupported / cudaErrorCooperativeLaunchTooLarge when that
-  // kernel does not apply (the caller falls back).
-  cudaError_t launch_stages_tma(double dt, int nSteps) {
+  // stages (k_fused_stage_tma<..., true>), from the current parities.  Where
+  // that kernel does not apply (cudaErrorNotSupported,
+  // cudaErrorCooperativeLaunchTooLarge) or a launch is refused, `done` steps
+  // have been issued and the caller runs the others otherwise.
+  cudaError_t launch_stages_tma(double dt, int nSteps, int& done) {
     cudaError_t e = cudaSuccess;
     if (!stepBar) e = cudaMalloc(&stepBar, sizeof(unsigned));
     if (e != cudaSuccess) return e;
     StageArgs a = base;
     a.mode = MODE_RK;
     constexpr int kChunk = 100000;  // steps per launch: the stage-end counter stays below 2^32
-    for (int done = 0; done < nSteps;) {
+    for (done = 0; done < nSteps;) {
       const int n = (nSteps - done) < kChunk ? (nSteps - done) : kChunk;
       e = cudaMemsetAsync(stepBar, 0, sizeof(unsigned), stream);
       if (e != cudaSuccess) return e;
@@ -816,25 +818,24 @@ int selfgpu_model2d_rk3(selfgpu_model2d* m, double dt, int nSteps) {
   cudaError_t e = cudaSuccess;
   if ((m->resident == m->RESIDENT_ON || (m->resident == m->RESIDENT_AUTO && !m->stagesChosen)) && nSteps > 0 &&
       m->avMode == AV_OFF && m->nHalo == 0 && m->symmetric && m->base.debugStarve != 1) {
-    e = m->launch_resident(dt, nSteps);
+    int done = 0;
+    e = m->launch_resident(dt, nSteps, done);
     if (e == cudaSuccess) return SELFGPU_OK;
+    // The mesh does not fit, or a cooperative launch is refused here: stage
+    // launches for what is left.  (An error of earlier work on the device stays
+    // and is reported by them.)
     cudaGetLastError();
-    if (e != cudaErrorCooperativeLaunchTooLarge)
-      return fail_cuda("selfgpu_model2d_rk3: resident launch", e);
-    // larger meshes: stage launches below
+    nSteps -= done;
   }
   if (m->multistage && nSteps > 0 && m->avMode == AV_OFF && m->nHalo == 0 && m->base.debugStarve != 1 &&
       m->cfg.allowTma) {
     e = m->valid ? cudaSuccess : m->prologue();
     if (e != cudaSuccess) return fail_cuda("selfgpu_model2d_rk3", e);
-    const int c0 = m->cur, v0 = m->vcur;
-    e = m->launch_stages_tma(dt, nSteps);
+    int done = 0;
+    e = m->launch_stages_tma(dt, nSteps, done);
     if (e == cudaSuccess) return SELFGPU_OK;
-    cudaGetLastError();
-    if (e != cudaErrorNotSupported && e != cudaErrorCooperativeLaunchTooLarge)
-      return fail_cuda("selfgpu_model2d_rk3: multi-stage launch", e);
-    m->cur = c0;  // nothing was launched: stage launches below
-    m->vcur = v0;
+    cudaGetLastError();  // as above
+    nSteps -= done;
   }
   if (!m->valid) {
     e = m->prologue();
