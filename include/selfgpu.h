@@ -341,6 +341,8 @@ int selfgpu_model2d_set_kernel(selfgpu_model2d* m, int persistent);
  * each other.  That is the default until set_kernel, set_launch or
  * set_multistage chooses among the stage launches; enable = 1 keeps it on
  * after those, 0 turns it off.  Results equal the stage launches bit for bit.
+ * A call of more than 1 000 steps is one launch per 1 000, and a device that
+ * refuses a cooperative launch runs stage launches.
  * The waits for neighbours' traces are bounded (set_wait_limit;
  * SELFGPU_ERR_TIMEOUT from sync). */
 int selfgpu_model2d_set_multistep(selfgpu_model2d* m, int enable);

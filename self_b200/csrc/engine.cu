@@ -382,7 +382,10 @@ struct selfgpu_model2d {
     ra.tiles = residentTiles;
     const size_t pub = publish_bytes();
     cudaError_t e = cudaSuccess;
-    constexpr int kChunk = 100000;  // steps per launch
+    // Steps per launch.  Its CTAs may fill the SMs, and work on other streams
+    // then waits for its end: at most some 40 ms (3 000 stages of up to 12.5 us).
+    // Starting again from memory costs a launch and a stage's traffic, 0.1 %.
+    constexpr int kChunk = 1000;
     for (done = 0; done < nSteps;) {
       const int k = (nSteps - done) < kChunk ? (nSteps - done) : kChunk;
       ra.nStages = 3 * k;

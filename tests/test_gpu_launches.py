@@ -42,3 +42,21 @@ def refused(nx):
 def test_a_refused_cooperative_launch_runs_stage_launches(nx, tmp_path):
     noted = launch_shim.run(tmp_path, f"from tests.test_gpu_launches import refused; refused({nx})", refuse=True)
     assert any(cooperative for _, cooperative in noted)
+
+
+@pytest.mark.parametrize("name", ["LSW", "SW"])
+def test_a_long_call_is_several_bounded_launches(name):
+    """An on-chip launch holds its SMs: 2 001 steps are three launches, with the state of the stage launches."""
+    import self_b200 as S
+    out = []
+    for pinned in (False, True):
+        m = model(name, 5, 3, S.FP64)
+        if pinned:
+            S.check(S.lib().selfgpu_model2d_set_launch(m._h, 1, 0))
+        l0 = m.LaunchCount()
+        m.ForwardStep(2001, 1e-5)
+        m.Sync()
+        assert pinned or m.LaunchCount() - l0 == 3
+        out.append((m.solution.clone(), m.workSol.clone()))
+    assert torch.isfinite(out[0][0]).all()
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
