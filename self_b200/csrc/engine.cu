@@ -395,14 +395,11 @@ struct selfgpu_model2d {
         ra.rkA[m] = kRK3a[m];
         ra.rkG[m] = kRK3g[m];
       }
-      // the parities that as many stage launches leave; one pair may serve as
-      // input and output, since a CTA writes its final traces only after its
-      // neighbours have read the initial ones
-      const int odd = ra.nStages & 1;
-      ra.trIn = tr[cur];
-      ra.velIn = vel[vcur];
-      ra.trOut = tr[cur ^ odd];
-      ra.velOut = vel[vcur ^ odd];
+      // One pair of caches is input and output, since a CTA writes its final
+      // traces (in the third stage or later) only after its neighbours have read
+      // the initial ones.  So a captured call, replayed, finds what it left.
+      ra.trIn = ra.trOut = tr[cur];
+      ra.velIn = ra.velOut = vel[vcur];
       ra.xch[0] = xch;
       ra.xch[1] = reinterpret_cast<char*>(xch) + pub;
       ra.epoch = reinterpret_cast<ResidentEpoch*>(reinterpret_cast<char*>(xch) + 2 * pub);
@@ -410,8 +407,6 @@ struct selfgpu_model2d {
       if (e != cudaSuccess) return e;
       ++launches;
       valid = true;
-      cur ^= odd;
-      if (model == SELFGPU_MODEL_SW) vcur ^= odd;
       done += k;
     }
     return cudaSuccess;

@@ -60,3 +60,31 @@ def test_a_long_call_is_several_bounded_launches(name):
         out.append((m.solution.clone(), m.workSol.clone()))
     assert torch.isfinite(out[0][0]).all()
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("n", [1, 2, 3])
+@pytest.mark.parametrize("name,nx,N", [("LSW", 8, 7), ("SW", 24, 7), ("SW", 90, 4), ("CIG", 50, 7), ("CIG", 9, 2)])
+def test_a_captured_call_replays(name, nx, N, n):
+    """An on-chip call captured into a CUDA graph, with an odd or an even number of steps, and replayed: the steps of
+    as many calls, bit for bit (one and several tiles per CTA)."""
+    import self_b200 as S
+    st = torch.cuda.Stream()
+    a, b = (model(name, nx, N, S.FP64, stream=s) for s in (st.cuda_stream, None))
+    torch.cuda.synchronize()
+    for m in (a, b):
+        m.ForwardStep(1, 1e-5)
+        m.Sync()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=st):
+        a.ForwardStep(n, 1e-5)
+    for _ in range(4):
+        graph.replay()
+    torch.cuda.synchronize()
+    a.ForwardStep(2, 1e-5)
+    a.Sync()
+    for _ in range(4):
+        b.ForwardStep(n, 1e-5)
+    b.ForwardStep(2, 1e-5)
+    b.Sync()
+    assert torch.isfinite(a.solution).all()
+    assert torch.equal(a.solution, b.solution) and torch.equal(a.workSol, b.workSol)
