@@ -384,7 +384,9 @@ int selfgpu_ensemble_destroy(selfgpu_ensemble* e);
  * its double-buffered staging tile) on RK-stage launches over this handle's
  * own data (a zero step on scratch copies of the solution and RK register;
  * the state is not modified), keeps the fastest, and reports it (persistent
- * 0/1, group count, microseconds per stage).  Allocates scratch memory. */
+ * 0/1, group count, microseconds per stage).  Allocates scratch memory.  The
+ * choice is for stage launches (and set_multistage's): where rk3 keeps the
+ * state on chip (set_multistep) it goes on doing so. */
 int selfgpu_model2d_autotune(selfgpu_model2d* m, int* persistent, int* groups, float* usPerStage);
 
 /* Failure detection.  Every wait inside the persistent kernel is bounded; a

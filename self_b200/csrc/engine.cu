@@ -329,6 +329,14 @@ struct selfgpu_model2d {
     }
   }
 
+  int stage_groups(const StageArgs& a, const StageLaunch& L) const {
+    switch (form) {
+      case SELFGPU_FP64: return stage_groups_fp64(model, P, a, L);
+      case SELFGPU_FP64_REF: return stage_groups_fp64_ref(model, P, a, L);
+      default: return stage_groups_fp32(model, P, a, L);
+    }
+  }
+
   // closure preparation of one stage: element viscosity (formNu: the first
   // stage of an RK step and tendency evaluations; the step's other stages
   // keep it), BR1 gradient, viscous volume flux and traces, from the
@@ -956,17 +964,18 @@ int selfgpu_model2d_autotune(selfgpu_model2d* m, int* persistent, int* groups, f
   // every consumer-group count from 2 up to what fits.  Each is timed on
   // RK-stage launches over scratch copies of the solution and RK register
   // (a zero step: the state is not modified); the stage writes the trace
-  // caches the next real stage rewrites anyway.
-  const size_t n = (size_t)m->P * m->P * nv_of(m->model) * m->nEl;
+  // caches the next real stage rewrites anyway.  Both copies start on a
+  // 16-byte boundary, as the persistent kernel needs (n may be odd).
+  const size_t n = (size_t)m->P * m->P * nv_of(m->model) * m->nEl, atG = (n + 1) / 2 * 2;
   double* scratch = nullptr;
-  cudaError_t e = cudaMalloc(&scratch, 2 * n * sizeof(double));
+  cudaError_t e = cudaMalloc(&scratch, (atG + n) * sizeof(double));
   if (e != cudaSuccess) return fail_cuda("selfgpu_model2d_autotune", e);
   e = cudaMemcpyAsync(scratch, m->base.q, n * sizeof(double), cudaMemcpyDeviceToDevice, m->stream);
   if (e == cudaSuccess) {
     if (m->gf)  // the FP32-bulk form's register (n floats fit the second half)
-      e = cudaMemcpyAsync(scratch + n, m->gf, n * sizeof(float), cudaMemcpyDeviceToDevice, m->stream);
+      e = cudaMemcpyAsync(scratch + atG, m->gf, n * sizeof(float), cudaMemcpyDeviceToDevice, m->stream);
     else
-      e = cudaMemcpyAsync(scratch + n, m->base.G, n * sizeof(double), cudaMemcpyDeviceToDevice, m->stream);
+      e = cudaMemcpyAsync(scratch + atG, m->base.G, n * sizeof(double), cudaMemcpyDeviceToDevice, m->stream);
   }
   if (e != cudaSuccess) {
     cudaFree(scratch);
@@ -982,8 +991,8 @@ int selfgpu_model2d_autotune(selfgpu_model2d* m, int* persistent, int* groups, f
   StageArgs a = m->base;
   a.mode = MODE_RK;
   a.q = scratch;
-  a.G = scratch + n;
-  if (m->gf) a.Gf = reinterpret_cast<float*>(scratch + n);
+  a.G = scratch + atG;
+  if (m->gf) a.Gf = reinterpret_cast<float*>(scratch + atG);
   a.rk_a = 0.0;
   a.rk_gdt = 0.0;
   a.rk_g = 0.0;
@@ -1006,26 +1015,19 @@ int selfgpu_model2d_autotune(selfgpu_model2d* m, int* persistent, int* groups, f
   const StageLaunch saved = m->cfg;
   float best = 1e30f;
   StageLaunch bestCfg = saved;
-  // consumer groups per CTA: up to 10 two-warp groups for P >= 6 (at P = 8, 14
-  // in the FP32-bulk form, 12 for the production FP64 ShallowWater models), up
-  // to 20 one-warp groups for P <= 4, 24 in FP32 (TmaTraits::kMaxGroups)
-  const bool twelve = m->P == 8 && (m->form == SELFGPU_FP32_BULK ||
-                                    (m->form == SELFGPU_FP64 && m->model != SELFGPU_MODEL_CIG));
-  const int maxCand = m->P <= 4 ? (m->form == SELFGPU_FP32_BULK ? 23 : 19)
-                                  : (m->form == SELFGPU_FP32_BULK && m->P == 8 ? 13 : twelve ? 11 : 9);
-  for (int cand = 0; cand <= maxCand; ++cand) {
+  StageLaunch most = saved;  // as many groups as the kernel's registers and shared memory allow
+  most.allowTma = true;
+  most.maxGroups = 0;
+  const int fit = m->stage_groups(a, most);
+  for (int groups = 0; groups <= fit; ++groups) {  // 0: the per-element-group kernel
+    if (groups == 1 && fit > 1) continue;
     StageLaunch c = saved;
-    if (cand == 0) {
-      c.allowTma = false;
-    } else {
-      c.allowTma = true;
-      c.maxGroups = cand + 1;  // capped by what fits in shared memory
-    }
+    c.allowTma = groups > 0;
+    if (groups > 0) c.maxGroups = groups;
     m->cfg = c;
     int tma = 0;
     e = selfgpu_model2d::launch_stage_form(m->form, m->model, m->P, a, c, m->stream, &tma);
     if (e != cudaSuccess) break;
-    if (cand > 0 && !tma) break;  // the persistent kernel does not apply
     cudaEventRecord(t0, m->stream);
     for (int r = 0; r < 3; ++r)
       selfgpu_model2d::launch_stage_form(m->form, m->model, m->P, a, c, m->stream, &tma);

@@ -67,6 +67,10 @@ cudaError_t launch_stage_fp64_ref(int model, int P, const StageArgs& a, const St
                                   int* usedTma);
 cudaError_t launch_stage_fp32(int model, int P, const StageArgs& a, const StageLaunch& L, cudaStream_t st,
                               int* usedTma);
+// consumer groups the persistent kernel would run with these arguments, 0 where it does not apply
+int stage_groups_fp64(int model, int P, const StageArgs& a, const StageLaunch& L);
+int stage_groups_fp64_ref(int model, int P, const StageArgs& a, const StageLaunch& L);
+int stage_groups_fp32(int model, int P, const StageArgs& a, const StageLaunch& L);
 // all stages of an rk3 call in one cooperative launch of k_fused_resident, per form
 struct ResidentArgs;
 cudaError_t launch_resident_fp64(int model, int P, const StageArgs& a, ResidentArgs& ra, const StageLaunch& L,

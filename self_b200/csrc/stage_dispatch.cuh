@@ -28,16 +28,22 @@ constexpr int elems_per_block() {
 
 inline bool aligned16(const void* p) { return ((uintptr_t)p % 16) == 0; }
 
+// Whether the persistent kernel runs a launch with these buffers, and its plan.
 template <int P, class Phys, typename R>
-cudaError_t launch_one(const StageArgs& a, const StageLaunch& L, cudaStream_t st, int* usedTma) {
-  *usedTma = 0;
-  if (a.mode == MODE_TRACES) return launch_traces<P, Phys, R>(a, st);
+bool plan_stage(const StageArgs& a, const StageLaunch& L, TmaPlan& pl) {
   bool ok = L.allowTma && a.geo != nullptr && aligned16(a.geo) && aligned16(a.q) &&
             aligned16(sizeof(R) == 4 ? (const void*)a.Gf : (const void*)a.G) && aligned16(a.trIn) &&
             (a.velIn == nullptr || aligned16(a.velIn));
   for (int k = 0; k < 5; ++k) ok = ok && (a.fld[k] == nullptr || aligned16(a.fld[k]));
+  return ok && make_tma_plan<P, Phys, R>(a, L.smemOptin, L.l2Bytes, pl, L.maxGroups);
+}
+
+template <int P, class Phys, typename R>
+cudaError_t launch_one(const StageArgs& a, const StageLaunch& L, cudaStream_t st, int* usedTma) {
+  *usedTma = 0;
+  if (a.mode == MODE_TRACES) return launch_traces<P, Phys, R>(a, st);
   TmaPlan pl{};
-  if (ok && make_tma_plan<P, Phys, R>(a, L.smemOptin, L.l2Bytes, pl, L.maxGroups)) {
+  if (plan_stage<P, Phys, R>(a, L, pl)) {
     // the shared-memory opt-in is per device: one bit per device that has it
     static std::atomic<unsigned long long> attrSet{0};  // one instantiation per (P, Phys, R)
     int dev = 0;
@@ -147,6 +153,32 @@ cudaError_t launch_stages_tma_impl(int model, int P, const StageArgs& a, const S
     case SELFGPU_MODEL_SW: return launch_stages_tma_P<PhysSW, R>(P, a, L, ms, st);
     case SELFGPU_MODEL_CIG: return launch_stages_tma_P<PhysCIG, R>(P, a, L, ms, st);
     default: return cudaErrorInvalidValue;
+  }
+}
+
+// Consumer groups of the persistent kernel for these arguments; 0 where it
+// does not apply.
+template <class Phys, typename R>
+int stage_groups_P(int P, const StageArgs& a, const StageLaunch& L) {
+  TmaPlan pl{};
+  switch (P) {
+    case 2: return plan_stage<2, Phys, R>(a, L, pl) ? pl.groups : 0;
+    case 3: return plan_stage<3, Phys, R>(a, L, pl) ? pl.groups : 0;
+    case 4: return plan_stage<4, Phys, R>(a, L, pl) ? pl.groups : 0;
+    case 5: return plan_stage<5, Phys, R>(a, L, pl) ? pl.groups : 0;
+    case 6: return plan_stage<6, Phys, R>(a, L, pl) ? pl.groups : 0;
+    case 7: return plan_stage<7, Phys, R>(a, L, pl) ? pl.groups : 0;
+    case 8: return plan_stage<8, Phys, R>(a, L, pl) ? pl.groups : 0;
+    default: return 0;
+  }
+}
+template <typename R>
+int stage_groups_impl(int model, int P, const StageArgs& a, const StageLaunch& L) {
+  switch (model) {
+    case SELFGPU_MODEL_LSW: return stage_groups_P<PhysLSW, R>(P, a, L);
+    case SELFGPU_MODEL_SW: return stage_groups_P<PhysSW, R>(P, a, L);
+    case SELFGPU_MODEL_CIG: return stage_groups_P<PhysCIG, R>(P, a, L);
+    default: return 0;
   }
 }
 

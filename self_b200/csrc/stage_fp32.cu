@@ -12,6 +12,9 @@ cudaError_t launch_stage_fp32(int model, int P, const StageArgs& a, const StageL
 cudaError_t launch_av_prep_fp32(int P, const AvArgs& a, cudaStream_t st, int numSMs, bool formNu) {
   return launch_av_prep_impl<float>(P, a, st, numSMs, formNu);
 }
+int stage_groups_fp32(int model, int P, const StageArgs& a, const StageLaunch& L) {
+  return stage_groups_impl<float>(model, P, a, L);
+}
 cudaError_t launch_resident_fp32(int model, int P, const StageArgs& a, ResidentArgs& ra, const StageLaunch& L,
                                  cudaStream_t st) {
   return launch_resident_impl<float>(model, P, a, ra, L, st);

@@ -53,6 +53,9 @@ cudaError_t launch_closure_features(const double* q, int P, int nEl, const AvArg
       return cudaErrorInvalidValue;
   }
 }
+int stage_groups_fp64_ref(int model, int P, const StageArgs& a, const StageLaunch& L) {
+  return stage_groups_impl<double>(model, P, a, L);
+}
 cudaError_t launch_resident_fp64_ref(int model, int P, const StageArgs& a, ResidentArgs& ra, const StageLaunch& L,
                                      cudaStream_t st) {
   return launch_resident_impl<double>(model, P, a, ra, L, st);

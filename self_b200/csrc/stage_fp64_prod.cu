@@ -12,6 +12,9 @@ cudaError_t launch_stage_fp64(int model, int P, const StageArgs& a, const StageL
                               int* usedTma) {
   return launch_stage_impl<double>(model, P, a, L, st, usedTma);
 }
+int stage_groups_fp64(int model, int P, const StageArgs& a, const StageLaunch& L) {
+  return stage_groups_impl<double>(model, P, a, L);
+}
 cudaError_t launch_resident_fp64(int model, int P, const StageArgs& a, ResidentArgs& ra, const StageLaunch& L,
                                  cudaStream_t st) {
   return launch_resident_impl<double>(model, P, a, ra, L, st);

@@ -17,7 +17,7 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void
   static FILE* log = 0;
   if (!real) {
     *(void**)&real = dlsym(dlopen("libcudart.so.12", RTLD_LAZY | RTLD_NOLOAD), "cudaLaunchKernelExC");
-    log = fopen(getenv("SHIM_LOG"), "w");
+    log = fopen(getenv("SHIM_LOG"), "a");
   }
   int cooperative = 0;
   for (unsigned k = 0; k < c->numAttrs; ++k)
@@ -31,8 +31,8 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void
 
 
 def run(tmp_path, code, refuse=False):
-    """Runs the Python code in a child process under the shim; returns the noted launches (threads per block,
-    cooperative)."""
+    """Runs the Python code in a child process under the shim; returns the launches it noted (threads per block,
+    cooperative), as one list per stretch between the child's calls of mark()."""
     src, so, log = tmp_path / "shim.c", tmp_path / "shim.so", tmp_path / "launches.log"
     src.write_text(SHIM)
     subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-I/usr/local/cuda/include", "-o", str(so), str(src), "-ldl"],
@@ -42,4 +42,10 @@ def run(tmp_path, code, refuse=False):
         env["SHIM_REFUSE"] = "1"
     out = subprocess.run([sys.executable, "-c", code], env=env, cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert out.returncode == 0, out.stdout + out.stderr
-    return [tuple(map(int, x.split())) for x in log.read_text().splitlines()]
+    stretches = log.read_text().split("mark\n")
+    return [[tuple(map(int, x.split())) for x in s.splitlines()] for s in stretches]
+
+
+def mark():
+    with open(os.environ["SHIM_LOG"], "a") as f:
+        f.write("mark\n")

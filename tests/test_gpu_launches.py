@@ -1,5 +1,8 @@
 """How the RK3 steps of a call reach the device: refused and bounded
 cooperative launches, captured calls, tuned launches."""
+import ctypes
+from collections import Counter
+
 import pytest
 import torch
 
@@ -41,7 +44,7 @@ def refused(nx):
 @pytest.mark.parametrize("nx", [9, 80])  # where the on-chip and where the multi-stage launch would run
 def test_a_refused_cooperative_launch_runs_stage_launches(nx, tmp_path):
     noted = launch_shim.run(tmp_path, f"from tests.test_gpu_launches import refused; refused({nx})", refuse=True)
-    assert any(cooperative for _, cooperative in noted)
+    assert any(cooperative for stretch in noted for _, cooperative in stretch)
 
 
 @pytest.mark.parametrize("name", ["LSW", "SW"])
@@ -88,3 +91,50 @@ def test_a_captured_call_replays(name, nx, N, n):
     b.Sync()
     assert torch.isfinite(a.solution).all()
     assert torch.equal(a.solution, b.solution) and torch.equal(a.workSol, b.workSol)
+
+
+def tuned(name, nx, ny, N, form_name):
+    """A step of stage launches as configured by default, the autotuner, and then steps of a new solution."""
+    import self_b200 as S
+    L = S.lib()
+    m = model(name, nx, N, getattr(S, form_name), ny=ny)
+    S.check(L.selfgpu_model2d_set_multistep(m._h, 0))
+    launch_shim.mark()
+    m.ForwardStep(1, 1e-5)
+    launch_shim.mark()
+    p, c, us = ctypes.c_int(), ctypes.c_int(), ctypes.c_float()
+    S.check(L.selfgpu_model2d_autotune(m._h, ctypes.byref(p), ctypes.byref(c), ctypes.byref(us)))
+    launch_shim.mark()
+    m.ForwardStep(1, 1e-5)
+    m.Sync()
+    assert (c.value > 0) == bool(p.value) and us.value > 0
+
+
+@pytest.mark.parametrize("name,nx,ny,N,form_name,threads", [
+    ("SW", 9, 7, 4, "FP32_BULK", 64),  # an odd number of values, twelve groups
+    ("LSW", 7, 5, 6, "FP64", 128), ("CIG", 9, 7, 2, "FP64", 96), ("SW", 8, 8, 7, "FP32_BULK", 64),
+    ("CIG", 6, 6, 3, "FP64", 32)])
+def test_the_autotuner_times_every_group_count_once(name, nx, ny, N, form_name, threads, tmp_path):
+    """Four launches with each number of consumer groups from two to the default, which is the most that fit."""
+    noted = launch_shim.run(tmp_path, "from tests.test_gpu_launches import tuned; "
+                                      f"tuned({name!r}, {nx}, {ny}, {N}, {form_name!r})")
+    _, default, candidates, _ = noted
+    assert len(default) == 3 and len(set(default)) == 1
+    fit = default[0][0] // threads
+    assert fit >= 2 and default[0][0] == fit * threads
+    assert Counter(candidates) == {(g * threads, 0): 4 for g in range(2, fit + 1)}
+
+
+def test_the_autotuner_leaves_the_on_chip_launch():
+    """Its choice is for stage launches: rk3 on a mesh that fits on chip stays one launch, with the same state."""
+    import self_b200 as S
+    L = S.lib()
+    a, b = (model("CIG", 9, 5, S.FP64) for _ in range(2))
+    p, c, us = ctypes.c_int(), ctypes.c_int(), ctypes.c_float()
+    S.check(L.selfgpu_model2d_autotune(a._h, ctypes.byref(p), ctypes.byref(c), ctypes.byref(us)))
+    for m in (a, b):
+        l0 = m.LaunchCount()
+        m.ForwardStep(3, 1e-5)
+        m.Sync()
+        assert m.LaunchCount() - l0 == 1
+    assert torch.equal(a.solution, b.solution)
