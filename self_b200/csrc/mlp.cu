@@ -20,8 +20,9 @@
 #include <cuda_runtime.h>
 
 #include <cstring>
+#include <memory>
+#include <new>
 #include <string>
-#include <vector>
 
 #include "av_closure.cuh"
 #include "selfgpu_internal.h"
@@ -369,10 +370,14 @@ int selfgpu_mlp_train_range(const float* features, const float* labels, int n, i
   const size_t rangeAt = NP + (size_t)epochs, back = rangeAt + (range ? 2 * IN : 0);
   const size_t scratch = range ? sizeof(RangeScratch) / sizeof(float) : 0;
   const size_t fixed = rangeAt + scratch + 2 * (size_t)NP, total = fixed + (size_t)blocks * (NPP + 1);
-  std::vector<float> host(back);
   float* buf = nullptr;
   cudaError_t e = cudaMalloc(&buf, total * sizeof(float));
   if (e != cudaSuccess) return fail("selfgpu_mlp_train", e);
+  const std::unique_ptr<float[]> host(new (std::nothrow) float[back]);
+  if (!host) {
+    cudaFree(buf);
+    return fail("selfgpu_mlp_train", cudaErrorMemoryAllocation);
+  }
   float *master = buf, *loss = buf + NP, *m1 = buf + rangeAt + scratch, *m2 = m1 + NP, *part = buf + fixed,
         *lossPart = part + (size_t)blocks * NPP;
   e = cudaMemsetAsync(buf, 0, fixed * sizeof(float), st);
@@ -394,14 +399,14 @@ int selfgpu_mlp_train_range(const float* features, const float* labels, int n, i
                              1.f - c1, 1.f - c2);
     }
   }
-  if (e == cudaSuccess) e = cudaMemcpyAsync(host.data(), buf, back * sizeof(float), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(host.get(), buf, back * sizeof(float), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   cudaFree(buf);
   if (e != cudaSuccess) return fail("selfgpu_mlp_train", e);
-  std::memcpy(params, host.data(), NP * sizeof(float));
+  std::memcpy(params, host.get(), NP * sizeof(float));
   if (lossPerEpoch)
     for (int ep = 0; ep < epochs; ++ep) lossPerEpoch[ep] = host[NP + ep] / (float)(stepsPerEpoch * batch);
-  if (range) std::memcpy(range, host.data() + rangeAt, 2 * IN * sizeof(float));
+  if (range) std::memcpy(range, host.get() + rangeAt, 2 * IN * sizeof(float));
   return SELFGPU_OK;
 }
 

@@ -135,3 +135,26 @@ def test_closure_off_equals_plain_tendency_and_mode2_with_indicator_nu_equals_mo
     np.testing.assert_array_equal(c.tendency(), t1)
     b.set_closure(1, c=0.0)  # zero viscosity: the viscous terms add exact zeros
     np.testing.assert_array_equal(b.tendency(), t0)
+
+
+def test_training_reports_a_shortage_of_host_memory():
+    """The losses of 2^31 - 1 epochs do not fit the address space left: an error code, no C++ exception through the C
+    entry.  (A child process without a device, whose address space is bounded once everything is loaded.)"""
+    import os
+    import subprocess
+    import sys
+    code = """
+import ctypes, resource
+import numpy as np
+from self_b200._lib import lib
+L = lib()
+size = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
+resource.setrlimit(resource.RLIMIT_AS, (size + (2 << 30),) * 2)
+p = np.zeros(2273, dtype=np.float32)
+at = p.ctypes.data_as(ctypes.c_void_p)
+assert L.selfgpu_mlp_train(at, at, 1, 2**31 - 1, 1, 1e-3, 1, at, None, None) != 0
+"""
+    root = os.path.abspath(os.path.join(os.path.dirname(__file__), ".."))
+    env = dict(os.environ, CUDA_VISIBLE_DEVICES="", PYTHONPATH=root)
+    out = subprocess.run([sys.executable, "-c", code], env=env, cwd=root, capture_output=True, text=True, timeout=120)
+    assert out.returncode == 0, out.stderr
