@@ -59,6 +59,45 @@ constexpr int kGradThreads = 256;
 constexpr int NPP = (NP + 31) / 32 * 32;  // stride of a block's partial sums
 constexpr int kMaxGradBlocks = 296;  // two blocks per SM; larger batches loop over tiles
 
+// Sums of eight values by pairs.
+__device__ __forceinline__ float pairwise(const float v[8]) {
+  return ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+}
+
+// A tile's products D[r][row] A[r][col + k], k < K, summed over its samples and
+// added to acc: chains of four samples, then by pairs, so that a value passes
+// through seven roundings at most (one chain over the tile would be 32, and as
+// many more for each further tile of the block).
+template <int K, int W>
+__device__ __forceinline__ void tile_sums(const float (*D)[H + 1], const float (*A)[W], int row, int col,
+                                          float acc[9]) {
+  float sum[K], half[K], oct[K];
+  auto octet = [&](int r0, float o[K]) {  // of samples r0 .. r0 + 7
+    float a[K], b[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) a[k] = b[k] = 0.f;
+#pragma unroll
+    for (int r = r0; r < r0 + 4; ++r) {
+      const float da = D[r][row], db = D[r + 4][row];
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        a[k] = fmaf(da, A[r][col + k], a[k]);
+        b[k] = fmaf(db, A[r + 4][col + k], b[k]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) o[k] = a[k] + b[k];
+  };
+  octet(0, sum);
+  octet(8, oct);
+#pragma unroll
+  for (int k = 0; k < K; ++k) sum[k] = sum[k] + oct[k];
+  octet(16, half);
+  octet(24, oct);
+#pragma unroll
+  for (int k = 0; k < K; ++k) acc[k] = acc[k] + (sum[k] + (half[k] + oct[k]));
+}
+
 // Latency bounds a step (a 4096-sample batch is 54 MFLOP): 128 tiles on as
 // many SMs.  Adding each sample's gradient to shared memory by warp shuffles
 // (2 273 five-step sums per warp, a block per 256 samples) took 390 us for a
@@ -160,24 +199,19 @@ __global__ void __launch_bounds__(kGradThreads) k_grad(const float* feat, const 
       D1[s][k] = H1[s][k] > 0.f ? a : 0.f;
     }
     __syncthreads();
-    if (half == 0) {
-#pragma unroll 4
-      for (int r = 0; r < kTile; ++r) {
-        const float d = D1[r][row];
+    if (half == 0) tile_sums<9, IN + 1>(D1, F, row, col, acc);
+    else tile_sums<8, H + 1>(D2, H1, row, col, acc);
+    if (t < 3 * H + 1) {
+      float v[kTile / 4];
 #pragma unroll
-        for (int k = 0; k < 9; ++k) acc[k] = fmaf(d, F[r][col + k], acc[k]);
-      }
-    } else {
-#pragma unroll 4
-      for (int r = 0; r < kTile; ++r) {
-        const float d = D2[r][row];
+      for (int q = 0; q < kTile / 4; ++q) {
+        v[q] = 0.f;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) acc[k] = fmaf(d, H1[r][col + k], acc[k]);
+        for (int r = 4 * q; r < 4 * q + 4; ++r)
+          v[q] = v[q] + (t < H ? D1[r][t] : t < 2 * H ? D2[r][t - H] : t < 3 * H ? sg[r] * H2[r][t - 2 * H] : sg[r]);
       }
+      accB = accB + pairwise(v);
     }
-    if (t < 3 * H + 1)
-      for (int r = 0; r < kTile; ++r)
-        accB = accB + (t < H ? D1[r][t] : t < 2 * H ? D2[r][t - H] : t < 3 * H ? sg[r] * H2[r][t - 2 * H] : sg[r]);
   }
   float* o = part + (size_t)NPP * blockIdx.x;
 #pragma unroll
@@ -189,7 +223,7 @@ __global__ void __launch_bounds__(kGradThreads) k_grad(const float* feat, const 
 }
 
 // 32 parameters per block: lane = parameter, warp = every eighth block's
-// partial sum, then the eight strips in order.
+// partial sum in four chains, then the eight strips by pairs.
 __global__ void __launch_bounds__(256) k_adam(float* master, const float* part, const float* lossPart, int blocks,
                                               float* m1, float* m2, float* loss, float lr, float c1, float c2) {
   __shared__ float strip[8][32];
@@ -202,15 +236,19 @@ __global__ void __launch_bounds__(256) k_adam(float* master, const float* part, 
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   float m1k = 0.f, m2k = 0.f, mk = 0.f;  // in flight during the sums
   if (w == 0 && k < NP) m1k = m1[k], m2k = m2[k], mk = master[k];
-  float s = 0.f;
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
   if (k < NP)
-    for (int r = w; r < blocks; r += 8) s += part[(size_t)NPP * r + k];
-  strip[w][lane] = s;
+    for (int r = w; r < blocks; r += 32)
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (r + 8 * q < blocks) s[q] += part[(size_t)NPP * (r + 8 * q) + k];
+  strip[w][lane] = (s[0] + s[1]) + (s[2] + s[3]);
   __syncthreads();
   if (w == 0 && k < NP) {
-    float gk = 0.f;
+    float v[8];
 #pragma unroll
-    for (int r = 0; r < 8; ++r) gk += strip[r][lane];
+    for (int r = 0; r < 8; ++r) v[r] = strip[r][lane];
+    const float gk = pairwise(v);
     m1[k] = m1k = b1 * m1k + (1.f - b1) * gk;
     m2[k] = m2k = b2 * m2k + (1.f - b2) * gk * gk;
     const float mh = m1k / c1, vh = m2k / c2;
