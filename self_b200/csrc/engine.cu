@@ -214,7 +214,8 @@ cudaError_t read_sum(int slot, double* result, cudaStream_t st) {
 }
 double* sum_target(int slot) { return sum_results() ? sum_results() + slot : nullptr; }
 
-// Entropy integrands (CalculateEntropy of the three models):
+// Entropy integrands (CalculateEntropy of the three models), each formed as the
+// reference forms it; the sum over the nodes is sum_grid's:
 //   LSW  0.5 (H (u^2 + v^2) + g eta^2) J w_i w_j  (src/models/SELF_LinearShallowWater.f90:171-216)
 //   SW   (0.5 (Hu^2/H + Hv^2/H) + 0.5 g H^2 - g H b) J w_i w_j  (src/models/SELF_ShallowWater.f90:149-188)
 //   CIG  rho (log p - gamma log rho) / (gamma - 1) w_i w_j J, p from the
@@ -231,21 +232,21 @@ __global__ void __launch_bounds__(kSumThreads) k_entropy(int model, const double
     int n;
     const long long e = element_of(k, PP, n);
     const double* qe = q + nv * PP * e + n;
-    const double wt = qw.w[n % P] * qw.w[n / P] * J[k];
+    const double wi = qw.w[n % P], wj = qw.w[n / P], Jac = J[k];
     if (model == SELFGPU_MODEL_LSW) {
       const double u = qe[0], v = qe[PP], eta = qe[2 * PP], H = aux[k];
-      s += 0.5 * (H * (u * u + v * v) + g * eta * eta) * wt;
+      s += 0.5 * (H * (u * u + v * v) + g * eta * eta) * Jac * wi * wj;
     } else if (model == SELFGPU_MODEL_SW) {
       const double Hu = qe[0], Hv = qe[PP], H = qe[2 * PP];
       const double b = aux ? aux[k] : 0.0;
-      s += (0.5 * (Hu * Hu / H + Hv * Hv / H) + 0.5 * g * H * H - g * H * b) * wt;
+      s += (0.5 * (Hu * Hu / H + Hv * Hv / H) + 0.5 * g * H * H - g * H * b) * Jac * wi * wj;
     } else {
       const double rhoU = qe[0], rhoV = qe[PP], rho = qe[2 * PP], rhoE = qe[3 * PP];
-      const double p = (gamma - 1.0) * (rhoE - 0.5 * (rhoU * rhoU + rhoV * rhoV) / rho);
-      s += rho * (log(p) - gamma * log(rho)) * wt;
+      const double u = rhoU / rho, v = rhoV / rho;
+      const double p = (gamma - 1.0) * (rhoE - 0.5 * (rhoU * u + rhoV * v));
+      s += rho * (log(p) - gamma * log(rho)) / (gamma - 1.0) * wi * wj * Jac;
     }
   }
-  if (model == SELFGPU_MODEL_CIG) s = s / (gamma - 1.0);
   sum_grid(s, &g_sumSlots[slot], out);
 }
 

@@ -316,3 +316,18 @@ def test_closure_lane_groups(N, nx, ny):
     nu = ref.get("avNu")
     assert np.abs(mod.ClosureState()[0].cpu().numpy() - nu).max() <= 1e-13 * nu.max()
     _check(got, t, S.FP64)
+
+
+def test_gas_entropy_of_a_state_whose_squares_overflow():
+    """The pressure is formed from rho u times u, as the reference forms it: momenta above 1.4e154, whose squares
+    overflow, in a fluid as dense."""
+    import self_b200 as S
+    mesh = S.Mesh2D(3, 2, periodic=(True, True))
+    m = S.CompressibleIdealGas2D(mesh, S.SEMQuad(S.Lagrange(3, S.GAUSS, 3, S.UNIFORM), mesh))
+    q = torch.empty_like(m.solution)
+    q[:, 0], q[:, 1], q[:, 2], q[:, 3] = 3e154, -2e154, 2e154, 1e155
+    m.SetSolution(q)
+    r, e = np.longdouble(2e154), np.longdouble(1e155)
+    p = 0.4 * (e - 0.5 * (np.longdouble(3e154) * 1.5 + np.longdouble(2e154)))
+    ref = float(r * (np.log(p) - 1.4 * np.log(r)) / 0.4)  # of a unit square
+    assert abs(m.CalculateEntropy() - ref) <= 1e-13 * abs(ref)
