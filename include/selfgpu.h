@@ -336,11 +336,15 @@ int selfgpu_model2d_set_kernel(selfgpu_model2d* m, int persistent);
 /* selfgpu_model2d_rk3 runs all 3 nSteps RK stages as ONE cooperative launch
  * that keeps the state on chip (k_fused_resident) where the mesh's tiles of
  * elements all fit resident CTAs: up to 4 736 elements at N = 7, 7 104 at
- * N = 5, 18 944 at N = 3 (148 SMs; three quarters of that with the reference's
- * roundings), without a closure or halo and with neighbour records that name
- * each other.  That is the default until set_kernel, set_launch or
+ * N = 5, 18 944 at N = 3 (148 SMs; three quarters of that or half with the
+ * reference's roundings and for CompressibleIdealGas2D at N = 2, 3 and 5),
+ * without a closure or halo and with neighbour records that name each other.
+ * On meshes of more than a quarter of those sizes, calls of one step, or of up
+ * to three with the reference's roundings, may run stage launches, which are
+ * then faster.  That is the default until set_kernel, set_launch or
  * set_multistage chooses among the stage launches; enable = 1 keeps it on
- * after those, 0 turns it off.  Results equal the stage launches bit for bit.
+ * after those and for calls of any length, 0 turns it off.  Results equal the
+ * stage launches bit for bit.
  * A call of more than 1 000 steps is one launch per 1 000, and a device that
  * refuses a cooperative launch runs stage launches.
  * The waits for neighbours' traces are bounded (set_wait_limit;

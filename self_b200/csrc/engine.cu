@@ -312,6 +312,7 @@ struct selfgpu_model2d {
   int resident = RESIDENT_AUTO;
   bool stagesChosen = false;
   int residentTiles = 0;          // tiles per CTA; 0 where the mesh does not fit
+  int residentSteps = 1;          // steps of the shortest call that gains from it
   bool symmetric = false;         // every exchanged side's neighbour exchanges with that side
   void* xch = nullptr;            // k_fused_resident's published traces and set counter
   void* caches = nullptr;         // the allocation that holds tr, vel and xch
@@ -377,6 +378,20 @@ struct selfgpu_model2d {
       case SELFGPU_FP64_REF: return launch_resident_fp64_ref(model, P, a, ra, cfg, stream);
       default: return launch_resident_fp32(model, P, a, ra, cfg, stream);
     }
+  }
+
+  // Whether an rk3 call tries the on-chip launch.  A call with stale traces
+  // saves their launch too, some 6 us: as much as two steps more.  A captured
+  // call always does: its stage launches would leave the traces in the other
+  // cache after an odd number of steps, and a replay would not find them.
+  bool run_resident(int nSteps) const {
+    if (nSteps <= 0 || residentTiles == 0 || avMode != AV_OFF || nHalo != 0 || !symmetric || base.debugStarve == 1)
+      return false;
+    if (resident != RESIDENT_AUTO) return resident == RESIDENT_ON;
+    if (stagesChosen) return false;
+    if (nSteps + (valid ? 0 : 2) >= residentSteps) return true;
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(stream, &s) == cudaSuccess && s == cudaStreamCaptureStatusActive;
   }
 
   // nSteps RK3 steps as one launch of k_fused_resident (it forms stale traces
@@ -539,6 +554,7 @@ struct selfgpu_model2d {
     StageArgs a{};
     a.nEl = nEl;
     residentTiles = nHalo == 0 && launch_resident_form(a, ra) == cudaSuccess ? ra.tiles : 0;
+    residentSteps = residentTiles ? ra.nStages / 3 : 1;
     cudaGetLastError();
     const size_t nb = 4 * (size_t)(nEl + nHalo), t = (trace_block_bytes() * nb + 255) / 256 * 256,
                  v = model == SELFGPU_MODEL_SW ? (vel_block_bytes() * nb + 255) / 256 * 256 : 0;
@@ -823,8 +839,7 @@ int selfgpu_model2d_rk3(selfgpu_model2d* m, double dt, int nSteps) {
   if (rc) return rc;
   if (nSteps < 0) return set_error(SELFGPU_ERR_ARG, "selfgpu_model2d_rk3: nSteps < 0");
   cudaError_t e = cudaSuccess;
-  if ((m->resident == m->RESIDENT_ON || (m->resident == m->RESIDENT_AUTO && !m->stagesChosen)) && nSteps > 0 &&
-      m->avMode == AV_OFF && m->nHalo == 0 && m->symmetric && m->base.debugStarve != 1) {
+  if (m->run_resident(nSteps)) {
     int done = 0;
     e = m->launch_resident(dt, nSteps, done);
     if (e == cudaSuccess) return SELFGPU_OK;

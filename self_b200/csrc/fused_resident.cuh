@@ -46,18 +46,49 @@ struct ResidentEpoch {
   unsigned done;
 };
 
-// Most tiles per CTA.  us per stage, stage launches -> this launch, for
-// CompressibleIdealGas2D FP64 at P = 8 (1 184 elements per tile of the CTAs):
-// one tile 6.9 -> 2.8 (34x34), two 9.7 -> 6.6 (48x48), three 12.6 -> 9.6,
-// four 13.7 -> 12.5, five 16.6 -> 16.5; at P = 6 (1 776) 9.7 -> 6.1, 13.7 ->
-// 11.7, 18.0 -> 17.4, six 25.4 -> 30.3; with the reference's roundings four
-// tiles are already 1 % slower.
-// At P = 3 (5 920) CompressibleIdealGas2D FP64 gains up to three (17.8 -> 18.0;
-// four 22.0 -> 26.8), the other models up to four (ShallowWater 16.3 -> 13.9).
+// Most tiles per CTA: four, three with the reference's roundings, fewer where
+// the smallest meshes of that many tiles were slower than their stage launches.
+// us per stage in calls of 20 steps on nx x nx meshes, stage launches -> this
+// launch, for CompressibleIdealGas2D FP64 at P = 8 (1 184 elements per tile of
+// the CTAs): one tile 6.9 -> 2.8 (34x34), two 9.7 -> 6.6 (48x48), three 10.3 ->
+// 8.9 (52x52), four 13.0 -> 11.7 (60x60).  Over all P, models and forms on 21
+// meshes each, the ratio is at worst 0.65 for one tile, 0.91 for two (0.99 for
+// CompressibleIdealGas2D FP32 at P = 3), 1.01 for three and 0.93 for four, but
+// for those excepted here:
+//   CompressibleIdealGas2D at P = 3: three 1.04 FP64, 1.06 reference roundings,
+//     1.12 FP32;
+//   CompressibleIdealGas2D FP64 at P = 4: three 1.02, four 1.22; at P = 6: four
+//     1.07;
+//   ShallowWater with the reference's roundings at P = 6: three 1.06.
+// Least steps of a call.  A call pays some 6 us to load and store the state and
+// to start all CTAs at once.  With one tile a single step wins that back (ratio
+// 0.91 at worst); with several it takes as many steps as the stages' gain needs
+// on the smallest meshes of the tile count.  us per call, stage launches -> this
+// launch, with the reference's roundings at P = 8: ShallowWater two tiles one
+// step 22.6 -> 26.8, two 45.2 -> 45.5; CompressibleIdealGas2D three tiles three
+// steps 123 -> 129, four 164 -> 169, 20 819 -> 816.  In the other forms one step
+// of three or four tiles: at P = 8 CompressibleIdealGas2D FP64 40.8 -> 41.3,
+// ShallowWater 35.0 -> 37.1, FP32 28.8 -> 31.1; at P = 6 LinearShallowWater FP64
+// 24.7 -> 26.8, CompressibleIdealGas2D FP32 30.8 -> 34.5, two steps 59.5 -> 61.7.  LinearShallowWater elsewhere and P = 5 and 7 gain with one step too
+// (P = 5 FP64 four tiles, ratio 0.81 to 0.96).
 inline namespace SELFGPU_FORM_NS {
 template <int P, class Phys, typename R>
 __host__ __device__ constexpr int resident_tiles() {
-  return ref_rounding<R>() || (P == 3 && Phys::NV == 4 && sizeof(R) == 8) ? 3 : 4;
+  constexpr bool cig = Phys::NV == 4, prod = sizeof(R) == 8 && !ref_rounding<R>();
+  if (cig && (P == 3 || (P == 4 && prod))) return 2;
+  if (ref_rounding<R>()) return P == 6 && Phys::kLaggedVelocity ? 2 : 3;
+  return cig && P == 6 && prod ? 3 : 4;
+}
+template <int P, class Phys, typename R>
+__host__ __device__ constexpr int resident_min_steps(int tiles) {
+  constexpr bool cig = Phys::NV == 4, lsw = !cig && !Phys::kLaggedVelocity;
+  if (tiles <= 1) return 1;
+  if (ref_rounding<R>()) {
+    if (P == 6 || P == 8) return tiles == 2 ? 2 : 4;
+    return tiles == 2 && (P == 5 || (P < 6 && lsw)) ? 1 : 2;
+  }
+  if (P == 5 || P == 7 || (lsw && !(P == 6 && sizeof(R) == 8))) return 1;
+  return tiles > 2 || (cig && P == 3 && sizeof(R) == 4) ? 2 : 1;
 }
 }  // namespace SELFGPU_FORM_NS
 

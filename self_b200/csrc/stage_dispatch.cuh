@@ -198,7 +198,8 @@ cudaError_t launch_P(int P, const StageArgs& a, const StageLaunch& L, cudaStream
 
 // All stages of an rk3 call in one cooperative launch of k_fused_resident with
 // ra.tiles tiles per CTA.  With ra.tiles = 0 nothing is launched: ra.tiles is
-// set to the fewest tiles per CTA with which the mesh fits resident CTAs, and
+// set to the fewest tiles per CTA with which the mesh fits resident CTAs and
+// ra.nStages to the stages of the shortest call that gains from them, and
 // cudaErrorCooperativeLaunchTooLarge returned when there is none.
 template <int P, class Phys, typename R>
 cudaError_t launch_resident_one(const StageArgs& a, ResidentArgs& ra, const StageLaunch& L, cudaStream_t st) {
@@ -211,17 +212,16 @@ cudaError_t launch_resident_one(const StageArgs& a, ResidentArgs& ra, const Stag
     int nb = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, one, T::TPE, 0);
     if (e != cudaSuccess) return e;
-    if (total <= (long long)nb * L.numSMs) {
-      ra.tiles = 1;
+    auto fits = [&](int tiles) {
+      ra.tiles = tiles;
+      ra.nStages = 3 * resident_min_steps<P, Phys, R>(tiles);
       return cudaSuccess;
-    }
+    };
+    if (total <= (long long)nb * L.numSMs) return fits(1);
     e = cudaFuncSetAttribute(many, cudaFuncAttributeMaxDynamicSharedMemorySize, resident_tiles<P, Phys, R>() * X::tileBytes);
     for (int k = 2; k <= resident_tiles<P, Phys, R>() && e == cudaSuccess; ++k) {
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, many, T::TPE, (size_t)k * X::tileBytes);
-      if (e == cudaSuccess && (total + k - 1) / k <= (long long)nb * L.numSMs) {
-        ra.tiles = k;
-        return cudaSuccess;
-      }
+      if (e == cudaSuccess && (total + k - 1) / k <= (long long)nb * L.numSMs) return fits(k);
     }
     return e != cudaSuccess ? e : cudaErrorCooperativeLaunchTooLarge;
   }

@@ -138,3 +138,32 @@ def test_the_autotuner_leaves_the_on_chip_launch():
         m.Sync()
         assert m.LaunchCount() - l0 == 1
     assert torch.equal(a.solution, b.solution)
+
+
+@pytest.mark.parametrize("name,nx,N,form_name,least", [
+    # several tiles per CTA
+    ("SW", 38, 7, "FP64_REF", 2), ("CIG", 52, 7, "FP64_REF", 4), ("CIG", 60, 7, "FP64", 2), ("LSW", 60, 5, "FP64", 2),
+    ("CIG", 60, 5, "FP32_BULK", 2), ("LSW", 60, 5, "FP32_BULK", 1), ("SW", 90, 4, "FP64", 1),
+    ("CIG", 80, 2, "FP32_BULK", 2),
+    # one tile; more than the launch gains from
+    ("SW", 30, 7, "FP64_REF", 1), ("CIG", 104, 3, "FP64", None), ("SW", 60, 5, "FP64_REF", None),
+    ("CIG", 120, 2, "FP32_BULK", None)])
+def test_a_call_runs_on_chip_where_that_is_faster(name, nx, N, form_name, least):
+    """Calls shorter than the on-chip launch needs to win back its start run stage launches (counted as two steps
+    longer where the traces are stale), as do meshes of more tiles than it gains from; the state is the same however
+    the steps are divided."""
+    import self_b200 as S
+    a, b = (model(name, nx, N, getattr(S, form_name)) for _ in range(2))
+    S.check(S.lib().selfgpu_model2d_set_launch(b._h, 1, 0))
+    stale = True
+    for n in (1, 1, 2, 3, 4, 1):
+        l0 = a.LaunchCount()
+        a.ForwardStep(n, 1e-6)
+        on_chip = least is not None and n + 2 * stale >= least
+        assert a.LaunchCount() - l0 == (1 if on_chip else 3 * n + stale), (n, stale)
+        stale = False
+        b.ForwardStep(n, 1e-6)
+    a.Sync()
+    b.Sync()
+    assert torch.isfinite(a.solution).all()
+    assert torch.equal(a.solution, b.solution) and torch.equal(a.workSol, b.workSol)
