@@ -65,37 +65,27 @@ __device__ __forceinline__ float pairwise(const float v[8]) {
 }
 
 // A tile's products D[r][row] A[r][col + k], k < K, summed over its samples and
-// added to acc: chains of four samples, then by pairs, so that a value passes
-// through seven roundings at most (one chain over the tile would be 32, and as
-// many more for each further tile of the block).
+// added to acc: four chains of eight samples, then by pairs, so that a value
+// passes through ten roundings at most (one chain over the tile would be 32, and
+// as many more for each further tile of the block).
 template <int K, int W>
 __device__ __forceinline__ void tile_sums(const float (*D)[H + 1], const float (*A)[W], int row, int col,
                                           float acc[9]) {
-  float sum[K], half[K], oct[K];
-  auto octet = [&](int r0, float o[K]) {  // of samples r0 .. r0 + 7
-    float a[K], b[K];
+  float c[4][K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) a[k] = b[k] = 0.f;
+  for (int q = 0; q < 4; ++q)
 #pragma unroll
-    for (int r = r0; r < r0 + 4; ++r) {
-      const float da = D[r][row], db = D[r + 4][row];
+    for (int k = 0; k < K; ++k) c[q][k] = 0.f;
+#pragma unroll 2
+  for (int r = 0; r < kTile / 4; ++r)
 #pragma unroll
-      for (int k = 0; k < K; ++k) {
-        a[k] = fmaf(da, A[r][col + k], a[k]);
-        b[k] = fmaf(db, A[r + 4][col + k], b[k]);
-      }
+    for (int q = 0; q < 4; ++q) {
+      const float d = D[r + kTile / 4 * q][row];
+#pragma unroll
+      for (int k = 0; k < K; ++k) c[q][k] = fmaf(d, A[r + kTile / 4 * q][col + k], c[q][k]);
     }
 #pragma unroll
-    for (int k = 0; k < K; ++k) o[k] = a[k] + b[k];
-  };
-  octet(0, sum);
-  octet(8, oct);
-#pragma unroll
-  for (int k = 0; k < K; ++k) sum[k] = sum[k] + oct[k];
-  octet(16, half);
-  octet(24, oct);
-#pragma unroll
-  for (int k = 0; k < K; ++k) acc[k] = acc[k] + (sum[k] + (half[k] + oct[k]));
+  for (int k = 0; k < K; ++k) acc[k] = acc[k] + ((c[0][k] + c[1][k]) + (c[2][k] + c[3][k]));
 }
 
 // Latency bounds a step (a 4096-sample batch is 54 MFLOP): 128 tiles on as
@@ -223,7 +213,7 @@ __global__ void __launch_bounds__(kGradThreads) k_grad(const float* feat, const 
 }
 
 // 32 parameters per block: lane = parameter, warp = every eighth block's
-// partial sum in four chains, then the eight strips by pairs.
+// partial sum in eight chains, then the eight strips by pairs.
 __global__ void __launch_bounds__(256) k_adam(float* master, const float* part, const float* lossPart, int blocks,
                                               float* m1, float* m2, float* loss, float lr, float c1, float c2) {
   __shared__ float strip[8][32];
@@ -236,13 +226,18 @@ __global__ void __launch_bounds__(256) k_adam(float* master, const float* part, 
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   float m1k = 0.f, m2k = 0.f, mk = 0.f;  // in flight during the sums
   if (w == 0 && k < NP) m1k = m1[k], m2k = m2[k], mk = master[k];
-  float s[4] = {0.f, 0.f, 0.f, 0.f};
-  if (k < NP)
-    for (int r = w; r < blocks; r += 32)
+  float s[8];
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (r + 8 * q < blocks) s[q] += part[(size_t)NPP * (r + 8 * q) + k];
-  strip[w][lane] = (s[0] + s[1]) + (s[2] + s[3]);
+  for (int q = 0; q < 8; ++q) s[q] = 0.f;
+  if (k < NP)
+    for (int r = w; r < blocks; r += 64) {  // (a batch of 4 096 samples: two rounds of loads)
+      float x[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) x[q] = r + 8 * q < blocks ? part[(size_t)NPP * (r + 8 * q) + k] : 0.f;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) s[q] = s[q] + x[q];
+    }
+  strip[w][lane] = pairwise(s);
   __syncthreads();
   if (w == 0 && k < NP) {
     float v[8];
