@@ -50,7 +50,7 @@ struct ResidentEpoch {
 // the smallest meshes of that many tiles were slower than their stage launches.
 // us per stage in calls of 20 steps on nx x nx meshes, stage launches -> this
 // launch, for CompressibleIdealGas2D FP64 at P = 8 (1 184 elements per tile of
-// the CTAs): one tile 6.9 -> 2.8 (34x34), two 9.7 -> 6.6 (48x48), three 10.3 ->
+// the CTAs): one tile 6.5 -> 2.7 (34x34), two 9.6 -> 6.2 (48x48), three 10.3 ->
 // 8.9 (52x52), four 13.0 -> 11.7 (60x60).  Over all P, models and forms on 21
 // meshes each, the ratio is at worst 0.65 for one tile, 0.91 for two (0.99 for
 // CompressibleIdealGas2D FP32 at P = 3), 1.01 for three and 0.93 for four, but
@@ -69,8 +69,9 @@ struct ResidentEpoch {
 // steps 123 -> 129, four 164 -> 169, 20 819 -> 816.  In the other forms one step
 // of three or four tiles: at P = 8 CompressibleIdealGas2D FP64 40.8 -> 41.3,
 // ShallowWater 35.0 -> 37.1, FP32 28.8 -> 31.1; at P = 6 LinearShallowWater FP64
-// 24.7 -> 26.8, CompressibleIdealGas2D FP32 30.8 -> 34.5, two steps 59.5 -> 61.7.  LinearShallowWater elsewhere and P = 5 and 7 gain with one step too
-// (P = 5 FP64 four tiles, ratio 0.81 to 0.96).
+// 24.7 -> 26.8, CompressibleIdealGas2D FP32 30.8 -> 34.5, two steps 59.5 -> 61.7.
+// LinearShallowWater elsewhere and P = 5 and 7 gain with one step too (P = 5
+// FP64 four tiles, ratio 0.81 to 0.96).
 inline namespace SELFGPU_FORM_NS {
 template <int P, class Phys, typename R>
 __host__ __device__ constexpr int resident_tiles() {
