@@ -381,17 +381,34 @@ struct selfgpu_model2d {
   }
 
   // Whether an rk3 call tries the on-chip launch.  A call with stale traces
-  // saves their launch too, some 6 us: as much as two steps more.  A captured
-  // call always does: its stage launches would leave the traces in the other
-  // cache after an odd number of steps, and a replay would not find them.
+  // saves their launch too, some 6 us: as much as two steps more.
   bool run_resident(int nSteps) const {
     if (nSteps <= 0 || residentTiles == 0 || avMode != AV_OFF || nHalo != 0 || !symmetric || base.debugStarve == 1)
       return false;
     if (resident != RESIDENT_AUTO) return resident == RESIDENT_ON;
-    if (stagesChosen) return false;
-    if (nSteps + (valid ? 0 : 2) >= residentSteps) return true;
+    return !stagesChosen && nSteps + (valid ? 0 : 2) >= residentSteps;
+  }
+
+  bool capturing() const {
     cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
     return cudaStreamIsCapturing(stream, &s) == cudaSuccess && s == cudaStreamCaptureStatusActive;
+  }
+
+  // nSteps RK3 steps into the graph that the caller is capturing: plain stage
+  // launches (a step's own graph cannot be captured inside it), which end in the
+  // caches they began with, so that a replay finds what it left.
+  cudaError_t capture_steps(double dt, int nSteps) {
+    const int c0 = cur, v0 = vcur;
+    cudaError_t e = cudaSuccess;
+    for (int s = 0; s < nSteps && e == cudaSuccess; ++s) e = step(dt);
+    const size_t blocks = 4 * (size_t)(nEl + nHalo);
+    if (e == cudaSuccess && cur != c0)
+      e = cudaMemcpyAsync(tr[c0], tr[cur], trace_block_bytes() * blocks, cudaMemcpyDeviceToDevice, stream);
+    if (e == cudaSuccess && vcur != v0)
+      e = cudaMemcpyAsync(vel[v0], vel[vcur], vel_block_bytes() * blocks, cudaMemcpyDeviceToDevice, stream);
+    cur = c0;
+    vcur = v0;
+    return e;
   }
 
   // nSteps RK3 steps as one launch of k_fused_resident (it forms stale traces
@@ -849,7 +866,8 @@ int selfgpu_model2d_rk3(selfgpu_model2d* m, double dt, int nSteps) {
     cudaGetLastError();
     nSteps -= done;
   }
-  if (m->multistage && nSteps > 0 && m->avMode == AV_OFF && m->nHalo == 0 && m->base.debugStarve != 1 &&
+  const bool captured = m->capturing();
+  if (m->multistage && !captured && nSteps > 0 && m->avMode == AV_OFF && m->nHalo == 0 && m->base.debugStarve != 1 &&
       m->cfg.allowTma) {
     e = m->valid ? cudaSuccess : m->prologue();
     if (e != cudaSuccess) return fail_cuda("selfgpu_model2d_rk3", e);
@@ -862,6 +880,10 @@ int selfgpu_model2d_rk3(selfgpu_model2d* m, double dt, int nSteps) {
   if (!m->valid) {
     e = m->prologue();
     if (e != cudaSuccess) return fail_cuda("selfgpu_model2d_rk3", e);
+  }
+  if (captured) {
+    e = m->capture_steps(dt, nSteps);
+    return e == cudaSuccess ? SELFGPU_OK : fail_cuda("selfgpu_model2d_rk3", e);
   }
   if (!(dt == m->graphDt)) m->drop_graphs();
   for (int s = 0; s < nSteps; ++s) {

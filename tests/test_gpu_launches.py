@@ -167,3 +167,34 @@ def test_a_call_runs_on_chip_where_that_is_faster(name, nx, N, form_name, least)
     b.Sync()
     assert torch.isfinite(a.solution).all()
     assert torch.equal(a.solution, b.solution) and torch.equal(a.workSol, b.workSol)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3])
+@pytest.mark.parametrize("name,nx,N,closure", [
+    ("CIG", 100, 3, False), ("SW", 100, 7, False), ("SW", 120, 4, False), ("CIG", 61, 7, False), ("CIG", 20, 5, True)])
+def test_captured_stage_launches_replay(name, nx, N, closure, n):
+    """Meshes and calls of stage launches (one of them where longer calls run on chip or as one launch), captured after
+    a call of another kind: the steps of as many calls, bit for bit."""
+    import self_b200 as S
+    st = torch.cuda.Stream()
+    a, b = (model(name, nx, N, S.FP64, stream=s) for s in (st.cuda_stream, None))
+    torch.cuda.synchronize()
+    for m in (a, b):
+        if closure:
+            m.SetClosure(S.CLOSURE_INDICATOR, c=1.0)
+        m.ForwardStep(5, 1e-5)
+        m.Sync()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=st):
+        a.ForwardStep(n, 1e-5)
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    a.ForwardStep(4, 1e-5)
+    a.Sync()
+    for _ in range(3):
+        b.ForwardStep(n, 1e-5)
+    b.ForwardStep(4, 1e-5)
+    b.Sync()
+    assert torch.isfinite(a.solution).all()
+    assert torch.equal(a.solution, b.solution) and torch.equal(a.workSol, b.workSol)
