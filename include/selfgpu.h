@@ -295,7 +295,9 @@ int selfgpu_model2d_tendency(selfgpu_model2d* m, double* dSdt);
 /* nSteps Williamson low-storage RK3 steps of size dt
  * (LowStorageRK3_timeIntegrator, src/SELF_Model.f90:704-732, stepped by
  * count): per stage one fused kernel does tendency + UpdateGRK3.  Steps are
- * replayed from a captured CUDA graph after the first call. */
+ * replayed from a captured CUDA graph after the first call, or run as one
+ * launch (set_multistep, set_multistage).  A call may be captured into the
+ * caller's graph; a replay continues from what the last one left. */
 int selfgpu_model2d_rk3(selfgpu_model2d* m, double dt, int nSteps);
 
 /* Wait for the engine's stream; returns the first pending CUDA error. */
